@@ -125,6 +125,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_calls = None
 
 
 def load() -> ctypes.CDLL:
@@ -146,3 +147,22 @@ def load() -> ctypes.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def calls():
+    """The compiled per-call functions (csrc/py_calls.cpp), built first if their source is newer."""
+    global _calls
+    if _calls is None:
+        load()
+        if _build.calls_stale():
+            try:
+                _build.build_calls()
+            except (RuntimeError, OSError):
+                if not _build.CALLS.exists():
+                    raise
+        import torch  # noqa: F401  (its libraries are what the module links against)
+
+        from . import _calls as module
+
+        _calls = module
+    return _calls

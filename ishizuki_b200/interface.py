@@ -14,11 +14,16 @@ and "declined" behaviour follow the reference:
 Where the reference returns nil ("declined, the caller falls back"), these return None for a
 shape guard and raise for anything else; there is no fallback path behind them. Device memory
 is held in torch tensors (plumbing only): every product is computed by libishizuki_cuda.so.
+
+What a decode loop calls per token (the products, the norm, the embedding rows, the EXL3 projection)
+goes through the compiled functions of csrc/py_calls.cpp: from tensor to launch in about 4 us where
+ctypes took 17. The rest is ctypes.
 """
 from __future__ import annotations
 
 import ctypes
 import enum
+import math
 from dataclasses import dataclass
 
 import torch
@@ -30,6 +35,9 @@ class IshizukiError(RuntimeError):
     def __init__(self, status: int, message: str):
         super().__init__(f"{_status_name(status)}: {message}")
         self.status = status
+
+
+_calls = None  # csrc/py_calls.cpp, loaded with the first context
 
 
 def _status_name(status: int) -> str:
@@ -100,6 +108,7 @@ class Context:
     _by_device: dict[int, "Context"] = {}
 
     def __init__(self, device: int = 0):
+        global _calls
         self.lib = _lib.load()
         if not torch.cuda.is_available():
             raise RuntimeError("ishizuki_b200 needs a CUDA device: there is no CPU path")
@@ -107,7 +116,11 @@ class Context:
         rc = self.lib.ishi_ctx_create(device, ctypes.byref(handle))
         if rc != _lib.OK:
             raise IshizukiError(rc, f"ishi_ctx_create({device}) failed")
+        if _calls is None:
+            _calls = _lib.calls()
+            _calls.set_error(IshizukiError)
         self.handle = handle
+        self.address = handle.value
         self.device = device
 
     @classmethod
@@ -117,6 +130,14 @@ class Context:
         if ctx is None:
             ctx = cls._by_device[device] = Context(device)
         return ctx
+
+    @classmethod
+    def of(cls, t: torch.Tensor) -> "Context":
+        """The context of the GPU a tensor lives on."""
+        if _calls is None:
+            return cls.get(t.device.index)
+        index = _calls.device_of(t)
+        return cls._by_device.get(index) or cls.get(index)
 
     def last_error(self) -> str:
         return self.lib.ishi_last_error(self.handle).decode()
@@ -141,7 +162,7 @@ class Context:
 
 
 def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_calls.current_stream(torch.cuda.current_device()))
 
 
 def _ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
@@ -167,43 +188,28 @@ class GGMLKernels:
 
     @staticmethod
     def dequantize(blocks: torch.Tensor, type: GGMLType, shape, dtype=torch.bfloat16):
-        ctx = Context.get(blocks.device.index)
-        count = 1
-        for s in shape:
-            count *= s
-        try:
-            type = GGMLType(type)
-        except ValueError:
+        ctx = Context.of(blocks)
+        count = math.prod(shape)
+        if type not in _lib.GGML_TYPE_SIZE:
             return None
+        type = GGMLType(type)
         if count % type.blockSize != 0:
             return None
         n_blocks = count // type.blockSize
         if blocks.numel() < n_blocks * type.typeSize:
             return None
-        out = torch.empty(count, dtype=dtype, device=blocks.device)
-        rc = ctx.lib.ishi_ggml_dequantize(ctx.handle, int(type), _ptr(blocks), n_blocks, _ptr(out),
-                                          _OUT_DT[dtype], _stream())
-        if not ctx.check(rc, declined=(_lib.E_SHAPE, _lib.E_UNSUPPORTED)):
-            return None
-        return out.reshape(tuple(shape))
+        return _calls.dequantize(ctx.address, blocks, type, n_blocks, shape, dtype)
 
     @staticmethod
     def gather(ids: torch.Tensor, blocks: torch.Tensor, type: GGMLType, inputDim: int, dtype=torch.bfloat16):  # noqa: N803
         """The rows named by ids, decoded into [ids.numel(), inputDim] (the embedding lookup)."""
-        try:
-            type = GGMLType(type)
-        except ValueError:
+        if type not in _lib.GGML_TYPE_SIZE:
             return None
+        type = GGMLType(type)
         if inputDim % type.blockSize != 0 or ids.numel() == 0:
             return None
-        ctx = Context.get(blocks.device.index)
-        idx = ids.reshape(-1).to(torch.int32).contiguous()
-        per_row = inputDim // type.blockSize * type.typeSize
-        table_rows = blocks.numel() // per_row
-        out = torch.empty((idx.numel(), inputDim), dtype=dtype, device=blocks.device)
-        rc = ctx.lib.ishi_ggml_gather(ctx.handle, _ptr(idx), idx.numel(), _ptr(blocks), blocks.numel(), int(type),
-                                      table_rows, inputDim, _ptr(out), _OUT_DT[dtype], _stream())
-        return out if ctx.check(rc, declined=(_lib.E_SHAPE, _lib.E_UNSUPPORTED)) else None
+        ctx = Context.of(blocks)
+        return _calls.gather(ctx.address, ids, blocks, type, inputDim // type.blockSize * type.typeSize, inputDim, dtype)
 
     @staticmethod
     def _product(fn_name: str, x, blocks, type, outputDim):
@@ -297,7 +303,11 @@ class PackedLinear:
         rc = self.ctx.lib.ishi_projection_create(self.ctx.handle, ctypes.byref(d), ctypes.byref(handle))
         if rc != _lib.OK:
             raise IshizukiError(rc, self.ctx.last_error())
+        self._bind(handle)
+
+    def _bind(self, handle) -> None:
         self.handle = handle
+        self._addresses = (self.ctx.address, handle.value)
 
     def _describe(self, weight, scales, biases, n) -> "_lib.WeightDesc":
         d = _lib.WeightDesc()
@@ -318,7 +328,7 @@ class PackedLinear:
         handle = getattr(self, "handle", None)
         if handle:
             self.ctx.lib.ishi_projection_destroy(handle)
-            self.handle = None
+            self.handle = self._addresses = None
 
     @property
     def weightBytes(self) -> int:  # noqa: N802
@@ -347,32 +357,16 @@ class PackedLinear:
         shape = tuple(x.shape)
         return x.reshape(-1, shape[-1]).contiguous(), shape
 
-    def _out(self, h: torch.Tensor, transposed: bool) -> torch.Tensor:
-        m = h.shape[0]
-        if transposed:
-            return torch.empty((self.outputDim, m), dtype=torch.float16, device=h.device)
-        return torch.empty((m, self.outputDim), dtype=torch.float16, device=h.device)
-
     def __call__(self, x: torch.Tensor, transposed: bool = False, out: torch.Tensor | None = None):
         """y = x . W^T for 1...16 rows of x, rotating x first when the pack is rotated."""
-        self.ctx.sync_route()
-        h, shape = self._rows(x)
-        y = self._out(h, transposed) if out is None else out
-        rc = self.ctx.lib.ishi_projection_apply(self.handle, _ptr(h), h.shape[0], _ptr(y), y.stride(0),
-                                                _lib.OUT_TRANSPOSED if transposed else 0, _stream())
-        if rc != _lib.OK:
-            raise IshizukiError(rc, self.ctx.last_error())
-        return y if transposed or out is not None else y.reshape(shape[:-1] + (self.outputDim,))
+        ctx, projection = self._addresses
+        return _calls.linear(ctx, projection, x, self.outputDim, BonsaiRuntime.route, BonsaiRuntime.crossoverRows, False,
+                             transposed, out)
 
     def argmax(self, x: torch.Tensor) -> torch.Tensor:
         """Per row of x the index of its largest logit (int32): the head of a greedy verify step."""
-        self.ctx.sync_route()
-        h, _ = self._rows(x)
-        out = torch.empty(h.shape[0], dtype=torch.int32, device=h.device)
-        rc = self.ctx.lib.ishi_projection_apply_argmax(self.handle, _ptr(h), h.shape[0], _ptr(out), _stream())
-        if rc != _lib.OK:
-            raise IshizukiError(rc, self.ctx.last_error())
-        return out
+        ctx, projection = self._addresses
+        return _calls.argmax(ctx, projection, x, BonsaiRuntime.route, BonsaiRuntime.crossoverRows)
 
     def rotate(self, x: torch.Tensor) -> torch.Tensor:
         h, shape = self._rows(x)
@@ -383,14 +377,8 @@ class PackedLinear:
         return xr.reshape(shape)
 
     def applyRotated(self, h: torch.Tensor) -> torch.Tensor:  # noqa: N802
-        self.ctx.sync_route()
-        rows, shape = self._rows(h)
-        y = self._out(rows, False)
-        rc = self.ctx.lib.ishi_projection_apply_rotated(self.handle, _ptr(rows), rows.shape[0], _ptr(y),
-                                                        y.stride(0), 0, _stream())
-        if rc != _lib.OK:
-            raise IshizukiError(rc, self.ctx.last_error())
-        return y.reshape(shape[:-1] + (self.outputDim,))
+        ctx, projection = self._addresses
+        return _calls.linear(ctx, projection, h, self.outputDim, BonsaiRuntime.route, BonsaiRuntime.crossoverRows, True, False, None)
 
     def apply_host(self, x_host, y_host) -> None:
         """Host-buffer form: x_host [M, K] and y_host [M, N] are C-contiguous fp16 numpy arrays."""
@@ -483,7 +471,7 @@ class FusedLinear(PackedLinear):
             rc = self.ctx.lib.ishi_projection_create_fused(self.ctx.handle, descs, len(triples), ctypes.byref(handle))
         if rc != _lib.OK:
             raise IshizukiError(rc, self.ctx.last_error())
-        self.handle = handle
+        self._bind(handle)
         self.weight = self.scales = self.biases = None  # the library keeps its own tiled copy
 
     def split(self, y: torch.Tensor, transposed: bool = False):
@@ -507,13 +495,7 @@ def hadamardRotate(x: torch.Tensor, block: int, signs: torch.Tensor | None) -> t
 def rmsNorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:  # noqa: N802
     """MLXFast.rmsNorm(x, weight:, eps:) ahead of a projection (TextModel.swift:151-161): fp32 or
     fp16 rows in, fp16 out."""
-    ctx = Context.get(x.device.index)
-    h = x.reshape(-1, x.shape[-1]).contiguous()
-    w = weight.contiguous()
-    y = torch.empty(h.shape, dtype=torch.float16, device=x.device)
-    ctx.check(ctx.lib.ishi_rms_norm(ctx.handle, _ptr(h), _OUT_DT[h.dtype], h.shape[0], h.shape[1], _ptr(w), _OUT_DT[w.dtype],
-                                    ctypes.c_float(eps), _ptr(y), _stream()), declined=())
-    return y.reshape(x.shape)
+    return _calls.rms_norm(Context.of(x).address, x, weight, eps)
 
 
 class EXL3Tensor:
@@ -582,12 +564,7 @@ class EXL3Kernels:
     @staticmethod
     def apply(x: torch.Tensor, t: EXL3Tensor) -> torch.Tensor:
         """rotate -> product -> rotate, 1...16 fp16 rows."""
-        ctx = Context.get(x.device.index)
-        shape = x.shape
-        h = x.reshape(-1, t.inputDim).to(torch.float16).contiguous()
-        y = torch.empty((h.shape[0], t.outputDim), dtype=torch.float16, device=x.device)
-        ctx.check(ctx.lib.ishi_exl3_apply(ctx.handle, ctypes.byref(t._desc()), _ptr(h), h.shape[0], _ptr(y), _stream()), declined=())
-        return y.reshape(shape[:-1] + (t.outputDim,))
+        return _calls.exl3_apply(Context.of(x).address, t.trellis, t.inputScales, t.outputScales, t.codebook, x)
 
 
 class EXL3Linear:

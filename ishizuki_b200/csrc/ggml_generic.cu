@@ -3,7 +3,9 @@
 // streaming kernel of their own, and the arg-max over a row of logits.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 
 #include "ggml_decode.cuh"
@@ -13,55 +15,127 @@ namespace ishi {
 
 namespace {
 
-template <typename OT>
-__device__ __forceinline__ OT to_out(float v);
-template <>
-__device__ __forceinline__ float to_out<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ __half to_out<__half>(float v) { return __float2half_rn(v); }
-template <>
-__device__ __forceinline__ __nv_bfloat16 to_out<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
-// One warp decodes one block and writes one contiguous run of 256 outputs
-// (Sources/IshizukiKit/Core/GGMLKernels.swift:391-401).
-template <int TYPE, typename OT>
-__global__ void __launch_bounds__(256) ggml_dequantize_kernel(const uint8_t *__restrict__ blocks, long long n_blocks,
-                                                              OT *__restrict__ y) {
-  constexpr int kBytes = ggml_type_bytes(TYPE);
-  const int lane = threadIdx.x & 31;
-  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long bi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; bi < n_blocks; bi += warps) {
-    float w[8];
-    decode8<TYPE>(blocks + bi * kBytes, lane, w);
-    OT *out = y + bi * 256 + 8 * lane;
+// Eight consecutive outputs, rounded once: 16-byte stores where the array allows.
+__device__ __forceinline__ void store8(float *y, const float (&w)[8], bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(y), "f"(w[0]), "f"(w[1]), "f"(w[2]), "f"(w[3]), "f"(w[4]),
+                 "f"(w[5]), "f"(w[6]), "f"(w[7])
+                 : "memory");
+    return;
+  }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) out[e] = to_out<OT>(w[e]);
+  for (int e = 0; e < 8; ++e) y[e] = w[e];
+}
+template <class H, class Round>
+__device__ __forceinline__ void store8_half(H *y, const float (&w)[8], bool wide, Round &&round) {
+  H h[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) h[e] = round(w[e]);
+  if (wide) {
+    uint4 v;
+    memcpy(&v, h, 16);
+    __stcs(reinterpret_cast<uint4 *>(y), v);
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) y[e] = h[e];
+}
+__device__ __forceinline__ void store8(__half *y, const float (&w)[8], bool wide) {
+  store8_half(y, w, wide, [](float v) { return __float2half_rn(v); });
+}
+__device__ __forceinline__ void store8(__nv_bfloat16 *y, const float (&w)[8], bool wide) {
+  store8_half(y, w, wide, [](float v) { return __float2bfloat16_rn(v); });
+}
+
+// `bytes` (even) bytes from anywhere into shared memory at a 16-byte boundary, by one warp, in the
+// widest pieces the source's alignment allows.
+__device__ __forceinline__ void stage_bytes(uint32_t dst, const uint8_t *src, int bytes, int lane) {
+  const uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(src);
+  int done = 0;
+  if ((low & 15u) == 0) {
+    constexpr int kAhead = 4;  // 8 blocks of any type in one batch of loads
+    for (int i0 = lane * 16; i0 < (bytes & ~15); i0 += kAhead * 512) {
+      uint4 v[kAhead];
+#pragma unroll
+      for (int e = 0; e < kAhead; ++e)
+        if (i0 + e * 512 + 16 <= bytes) v[e] = __ldg(reinterpret_cast<const uint4 *>(src + i0 + e * 512));
+#pragma unroll
+      for (int e = 0; e < kAhead; ++e)
+        if (i0 + e * 512 + 16 <= bytes) sts128u(dst + i0 + e * 512, v[e]);
+    }
+    done = bytes & ~15;
+  } else if ((low & 3u) == 0) {
+    constexpr int kAhead = 7;
+    for (int i0 = lane * 4; i0 < (bytes & ~3); i0 += kAhead * 128) {
+      uint32_t v[kAhead];
+#pragma unroll
+      for (int e = 0; e < kAhead; ++e)
+        if (i0 + e * 128 + 4 <= bytes) v[e] = __ldg(reinterpret_cast<const uint32_t *>(src + i0 + e * 128));
+#pragma unroll
+      for (int e = 0; e < kAhead; ++e)
+        if (i0 + e * 128 + 4 <= bytes) sts32(dst + i0 + e * 128, v[e]);
+    }
+    done = bytes & ~3;
+  }
+  for (int i = done + 2 * lane; i < bytes; i += 64) {
+    const uint32_t v = (low & 1u) ? (uint32_t)src[i] | ((uint32_t)src[i + 1] << 8) : *reinterpret_cast<const uint16_t *>(src + i);
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + i), "h"((uint16_t)v) : "memory");
   }
 }
 
-// Rows of a quantized table by id (GGMLKernels.swift:102-138, 404-420): a work item is one block
-// of one requested row. Ids outside the table give zeros.
-template <int TYPE, typename OT>
-__global__ void __launch_bounds__(256) ggml_gather_kernel(const int *__restrict__ ids, long long count,
-                                                          const uint8_t *__restrict__ blocks, long long table_rows,
-                                                          long long per_row, OT *__restrict__ y) {
-  constexpr int kBytes = ggml_type_bytes(TYPE);
-  const int lane = threadIdx.x & 31;
-  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const long long work = count * per_row;
-  for (long long wi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wi < work; wi += warps) {
-    const long long i = wi / per_row, b = wi - i * per_row;
-    const long long row = ids[i];
+// Dense decode (Sources/IshizukiKit/Core/GGMLKernels.swift:391-401), and with ids the rows of a
+// quantized table (GGMLKernels.swift:102-138, 404-420; an id outside the table gives zeros). A
+// warp's work item is a run of up to `chunk` consecutive blocks of a row: their bytes come into
+// shared memory in 16-byte pieces (eight blocks of any type are a multiple of 16), are decoded from
+// there a lane eight weights, and leave in 16-byte stores.
+//
+// Bound: HBM on the output. A Q6_K weight of 17408 x 5120 to bf16 takes 43 us (5.8 TB/s), to fp32
+// 68 (6.3 TB/s); reading the blocks byte by byte from global memory and storing value by value took
+// 129 and 185: the load/store unit was what was busy, with eighteen byte loads and eight stores per
+// eight weights against nine and one here.
+constexpr int kExpandChunk = 8, kExpandWarps = 8;  // most blocks of an item, warps of a thread block
+template <int TYPE>
+constexpr int kExpandSlot = (kExpandChunk * ggml_type_bytes(TYPE) + 31) & ~15;  // a reader may look at the words behind a block
+template <int TYPE, typename OT, bool ROWS>
+__global__ void __launch_bounds__(kExpandWarps * 32) ggml_expand_kernel(const int *__restrict__ ids, long long rows,
+                                                                        const uint8_t *__restrict__ blocks, long long table_rows,
+                                                                        long long per_row, int chunk_log, OT *__restrict__ y) {
+  constexpr int kBytes = ggml_type_bytes(TYPE), kTable = ggml_table_bytes(TYPE);
+  __shared__ __align__(16) uint8_t s_blocks[kExpandWarps][kExpandSlot<TYPE>];
+  __shared__ __align__(16) uint8_t s_table[kTable ? kTable : 16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t table = smem_u32(s_table);
+  if (kTable) {
+    ggml_table_fill<TYPE>(table);
+    __syncthreads();
+    table = stage_acquire(table);
+  }
+  const uint32_t slot = smem_u32(s_blocks[warp]);
+  const bool wide = (reinterpret_cast<uintptr_t>(y) & (8 * sizeof(OT) - 1)) == 0;
+  const int chunk = 1 << chunk_log;
+  const long long chunks = (per_row + chunk - 1) >> chunk_log, work = rows * chunks;
+  for (long long wi = (long long)blockIdx.x * kExpandWarps + warp; wi < work; wi += (long long)gridDim.x * kExpandWarps) {
+    const long long i = !ROWS ? 0 : work >> 32 ? wi / chunks : (long long)((uint32_t)wi / (uint32_t)chunks);
+    const long long b0 = (wi - i * chunks) << chunk_log;
+    const int nb = (int)(per_row - b0 < chunk ? per_row - b0 : chunk);
+    const long long row = ROWS ? ids[i] : 0;
+    OT *out = y + (i * per_row + b0) * 256 + 8 * lane;
     float w[8];
-    if (row >= 0 && row < table_rows) {
-      decode8<TYPE>(blocks + (row * per_row + b) * kBytes, lane, w);
-    } else {
+    if (ROWS && (row < 0 || row >= table_rows)) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) w[e] = 0.f;
+      for (int b = 0; b < nb; ++b) store8(out + b * 256, w, wide);
+      continue;
     }
-    OT *out = y + wi * 256 + 8 * lane;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) out[e] = to_out<OT>(w[e]);
+    __syncwarp();  // every lane is done with the last item's blocks
+    stage_bytes(slot, blocks + (row * per_row + b0) * kBytes, nb * kBytes, lane);
+    __syncwarp();
+    const uint32_t a = stage_acquire(slot);
+#pragma unroll 2
+    for (int b = 0; b < nb; ++b) {
+      decode8<TYPE>(BlockShared<TYPE>{a + b * kBytes, table}, lane, w);
+      store8(out + b * 256, w, wide);
+    }
   }
 }
 
@@ -214,33 +288,45 @@ cudaError_t with_type(int type, F &&f) {
 
 int ggml_type_size(int type) { return ggml_type_bytes(type); }
 
-cudaError_t launch_ggml_dequantize(int type, const uint8_t *blocks, long long n_blocks, void *out, int out_dtype, int sm_count,
-                                   cudaStream_t st) {
-  const long long want = (n_blocks * 32 + 255) / 256;
-  const int grid = (int)(want < (long long)sm_count * 32 ? want : (long long)sm_count * 32);
+// Blocks per work item (their logarithm): eight where that leaves every SM eight warps or more, fewer
+// for small arrays (a warp decodes its blocks one after the other: a short array is done sooner by
+// more warps). Measured on 2048 rows of 5120 in Q6_K: eight blocks 7.4 us, four 7.7, two 10.2.
+static int expand_chunk_log(long long rows, long long per_row, int sm_count) {
+  int log = 3;
+  while (log > 0 && rows * ((per_row + (1 << log) - 1) >> log) < (long long)sm_count * 8) --log;
+  return log;
+}
+
+template <bool ROWS>
+static cudaError_t launch_expand(int type, const int *ids, long long rows, const uint8_t *blocks, long long table_rows,
+                                 long long per_row, void *out, int out_dtype, int sm_count, cudaStream_t st) {
+  const int chunk_log = expand_chunk_log(rows, per_row, sm_count);
+  const long long want = (rows * ((per_row + (1 << chunk_log) - 1) >> chunk_log) + kExpandWarps - 1) / kExpandWarps;
+  // Two items per warp in long 16-bit arrays: a thread block's start and its codebook are then paid
+  // half as often (17408 x 5120 Q6_K to bf16 44.9 -> 43.1 us, IQ2_XS 45.1 -> 41.6); one item in fp32,
+  // which is bound by its output (67.8 against 69.8 us). More items leave a longer last wave.
+  const int rounds = out_dtype != 2 && want >= (long long)sm_count * 16 ? 2 : 1;
+  const long long grid = std::min((want + rounds - 1) / rounds, 0x7fffffffll);
   return with_type(type, [&](auto t) {
     constexpr int T = decltype(t)::value;
-    if (out_dtype == 0) ggml_dequantize_kernel<T, __half><<<grid, 256, 0, st>>>(blocks, n_blocks, static_cast<__half *>(out));
-    else if (out_dtype == 1)
-      ggml_dequantize_kernel<T, __nv_bfloat16><<<grid, 256, 0, st>>>(blocks, n_blocks, static_cast<__nv_bfloat16 *>(out));
-    else ggml_dequantize_kernel<T, float><<<grid, 256, 0, st>>>(blocks, n_blocks, static_cast<float *>(out));
+    auto launch = [&](auto *y) {
+      ggml_expand_kernel<T, std::remove_pointer_t<decltype(y)>, ROWS>
+          <<<(unsigned)grid, kExpandWarps * 32, 0, st>>>(ids, rows, blocks, table_rows, per_row, chunk_log, y);
+    };
+    if (out_dtype == 0) launch(static_cast<__half *>(out));
+    else if (out_dtype == 1) launch(static_cast<__nv_bfloat16 *>(out));
+    else launch(static_cast<float *>(out));
   });
+}
+
+cudaError_t launch_ggml_dequantize(int type, const uint8_t *blocks, long long n_blocks, void *out, int out_dtype, int sm_count,
+                                   cudaStream_t st) {
+  return launch_expand<false>(type, nullptr, 1, blocks, 1, n_blocks, out, out_dtype, sm_count, st);
 }
 
 cudaError_t launch_ggml_gather(int type, const int *ids, long long count, const uint8_t *blocks, long long table_rows,
                                long long k, void *out, int out_dtype, int sm_count, cudaStream_t st) {
-  const long long per_row = k / 256;
-  const long long want = (count * per_row * 32 + 255) / 256;
-  const int grid = (int)(want < (long long)sm_count * 32 ? want : (long long)sm_count * 32);
-  return with_type(type, [&](auto t) {
-    constexpr int T = decltype(t)::value;
-    if (out_dtype == 0)
-      ggml_gather_kernel<T, __half><<<grid, 256, 0, st>>>(ids, count, blocks, table_rows, per_row, static_cast<__half *>(out));
-    else if (out_dtype == 1)
-      ggml_gather_kernel<T, __nv_bfloat16>
-          <<<grid, 256, 0, st>>>(ids, count, blocks, table_rows, per_row, static_cast<__nv_bfloat16 *>(out));
-    else ggml_gather_kernel<T, float><<<grid, 256, 0, st>>>(ids, count, blocks, table_rows, per_row, static_cast<float *>(out));
-  });
+  return launch_expand<true>(type, ids, count, blocks, table_rows, k / 256, out, out_dtype, sm_count, st);
 }
 
 cudaError_t launch_ggml_rowdot(int type, const uint8_t *blocks, long long n, long long k, const __half *x, int rows, __half *y,

@@ -9,7 +9,8 @@ import torch
 
 from ishizuki_b200 import synth
 from ishizuki_b200 import _lib
-from ishizuki_b200.interface import BonsaiRuntime, FusedLinear, GGMLKernels, GGMLType, GGUFBlocks, IshizukiError, PackedLinear
+from ishizuki_b200.interface import (BonsaiRuntime, Context, FusedLinear, GGMLKernels, GGMLType, GGUFBlocks, IshizukiError,
+                                     PackedLinear, _ptr, _stream)
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -51,6 +52,25 @@ def test_decode_matches_oracle_on_a_projection(type_id):
     assert same_bits(got.cpu().numpy(), want)
     half = GGMLKernels.dequantize(dev(blocks), type_id, [n, k], dtype=torch.float16)
     assert np.array_equal(half.cpu().numpy().view(np.uint16), want.astype(np.float16).view(np.uint16))
+
+
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("offset,n_blocks", [(0, 1), (4, 9), (2, 65), (1, 13), (0, 9475)])
+def test_decode_from_any_address_and_count(type_id, offset, n_blocks):
+    """Blocks at every alignment the staging tells apart, counts that end inside a run of eight, the
+    three output types, and outputs that are not 16-byte aligned."""
+    raw = synth.ggml_blocks(np.random.default_rng(n_blocks), int(type_id), n_blocks, 256)
+    blocks = torch.zeros(raw.size + offset, dtype=torch.uint8, device="cuda")
+    blocks[offset:] = dev(raw)
+    want = torch.from_numpy(oracle.dequantize(int(type_id), raw))
+    for dtype in (torch.float32, torch.float16, torch.bfloat16):
+        got = GGMLKernels.dequantize(blocks[offset:], type_id, [n_blocks, 256], dtype=dtype)
+        assert torch.equal(got.cpu().view(-1), want.to(dtype))
+    ctx = Context.get(0)
+    out = torch.zeros(n_blocks * 256 + 9, dtype=torch.float16, device="cuda")
+    assert ctx.check(ctx.lib.ishi_ggml_dequantize(ctx.handle, int(type_id), _ptr(blocks[offset:]), n_blocks, _ptr(out[1:]),
+                                                  _lib.DT_F16, _stream()))
+    assert torch.equal(out[1:-8].cpu(), want.to(torch.float16)) and not out[-8:].any() and not out[0]
 
 
 def test_decode_refuses_what_the_reference_refuses():

@@ -41,9 +41,10 @@ struct FragAffine {
   static constexpr int kRowHeader = 4 * kGroups;     // bytes per row there
   static constexpr int kTileBytes = kHeader + 16 * kRowHeader;
   static constexpr int kSums = 4096;                 // offset of the group sums of x: [group][activation row] fp32
-  static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the per-unit staging
+  static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
+  static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
-  static constexpr int kXBytes = 4096 + (32 * kGroups > 128 ? 32 * kGroups : 128);
+  static constexpr int kXBytes = 4096 + (32 * kGroups > 128 ? 32 * kGroups : 128), kXFixed = 0;  // per unit of a staged region
 
   static __device__ __forceinline__ uint16_t tile_halfword(const FragSrc &s, long long p, int u, int hw) {
     if (hw < kHeader / 2) {
@@ -83,29 +84,24 @@ struct FragAffine {
   // row): lane l loads the eight values k = 8l .. 8l + 7. The fragment of k-step st = kMasks * q + m
   // sits at st * 256 + ((g ^ (q & 3)) * 4 + t) * 8: the xor spreads a store's quads over the banks,
   // and a k-step's 32 lanes still read one 256-byte run.
-  // after_loads() runs once, when the first batch of loads is in flight and before their values are
-  // used (the kernel issues its first weight copies there, behind the activations).
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     if (BITS == 2 && GS == 128 && a.rot_block == 128 && !a.rot_signs) {
-      stage_x_rot128(a, xfrag, ub0, uc, after_loads);
+      stage_x_rot128(a, x, M, xfrag, ub0, uc);
       return;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int tasks = uc * 8;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
-    if (warp >= tasks) after_loads();  // a warp without a task
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -144,7 +140,7 @@ struct FragAffine {
             sts64(dst + 256u, scale_down<2>(prmt(ea, eb, 0x7632u)), scale_down<2>(prmt(ec, ed, 0x7632u)));
           }
         }
-        // fp32 sums of x over the groups (GS / 8 lanes each), for the bias term
+        // fp32 sums of x over the groups (GS / 8 lanes each) in the codes' unit, for the bias term
         const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].x));
         const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].y));
         const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].z));
@@ -153,7 +149,7 @@ struct FragAffine {
 #pragma unroll
         for (int d = 1; d < GS / 8; d *= 2) s += __shfl_xor_sync(0xffffffffu, s, d);
         if ((lane & (GS / 8 - 1)) == 0)
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kSums + (uint32_t)((lane / (GS / 8)) * 8 + g) * 4u), "f"(s)
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kSums + (uint32_t)((lane / (GS / 8)) * 8 + g) * 4u), "f"(s * (1.f / 16777216.f))
                        : "memory");
       }
     }
@@ -180,8 +176,7 @@ struct FragAffine {
   // to fp32 rounding. Lane (g, t) ends up with the values k' = 16 (4 h + t) + g and + 8 of each
   // block: the codes g and g + 8 of the block's word 4 h + t, which are one B register of the
   // product's k-step (quad 2 block + h, mask g % 4), low register when g < 4.
-  template <class F>
-  static __device__ __forceinline__ void stage_x_rot128(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  static __device__ __forceinline__ void stage_x_rot128(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int tasks = uc * 8;
@@ -198,20 +193,18 @@ struct FragAffine {
     const uint32_t down1 = (uint32_t)(15 - 2 * m) << 10;  // 2^-(2 m) in fp16
     const uint32_t down = down1 | (down1 << 16);
     const float scale = 1.0f / sqrtf(128.f);
-    const uint32_t *xl = reinterpret_cast<const uint32_t *>(a.x + (long long)ub0 * 256) + lane;
+    const uint32_t *xl = reinterpret_cast<const uint32_t *>(x + (long long)ub0 * 256) + lane;
     const long long row_words = a.K >> 1;
-    if (warp >= tasks) after_loads();
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint32_t v[kBatch][4];  // [block * 2 + half]
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
-        const bool live = i < tasks && (i & 7) < a.M;
+        const bool live = i < tasks && (i & 7) < M;
         const uint32_t *src = xl + (long long)(i & 7) * row_words + (i >> 3) * 128;
 #pragma unroll
         for (int c = 0; c < 4; ++c) v[e][c] = live ? __ldg(src + 32 * c) : 0u;
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -256,7 +249,7 @@ struct FragAffine {
 #pragma unroll
         for (int d = 8; d; d >>= 1) keep += __shfl_xor_sync(0xffffffffu, keep, d);
         if ((lane & 15) == 0)
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kSums + (uint32_t)((lane >> 4) * 8 + r) * 4u), "f"(keep) : "memory");
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kSums + (uint32_t)((lane >> 4) * 8 + r) * 4u), "f"(keep * (1.f / 16777216.f)) : "memory");
       }
     }
   }
@@ -270,9 +263,9 @@ struct FragAffine {
 
   // One tile against the activations of its unit. acc: the warp's C fragment (MODE 0) or this
   // lane's partial dot products of rows g (acc[0]) and g + 8 (acc[2]) (MODE 1).
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t xu = xbase + (uint32_t)uq * kXBytes;
     // scales and biases of the two rows: kGroups halfwords of each, packed in pairs
     uint32_t hdr0[kRowHeader / 4], hdr1[kRowHeader / 4];
@@ -289,7 +282,7 @@ struct FragAffine {
       }
     }
     const uint32_t xl = xu + (uint32_t)(MODE == 0 ? lane : t) * 8u;  // single row: the fragments of activation row 0
-    float part[4];
+    float part[NB][4];
 
 #pragma unroll
     for (int j = 0; j < BITS; ++j) {
@@ -304,41 +297,49 @@ struct FragAffine {
         for (int m = 0; m < kMasks; ++m) {
           const uint32_t mask = (BITS == 4 ? 0x000f000fu : 0x00030003u) << (BITS * m);
           const uint32_t a0 = x0 & mask, a1 = x1 & mask, a2 = y0 & mask, a3 = y1 & mask;
-          const uint2 b = lds64(xq + (uint32_t)(kMasks * q + m) * 256u);
           const bool first = (q * kQuadK) % GS == 0 && m == 0;  // first k-step of a group
           if (MODE == 0) {
-            if (first) mma16816_first(part, a0, a1, a2, a3, b.x, b.y);
-            else mma16816(part, a0, a1, a2, a3, b.x, b.y);
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb) {
+              const uint2 b = lds64(xq + nb * a.xregion + (uint32_t)(kMasks * q + m) * 256u);
+              if (first) mma16816_first(part[nb], a0, a1, a2, a3, b.x, b.y);
+              else mma16816(part[nb], a0, a1, a2, a3, b.x, b.y);
+            }
           } else {
-            if (first) part[0] = part[1] = part[2] = part[3] = 0.f;
-            part[0] = fmaf(half_lo(a0), half_lo(b.x), part[0]);
-            part[0] = fmaf(half_hi(a0), half_hi(b.x), part[0]);
-            part[0] = fmaf(half_lo(a2), half_lo(b.y), part[0]);
-            part[0] = fmaf(half_hi(a2), half_hi(b.y), part[0]);
-            part[2] = fmaf(half_lo(a1), half_lo(b.x), part[2]);
-            part[2] = fmaf(half_hi(a1), half_hi(b.x), part[2]);
-            part[2] = fmaf(half_lo(a3), half_lo(b.y), part[2]);
-            part[2] = fmaf(half_hi(a3), half_hi(b.y), part[2]);
+            const uint2 b = lds64(xq + (uint32_t)(kMasks * q + m) * 256u);
+            float(&d)[4] = part[0];
+            if (first) d[0] = d[1] = d[2] = d[3] = 0.f;
+            d[0] = fmaf(half_lo(a0), half_lo(b.x), d[0]);
+            d[0] = fmaf(half_hi(a0), half_hi(b.x), d[0]);
+            d[0] = fmaf(half_lo(a2), half_lo(b.y), d[0]);
+            d[0] = fmaf(half_hi(a2), half_hi(b.y), d[0]);
+            d[2] = fmaf(half_lo(a1), half_lo(b.x), d[2]);
+            d[2] = fmaf(half_hi(a1), half_hi(b.x), d[2]);
+            d[2] = fmaf(half_lo(a3), half_lo(b.y), d[2]);
+            d[2] = fmaf(half_hi(a3), half_hi(b.y), d[2]);
           }
         }
         if (((q + 1) * kQuadK) % GS == 0) {
           // the group is complete: scale its code sum, add bias times the group's sum of x
           const int grp = (q * kQuadK) / GS;
-          const float s0 = param(hdr0[grp >> 1], grp & 1) * 16777216.f;
-          const float s1 = param(hdr1[grp >> 1], grp & 1) * 16777216.f;
+          const float s0 = param(hdr0[grp >> 1], grp & 1);
+          const float s1 = param(hdr1[grp >> 1], grp & 1);
           const float b0 = param(hdr0[(kGroups + grp) >> 1], (kGroups + grp) & 1);
           const float b1 = param(hdr1[(kGroups + grp) >> 1], (kGroups + grp) & 1);
           if (MODE == 0) {
-            const float2 xs = lds64f(xu + kSums + (uint32_t)(grp * 8 + 2 * t) * 4u);
-            acc[0] += s0 * part[0] + b0 * xs.x;
-            acc[1] += s0 * part[1] + b0 * xs.y;
-            acc[2] += s1 * part[2] + b1 * xs.x;
-            acc[3] += s1 * part[3] + b1 * xs.y;
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb) {
+              const float2 xs = lds64f(xu + nb * a.xregion + kSums + (uint32_t)(grp * 8 + 2 * t) * 4u);
+              acc[nb][0] += s0 * part[nb][0] + b0 * xs.x;
+              acc[nb][1] += s0 * part[nb][1] + b0 * xs.y;
+              acc[nb][2] += s1 * part[nb][2] + b1 * xs.x;
+              acc[nb][3] += s1 * part[nb][3] + b1 * xs.y;
+            }
           } else {
             // the bias term enters once per row: lane t = 0 adds it
             const float xs = t == 0 ? lds32f(xu + kSums + (uint32_t)(grp * 8) * 4u) : 0.f;
-            acc[0] += s0 * part[0] + b0 * xs;
-            acc[2] += s1 * part[2] + b1 * xs;
+            acc[0][0] += s0 * part[0][0] + b0 * xs;
+            acc[0][2] += s1 * part[0][2] + b1 * xs;
           }
         }
       }

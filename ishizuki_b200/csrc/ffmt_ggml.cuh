@@ -28,8 +28,9 @@ struct FragGGML {
   static constexpr int kBlock = ggml_type_bytes(TYPE);
   static_assert(kBlock > 0, "a GGML type with a decoder");
   static constexpr int kTileBytes = 16 * kBlock;
-  static constexpr int kXBytes = 8 * 512;  // per unit: eight rows of 512 bytes
-  static constexpr int kExtraBytes = 8 * 16;  // the rows' 16-byte skews
+  static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 16;  // a staged region: per unit eight rows of 512 bytes; the rows' skews
+  static constexpr double kUnit = 1.0;  // unit of the tile results
+  static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;     // one activation row runs through the MMA path as well
 
   static __device__ __forceinline__ uint8_t tile_byte(const FragSrc &s, long long p, int u, int b) {
@@ -49,26 +50,22 @@ struct FragGGML {
   static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t) {}
 
   // Activations of the CTA's column range as they lie in x (rows past M as zeros). A warp task is
-  // (unit, activation row): lane l loads and stores k = 8l .. 8l + 7. after_loads() runs once,
-  // when the first batch of loads is in flight. GGML blocks have no input rotation.
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  // (unit, activation row): lane l loads and stores k = 8l .. 8l + 7. GGML blocks have no input rotation.
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const uint32_t R = row_stride(a);
     const int tasks = uc * 8;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
-    if (warp >= tasks) after_loads();  // a warp without a task
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -88,9 +85,9 @@ struct FragGGML {
   }
 
   // One tile against the activations of its unit; acc is the warp's C fragment.
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     (void)lane;
     const uint32_t R = row_stride(a);
     const uint32_t xrow = xbase + (uint32_t)g * R + (uint32_t)uq * 512u + (uint32_t)t * 32u;
@@ -109,11 +106,15 @@ struct FragGGML {
       pack(lo1, w);
       decode8<TYPE>(blk1, 2 * sb + 1, w);
       pack(hi1, w);
-      const uint4 b0 = lds128(xrow + (uint32_t)j * 128u), b1 = lds128(xrow + (uint32_t)j * 128u + 16u);
-      mma16816(acc, lo0[0], lo1[0], lo0[1], lo1[1], b0.x, b0.y);
-      mma16816(acc, lo0[2], lo1[2], lo0[3], lo1[3], b0.z, b0.w);
-      mma16816(acc, hi0[0], hi1[0], hi0[1], hi1[1], b1.x, b1.y);
-      mma16816(acc, hi0[2], hi1[2], hi0[3], hi1[3], b1.z, b1.w);
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) {
+        const uint32_t xj = xrow + nb * a.xregion + (uint32_t)j * 128u;
+        const uint4 b0 = lds128(xj), b1 = lds128(xj + 16u);
+        mma16816(acc[nb], lo0[0], lo1[0], lo0[1], lo1[1], b0.x, b0.y);
+        mma16816(acc[nb], lo0[2], lo1[2], lo0[3], lo1[3], b0.z, b0.w);
+        mma16816(acc[nb], hi0[0], hi1[0], hi0[1], hi1[1], b1.x, b1.y);
+        mma16816(acc[nb], hi0[2], hi1[2], hi0[3], hi1[3], b1.z, b1.w);
+      }
     }
   }
 };

@@ -40,9 +40,10 @@ struct FragIQ1 {
   static constexpr int kBlock = TYPE == 19 ? 50 : 56;
   static constexpr int kD = 1024;
   static constexpr int kTileBytes = kD + 32;
-  static constexpr int kXBytes = 8 * 512 + 1024;  // per unit: eight rows of 512 bytes, and the entry sums
-  static constexpr int kGrid = 8 * 16;            // first in the extra region: the rows' 16-byte skews
-  static constexpr int kExtraBytes = kGrid + 2048 * 32;  // then the grid, four copies interleaved
+  // a staged region: per unit eight rows of 512 bytes and the entry sums; the rows' 16-byte skews
+  static constexpr int kXBytes = 8 * 512 + 1024, kXFixed = 8 * 16;
+  static constexpr double kUnit = 1.0;  // unit of the tile results
+  static constexpr int kExtraBytes = 2048 * 32;  // the grid, four copies interleaved
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {
@@ -98,39 +99,34 @@ struct FragIQ1 {
 
   // the grid (each value + 128), set up ahead of the dependency wait; four consecutive threads
   // store the four copies of an entry
-  static __device__ __forceinline__ void before_wait(const FragArgs &a, uint32_t xfrag) {
-    const uint32_t grid = xfrag + (uint32_t)a.umax * kXBytes + kGrid;
+  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t tables) {
     for (int i = threadIdx.x; i < 2048 * 4; i += blockDim.x) {
       const uint64_t v = d_iq1s_grid[i >> 2] ^ 0x8080808080808080ull;
-      sts64(grid + (uint32_t)i * 8u, (uint32_t)v, (uint32_t)(v >> 32));
+      sts64(tables + (uint32_t)i * 8u, (uint32_t)v, (uint32_t)(v >> 32));
     }
   }
 
   // Activations of the CTA's column range as they lie in x (rows past M as zeros), and per entry
   // (the eight values of one lane) their sum as fp16 high and low parts, where the MMA over the
   // entries reads them: entry E = 2 (4 j + t) + e is slot 2t + e + 8 (j % 2) of k-step j / 2, i.e.
-  // register j % 2, half e, of lane (r, t). after_loads() runs once, when the first batch of loads
-  // is in flight. No rotation here.
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  // register j % 2, half e, of lane (r, t). No rotation here.
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const uint32_t R = row_stride(a);
     const int tasks = uc * 8;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     const int sb = lane >> 1, j = sb >> 2, t = sb & 3;
     const uint32_t slot = (uint32_t)((j >> 1) * 512 + t * 16 + (j & 1) * 4 + (lane & 1) * 2);
-    if (warp >= tasks) after_loads();  // a warp without a task
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -164,13 +160,13 @@ struct FragIQ1 {
   }
 
   // One tile against the activations of its unit; acc is the warp's C fragment.
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t R = row_stride(a);
-    const uint32_t grid = xbase + (uint32_t)a.umax * kXBytes + kGrid + (uint32_t)(lane & 3) * 8u;
+    const uint32_t grid = tables + (uint32_t)(lane & 3) * 8u;
     const uint32_t xrow = xbase + (uint32_t)g * R + (uint32_t)uq * 512u + (uint32_t)t * 32u;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    float c[NB][4];
     uint32_t da[2][4];  // the A registers of the two k-steps over the entries: +-(2 s + 1)
 #pragma unroll
     for (int pc = 0; pc < 2; ++pc) {
@@ -191,33 +187,40 @@ struct FragIQ1 {
         // the two entries' +-(2 s + 1): the delta's sign bits 27 and 28 to bits 15 and 31
         da[j >> 1][(j & 1) * 2] = *reinterpret_cast<const uint32_t *>(&s0) ^ (((q0 >> 12) & 0x8000u) | ((q0 << 3) & 0x80000000u));
         da[j >> 1][(j & 1) * 2 + 1] = *reinterpret_cast<const uint32_t *>(&s1) ^ (((q1 >> 12) & 0x8000u) | ((q1 << 3) & 0x80000000u));
-        const uint4 x0 = lds128(xrow + (uint32_t)j * 128u), x1 = lds128(xrow + (uint32_t)j * 128u + 16u);
-        if (j == 0)
-          mma16816_first(c, lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
-        else
-          mma16816(c, lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
-        mma16816(c, lo0[2], lo1[2], lo0[3], lo1[3], x0.z, x0.w);
-        mma16816(c, hi0[0], hi1[0], hi0[1], hi1[1], x1.x, x1.y);
-        mma16816(c, hi0[2], hi1[2], hi0[3], hi1[3], x1.z, x1.w);
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          const uint32_t xj = xrow + nb * a.xregion + (uint32_t)j * 128u;
+          const uint4 x0 = lds128(xj), x1 = lds128(xj + 16u);
+          if (j == 0)
+            mma16816_first(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
+          else
+            mma16816(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
+          mma16816(c[nb], lo0[2], lo1[2], lo0[3], lo1[3], x0.z, x0.w);
+          mma16816(c[nb], hi0[0], hi1[0], hi0[1], hi1[1], x1.x, x1.y);
+          mma16816(c[nb], hi0[2], hi1[2], hi0[3], hi1[3], x1.z, x1.w);
+        }
       }
     }
     // sum_E +-(2 s + 1) * (sum of x over entry E): da[ks] = {row g: j = 2 ks, row g + 8: j = 2 ks,
     // row g: j = 2 ks + 1, row g + 8: j = 2 ks + 1} = the registers a0, a1, a2, a3 of k-step ks
     const uint32_t sums = sums_of(a, xbase, uq) + (uint32_t)lane * 16u;
-    float cm[4];
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
-      const uint4 bs = lds128(sums + (uint32_t)ks * 512u);
-      if (ks == 0) mma16816_first(cm, da[ks][0], da[ks][1], da[ks][2], da[ks][3], bs.x, bs.y);
-      else mma16816(cm, da[ks][0], da[ks][1], da[ks][2], da[ks][3], bs.x, bs.y);
-      mma16816(cm, da[ks][0], da[ks][1], da[ks][2], da[ks][3], bs.z, bs.w);
-    }
     const uint32_t dd = lds32(tile + (uint32_t)kD + (uint32_t)g * 4u);
     const float d0 = half_bits_to_float(dd & 0xffffu), d1 = half_bits_to_float(dd >> 16);
-    acc[0] = fmaf(d0, fmaf(0.125f, cm[0], c[0]), acc[0]);
-    acc[1] = fmaf(d0, fmaf(0.125f, cm[1], c[1]), acc[1]);
-    acc[2] = fmaf(d1, fmaf(0.125f, cm[2], c[2]), acc[2]);
-    acc[3] = fmaf(d1, fmaf(0.125f, cm[3], c[3]), acc[3]);
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      float cm[4];
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        const uint4 bs = lds128(sums + nb * a.xregion + (uint32_t)ks * 512u);
+        if (ks == 0) mma16816_first(cm, da[ks][0], da[ks][1], da[ks][2], da[ks][3], bs.x, bs.y);
+        else mma16816(cm, da[ks][0], da[ks][1], da[ks][2], da[ks][3], bs.x, bs.y);
+        mma16816(cm, da[ks][0], da[ks][1], da[ks][2], da[ks][3], bs.z, bs.w);
+      }
+      acc[nb][0] = fmaf(d0, fmaf(0.125f, cm[0], c[nb][0]), acc[nb][0]);
+      acc[nb][1] = fmaf(d0, fmaf(0.125f, cm[1], c[nb][1]), acc[nb][1]);
+      acc[nb][2] = fmaf(d1, fmaf(0.125f, cm[2], c[nb][2]), acc[nb][2]);
+      acc[nb][3] = fmaf(d1, fmaf(0.125f, cm[3], c[nb][3]), acc[nb][3]);
+    }
   }
 };
 

@@ -61,9 +61,9 @@ struct FragIQ2 {
   static constexpr int kScales = 1024;                       // offset of the per-lane scale bytes
   static constexpr int kD = kScales + (kWide ? 256 : 128);   // offset of d
   static constexpr int kTileBytes = kD + 32;
-  static constexpr int kXBytes = 8 * 512;        // per unit: eight rows of 512 bytes
-  static constexpr int kGrid = 8 * 16;           // first in the extra region: the rows' 16-byte skews
-  static constexpr int kExtraBytes = kGrid + kEntries * kCopies * 16;  // then the grid as fp16, its copies interleaved
+  static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 16;    // a staged region: per unit eight rows of 512 bytes; the rows' skews
+  static constexpr double kUnit = 0.125;         // tile results come in units of 1/8
+  static constexpr int kExtraBytes = kEntries * kCopies * 16;  // the grid as fp16, its copies interleaved
   static constexpr bool kRowMode = false;        // one activation row runs through the MMA path as well
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {
@@ -134,8 +134,7 @@ struct FragIQ2 {
   // What does not depend on the launches before this one, set up ahead of the dependency wait:
   // the grid. Entry i = eight fp16 magnitudes (the codes are 2 bits each: 0, 1, 2 -> 8, 25, 43);
   // eight consecutive threads store the eight copies of an entry, 128 contiguous bytes.
-  static __device__ __forceinline__ void before_wait(const FragArgs &a, uint32_t xfrag) {
-    const uint32_t grid = xfrag + (uint32_t)a.umax * kXBytes + kGrid;
+  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t tables) {
     for (int i = threadIdx.x; i < kEntries * kCopies; i += blockDim.x) {
       const int entry = i / kCopies;
       uint32_t w[4];
@@ -157,31 +156,28 @@ struct FragIQ2 {
           w[r] = *reinterpret_cast<const uint32_t *>(&h);
         }
       }
-      sts128u(grid + (uint32_t)i * 16u, make_uint4(w[0], w[1], w[2], w[3]));
+      sts128u(tables + (uint32_t)i * 16u, make_uint4(w[0], w[1], w[2], w[3]));
     }
   }
 
   // Activations of the CTA's column range as they lie in x (rows past M as zeros).
   // A warp task is (unit, activation row): lane l loads and stores k = 8l .. 8l + 7.
-  // after_loads() runs once, when the first batch of loads is in flight. IQ2_XS has no rotation.
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  // IQ2_XS has no rotation.
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const uint32_t R = row_stride(a);
     const int tasks = uc * 8;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
-    if (warp >= tasks) after_loads();  // a warp without a task
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -217,11 +213,11 @@ struct FragIQ2 {
   }
 
   // One tile against the activations of its unit; acc is the warp's C fragment.
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t R = row_stride(a);
-    const uint32_t grid = xbase + (uint32_t)a.umax * kXBytes + kGrid + (uint32_t)(lane & (kCopies - 1)) * 16u;
+    const uint32_t grid = tables + (uint32_t)(lane & (kCopies - 1)) * 16u;
     const uint32_t xrow = xbase + (uint32_t)g * R + (uint32_t)uq * 512u + (uint32_t)t * 32u;
     // scales: nibbles j of row g in the low half, of row g + 8 in the high half; IQ2_S: a byte per
     // sub-block (scale | high index bits << 4), row g in sw.x, row g + 8 in sw.y
@@ -229,7 +225,7 @@ struct FragIQ2 {
     uint2 sw = make_uint2(0u, 0u);
     if (kWide) sw = lds64(tile + kScales + (uint32_t)lane * 8u);
     else sn = lds32(tile + kScales + (uint32_t)lane * 4u);
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    float c[NB][4];
 #pragma unroll
     for (int pc = 0; pc < 2; ++pc) {
       const uint4 w = lds128(tile + (uint32_t)pc * 512u + (uint32_t)lane * 16u);
@@ -252,22 +248,29 @@ struct FragIQ2 {
           entry(lo1, q1 & 0xffffu, grid, s1);
           entry(hi1, q1 >> 16, grid, s1);
         }
-        const uint4 b0 = lds128(xrow + (uint32_t)j * 128u), b1 = lds128(xrow + (uint32_t)j * 128u + 16u);
-        if (j == 0)
-          mma16816_first(c, lo0[0], lo1[0], lo0[1], lo1[1], b0.x, b0.y);
-        else
-          mma16816(c, lo0[0], lo1[0], lo0[1], lo1[1], b0.x, b0.y);
-        mma16816(c, lo0[2], lo1[2], lo0[3], lo1[3], b0.z, b0.w);
-        mma16816(c, hi0[0], hi1[0], hi0[1], hi1[1], b1.x, b1.y);
-        mma16816(c, hi0[2], hi1[2], hi0[3], hi1[3], b1.z, b1.w);
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          const uint32_t xj = xrow + nb * a.xregion + (uint32_t)j * 128u;
+          const uint4 x0 = lds128(xj), x1 = lds128(xj + 16u);
+          if (j == 0)
+            mma16816_first(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
+          else
+            mma16816(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
+          mma16816(c[nb], lo0[2], lo1[2], lo0[3], lo1[3], x0.z, x0.w);
+          mma16816(c[nb], hi0[0], hi1[0], hi0[1], hi1[1], x1.x, x1.y);
+          mma16816(c[nb], hi0[2], hi1[2], hi0[3], hi1[3], x1.z, x1.w);
+        }
       }
     }
     const uint32_t dd = lds32(tile + (uint32_t)kD + (uint32_t)g * 4u);
-    const float d0 = half_bits_to_float(dd & 0xffffu) * 0.125f, d1 = half_bits_to_float(dd >> 16) * 0.125f;
-    acc[0] = fmaf(d0, c[0], acc[0]);
-    acc[1] = fmaf(d0, c[1], acc[1]);
-    acc[2] = fmaf(d1, c[2], acc[2]);
-    acc[3] = fmaf(d1, c[3], acc[3]);
+    const float d0 = half_bits_to_float(dd & 0xffffu), d1 = half_bits_to_float(dd >> 16);
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      acc[nb][0] = fmaf(d0, c[nb][0], acc[nb][0]);
+      acc[nb][1] = fmaf(d0, c[nb][1], acc[nb][1]);
+      acc[nb][2] = fmaf(d1, c[nb][2], acc[nb][2]);
+      acc[nb][3] = fmaf(d1, c[nb][3], acc[nb][3]);
+    }
   }
 };
 

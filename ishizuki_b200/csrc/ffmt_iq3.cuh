@@ -36,9 +36,9 @@ struct FragIQ3 {
   static constexpr int kEntries = kNine ? 512 : 256;
   static constexpr int kSigns = 1024, kScales = 1536, kD = 1792;
   static constexpr int kTileBytes = kD + 32;
-  static constexpr int kXBytes = 8 * 512;  // per unit: eight rows of 512 bytes
-  static constexpr int kGrid = 8 * 16;     // first in the extra region: the rows' 16-byte skews
-  static constexpr int kExtraBytes = kGrid + kEntries * 128;  // then the grid as fp16, sixteen copies interleaved
+  static constexpr int kXBytes = FragIQ2<17>::kXBytes, kXFixed = FragIQ2<17>::kXFixed;
+  static constexpr double kUnit = kNine ? 1.0 : 0.25;  // unit of the tile results
+  static constexpr int kExtraBytes = kEntries * 128;  // the grid as fp16, sixteen copies interleaved
   static constexpr bool kRowMode = false;  // one activation row runs through the MMA path as well
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {
@@ -97,20 +97,18 @@ struct FragIQ3 {
 
   // the grid, set up ahead of the dependency wait; sixteen consecutive threads store the sixteen
   // copies of an entry, 128 contiguous bytes
-  static __device__ __forceinline__ void before_wait(const FragArgs &a, uint32_t xfrag) {
-    const uint32_t grid = xfrag + (uint32_t)a.umax * kXBytes + kGrid;
+  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t tables) {
     for (int i = threadIdx.x; i < kEntries * 16; i += blockDim.x) {
       const uint32_t bytes = kNine ? d_iq3s_grid[i >> 4] : d_iq3xxs_grid[i >> 4];  // four magnitudes, a byte each
       const __half2 lo = __halves2half2(__int2half_rn((int)(bytes & 0xffu)), __int2half_rn((int)((bytes >> 8) & 0xffu)));
       const __half2 hi = __halves2half2(__int2half_rn((int)((bytes >> 16) & 0xffu)), __int2half_rn((int)(bytes >> 24)));
-      sts64(grid + (uint32_t)i * 8u, *reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+      sts64(tables + (uint32_t)i * 8u, *reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
     }
   }
 
   // the activations as for IQ2_XS: the rows as they lie in x
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
-    FragIQ2<17>::stage_x(a, xfrag, ub0, uc, after_loads);
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
+    FragIQ2<17>::stage_x(a, x, M, xfrag, ub0, uc);
   }
 
   // eight weights as four A registers, magnitude * (2 s + 1) * sign: the two grid indices (this
@@ -133,16 +131,16 @@ struct FragIQ3 {
   }
 
   // One tile against the activations of its unit; acc is the warp's C fragment.
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t R = row_stride(a);
-    const uint32_t grid = xbase + (uint32_t)a.umax * kXBytes + kGrid + (uint32_t)(lane & 15) * 8u;
+    const uint32_t grid = tables + (uint32_t)(lane & 15) * 8u;
     const uint32_t xrow = xbase + (uint32_t)g * R + (uint32_t)uq * 512u + (uint32_t)t * 32u;
     const uint4 sg = lds128(tile + kSigns + (uint32_t)lane * 16u);  // word j: sign bytes of row g (low half), of row g + 8
     const uint2 sw = lds64(tile + kScales + (uint32_t)lane * 8u);   // byte j: scale | ninth bits << 4; row g, row g + 8
     const uint32_t sgw[4] = {sg.x, sg.y, sg.z, sg.w};
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    float c[NB][4];
 #pragma unroll
     for (int pc = 0; pc < 2; ++pc) {
       const uint4 w = lds128(tile + (uint32_t)pc * 512u + (uint32_t)lane * 16u);
@@ -157,23 +155,29 @@ struct FragIQ3 {
         entry(hi0, index_of(q0, y0, 2), index_of(q0, y0, 3), (sgw[j] >> 8) & 0xffu, grid, s0);
         entry(lo1, index_of(q1, y1, 0), index_of(q1, y1, 1), (sgw[j] >> 16) & 0xffu, grid, s1);
         entry(hi1, index_of(q1, y1, 2), index_of(q1, y1, 3), sgw[j] >> 24, grid, s1);
-        const uint4 b0 = lds128(xrow + (uint32_t)j * 128u), b1 = lds128(xrow + (uint32_t)j * 128u + 16u);
-        if (j == 0)
-          mma16816_first(c, lo0[0], lo1[0], lo0[1], lo1[1], b0.x, b0.y);
-        else
-          mma16816(c, lo0[0], lo1[0], lo0[1], lo1[1], b0.x, b0.y);
-        mma16816(c, lo0[2], lo1[2], lo0[3], lo1[3], b0.z, b0.w);
-        mma16816(c, hi0[0], hi1[0], hi0[1], hi1[1], b1.x, b1.y);
-        mma16816(c, hi0[2], hi1[2], hi0[3], hi1[3], b1.z, b1.w);
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          const uint32_t xj = xrow + nb * a.xregion + (uint32_t)j * 128u;
+          const uint4 x0 = lds128(xj), x1 = lds128(xj + 16u);
+          if (j == 0)
+            mma16816_first(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
+          else
+            mma16816(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
+          mma16816(c[nb], lo0[2], lo1[2], lo0[3], lo1[3], x0.z, x0.w);
+          mma16816(c[nb], hi0[0], hi1[0], hi0[1], hi1[1], x1.x, x1.y);
+          mma16816(c[nb], hi0[2], hi1[2], hi0[3], hi1[3], x1.z, x1.w);
+        }
       }
     }
     const uint32_t dd = lds32(tile + (uint32_t)kD + (uint32_t)g * 4u);
-    const float f = kNine ? 1.0f : 0.25f;
-    const float d0 = half_bits_to_float(dd & 0xffffu) * f, d1 = half_bits_to_float(dd >> 16) * f;
-    acc[0] = fmaf(d0, c[0], acc[0]);
-    acc[1] = fmaf(d0, c[1], acc[1]);
-    acc[2] = fmaf(d1, c[2], acc[2]);
-    acc[3] = fmaf(d1, c[3], acc[3]);
+    const float d0 = half_bits_to_float(dd & 0xffffu), d1 = half_bits_to_float(dd >> 16);
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      acc[nb][0] = fmaf(d0, c[nb][0], acc[nb][0]);
+      acc[nb][1] = fmaf(d0, c[nb][1], acc[nb][1]);
+      acc[nb][2] = fmaf(d1, c[nb][2], acc[nb][2]);
+      acc[nb][3] = fmaf(d1, c[nb][3], acc[nb][3]);
+    }
   }
 };
 

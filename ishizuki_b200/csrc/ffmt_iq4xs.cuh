@@ -26,7 +26,8 @@ namespace ishi {
 
 struct FragIQ4XS {
   static constexpr int kTileBytes = 2048 + 128 + 32;
-  static constexpr int kXBytes = 4096;                // per unit: sixteen k-steps of 256 bytes
+  static constexpr int kXBytes = 4096, kXFixed = 0;   // a staged region: per unit sixteen k-steps of 256 bytes
+  static constexpr double kUnit = 1.0;  // unit of the tile results
   static constexpr int kExtraBytes = 256 * 128;       // the pair table: entry e of lane l's copy at e * 128 + l * 4
   static constexpr bool kRowMode = false;             // one activation row runs through the MMA path as well
 
@@ -65,12 +66,11 @@ struct FragIQ4XS {
   }
 
   // the pair table, filled ahead of the dependency wait: it depends on no earlier launch
-  static __device__ __forceinline__ void before_wait(const FragArgs &a, uint32_t xfrag) {
-    const uint32_t table = xfrag + (uint32_t)a.umax * kXBytes;
+  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t tables) {
     for (int i = threadIdx.x; i < 256 * 32; i += blockDim.x) {
       const int e = i >> 5;  // consecutive threads store one entry's 32 copies: consecutive banks
       const __half2 pair = __halves2half2(__int2half_rn((int)d_kvalues_iq4nl[e & 15]), __int2half_rn((int)d_kvalues_iq4nl[e >> 4]));
-      sts32(table + (uint32_t)i * 4u, *reinterpret_cast<const uint32_t *>(&pair));
+      sts32(tables + (uint32_t)i * 4u, *reinterpret_cast<const uint32_t *>(&pair));
     }
   }
 
@@ -81,27 +81,24 @@ struct FragIQ4XS {
   // builds the pairs of t = 2 (l % 4), the second those of t + 1. The B registers of k-step
   // ks = 2 ib + s and quad row r lie at ks * 256 + ((r ^ (ks % 8)) * 4 + t) * 8; the xor spreads the
   // stores over the banks, a warp's read of one k-step is still one 256-byte run.
-  // after_loads() runs once, when the first loads are in flight. No rotation here.
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  // No rotation here.
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int tasks = uc * 8;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     const int ib = lane >> 2, r4 = lane & 3;
     const bool second = r4 >= 2;
     const int t = second ? 2 * (r4 - 2) + 1 : 2 * r4;
-    if (warp >= tasks) after_loads();  // a warp without a task
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -132,13 +129,15 @@ struct FragIQ4XS {
   }
 
   // One tile against the activations of its unit; acc is the warp's C fragment.
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t xu = xbase + (uint32_t)uq * kXBytes;
-    const uint32_t table = xbase + (uint32_t)a.umax * kXBytes + (uint32_t)lane * 4u;
+    const uint32_t table = tables + (uint32_t)lane * 4u;
     const uint2 sc0 = lds64(tile + 2048u + (uint32_t)g * 8u), sc1 = lds64(tile + 2048u + (uint32_t)(g + 8) * 8u);
-    float su[4] = {0.f, 0.f, 0.f, 0.f};  // sum over the sub-blocks of (ls - 32) * (sum of value * x), d follows at the end
+    float su[NB][4];  // sum over the sub-blocks of (ls - 32) * (sum of value * x), d follows at the end
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = su[nb][2] = su[nb][3] = 0.f;
     const uint32_t xl = xu + (uint32_t)t * 8u;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -147,26 +146,35 @@ struct FragIQ4XS {
       for (int e = 0; e < 2; ++e) {
         const int sb = 2 * j + e;
         const uint32_t w0 = e ? q.y : q.x, w1 = e ? q.w : q.z;
-        float part[4];
+        float part[NB][4];
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
           const int ks = 2 * sb + s;
-          const uint2 b = lds64(xl + (uint32_t)ks * 256u + (uint32_t)((g ^ (ks & 7)) * 32));
           const uint32_t a0 = pair_of(w0, 2 * s, table), a2 = pair_of(w0, 2 * s + 1, table);
           const uint32_t a1 = pair_of(w1, 2 * s, table), a3 = pair_of(w1, 2 * s + 1, table);
-          if (s == 0) mma16816_first(part, a0, a1, a2, a3, b.x, b.y);
-          else mma16816(part, a0, a1, a2, a3, b.x, b.y);
+#pragma unroll
+          for (int nb = 0; nb < NB; ++nb) {
+            const uint2 b = lds64(xl + nb * a.xregion + (uint32_t)ks * 256u + (uint32_t)((g ^ (ks & 7)) * 32));
+            if (s == 0) mma16816_first(part[nb], a0, a1, a2, a3, b.x, b.y);
+            else mma16816(part[nb], a0, a1, a2, a3, b.x, b.y);
+          }
         }
         const float f0 = byte_float(sb < 4 ? sc0.x : sc0.y, sb & 3) - 8388640.f;  // ls - 32, exact
         const float f1 = byte_float(sb < 4 ? sc1.x : sc1.y, sb & 3) - 8388640.f;
-        su[0] = fmaf(f0, part[0], su[0]), su[1] = fmaf(f0, part[1], su[1]);
-        su[2] = fmaf(f1, part[2], su[2]), su[3] = fmaf(f1, part[3], su[3]);
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          su[nb][0] = fmaf(f0, part[nb][0], su[nb][0]), su[nb][1] = fmaf(f0, part[nb][1], su[nb][1]);
+          su[nb][2] = fmaf(f1, part[nb][2], su[nb][2]), su[nb][3] = fmaf(f1, part[nb][3], su[nb][3]);
+        }
       }
     }
     const uint32_t dd = lds32(tile + 2176u + (uint32_t)g * 4u);
     const float d0 = half_bits_to_float(dd & 0xffffu), d1 = half_bits_to_float(dd >> 16);
-    acc[0] = fmaf(d0, su[0], acc[0]), acc[1] = fmaf(d0, su[1], acc[1]);
-    acc[2] = fmaf(d1, su[2], acc[2]), acc[3] = fmaf(d1, su[3], acc[3]);
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      acc[nb][0] = fmaf(d0, su[nb][0], acc[nb][0]), acc[nb][1] = fmaf(d0, su[nb][1], acc[nb][1]);
+      acc[nb][2] = fmaf(d1, su[nb][2], acc[nb][2]), acc[nb][3] = fmaf(d1, su[nb][3], acc[nb][3]);
+    }
   }
 };
 

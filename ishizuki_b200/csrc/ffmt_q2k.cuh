@@ -30,7 +30,8 @@ namespace ishi {
 struct FragQ2K {
   static constexpr int kTileBytes = 16 * 84;
   static constexpr int kXSums = 4096;           // after the activations: [lane][hi hi | lo lo] sub-block sums
-  static constexpr int kXBytes = kXSums + 512;  // per unit
+  static constexpr int kXBytes = kXSums + 512, kXFixed = 0;  // per unit of a staged region
+  static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;       // one activation row runs through the MMA path as well
 
@@ -74,29 +75,25 @@ struct FragQ2K {
   // t = 2 (l % 2) and t + 1 of quad r multiply in k-step is; stored divided by 4^j at
   // is * 256 + ((r ^ (is % 8)) * 4 + t) * 8 (the xor spreads the stores over the banks, a warp's read
   // of one k-step is still one 256-byte run). Then the sub-block sums of the undivided values
-  // (fp16 hi + lo) for the MMA over sub-blocks. after_loads() runs once, when the first loads are
-  // in flight. No rotation here.
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  // (fp16 hi + lo) for the MMA over sub-blocks. No rotation here.
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int tasks = uc * 8;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     const int j = (lane >> 2) & 3;
     const int is = 8 * (lane >> 4) + 2 * j + ((lane & 3) >> 1);
     const uint32_t down1 = (uint32_t)(15 - 2 * j) << 10;  // 4^-j in fp16
     const uint32_t down = down1 | (down1 << 16);
-    if (warp >= tasks) after_loads();  // a warp without a task
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -135,25 +132,19 @@ struct FragQ2K {
   static __device__ __forceinline__ float byte_float(uint32_t w, int byte) {
     return __uint_as_float(prmt(w, 0x4b000000u, 0x7440u | (uint32_t)byte));
   }
-  // two bytes (each < 16) of a word as a half2: the bits of 1024 + b, minus 1024
-  static __device__ __forceinline__ uint32_t byte_pair(uint32_t w, uint32_t selector) {
-    const uint32_t bits = prmt(w, 0x64646464u, selector);
-    const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&bits), __float2half2_rn(1024.f));
-    return *reinterpret_cast<const uint32_t *>(&v);
-  }
-
   // One tile against the activations of its unit; acc is the warp's C fragment.
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
-    (void)a;
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t xu = xbase + (uint32_t)uq * kXBytes;
     const uint4 h0 = lds128(tile + 1024u + (uint32_t)g * 16u), h1 = lds128(tile + 1024u + (uint32_t)(g + 8) * 16u);
     // the scales (low nibbles), word tw = sub-blocks (2 tw, 2 tw + 1, 2 tw + 8, 2 tw + 9)
     const uint32_t sl0[4] = {h0.x & 0x0f0f0f0fu, h0.y & 0x0f0f0f0fu, h0.z & 0x0f0f0f0fu, h0.w & 0x0f0f0f0fu};
     const uint32_t sl1[4] = {h1.x & 0x0f0f0f0fu, h1.y & 0x0f0f0f0fu, h1.z & 0x0f0f0f0fu, h1.w & 0x0f0f0f0fu};
     const uint32_t xl = xu + (uint32_t)t * 8u;
-    float su[4] = {0.f, 0.f, 0.f, 0.f};
+    float su[NB][4];
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = su[nb][2] = su[nb][3] = 0.f;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const uint4 q = lds128(tile + (uint32_t)n * 512u + (uint32_t)lane * 16u);
@@ -165,13 +156,16 @@ struct FragQ2K {
         for (int j = 0; j < 4; ++j) {
           const int is = 8 * n + 2 * j + h;
           const uint32_t mask = 0x00030003u << (2 * j);
-          const uint2 b = lds64(xl + (uint32_t)is * 256u + (uint32_t)((g ^ (is & 7)) * 32));
-          float part[4];
-          mma16816_first(part, w0 & mask, w1 & mask, y0 & mask, y1 & mask, b.x, b.y);
           const int tw = (is & 7) >> 1, e = (is & 1) + 2 * (is >> 3);
           const float f0 = byte_float(sl0[tw], e) - 8388608.f, f1 = byte_float(sl1[tw], e) - 8388608.f;
-          su[0] = fmaf(f0, part[0], su[0]), su[1] = fmaf(f0, part[1], su[1]);
-          su[2] = fmaf(f1, part[2], su[2]), su[3] = fmaf(f1, part[3], su[3]);
+#pragma unroll
+          for (int nb = 0; nb < NB; ++nb) {
+            const uint2 b = lds64(xl + nb * a.xregion + (uint32_t)is * 256u + (uint32_t)((g ^ (is & 7)) * 32));
+            float part[4];
+            mma16816_first(part, w0 & mask, w1 & mask, y0 & mask, y1 & mask, b.x, b.y);
+            su[nb][0] = fmaf(f0, part[0], su[nb][0]), su[nb][1] = fmaf(f0, part[1], su[nb][1]);
+            su[nb][2] = fmaf(f1, part[2], su[nb][2]), su[nb][3] = fmaf(f1, part[3], su[nb][3]);
+          }
         }
       }
     }
@@ -179,19 +173,23 @@ struct FragQ2K {
     // sub-blocks 2t, 2t + 1, 2t + 8, 2t + 9, the word t of each row's sixteen bytes, high nibbles
     const uint32_t m0 = ((t == 0 ? h0.x : t == 1 ? h0.y : t == 2 ? h0.z : h0.w) >> 4) & 0x0f0f0f0fu;
     const uint32_t m1 = ((t == 0 ? h1.x : t == 1 ? h1.y : t == 2 ? h1.z : h1.w) >> 4) & 0x0f0f0f0fu;
-    const uint4 bs = lds128(xu + kXSums + (uint32_t)lane * 16u);
-    float cm[4];
-    const uint32_t a0 = byte_pair(m0, 0x4140u), a1 = byte_pair(m1, 0x4140u);
-    const uint32_t a2 = byte_pair(m0, 0x4342u), a3 = byte_pair(m1, 0x4342u);
-    mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
-    mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);
+    // (a byte as the low bits of an fp16 is the subnormal number m * 2^-24, as the codes are)
+    const uint32_t a0 = prmt(m0, 0u, 0x4140u), a1 = prmt(m1, 0u, 0x4140u);
+    const uint32_t a2 = prmt(m0, 0u, 0x4342u), a3 = prmt(m1, 0u, 0x4342u);
     const uint32_t dd = lds32(tile + 1280u + (uint32_t)g * 4u), mm = lds32(tile + 1312u + (uint32_t)g * 4u);
-    const float d0 = half_bits_to_float(dd & 0xffffu) * 16777216.f, d1 = half_bits_to_float(dd >> 16) * 16777216.f;
+    const float d0 = half_bits_to_float(dd & 0xffffu), d1 = half_bits_to_float(dd >> 16);
     const float n0 = -half_bits_to_float(mm & 0xffffu), n1 = -half_bits_to_float(mm >> 16);
-    acc[0] = fmaf(d0, su[0], fmaf(n0, cm[0], acc[0]));
-    acc[1] = fmaf(d0, su[1], fmaf(n0, cm[1], acc[1]));
-    acc[2] = fmaf(d1, su[2], fmaf(n1, cm[2], acc[2]));
-    acc[3] = fmaf(d1, su[3], fmaf(n1, cm[3], acc[3]));
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      const uint4 bs = lds128(xu + nb * a.xregion + kXSums + (uint32_t)lane * 16u);
+      float cm[4];
+      mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
+      mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);
+      acc[nb][0] = fmaf(d0, su[nb][0], fmaf(n0, cm[0], acc[nb][0]));
+      acc[nb][1] = fmaf(d0, su[nb][1], fmaf(n0, cm[1], acc[nb][1]));
+      acc[nb][2] = fmaf(d1, su[nb][2], fmaf(n1, cm[2], acc[nb][2]));
+      acc[nb][3] = fmaf(d1, su[nb][3], fmaf(n1, cm[3], acc[nb][3]));
+    }
   }
 };
 

@@ -43,13 +43,14 @@ namespace ishi {
 
 struct FragQ4K {
   static constexpr int kTileBytes = 2048 + 16 * 16 + 16 * 4;
-  static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the per-unit staging
+  static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
+  static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
   static constexpr int kSumBytes = 384;  // per unit: sub-block sums as fp16 hi / lo pairs, [lane][8 bytes], then
                                          // the fp32 sub-block sums of row 0 (single-row kernel) @256
-  // shared memory the kernel sets aside per unit of the column range: eight rows of 512 bytes, the
-  // sums, and a share of the rows' 64-byte skew (8 * 64 <= 512 for any range of one unit or more)
-  static constexpr int kXBytes = 8 * 512 + kSumBytes + 512;
+  // a staged region: per unit of the column range eight rows of 512 bytes and the sums, and once the
+  // rows' 64-byte skews
+  static constexpr int kXBytes = 8 * 512 + kSumBytes, kXFixed = 512;
 
   // ggml's get_scale_min_k4 on the twelve packed bytes of a block
   static __device__ __forceinline__ void scale_min(const uint8_t *q, int j, uint32_t *sc, uint32_t *m) {
@@ -99,31 +100,27 @@ struct FragQ4K {
 
   // Activations of the CTA's column range. A warp task is (unit, activation row): lane l loads
   // k = 8l .. 8l + 7 of it, stores them as they lie in x (rows past M as zeros) and the warp adds up
-  // every sub-block for the minimum term. after_loads() runs once, when the first batch of loads is
-  // in flight. Q4_K has no input rotation.
+  // every sub-block for the minimum term. Q4_K has no input rotation.
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
   // nothing to set up ahead of the dependency wait
   static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t) {}
 
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const uint32_t R = row_stride(a), sums = xfrag + 8u * R;
     const int tasks = uc * 8, jj = lane >> 3;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
-    if (warp >= tasks) after_loads();  // a warp without a task
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -158,9 +155,9 @@ struct FragQ4K {
 
   // One tile against the activations of its unit. acc: the warp's C fragment (MODE 0) or this
   // lane's partial dot products of rows g (acc[0]) and g + 8 (acc[2]) (MODE 1).
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     // this lane's sub-blocks 2t, 2t + 1 of rows g and g + 8: bytes m_lo, sc_lo, m_hi, sc_hi
     const uint32_t v0 = lds32(tile + 2048u + (uint32_t)lane * 4u), v1 = lds32(tile + 2048u + 128u + (uint32_t)lane * 4u);
     const uint32_t dd0 = lds32(tile + 2304u + (uint32_t)g * 4u), dd1 = lds32(tile + 2304u + 32u + (uint32_t)g * 4u);
@@ -177,18 +174,20 @@ struct FragQ4K {
     const uint32_t xrow = xbase + (uint32_t)(MODE == 0 ? g : 0) * R + (uint32_t)t * 144u + (uint32_t)uq * 512u;
     const uint32_t xsum = xbase + 8u * R + (uint32_t)uq * kSumBytes;
 
-    float c[4] = {0.f, 0.f, 0.f, 0.f};  // one MMA chain over the whole tile
+    float c[NB][4];  // one MMA chain over the whole tile (MODE 1: four partial dot products)
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) c[nb][0] = c[nb][1] = c[nb][2] = c[nb][3] = 0.f;
 #pragma unroll
     for (int jj = 0; jj < 4; ++jj) {
       const uint4 w = lds128(tile + (uint32_t)jj * 512u + (uint32_t)lane * 16u);  // row g: w.x, w.y; row g + 8: w.z, w.w
       const uint32_t xj = xrow ^ (uint32_t)(jj << 4);        // piece jj ^ t of the chunk
-      const uint4 blo = lds128(xj), bhi = lds128(xj + 64u);  // k-steps (s = 0, 1) of the low / high sub-block
+      uint4 blo[NB], bhi[NB];  // k-steps (s = 0, 1) of the low / high sub-block
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) blo[nb] = lds128(xj + nb * a.xregion), bhi[nb] = lds128(xj + nb * a.xregion + 64u);
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         const uint32_t x0 = s ? w.y : w.x, x1 = s ? w.w : w.z;
         const uint32_t y0 = x0 >> 8, y1 = x1 >> 8;
-        const uint32_t bl0 = s ? blo.z : blo.x, bl1 = s ? blo.w : blo.y;
-        const uint32_t bh0 = s ? bhi.z : bhi.x, bh1 = s ? bhi.w : bhi.y;
         // low nibbles: q * sc as an integer in each half (a subnormal fp16 bit pattern, x 2^-24)
         const uint32_t a0 = (x0 & 0x000f000fu) * sl0, a1 = (x1 & 0x000f000fu) * sl1;
         const uint32_t a2 = (y0 & 0x000f000fu) * sl0, a3 = (y1 & 0x000f000fu) * sl1;
@@ -201,53 +200,64 @@ struct FragQ4K {
         const uint32_t e0 = *reinterpret_cast<const uint32_t *>(&c0), e1 = *reinterpret_cast<const uint32_t *>(&c1);
         const uint32_t e2 = *reinterpret_cast<const uint32_t *>(&c2), e3 = *reinterpret_cast<const uint32_t *>(&c3);
         if (MODE == 0) {
-          if (jj == 0 && s == 0)
-            mma16816_first(c, a0, a1, a2, a3, bl0, bl1);
-          else
-            mma16816(c, a0, a1, a2, a3, bl0, bl1);
-          mma16816(c, e0, e1, e2, e3, bh0, bh1);
+#pragma unroll
+          for (int nb = 0; nb < NB; ++nb) {
+            const uint32_t bl0 = s ? blo[nb].z : blo[nb].x, bl1 = s ? blo[nb].w : blo[nb].y;
+            const uint32_t bh0 = s ? bhi[nb].z : bhi[nb].x, bh1 = s ? bhi[nb].w : bhi[nb].y;
+            if (jj == 0 && s == 0)
+              mma16816_first(c[nb], a0, a1, a2, a3, bl0, bl1);
+            else
+              mma16816(c[nb], a0, a1, a2, a3, bl0, bl1);
+            mma16816(c[nb], e0, e1, e2, e3, bh0, bh1);
+          }
         } else {
-          c[0] = fmaf(half_lo(a0), half_lo(bl0), c[0]);
-          c[0] = fmaf(half_hi(a0), half_hi(bl0), c[0]);
-          c[0] = fmaf(half_lo(a2), half_lo(bl1), c[0]);
-          c[0] = fmaf(half_hi(a2), half_hi(bl1), c[0]);
-          c[2] = fmaf(half_lo(a1), half_lo(bl0), c[2]);
-          c[2] = fmaf(half_hi(a1), half_hi(bl0), c[2]);
-          c[2] = fmaf(half_lo(a3), half_lo(bl1), c[2]);
-          c[2] = fmaf(half_hi(a3), half_hi(bl1), c[2]);
-          c[1] = fmaf(half_lo(e0), half_lo(bh0), c[1]);
-          c[1] = fmaf(half_hi(e0), half_hi(bh0), c[1]);
-          c[1] = fmaf(half_lo(e2), half_lo(bh1), c[1]);
-          c[1] = fmaf(half_hi(e2), half_hi(bh1), c[1]);
-          c[3] = fmaf(half_lo(e1), half_lo(bh0), c[3]);
-          c[3] = fmaf(half_hi(e1), half_hi(bh0), c[3]);
-          c[3] = fmaf(half_lo(e3), half_lo(bh1), c[3]);
-          c[3] = fmaf(half_hi(e3), half_hi(bh1), c[3]);
+          float (&d)[4] = c[0];
+          const uint32_t bl0 = s ? blo[0].z : blo[0].x, bl1 = s ? blo[0].w : blo[0].y;
+          const uint32_t bh0 = s ? bhi[0].z : bhi[0].x, bh1 = s ? bhi[0].w : bhi[0].y;
+          d[0] = fmaf(half_lo(a0), half_lo(bl0), d[0]);
+          d[0] = fmaf(half_hi(a0), half_hi(bl0), d[0]);
+          d[0] = fmaf(half_lo(a2), half_lo(bl1), d[0]);
+          d[0] = fmaf(half_hi(a2), half_hi(bl1), d[0]);
+          d[2] = fmaf(half_lo(a1), half_lo(bl0), d[2]);
+          d[2] = fmaf(half_hi(a1), half_hi(bl0), d[2]);
+          d[2] = fmaf(half_lo(a3), half_lo(bl1), d[2]);
+          d[2] = fmaf(half_hi(a3), half_hi(bl1), d[2]);
+          d[1] = fmaf(half_lo(e0), half_lo(bh0), d[1]);
+          d[1] = fmaf(half_hi(e0), half_hi(bh0), d[1]);
+          d[1] = fmaf(half_lo(e2), half_lo(bh1), d[1]);
+          d[1] = fmaf(half_hi(e2), half_hi(bh1), d[1]);
+          d[3] = fmaf(half_lo(e1), half_lo(bh0), d[3]);
+          d[3] = fmaf(half_hi(e1), half_hi(bh0), d[3]);
+          d[3] = fmaf(half_lo(e3), half_lo(bh1), d[3]);
+          d[3] = fmaf(half_hi(e3), half_hi(bh1), d[3]);
         }
       }
     }
 
-    const float d0 = half_bits_to_float(dd0 & 0xffffu) * 16777216.f, d1 = half_bits_to_float(dd1 & 0xffffu) * 16777216.f;
+    const float d0 = half_bits_to_float(dd0 & 0xffffu), d1 = half_bits_to_float(dd1 & 0xffffu);
     const float n0 = half_bits_to_float(dd0 >> 16), n1 = half_bits_to_float(dd1 >> 16);
     if (MODE == 0) {
       // minimum term: one MMA whose k index runs over sub-blocks (hi parts in k 0..7, lo in 8..15);
       // this lane's slots are sub-blocks 2t and 2t + 1, exactly the minima it holds
       const uint32_t ma = v0 & 0x00ff00ffu, mb = v1 & 0x00ff00ffu;
-      const uint2 xs = lds64(xsum + (uint32_t)lane * 8u);
-      float cm[4];
-      mma16816_first(cm, ma, mb, ma, mb, xs.x, xs.y);
-      const float m0 = n0 * -16777216.f, m1 = n1 * -16777216.f;
-      acc[0] = fmaf(d0, c[0], fmaf(m0, cm[0], acc[0]));
-      acc[1] = fmaf(d0, c[1], fmaf(m0, cm[1], acc[1]));
-      acc[2] = fmaf(d1, c[2], fmaf(m1, cm[2], acc[2]));
-      acc[3] = fmaf(d1, c[3], fmaf(m1, cm[3], acc[3]));
+      const float m0 = -n0, m1 = -n1;  // (the minima, integers in place, are subnormal numbers m * 2^-24 as well)
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) {
+        const uint2 xs = lds64(xsum + nb * a.xregion + (uint32_t)lane * 8u);
+        float cm[4];
+        mma16816_first(cm, ma, mb, ma, mb, xs.x, xs.y);
+        acc[nb][0] = fmaf(d0, c[nb][0], fmaf(m0, cm[0], acc[nb][0]));
+        acc[nb][1] = fmaf(d0, c[nb][1], fmaf(m0, cm[1], acc[nb][1]));
+        acc[nb][2] = fmaf(d1, c[nb][2], fmaf(m1, cm[2], acc[nb][2]));
+        acc[nb][3] = fmaf(d1, c[nb][3], fmaf(m1, cm[3], acc[nb][3]));
+      }
     } else {
       // the lane's share of the rows' minimum terms: its two sub-blocks
       const float2 xs = lds64f(xsum + 256u + (uint32_t)t * 8u);
       const float mt0 = (float)(v0 & 255u) * xs.x + (float)((v0 >> 16) & 255u) * xs.y;
       const float mt1 = (float)(v1 & 255u) * xs.x + (float)((v1 >> 16) & 255u) * xs.y;
-      acc[0] += d0 * (c[0] + c[1]) - n0 * mt0;
-      acc[2] += d1 * (c[2] + c[3]) - n1 * mt1;
+      acc[0][0] += d0 * (c[0][0] + c[0][1]) - n0 * (1.f / 16777216.f) * mt0;
+      acc[0][2] += d1 * (c[0][2] + c[0][3]) - n1 * (1.f / 16777216.f) * mt1;
     }
   }
 };

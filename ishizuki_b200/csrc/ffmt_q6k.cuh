@@ -39,8 +39,9 @@ namespace ishi {
 struct FragQ6K {
   static constexpr int kTileBytes = 16 * 210;
   static constexpr int kXSums = 4096;             // after the activations: [lane][hi hi | lo lo] group sums
-  static constexpr int kXBytes = kXSums + 512;    // per unit
-  static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the per-unit staging
+  static constexpr int kXBytes = kXSums + 512, kXFixed = 0;  // per unit of a staged region
+  static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
+  static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
 
   // the 6-bit code of weight k of a block
@@ -119,24 +120,21 @@ struct FragQ6K {
   // t + 1 of quad r multiply in k-step l / 2. The pair of k-steps i = l / 4 lies at
   // i * 512 + ((r ^ i) * 4 + t) * 16 (+ 8 for the odd k-step); the xor spreads the stores over the
   // banks and a warp's read of one pair is still one 512-byte run. Then the group sums (fp16 hi +
-  // lo) for the MMA over groups. after_loads() runs once, when the first loads are in flight.
-  template <class F>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, uint32_t xfrag, int ub0, int uc, F &&after_loads) {
+  // lo) for the MMA over groups.
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int tasks = uc * 8;
     constexpr int kBatch = 8;
-    const __half *xl = a.x + (long long)ub0 * 256 + lane * 8;
-    if (warp >= tasks) after_loads();  // a warp without a task
+    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint4 v[kBatch];
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < a.M)
+        if (i < tasks && (i & 7) < M)
           v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
       }
-      if (i0 == warp) after_loads();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -176,15 +174,16 @@ struct FragQ6K {
   }
 
   // One tile against the activations of its unit; acc is the warp's C fragment.
-  template <int MODE>
-  static __device__ __forceinline__ void unit(float (&acc)[4], const FragArgs &a, uint32_t tile, uint32_t xbase, int uq,
-                                              int g, int t, int lane) {
-    (void)a;
+  template <int MODE, int NB>
+  static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
+                                              uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t xu = xbase + (uint32_t)uq * kXBytes;
     const uint4 h0 = lds128(tile + 3072u + (uint32_t)g * 16u), h1 = lds128(tile + 3072u + (uint32_t)(g + 8) * 16u);
     const uint32_t hw0[4] = {h0.x, h0.y, h0.z, h0.w}, hw1[4] = {h1.x, h1.y, h1.z, h1.w};
     const uint32_t lane_off = (uint32_t)g * 64u + (uint32_t)t * 16u;
-    float su[4] = {0.f, 0.f, 0.f, 0.f};
+    float su[NB][4];
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = su[nb][2] = su[nb][3] = 0.f;
 #pragma unroll
     for (int pp = 0; pp < 4; ++pp) {
       const uint4 q = lds128(tile + (uint32_t)pp * 512u + (uint32_t)lane * 16u);
@@ -193,40 +192,48 @@ struct FragQ6K {
       for (int e = 0; e < 2; ++e) {
         const int pi = 2 * pp + e;
         const uint32_t x1 = e ? q.z : q.x, x2 = e ? q.w : q.y, h = e ? hh.y : hh.x;
-        const uint4 b = lds128(xu + (uint32_t)pi * 512u + (lane_off ^ (uint32_t)(pi << 6)));
         const uint32_t y1 = x1 >> 8, y2 = x2 >> 8;
         const uint32_t r2 = __funnelshift_r(h, h, 2), r8 = __funnelshift_r(h, h, 8), r10 = __funnelshift_r(h, h, 10);
-        float c0[4], c1[4];
-        mma16816_first(c0, (x1 & 0x000f000fu) | (h & 0x00300030u), (x2 & 0x000f000fu) | (r8 & 0x00300030u),
-                       (y1 & 0x000f000fu) | (r2 & 0x00300030u), (y2 & 0x000f000fu) | (r10 & 0x00300030u), b.x, b.y);
-        mma16816_first(c1, (x1 & 0x00f000f0u) | (h & 0x03000300u), (x2 & 0x00f000f0u) | (r8 & 0x03000300u),
-                       (y1 & 0x00f000f0u) | (r2 & 0x03000300u), (y2 & 0x00f000f0u) | (r10 & 0x03000300u), b.z, b.w);
+        const uint32_t a0 = (x1 & 0x000f000fu) | (h & 0x00300030u), a1 = (x2 & 0x000f000fu) | (r8 & 0x00300030u);
+        const uint32_t a2 = (y1 & 0x000f000fu) | (r2 & 0x00300030u), a3 = (y2 & 0x000f000fu) | (r10 & 0x00300030u);
+        const uint32_t e0 = (x1 & 0x00f000f0u) | (h & 0x03000300u), e1 = (x2 & 0x00f000f0u) | (r8 & 0x03000300u);
+        const uint32_t e2 = (y1 & 0x00f000f0u) | (r2 & 0x03000300u), e3 = (y2 & 0x00f000f0u) | (r10 & 0x03000300u);
         // scales of groups 2 pi and 2 pi + 1: word pi % 4 of the row's sixteen, bytes 2 (pi / 4) and + 1
         const float s00 = scale_of(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1) * 0.0625f;
         const float s10 = scale_of(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1) * 0.0625f;
-        su[0] = fmaf(s00, c0[0], su[0]), su[1] = fmaf(s00, c0[1], su[1]);
-        su[2] = fmaf(s10, c0[2], su[2]), su[3] = fmaf(s10, c0[3], su[3]);
-        su[0] = fmaf(s01, c1[0], su[0]), su[1] = fmaf(s01, c1[1], su[1]);
-        su[2] = fmaf(s11, c1[2], su[2]), su[3] = fmaf(s11, c1[3], su[3]);
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          const uint4 b = lds128(xu + nb * a.xregion + (uint32_t)pi * 512u + (lane_off ^ (uint32_t)(pi << 6)));
+          float c0[4], c1[4];
+          mma16816_first(c0, a0, a1, a2, a3, b.x, b.y);
+          mma16816_first(c1, e0, e1, e2, e3, b.z, b.w);
+          su[nb][0] = fmaf(s00, c0[0], su[nb][0]), su[nb][1] = fmaf(s00, c0[1], su[nb][1]);
+          su[nb][2] = fmaf(s10, c0[2], su[nb][2]), su[nb][3] = fmaf(s10, c0[3], su[nb][3]);
+          su[nb][0] = fmaf(s01, c1[0], su[nb][0]), su[nb][1] = fmaf(s01, c1[1], su[nb][1]);
+          su[nb][2] = fmaf(s11, c1[2], su[nb][2]), su[nb][3] = fmaf(s11, c1[3], su[nb][3]);
+        }
       }
     }
     // sum_g scale_g * (sum of x over group g): the MMA over groups; this lane's slots are groups
     // 2t, 2t + 1, 2t + 8, 2t + 9, the word t of each row's scales
     const uint32_t w0 = (t == 0 ? h0.x : t == 1 ? h0.y : t == 2 ? h0.z : h0.w) ^ 0x80808080u;
     const uint32_t w1 = (t == 0 ? h1.x : t == 1 ? h1.y : t == 2 ? h1.z : h1.w) ^ 0x80808080u;
-    const uint4 bs = lds128(xu + kXSums + (uint32_t)lane * 16u);
-    float cm[4];
     const uint32_t a0 = scale_pair(w0, 0x4140u), a1 = scale_pair(w1, 0x4140u);
     const uint32_t a2 = scale_pair(w0, 0x4342u), a3 = scale_pair(w1, 0x4342u);
-    mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
-    mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);
     const uint32_t dd = lds32(tile + 3328u + (uint32_t)g * 4u);
     const float d0 = half_bits_to_float(dd & 0xffffu), d1 = half_bits_to_float(dd >> 16);
-    const float dl0 = d0 * 16777216.f, dl1 = d1 * 16777216.f, dm0 = d0 * -32.f, dm1 = d1 * -32.f;
-    acc[0] = fmaf(dl0, su[0], fmaf(dm0, cm[0], acc[0]));
-    acc[1] = fmaf(dl0, su[1], fmaf(dm0, cm[1], acc[1]));
-    acc[2] = fmaf(dl1, su[2], fmaf(dm1, cm[2], acc[2]));
-    acc[3] = fmaf(dl1, su[3], fmaf(dm1, cm[3], acc[3]));
+    const float dm0 = d0 * (-32.f / 16777216.f), dm1 = d1 * (-32.f / 16777216.f);
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      const uint4 bs = lds128(xu + nb * a.xregion + kXSums + (uint32_t)lane * 16u);
+      float cm[4];
+      mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
+      mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);
+      acc[nb][0] = fmaf(d0, su[nb][0], fmaf(dm0, cm[0], acc[nb][0]));
+      acc[nb][1] = fmaf(d0, su[nb][1], fmaf(dm0, cm[1], acc[nb][1]));
+      acc[nb][2] = fmaf(d1, su[nb][2], fmaf(dm1, cm[2], acc[nb][2]));
+      acc[nb][3] = fmaf(d1, su[nb][3], fmaf(dm1, cm[3], acc[nb][3]));
+    }
   }
 };
 

@@ -65,13 +65,20 @@ struct RowPlan {
   size_t smem = 0, scratch_floats = 0, counters = 0, tiles_bytes = 0;
 };
 
-// Launch plan of the warp-level kernel (fragment-order tiles, 16-row panels, clusters of S CTAs).
+// Launch plan of the warp-level kernel (fragment-order tiles, 16-row panels, clusters of S CTAs) for
+// NB column groups of eight activation rows.
 struct FragPlan {
   bool ok = false;
   const FragOps *ops = nullptr;  // the format's kernels
-  int units = 0, S = 1, P = 0, NC = 1, Wu = 1, PP = 1, G = 1, ring = 3, umax = 0, tile_bytes = 0;
+  int units = 0, S = 1, P = 0, NC = 1, W = 1, NB = 1, ring = 3, umax = 0, led = 0, tile_bytes = 0;
+  int lane_warps = 1;  // W as ishi_projection_plan reports it: lane_warps * (W / lane_warps)
+  uint32_t xregion = 0;
   size_t smem = 0, tiles_bytes = 0;
   double cost = 0;
+};
+// one for up to eight rows, one for nine to sixteen (not ok: such a call runs as two launches of the first)
+struct FragPlans {
+  FragPlan few, many;
 };
 
 }  // namespace
@@ -97,9 +104,9 @@ struct ishi_ctx {
   std::vector<cudaEvent_t> ev_in, ev_done;
   cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
   std::mutex lock;
-  // launch plans already measured on this device, by (format's kernels, output rows, input width):
-  // {K split, warps per panel, panels in parallel, ring}
-  std::map<std::tuple<const void *, long long, long long>, std::array<int, 4>> tuned;
+  // launch plans already measured on this device, by (format's kernels, output rows, input width,
+  // column groups): {K split, warps, ring}
+  std::map<std::tuple<const void *, long long, long long, int>, std::array<int, 3>> tuned;
   char last_error[256] = {0};
 };
 
@@ -108,7 +115,7 @@ struct ishi_projection {
   ishi_weight_desc d;
   int fmt = 0;
   RowPlan plan;          // tcgen05 kernel (formats without a fragment decoder)
-  FragPlan frag;         // warp-level kernel
+  FragPlans frag;        // warp-level kernel
   bool generic = false;  // neither: the one-warp-per-row kernel reads a plain copy of the blocks (ws.tiles)
   bool gated = false;    // gate and up interleaved by eights, the kernel's epilogue writes silu(gate) * up: d.n / 2 output rows
   __half *logits = nullptr;  // [16][n] of apply_argmax, allocated by its first call
@@ -432,93 +439,98 @@ const FragOps *frag_ops_for(const ishi_weight_desc &d) {
 }
 
 // how many clusters of s CTAs with this much shared memory the device runs at once
-int max_frag_clusters(ishi_ctx *ctx, const FragOps *ops, int s, int warps, size_t smem) {
-  static std::map<std::tuple<int, const void *, int, int, size_t>, int> cache;
+int max_frag_clusters(ishi_ctx *ctx, const FragOps *ops, int s, int warps, int groups, size_t smem) {
+  static std::map<std::tuple<int, const void *, int, int, int, size_t>, int> cache;
   static std::mutex lock;
   std::lock_guard<std::mutex> g(lock);
-  const auto key = std::make_tuple(ctx->device, (const void *)ops, s, warps, smem);
+  const auto key = std::make_tuple(ctx->device, (const void *)ops, s, warps, groups, smem);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
-  const int n = ops->max_clusters(s, warps, smem, ctx->sm_count);
+  const int n = ops->max_clusters(s, warps, groups, smem, ctx->sm_count);
   cache[key] = n;
   return n;
 }
 
-// Picks the K split S (= cluster size), the warps per panel and the panels a CTA works on in
-// parallel. The estimate counts tile times on the longest warp (panels of the fullest cluster x
-// units per warp), stretched where the warps outnumber what the issue slots sustain.
-bool make_frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, FragPlan *pl, std::vector<FragPlan> *all = nullptr) {
+// The plan with K split s (= cluster size) and w warps per CTA, or false if it does not fit. ring:
+// tiles per warp, 0 for the deepest ring that fits.
+bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int w, int ring, FragPlan *out) {
   const FragOps *ops = frag_ops_for(d);
   if (!ops) return false;
   const size_t budget = (size_t)std::min(kSmemPerSm, ctx->smem_optin) - 1024;
   if (configure_once(ctx, ops, ops->configure, (int)budget) != ISHI_OK) return false;
-  const int xbytes = ops->x_bytes;
-  FragPlan best;
-  const int tile_bytes = ops->tile_bytes;
-  const int units = (int)(d.k / 256);
-  const int P = (int)((d.n + kFragRows - 1) / kFragRows);
+  FragPlan c;
+  c.ops = ops;
+  c.units = (int)(d.k / 256);
+  c.P = (int)((d.n + kFragRows - 1) / kFragRows);
+  c.S = s, c.W = w, c.NB = groups;
+  c.tile_bytes = ops->tile_bytes;
+  if (s < 1 || s > kFragMaxSplit || s > c.units || w < 1 || w > (groups == 2 ? kFragFewWarps : kFragMaxWarps)) return false;
   // the kernel divides by multiplication, exact while (clusters + 1) * P < 2^32 / clusters
-  if ((long long)P * (ctx->sm_count + 1) * ctx->sm_count >= (1ll << 32)) return false;
-  const char *force = getenv("ISHI_FRAG_PLAN");  // "S,per,PP[,ring]" for tuning runs
-  int fs = 0, fper = 0, fpp = 0, fring = 0;
-  if (force) sscanf(force, "%d,%d,%d,%d", &fs, &fper, &fpp, &fring);
-  for (int s = 1; s <= kFragMaxSplit && s <= units; ++s) {
-    if (fs && s != fs) continue;
-    const int umax = (units + s - 1) / s;
-    const int per_min = (umax + kFragMaxWarps - 1) / kFragMaxWarps;
-    // units per warp: a few around the fewest that fit the warps, and the whole range and half of
-    // it in one warp (no or little adding up between the warps of a panel)
-    const int per_hi = std::min(per_min + 2, kFragGroup);
-    for (int per = per_min; per <= umax; ++per) {
-      if (fper ? per != fper : (per > per_hi && per != umax && per != (umax + 1) / 2)) continue;
-      const int wu = (umax + per - 1) / per;
-      for (int pp = 1; pp <= kFragMaxPanels && wu * pp <= kFragMaxWarps; ++pp) {
-        if (fpp && pp != fpp) continue;
-        FragPlan c;
-        c.ops = ops;
-        c.units = units;
-        c.P = P;
-        c.S = s;
-        c.tile_bytes = tile_bytes;
-        c.umax = umax;
-        c.Wu = wu;
-        c.PP = pp;
-        const int w = wu * pp;
-        // the deepest tile ring that fits, then the larger inbox generation
-        bool fits = false;
-        for (int ring = fring ? fring : 3; ring >= (fring ? fring : 2) && !fits; --ring)
-          for (int gen = 2; gen >= 1 && !fits; --gen) {
-            const size_t need = frag_smem_bytes((size_t)umax * xbytes + ops->x_extra, w, pp, gen, s, tile_bytes, ring);
-            if (need <= budget) {
-              fits = true;
-              c.ring = ring, c.G = gen, c.smem = need;
-            }
-          }
-        if (!fits) continue;
-        // one CTA per SM: two would stage the activations twice and split the issue slots
-        c.NC = std::min(std::min(max_frag_clusters(ctx, ops, s, w, c.smem), ctx->sm_count / s), P);
-        if (c.NC < 1) continue;
-        // Estimate in microseconds, fitted to measurements on the 27B shapes: an SM passes about
-        // 13 tiles per microsecond when enough warps are busy; one warp alone needs about a
-        // microsecond per tile; every panel of a lane costs a reduction over its wu warps.
-        const int panels = (P + c.NC - 1) / c.NC;
-        const int rounds = (panels + pp - 1) / pp;  // panels one warp walks
-        const double throughput = 0.075 * panels * umax * std::max(1.0, 14.0 / w);
-        const double longest = 1.0 * rounds * per;
-        c.cost = std::max(throughput, longest) + rounds * (0.05 * wu + (s > 1 ? 0.05 : 0.0)) + 0.02 * umax;
-        c.ok = true;
-        c.tiles_bytes = (size_t)P * units * tile_bytes;
-        if (all) all->push_back(c);
-        if (!best.ok || c.cost < best.cost) best = c;
-      }
+  if ((long long)c.P * (ctx->sm_count + 1) * ctx->sm_count >= (1ll << 32)) return false;
+  c.umax = (c.units + s - 1) / s;
+  c.xregion = (uint32_t)(c.umax * ops->x_bytes + ops->x_fixed);
+  c.NC = std::min(ctx->sm_count / s, c.P);
+  // shared memory depends on the clusters (fewer of them lead more panels each), which depend on it
+  for (int tries = 0; tries < 3; ++tries) {
+    const int panels = (c.P + c.NC - 1) / c.NC;
+    if ((long long)panels * c.umax * (kFragMaxWarps + 1) >= (1ll << 31)) return false;
+    c.led = s > 1 ? (panels + s - 1) / s : 0;
+    bool fits = false;
+    for (int r = ring ? ring : kFragMaxRing; r >= (ring ? ring : 2) && !fits; --r) {
+      if (r * frag_ring_stride(c.tile_bytes) < groups * 1024) break;  // a drained ring holds a partial tile
+      c.ring = r;
+      c.smem = frag_smem_bytes((size_t)groups * c.xregion + ops->x_extra, w, c.led, s, groups, c.tile_bytes, r);
+      fits = c.smem <= budget;
     }
+    if (!fits) return false;
+    // one CTA per SM: two would stage the activations twice and split the issue slots
+    const int most = std::min(c.NC, max_frag_clusters(ctx, ops, s, w, groups, c.smem));
+    if (most < 1) return false;
+    if (most == c.NC) {
+      // Estimate in microseconds: the warps' runs of tiles, a tile every 0.075 us of an SM that is
+      // full of warps or one per 0.9 us and warp in one that is not; staging; the hand-over in a cluster.
+      const double run = (double)((panels * c.umax + w - 1) / w);
+      c.cost = run * std::max(0.9, 0.075 * w) * (groups == 2 ? 1.3 : 1.0) + 0.05 * c.umax * groups + (s > 1 ? 0.5 + 0.05 * s : 0.0);
+      c.tiles_bytes = (size_t)c.P * c.units * c.tile_bytes;
+      c.ok = true;
+      *out = c;
+      return true;
+    }
+    c.NC = most;
   }
+  return false;
+}
+
+// The K split and the number of warps: the estimate's choice, and all plans that fit for the
+// measurement. ISHI_FRAG_PLAN = "S,per,PP[,ring]" forces ceil(units of a range / per) * PP warps.
+bool make_frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, FragPlan *pl, std::vector<FragPlan> *all = nullptr) {
+  FragPlan best;
+  int fs = 0, fper = 0, fpp = 0, fring = 0;
+  if (const char *force = getenv("ISHI_FRAG_PLAN")) sscanf(force, "%d,%d,%d,%d", &fs, &fper, &fpp, &fring);
+  const int units = (int)(d.k / 256);
+  if (fs > 0 && fper > 0 && fpp > 0) {
+    const int lane = ((units + fs - 1) / fs + fper - 1) / fper;
+    if (!frag_plan(ctx, d, groups, fs, lane * fpp, fring, &best)) return false;
+    best.lane_warps = lane;
+    *pl = best;
+    return true;
+  }
+  for (int s = 1; s <= kFragMaxSplit && s <= units; ++s)
+    for (int w : {24, 20, 16, 12, 8, 4}) {
+      FragPlan c;
+      if (!frag_plan(ctx, d, groups, s, w, 0, &c)) continue;
+      if (all) all->push_back(c);
+      if (!best.ok || c.cost < best.cost) best = c;
+    }
   if (!best.ok) return false;
-  best.tiles_bytes = (size_t)P * units * tile_bytes;
-  if (getenv("ISHI_DEBUG_PLAN"))
-    fprintf(stderr, "ishi plan n=%lld k=%lld: split %d, clusters %d, warps %d x %d, generation %d, ring %d, smem %zu\n",
-            (long long)d.n, (long long)d.k, best.S, best.NC, best.Wu, best.PP, best.G, best.ring, best.smem);
   *pl = best;
+  return true;
+}
+
+// Both launches of a weight; false: the warp-level kernel does not take it.
+bool make_frag_plans(ishi_ctx *ctx, const ishi_weight_desc &d, FragPlans *pl) {
+  if (!make_frag_plan(ctx, d, 1, &pl->few)) return false;
+  make_frag_plan(ctx, d, 2, &pl->many);
   return true;
 }
 
@@ -577,10 +589,12 @@ bool single_row_on_cuda_cores(const ishi_ctx *ctx) {
 }
 
 // rows 1...16 through the warp-level kernel; gemv picks the CUDA-core variant for a single row
-ishi_status run_frag(ishi_ctx *ctx, const FragPlan &pl, const Workspace &ws, const ishi_weight_desc &d, const void *x,
+ishi_status run_frag(ishi_ctx *ctx, const FragPlans &plans, const Workspace &ws, const ishi_weight_desc &d, const void *x,
                      int rows, void *y, long long ldy, int flags, bool gemv, bool early, bool rotate, cudaStream_t st,
                      const PeerOut *peers = nullptr, bool gated = false) {
-  for (int r0 = 0; r0 < rows; r0 += 8) {
+  const bool whole = rows <= 8 || plans.many.ok;  // one launch, or pieces of eight rows
+  for (int r0 = 0; r0 < rows; r0 += whole ? 16 : 8) {
+    const FragPlan &pl = whole && rows > 8 ? plans.many : plans.few;
     FragArgs a;
     memset(&a, 0, sizeof(a));
     a.tiles = ws.tiles;
@@ -588,21 +602,18 @@ ishi_status run_frag(ishi_ctx *ctx, const FragPlan &pl, const Workspace &ws, con
     a.y = static_cast<__half *>(y) + ((flags & ISHI_OUT_TRANSPOSED) ? (long long)r0 : (long long)r0 * ldy);
     a.ldy = ldy;
     a.out_transposed = (flags & ISHI_OUT_TRANSPOSED) ? 1 : 0;
-    a.M = std::min(8, rows - r0);
+    a.M = whole ? rows : std::min(8, rows - r0);
     a.N = (int)d.n;
     a.K = (int)d.k;
     a.units = pl.units;
     a.S = pl.S;
     a.P = pl.P;
     a.NC = pl.NC;
-    a.Wu = pl.Wu;
-    a.PP = pl.PP;
-    a.G = pl.G;
     a.ring = pl.ring;
+    a.led = pl.led;
+    a.xregion = pl.xregion;
     a.inv_s = frag_inverse(pl.S);
     a.inv_nc = frag_inverse(pl.NC);
-    a.inv_wu = frag_inverse(pl.Wu);
-    a.inv_pp = frag_inverse(pl.PP);
     a.umax = pl.umax;
     a.group_size = d.group_size;
     a.scale_dtype = d.scale_dtype;
@@ -616,7 +627,7 @@ ishi_status run_frag(ishi_ctx *ctx, const FragPlan &pl, const Workspace &ws, con
     if (peers) {
       a.world = peers->world;
       a.rank = peers->rank;
-      a.peer_ld = rows > 8 ? 16 : 8;  // the second piece of eight rows lies beside the first
+      a.peer_ld = rows > 8 ? 16 : 8;
       for (int q = 0; q < peers->world; ++q) {
         a.peer_y[q] = peers->y[q] + r0;
         a.peer_flags[q] = peers->flags[q];
@@ -630,7 +641,7 @@ ishi_status run_frag(ishi_ctx *ctx, const FragPlan &pl, const Workspace &ws, con
     FragLaunch l;
     l.clusters = pl.NC;
     l.split = pl.S;
-    l.warps = pl.Wu * pl.PP;
+    l.warps = pl.W;
     l.smem = pl.smem;
     l.mode = (gemv && rows == 1) ? 1 : 0;
     l.early = early;
@@ -655,11 +666,11 @@ ishi_status raw_product(ishi_ctx *ctx, const ishi_weight_desc &d, const void *x,
   if (s != ISHI_OK) return s;
   std::lock_guard<std::mutex> g(ctx->lock);
   ISHI_CUDA(ctx, cudaSetDevice(ctx->device));
-  FragPlan fp;
-  if (make_frag_plan(ctx, d, &fp)) {
-    s = ensure_workspace(ctx, &ctx->ws, 0, 0, fp.tiles_bytes, st);
+  FragPlans fp;
+  if (make_frag_plans(ctx, d, &fp)) {
+    s = ensure_workspace(ctx, &ctx->ws, 0, 0, fp.few.tiles_bytes, st);
     if (s != ISHI_OK) return s;
-    s = tile_weight_frag(ctx, fp, &d, 1, d.n, ctx->ws.tiles, st);
+    s = tile_weight_frag(ctx, fp.few, &d, 1, d.n, ctx->ws.tiles, st);
     if (s != ISHI_OK) return s;
     return run_frag(ctx, fp, ctx->ws, d, x, rows, y, d.n, 0, gemv || single_row_on_cuda_cores(ctx), false, false, st);
   }
@@ -702,7 +713,7 @@ ishi_status ggml_raw(ishi_ctx *ctx, const void *x, int rows, const void *blocks,
 // the GGUF decoders' staging does not, their input is rotated by the stand-alone kernel first.
 bool rotates_in_kernel(const ishi_projection *p) {
   const int b = p->d.hadamard_block;
-  return p->frag.ok && p->d.kind == ISHI_KIND_AFFINE && b >= 8 && b <= 256 && (b & (b - 1)) == 0;
+  return p->frag.few.ok && p->d.kind == ISHI_KIND_AFFINE && b >= 8 && b <= 256 && (b & (b - 1)) == 0;
 }
 
 // rotate: x is unrotated and the projection's rotation is applied inside the product kernel
@@ -714,7 +725,7 @@ ishi_status projection_matmul(ishi_projection *p, const void *x, int rows, void 
   const int64_t need_ld = (flags & ISHI_OUT_TRANSPOSED) ? rows : out_rows(p);
   if (ldy < need_ld) return fail(ctx, ISHI_E_SHAPE, "ldy %lld shorter than %lld", (long long)ldy, (long long)need_ld);
   ISHI_CUDA(ctx, cudaSetDevice(ctx->device));
-  if (p->frag.ok)
+  if (p->frag.few.ok)
     return run_frag(ctx, p->frag, p->ws, p->d, x, rows, y, ldy, flags, single_row_on_cuda_cores(ctx),
                     getenv("ISHI_NO_EARLY_LAUNCH") == nullptr, rotate, st, nullptr, p->gated);
   if (p->generic) {
@@ -942,34 +953,39 @@ ishi_status ishi_verify_matmul(ishi_ctx *ctx, const void *x, int rows, const voi
 
 // The tile layout does not depend on the launch plan, so the plan can be chosen by measurement:
 // the planner's best candidates run a few times on the projection's own tiles (activations of
-// zeros, eight rows) and the fastest stays. The estimate alone is within ~15 % of the best plan.
-static void tune_frag_plan(ishi_ctx *ctx, ishi_projection *p, std::vector<FragPlan> *candidates) {
-  constexpr size_t kTuned = 24;
+// zeros, eight or sixteen rows) and the fastest stays.
+static void tune_frag_plan(ishi_ctx *ctx, ishi_projection *p, int groups, std::vector<FragPlan> *candidates) {
+  constexpr size_t kTuned = 16;
   constexpr int kLaunches = 4;
+  FragPlan *plan = groups == 2 ? &p->frag.many : &p->frag.few;
   if (candidates->size() < 2) return;
   // a shape measured before on this context keeps its plan (all layers of a model then agree)
-  const auto key = std::make_tuple((const void *)p->frag.ops, (long long)p->d.n, (long long)p->d.k);
+  const auto key = std::make_tuple((const void *)plan->ops, (long long)p->d.n, (long long)p->d.k, groups);
   const auto known = ctx->tuned.find(key);
   if (known != ctx->tuned.end()) {
     for (const FragPlan &c : *candidates)
-      if (c.S == known->second[0] && c.Wu == known->second[1] && c.PP == known->second[2] && c.ring == known->second[3]) {
-        p->frag = c;
+      if (c.S == known->second[0] && c.W == known->second[1] && c.ring == known->second[2]) {
+        *plan = c;
         return;
       }
   }
   std::sort(candidates->begin(), candidates->end(), [](const FragPlan &a, const FragPlan &b) { return a.cost < b.cost; });
   if (candidates->size() > kTuned) candidates->resize(kTuned);
+  const int rows = 8 * groups;
   __half *x = nullptr, *y = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  bool ok = cudaMalloc(&x, (size_t)8 * p->d.k * sizeof(__half)) == cudaSuccess &&
-            cudaMalloc(&y, (size_t)8 * p->d.n * sizeof(__half)) == cudaSuccess &&
-            cudaMemset(x, 0, (size_t)8 * p->d.k * sizeof(__half)) == cudaSuccess && cudaEventCreate(&e0) == cudaSuccess &&
+  bool ok = cudaMalloc(&x, (size_t)rows * p->d.k * sizeof(__half)) == cudaSuccess &&
+            cudaMalloc(&y, (size_t)rows * p->d.n * sizeof(__half)) == cudaSuccess &&
+            cudaMemset(x, 0, (size_t)rows * p->d.k * sizeof(__half)) == cudaSuccess && cudaEventCreate(&e0) == cudaSuccess &&
             cudaEventCreate(&e1) == cudaSuccess;
   // one timing: a warm-up launch, then `launches` back to back between two events
   auto time_plan = [&](const FragPlan &c, int launches, float *ms_per_launch) {
-    bool fine = run_frag(ctx, c, p->ws, p->d, x, 8, y, p->d.n, 0, false, true, false, 0) == ISHI_OK;
+    FragPlans both;
+    both.few = both.many = c;
+    auto launch = [&] { return run_frag(ctx, both, p->ws, p->d, x, rows, y, p->d.n, 0, false, true, false, 0) == ISHI_OK; };
+    bool fine = launch();
     if (fine) fine = cudaEventRecord(e0, 0) == cudaSuccess;
-    for (int r = 0; fine && r < launches; ++r) fine = run_frag(ctx, c, p->ws, p->d, x, 8, y, p->d.n, 0, false, true, false, 0) == ISHI_OK;
+    for (int r = 0; fine && r < launches; ++r) fine = launch();
     if (fine) fine = cudaEventRecord(e1, 0) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess;
     float ms = 0.f;
     if (fine) fine = cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess;
@@ -1005,11 +1021,14 @@ static void tune_frag_plan(ishi_ctx *ctx, ishi_projection *p, std::vector<FragPl
     for (const auto &f : finals)
       if (f.first <= best_ms * (1.f + tie) && f.second->S < best->S) best = f.second;
   if (ok && best) {
-    p->frag = *best;
-    ctx->tuned[key] = {best->S, best->Wu, best->PP, best->ring};
-    if (getenv("ISHI_DEBUG_PLAN"))
-      fprintf(stderr, "ishi plan n=%lld k=%lld measured: split %d, warps %d x %d, ring %d: %.2f us\n", (long long)p->d.n,
-              (long long)p->d.k, best->S, best->Wu, best->PP, best->ring, best_ms * 1e3f);
+    *plan = *best;
+    ctx->tuned[key] = {best->S, best->W, best->ring};
+    if (getenv("ISHI_DEBUG_PLAN")) {
+      fprintf(stderr, "ishi plan n=%lld k=%lld rows<=%d measured: split %d, %d clusters, %d warps, ring %d: %.2f us;", (long long)p->d.n,
+              (long long)p->d.k, rows, best->S, best->NC, best->W, best->ring, best_ms * 1e3f);
+      for (const auto &c : timed) fprintf(stderr, " %d/%d/%d:%.1f", c.second->S, c.second->W, c.second->ring, c.first * 1e3f);
+      fprintf(stderr, "\n");
+    }
   } else {
     cudaGetLastError();  // keep the estimate's choice
   }
@@ -1053,11 +1072,15 @@ static ishi_status create_projection(ishi_ctx *ctx, const ishi_weight_desc *desc
   ishi_status s = ISHI_OK;
   // Re-tile the weight once, for the kernel this format runs on; the caller's buffers are not read
   // again afterwards.
-  std::vector<FragPlan> candidates;
-  if (make_frag_plan(ctx, p->d, &p->frag, &candidates)) {
-    s = ensure_workspace(ctx, &p->ws, 0, 0, p->frag.tiles_bytes, 0);
-    if (s == ISHI_OK) s = tile_weight_frag(ctx, p->frag, descs, count, n_total, p->ws.tiles, 0, gated);
-    if (s == ISHI_OK && !getenv("ISHI_NO_AUTOTUNE") && !getenv("ISHI_FRAG_PLAN")) tune_frag_plan(ctx, p, &candidates);
+  std::vector<FragPlan> few, many;
+  if (make_frag_plan(ctx, p->d, 1, &p->frag.few, &few)) {
+    make_frag_plan(ctx, p->d, 2, &p->frag.many, &many);
+    s = ensure_workspace(ctx, &p->ws, 0, 0, p->frag.few.tiles_bytes, 0);
+    if (s == ISHI_OK) s = tile_weight_frag(ctx, p->frag.few, descs, count, n_total, p->ws.tiles, 0, gated);
+    if (s == ISHI_OK && !getenv("ISHI_NO_AUTOTUNE") && !getenv("ISHI_FRAG_PLAN")) {
+      tune_frag_plan(ctx, p, 1, &few);
+      tune_frag_plan(ctx, p, 2, &many);
+    }
   } else if (count > 1) {
     delete p;
     return fail(ctx, ISHI_E_UNSUPPORTED, "only the warp-level kernel's formats can be stacked into one projection");
@@ -1134,27 +1157,30 @@ int ishi_projection_crossover_rows(const ishi_projection *p) {
 ishi_status ishi_projection_plan(const ishi_projection *p, int plan[4]) {
   if (!p || !plan) return ISHI_E_INVALID;
   plan[0] = plan[1] = plan[2] = plan[3] = 0;
-  if (p->frag.ok) plan[0] = p->frag.S, plan[1] = p->frag.Wu, plan[2] = p->frag.PP, plan[3] = p->frag.ring;
+  const FragPlan &f = p->frag.few, &m = p->frag.many;
+  if (f.ok) {
+    plan[0] = f.S, plan[1] = f.lane_warps, plan[2] = f.W / f.lane_warps;
+    plan[3] = f.ring | (m.ok ? m.ring << 8 | m.S << 12 | m.W << 16 : 0);
+  }
   return ISHI_OK;
 }
 
 ishi_status ishi_projection_set_plan(ishi_projection *p, const int plan[4]) {
   if (!p || !plan) return ISHI_E_INVALID;
   ishi_ctx *ctx = p->ctx;
-  if (!p->frag.ok) return fail(ctx, ISHI_E_UNSUPPORTED, "this projection's kernel has one launch plan only");
+  if (!p->frag.few.ok) return fail(ctx, ISHI_E_UNSUPPORTED, "this projection's kernel has one launch plan only");
   std::lock_guard<std::mutex> g(ctx->lock);
-  ishi_weight_desc d = p->d;
-  d.weight_dev = p->ws.tiles;  // the planner looks at sizes only
-  std::vector<FragPlan> all;
-  FragPlan best;
-  if (!make_frag_plan(ctx, d, &best, &all)) return fail(ctx, ISHI_E_SHAPE, "no launch plan fits");
-  for (const FragPlan &c : all)
-    if (c.S == plan[0] && c.Wu == plan[1] && c.PP == plan[2] && c.ring == plan[3]) {
-      p->frag = c;
-      return ISHI_OK;
-    }
-  return fail(ctx, ISHI_E_INVALID, "plan %d,%d,%d,%d is not among this projection's launch plans", plan[0], plan[1], plan[2],
-              plan[3]);
+  const int many = plan[3] >> 8;
+  FragPlans both;
+  bool fine = plan[1] > 0 && plan[2] > 0 && plan[1] <= kFragMaxWarps && plan[2] <= kFragMaxWarps &&
+              frag_plan(ctx, p->d, 1, plan[0], plan[1] * plan[2], plan[3] & 255, &both.few);
+  if (fine && many > 0) fine = frag_plan(ctx, p->d, 2, (many >> 4) & 15, many >> 8, many & 15, &both.many);
+  if (!fine)
+    return fail(ctx, ISHI_E_INVALID, "plan %d,%d,%d,%d is not among this projection's launch plans", plan[0], plan[1], plan[2], plan[3]);
+  both.few.lane_warps = plan[1];
+  if (many == 0) make_frag_plan(ctx, p->d, 2, &both.many);
+  p->frag = both;
+  return ISHI_OK;
 }
 
 ishi_status ishi_projection_rotate(ishi_projection *p, const void *x, int rows, void *xr, void *stream) {
@@ -1456,7 +1482,7 @@ ishi_status ishi_exchange_apply(ishi_exchange *ex, ishi_projection *p, const voi
   if (p->ctx != ctx) return fail(ctx, ISHI_E_INVALID, "projection and exchange belong to different contexts");
   if (!ex->connected) return fail(ctx, ISHI_E_INVALID, "exchange not connected");
   if (!x) return fail(ctx, ISHI_E_INVALID, "null pointer");
-  if (!p->frag.ok) {
+  if (!p->frag.few.ok) {
     // The other kernels do not store to peers themselves: the product goes into this rank's own
     // copy and a small kernel passes the rows on and publishes them.
     if (rows < 1 || rows > 8) return fail(ctx, ISHI_E_SHAPE, "rows %d outside 1...8 for this weight format", rows);

@@ -9,15 +9,27 @@ namespace ishi {
 
 template <class Fmt>
 struct FragOpsOf {
-  static cudaError_t configure(int max_smem) {
-    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(frag_kernel<Fmt, 0, kFragFewWarps>, attr, max_smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(frag_kernel<Fmt, 0, kFragMaxWarps>, attr, max_smem);
+  // the variant that serves a launch: column groups of eight rows, CUDA cores or not, block size.
+  // Two column groups keep twice the accumulators: at most kFragFewWarps warps.
+  static const void *kernel(int groups, int mode, int warps) {
+    const bool few = warps <= kFragFewWarps;
+    if (groups == 2) return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 2> : nullptr;
     if constexpr (Fmt::kRowMode) {
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(frag_kernel<Fmt, 1, kFragFewWarps>, attr, max_smem);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(frag_kernel<Fmt, 1, kFragMaxWarps>, attr, max_smem);
+      // (a format without a CUDA-core variant for one activation row runs that row through the MMA path)
+      if (mode == 1) return few ? (const void *)frag_kernel<Fmt, 1, kFragFewWarps, 1> : (const void *)frag_kernel<Fmt, 1, kFragMaxWarps, 1>;
     }
-    return e;
+    return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 1> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1>;
+  }
+
+  static cudaError_t configure(int max_smem) {
+    for (int groups = 1; groups <= 2; ++groups)
+      for (int mode = 0; mode < 2; ++mode)
+        for (int warps : {kFragFewWarps, kFragMaxWarps})
+          if (const void *k = kernel(groups, mode, warps)) {
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+            if (e != cudaSuccess) return e;
+          }
+    return cudaSuccess;
   }
 
   static void fill(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at, int clusters, int split, int warps, size_t smem) {
@@ -33,14 +45,13 @@ struct FragOpsOf {
     cfg->numAttrs = 1;
   }
 
-  static int max_clusters(int split, int warps, size_t smem, int sm_count) {
+  static int max_clusters(int split, int warps, int groups, size_t smem, int sm_count) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
     fill(&cfg, at, sm_count, split, warps, smem);
     int n = 0;
-    const cudaError_t e = warps <= kFragFewWarps
-                              ? cudaOccupancyMaxActiveClusters(&n, frag_kernel<Fmt, 0, kFragFewWarps>, &cfg)
-                              : cudaOccupancyMaxActiveClusters(&n, frag_kernel<Fmt, 0, kFragMaxWarps>, &cfg);
+    const void *k = kernel(groups, 0, warps);
+    const cudaError_t e = k ? cudaOccupancyMaxActiveClusters(&n, k, &cfg) : cudaErrorInvalidValue;
     if (e != cudaSuccess) {
       cudaGetLastError();
       return 0;
@@ -59,15 +70,8 @@ struct FragOpsOf {
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = l.early ? 2 : 1;
-    // a format without a CUDA-core variant for one activation row runs that row through the MMA path
-    const bool few = l.warps <= kFragFewWarps;
-    if constexpr (Fmt::kRowMode) {
-      if (l.mode == 1)
-        return few ? cudaLaunchKernelEx(&cfg, frag_kernel<Fmt, 1, kFragFewWarps>, args)
-                   : cudaLaunchKernelEx(&cfg, frag_kernel<Fmt, 1, kFragMaxWarps>, args);
-    }
-    return few ? cudaLaunchKernelEx(&cfg, frag_kernel<Fmt, 0, kFragFewWarps>, args)
-               : cudaLaunchKernelEx(&cfg, frag_kernel<Fmt, 0, kFragMaxWarps>, args);
+    void *params[1] = {const_cast<FragArgs *>(&args)};
+    return cudaLaunchKernelExC(&cfg, kernel(args.M > 8 ? 2 : 1, l.mode, l.warps), params);
   }
 
   static cudaError_t prepare(const FragSrc &src, int units, uint8_t *dst, int grid, cudaStream_t stream) {
@@ -76,7 +80,7 @@ struct FragOpsOf {
   }
 
   static constexpr FragOps ops() {
-    return FragOps{Fmt::kTileBytes, Fmt::kXBytes, Fmt::kExtraBytes, &configure, &max_clusters, &launch, &prepare};
+    return FragOps{Fmt::kTileBytes, Fmt::kXBytes, Fmt::kXFixed, Fmt::kExtraBytes, &configure, &max_clusters, &launch, &prepare};
   }
 };
 

@@ -18,23 +18,32 @@
 // Work. K is cut into S column ranges and the kernel is launched as thread-block clusters of S
 // CTAs (S = 1: no cluster): CTA r of a cluster stages the activations of column range r into shared
 // memory once, laid out as its format's decoder reads them, and all CTAs of a cluster walk the same
-// run of 16-row panels, dealt to the clusters in equal contiguous runs. A CTA works on PP panels at a time ("panel lanes"), Wu warps
-// per lane: warp (lane wp, position wu) takes panels wp, wp + PP, ... of the cluster's run and in
-// each the units wu, wu + Wu, ... of the CTA's column range, streaming its tiles through a private
-// ring in shared memory: one bulk async copy per tile (the copy engine, not the load/store unit,
-// moves the bytes), completion counted on the ring slot's own mbarrier. No producer warp, no
-// cross-warp wait on the data path.
+// run of 16-row panels, dealt to the clusters in equal contiguous runs. A CTA's tiles, panel after
+// panel and in each its units in order, are one sequence, and every warp takes an equal contiguous
+// run of it, whatever panel it begins and ends in: with 14.7 panels per SM (a 27B gate and up pair) 24
+// warps walk 12 or 13 tiles each, where whole panels per warp kept 15 of 20 warps busy with 20 tiles.
+// A warp streams its run through a private ring in shared memory: its lanes copy a tile with a few
+// 16-byte async copies (cp.async), one commit group per tile. What bounds the loop is instruction
+// issue, so the copy has to be cheap: a bulk copy per tile on an mbarrier moves the same bytes with
+// one instruction, but moving its operands to uniform registers, electing the lane, counting the
+// bytes in and polling the barrier made about 100 of the loop's 365 instructions per Q4_K tile. No
+// producer warp, no cross-warp wait on the data path.
 //
-// Reduction, without a CTA-wide barrier. With Wu = 1 a warp owns its panels whole and there is
-// nothing to add up inside the CTA. Else a warp that has finished a panel parks its 16 x 8 partial
-// tile in the lane's slot ring and bumps the slot's arrival counter; the warp that arrives last
-// adds the lane's partials in warp order. With S > 1 it sends the CTA's partial panel into the
+// Reduction, without a CTA-wide barrier. A panel that lies inside one warp's run is complete when
+// the warp leaves it. The others (at most two per run: the one it begins in and the one it ends
+// in) are parked as partial 16 x 8 tiles, the first in a slot of the warp's, the last in its ring,
+// which is empty by then; the warp that arrives last at the panel's counter adds the partials in
+// warp order. The tiles' fp32 results are added up in fp64: where a panel is cut depends on where it
+// lies in the CTA's sequence, and the sums must not (a gated pair and the same two weights
+// stacked give the same products). With S > 1 the CTA's partial panel goes into the
 // shared memory of the panel's leader CTA (distributed shared memory, st.async counted on an
-// mbarrier there); the leader's last-arriving warp waits for the S partials, adds them in rank
-// order and writes y. Inbox slots are recycled two "generations" (G panels of a lane) later; a
-// relaxed cluster barrier, arrived at the end of a generation and waited for one generation
-// later, tells a sender that every leader is done with the slot it is about to overwrite. No
-// global scratch, no atomics on values, every y element written once, the summation order fixed.
+// mbarrier there), an inbox slot per panel and rank; when a CTA's warps are through their runs they
+// add the S partials of the panels it leads in rank order and write y. Every slot, counter and
+// mbarrier is used once per launch: nothing is recycled and nobody waits for room. No global
+// scratch, no atomics on values, every y element written once, the summation order fixed by the plan.
+//
+// Activation rows 9 ... 16 are a second column group: the same A fragments, decoded once, multiply
+// a second staged region (NB = 2).
 #pragma once
 #include "ishi_stream.cuh"
 
@@ -51,10 +60,6 @@ constexpr int kFragMaxWarps = ISHI_FRAG_MAX_WARPS;
 constexpr int kFragFewWarps = 20;
 constexpr int kFragMaxRing = 4;   // most tiles per warp-private ring (FragArgs::ring of them are used:
                                   // one is decoded while the others are in flight)
-constexpr int kFragMaxPanels = 24; // most panels a CTA works on in parallel (one warp each, then)
-constexpr int kFragGroup = 4;     // most units per warp the planner considers
-constexpr int kFragRed = 2;       // partial-tile slots per panel lane: a warp may run this many panels ahead of the slowest
-constexpr int kFragMaxGen = 4;    // most panels of a lane per generation of inbox slots
 constexpr int kFragMaxSplit = 8;  // portable cluster size
 constexpr int kFragMaxPeers = 8;  // GPUs of one NVSwitch box
 
@@ -66,11 +71,12 @@ struct FragArgs {
   int out_transposed;
   int M, N, K;
   int units, S, P, NC;  // NC clusters of S CTAs
-  int Wu, PP, G;        // warps per panel, panels in parallel (Wu * PP warps per CTA), panels of a lane per inbox generation
   int ring;             // tiles per warp-private ring, 2 ... kFragMaxRing
-  // ceil(2^32 / d) for d = S, NC, Wu, PP, or 0 for d = 1: see frag_div()
-  unsigned inv_s, inv_nc, inv_wu, inv_pp;
+  int led;              // most panels a CTA leads (S > 1)
+  // ceil(2^32 / d) for d = S, NC, or 0 for d = 1: see frag_div()
+  unsigned inv_s, inv_nc;
   int umax;             // most units in a column range
+  uint32_t xregion;     // bytes of one staged region: umax * Fmt::kXBytes + Fmt::kXFixed
   int group_size, scale_dtype;
   int *err;             // raised when a bounded wait gives up
   // Block Hadamard rotation of x while it is staged (0: none): xr = WHT_block(x * signs) / sqrt(block)
@@ -129,12 +135,27 @@ struct FragArgs {
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
+// a tile of BYTES (a multiple of 16) bytes by one warp; src and dst are this lane's: offset by 16 * lane
+template <int BYTES>
+__device__ __forceinline__ void cp_async_tile(uint32_t dst, const uint8_t *src, int lane) {
+#pragma unroll
+  for (int i = 0; i < BYTES / 512; ++i) cp_async16(dst + 512u * i, src + 512 * i);
+  if (BYTES % 512 && lane < BYTES % 512 / 16) cp_async16(dst + BYTES / 512 * 512u, src + BYTES / 512 * 512);
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+__device__ __forceinline__ void sts128d(uint32_t addr, double a, double b) {
+  asm volatile("st.shared.v2.f64 [%0], {%1,%2};" ::"r"(addr), "d"(a), "d"(b) : "memory");
+}
 // (not volatile: callers tie the address to the barrier that publishes the data)
+__device__ __forceinline__ double2 lds128d(uint32_t addr) {
+  double2 v;
+  asm("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ float lds32f(uint32_t addr) {
   float v;
   asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
@@ -176,19 +197,18 @@ __device__ __forceinline__ int frag_div(unsigned n, unsigned inv) { return inv ?
 __host__ inline unsigned frag_inverse(int d) { return d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
 
 __host__ __device__ inline int frag_column_begin(int c, int units, int S) { return (c * units) / S; }
-__host__ __device__ inline int frag_ring_stride(int tile_bytes) { return (tile_bytes + 127) & ~127; }
+__host__ __device__ inline int frag_ring_stride(int tile_bytes) { return (tile_bytes + 15) & ~15; }
 
-// shared memory of one CTA, in order: activations, the lanes' partial-tile slots, the inbox for the
-// partial panels of the cluster's CTAs, a control block (inbox mbarriers, arrival counters,
-// progress words, abort word), the warps' rings
-// control block (PP <= 24, G <= 2): inbox mbarriers [PP][2G] @0, phases used of each [PP][2G] @768,
-// arrival counters [PP][kFragRed] @1152, done [PP] @1344, abort @1440, ring mbarriers
-// [warp][kFragMaxRing] @1472
-constexpr uint32_t kFragCtrlBytes = 2304;
-// xregion: the format's activation staging, umax * Fmt::kXBytes + Fmt::kExtraBytes
-// (a panel lane of one warp parks nothing and has no slots)
-__host__ __device__ inline size_t frag_smem_bytes(size_t xregion, int W, int PP, int G, int S, int tile_bytes, int ring) {
-  return xregion + (W > PP ? (size_t)W * kFragRed * 512 : 0) + (S > 1 ? (size_t)PP * 2 * G * S * 512 : 0) + kFragCtrlBytes +
+// shared memory of one CTA, in order: the staged activations (a region per group of eight rows),
+// the format's tables, the warps' partial-tile slots, the inbox for the partial panels of the
+// cluster's CTAs, a control block, the warps' rings
+// control block: arrival counters [warp] @0, abort @96, inbox mbarriers [led] @128
+constexpr uint32_t kFragCtrlAbort = 96, kFragCtrlInbox = 128;
+static_assert(4 * kFragMaxWarps <= (int)kFragCtrlAbort, "control block");
+__host__ __device__ inline uint32_t frag_ctrl_bytes(int led) { return (kFragCtrlInbox + 8u * (uint32_t)led + 127u) & ~127u; }
+// x: the staged regions and the format's tables; led: most panels a CTA leads; NB: groups of eight rows
+__host__ __device__ inline size_t frag_smem_bytes(size_t x, int W, int led, int S, int NB, int tile_bytes, int ring) {
+  return x + (size_t)W * NB * 1024 + (S > 1 ? (size_t)led * S * NB * 512 : 0) + frag_ctrl_bytes(S > 1 ? led : 0) +
          (size_t)W * ring * frag_ring_stride(tile_bytes);
 }
 
@@ -217,7 +237,8 @@ __device__ __forceinline__ float frag_swiglu(float gate, float up) {
 // v.z, v.w = weight row g + 8, the same activation rows. Called by all 32 lanes of a warp.
 // With an output exchange the four lanes of a weight row gather its eight values and one of them
 // stores the 16 bytes into every rank's copy.
-__device__ __forceinline__ void frag_write(const FragArgs &a, int p, int lane, float4 v) {
+// m0: the first activation row of the tile's columns.
+__device__ __forceinline__ void frag_write(const FragArgs &a, int p, int lane, float4 v, int m0) {
   const int g = lane >> 2, t = lane & 3;
   const long long n0 = (long long)p * kFragRows + g;
   if (a.swiglu) {
@@ -232,12 +253,12 @@ __device__ __forceinline__ void frag_write(const FragArgs &a, int p, int lane, f
       row.x = __shfl_sync(0xffffffffu, ph, base), row.y = __shfl_sync(0xffffffffu, ph, base + 1);
       row.z = __shfl_sync(0xffffffffu, ph, base + 2), row.w = __shfl_sync(0xffffffffu, ph, base + 3);
       if (n < a.N / 2 && t < 2)  // lanes t = 0, 1 store to the even / odd ranks
-        for (int q = t; q < a.world; q += 2) *reinterpret_cast<uint4 *>(a.peer_y[q] + (a.row_offset + n) * a.peer_ld) = row;
+        for (int q = t; q < a.world; q += 2) *reinterpret_cast<uint4 *>(a.peer_y[q] + (a.row_offset + n) * a.peer_ld + m0) = row;
       return;
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int m = 2 * t + i;
+      const int m = m0 + 2 * t + i;
       if (n < a.N / 2 && m < a.M) {
         const __half h = __float2half_rn(i ? v.y : v.x);
         if (a.out_transposed) a.y[n * a.ldy + m] = h;
@@ -259,7 +280,7 @@ __device__ __forceinline__ void frag_write(const FragArgs &a, int p, int lane, f
     const long long n = n0 + ((t & 2) ? 8 : 0);
     if (n < a.N) {
       const uint4 row = (t & 2) ? rhi : rlo;
-      for (int q = t & 1; q < a.world; q += 2) *reinterpret_cast<uint4 *>(a.peer_y[q] + (a.row_offset + n) * a.peer_ld) = row;
+      for (int q = t & 1; q < a.world; q += 2) *reinterpret_cast<uint4 *>(a.peer_y[q] + (a.row_offset + n) * a.peer_ld + m0) = row;
     }
     return;
   }
@@ -267,7 +288,7 @@ __device__ __forceinline__ void frag_write(const FragArgs &a, int p, int lane, f
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const long long n = n0 + ((i & 2) ? 8 : 0);
-    const int m = 2 * t + (i & 1);
+    const int m = m0 + 2 * t + (i & 1);
     if (n < a.N && m < a.M) {
       const __half h = __float2half_rn(e[i]);
       if (a.out_transposed) a.y[n * a.ldy + m] = h;
@@ -329,105 +350,90 @@ __device__ __forceinline__ void st_async128(uint32_t addr, float4 v, uint32_t mb
                : "memory");
 }
 
-// MODE 0: tensor-core (rows 1..8); MODE 1: CUDA-core FMA for a single row. MAXW: most warps of a block.
-template <class Fmt, int MODE, int MAXW>
+// MODE 0: tensor-core (up to eight rows per column group); MODE 1: CUDA-core FMA for a single row.
+// MAXW: most warps of a block. NB: column groups of eight activation rows, 1 or 2.
+template <class Fmt, int MODE, int MAXW, int NB>
 __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
+  static_assert(MODE == 0 || NB == 1, "the CUDA-core variant takes one row");
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kTile = Fmt::kTileBytes;
-  constexpr uint32_t kStride = (uint32_t)((kTile + 127) & ~127);
-  const int warp = threadIdx.x >> 5;
+  constexpr uint32_t kStride = (uint32_t)((kTile + 15) & ~15), kPart = NB * 512u, kPark = NB * 1024u;  // bytes of a partial tile in fp32, fp64
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // (a broadcast: the compiler sees that it is uniform)
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int S = a.S, Wu = a.Wu, PP = a.PP, G = a.G;
-  const int W = Wu * PP;
-  // This warp's position wu in its panel lane wp. The lanes are dealt round robin over the warps,
-  // so that with 2 or 4 lanes all warps of an SM sub-partition (warp % 4) belong to one lane: the
-  // scheduler's preference for its oldest warps then cannot starve a whole lane.
-  const int wu = frag_div((unsigned)warp, a.inv_pp), wp = warp - wu * PP;
+  const int S = a.S, W = (int)(blockDim.x >> 5);
 
-  const uint32_t xfrag = smem_u32(smem);                                   // [umax][Fmt::kXBytes], then Fmt::kExtraBytes
-  const uint32_t red = xfrag + (uint32_t)a.umax * Fmt::kXBytes + Fmt::kExtraBytes;  // [PP][kFragRed][Wu][128 floats]
-  const uint32_t inbox = red + (Wu > 1 ? (uint32_t)(W * kFragRed) * 512u : 0u);  // [PP][2G][S][128 floats]
-  const uint32_t ctrl = inbox + (S > 1 ? (uint32_t)(PP * 2 * G * S) * 512u : 0u);
+  const uint32_t xfrag = smem_u32(smem);                                // [NB][a.xregion]
+  const uint32_t tables = xfrag + NB * a.xregion;                       // Fmt::kExtraBytes
+  const uint32_t red = tables + Fmt::kExtraBytes;                       // [warp][kPark]: the panel this warp's run begins inside of
+  const uint32_t inbox = red + (uint32_t)W * kPark;                     // [led][S][kPart]
+  const uint32_t ctrl = inbox + (S > 1 ? (uint32_t)(a.led * S) * kPart : 0u);
   const int R = a.ring;  // tiles in this warp's ring
-  const uint32_t ring = ctrl + kFragCtrlBytes + (uint32_t)(warp * R) * kStride;
-  uint8_t *ctrl_p = smem + (ctrl - xfrag);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(ctrl_p);                   // [PP][2G]
-  int *cnt = reinterpret_cast<int *>(ctrl_p + 1152);                       // [PP][kFragRed] arrivals of the lane's warps
-  volatile int *done = reinterpret_cast<volatile int *>(ctrl_p + 1344);    // [PP] panels of the lane whose partials were added
-  volatile int *abort_word = reinterpret_cast<volatile int *>(ctrl_p + 1440);
-  volatile int *uses = reinterpret_cast<volatile int *>(ctrl_p + 768);     // [PP][2G] completed phases of each inbox mbarrier
+  const uint32_t rings = ctrl + frag_ctrl_bytes(S > 1 ? a.led : 0), ring = rings + (uint32_t)(warp * R) * kStride;
+  int *cnt = reinterpret_cast<int *>(smem + (ctrl - xfrag));  // [warp]: arrivals at the panel that begins in this warp's run and goes on
+  volatile int *abort_word = reinterpret_cast<volatile int *>(smem + (ctrl - xfrag) + kFragCtrlAbort);
 
   // (divisions by multiplication: the host checks the ranges)
   const int cid = frag_div(blockIdx.x, a.inv_s);
   const int r = (int)blockIdx.x - cid * S;  // rank in the cluster = column range
-  const int ub0 = frag_div((unsigned)(r * a.units), a.inv_s);  // = frag_column_begin(r, units, S)
+  const int ub0 = frag_div((unsigned)(r * a.units), a.inv_s);
   const int uc = frag_div((unsigned)((r + 1) * a.units), a.inv_s) - ub0;
   // the cluster's panels: pa .. pa + np - 1
   const int pa = frag_div((unsigned)cid * (unsigned)a.P, a.inv_nc);
   const int np = frag_div((unsigned)(cid + 1) * (unsigned)a.P, a.inv_nc) - pa;
-  const int per = frag_div((unsigned)(uc - 1 - wu + Wu), a.inv_wu);  // units of a panel this warp owns: wu + i * Wu < uc
-  const int contributors = min(Wu, uc);                              // warps of a lane that own a unit
-  const int rounds = frag_div((unsigned)(np + PP - 1), a.inv_pp);    // panels of the fullest lane
-  const int npw = np > wp ? frag_div((unsigned)(np - wp + PP - 1), a.inv_pp) : 0;  // panels this warp takes: wp, wp + PP, ...
+  const int led = S > 1 ? frag_div((unsigned)(np - 1 - r + S), a.inv_s) : 0;  // panels this CTA leads: r, r + S, ...
+  // the CTA's tiles, and this warp's run of them
+  const unsigned T = (unsigned)(np * uc), We = min((unsigned)W, T);
+  const int t0 = (unsigned)warp < We ? (int)(T * (unsigned)warp / We) : (int)T;
+  const int t1 = (unsigned)warp < We ? (int)(T * (unsigned)(warp + 1) / We) : (int)T;
+  const int q0 = (int)((unsigned)t0 / (unsigned)uc);  // the run's first panel
 
   ISHI_STAMP(0);
   // Let the next kernel on the stream start its own prologue as SMs fall free.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  if (threadIdx.x < 32) {  // the control block, a word or a barrier per lane of warp 0
-    for (int i = threadIdx.x; i < PP * 2 * G; i += 32) {
-      mbar_init(bars + i, 1);
-      uses[i] = 0;
+  if (threadIdx.x < 32) {  // the control block
+    for (int i = threadIdx.x; i < led; i += 32) {
+      // each led panel's mbarrier: S partial panels, known now
+      mbar_init_u32(ctrl + kFragCtrlInbox + 8u * i, 1);
+      mbar_arrive_expect_tx_u32(ctrl + kFragCtrlInbox + 8u * i, (uint32_t)S * kPart);
     }
-    for (int i = threadIdx.x; i < PP * kFragRed; i += 32) cnt[i] = 0;
-    if ((int)threadIdx.x < PP) done[threadIdx.x] = 0;
+    if ((int)threadIdx.x < W) cnt[threadIdx.x] = 0;
     if (threadIdx.x == 0) *abort_word = 0;
     mbar_fence_init();
+    __syncwarp();
   }
   // Shared memory of another CTA may be written only once that CTA runs and has set up its
-  // barriers: every CTA arrives here, and waits before its first panel.
+  // barriers: every CTA arrives here, and a warp waits before its first partial panel.
   if (S > 1) cluster_arrive_relaxed();  // the init fence above is what the peers need; nothing else to publish yet
 
-  // This warp's tile sequence: its panels in order, in each its units wu + qi * Wu. The fetch
-  // cursor runs R - 1 tiles ahead of the compute cursor. Lane 0 issues the copies; every
-  // lane keeps the cursor.
-  const uint32_t wbar = ctrl + 1472u + (uint32_t)warp * kFragMaxRing * 8u;  // this warp's ring mbarriers
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < kFragMaxRing; ++i) mbar_init_u32(wbar + 8u * i, 1);
-    mbar_fence_init();
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copy engine sees the barriers initialised
-  }
-  __syncwarp();
-  int f_left = npw * per, f_qi = 0, f_idx = 0;
-  uint32_t f_slot = ring;
-  const uint8_t *f_src = a.tiles + ((long long)(pa + wp) * a.units + ub0 + wu) * (long long)kTile;
-  const long long step_unit = (long long)Wu * kTile;
-  const long long step_panel = ((long long)PP * a.units - (long long)per * Wu) * kTile;
-  auto fetch = [&]() {
-    bulk_g2s_if(f_left > 0 && lane == 0, f_slot, f_src, (uint32_t)kTile, wbar + 8u * f_idx);
+  // This warp's run of tiles. The fetch cursor runs R - 1 tiles ahead of the compute cursor: a tile is
+  // fetched into the slot of the tile decoded last. One commit group per tile, empty past the end.
+  int f_left = t1 - t0, f_u = t0 - q0 * uc;
+  const uint8_t *f_src = a.tiles + ((long long)(pa + q0) * a.units + ub0 + f_u) * (long long)kTile + lane * 16;
+  const long long step_panel = (long long)(a.units - uc) * kTile;  // from the end of a panel's column range to the next one's
+  auto fetch = [&](uint32_t slot) {
+    if (f_left > 0) {
+      cp_async_tile<kTile>(slot + (uint32_t)lane * 16u, f_src, lane);
+      f_src += kTile;
+      if (++f_u == uc) {
+        f_u = 0;
+        f_src += step_panel;
+      }
+    }
     --f_left;
-    f_src += step_unit;
-    if (++f_qi == per) {
-      f_qi = 0;
-      f_src += step_panel;
-    }
-    f_slot += kStride;
-    if (++f_idx == R) {
-      f_idx = 0;
-      f_slot = ring;
-    }
+    cp_async_commit();
   };
-  // The weight tiles are written by no earlier kernel: their first copies go out at once.
-  for (int i = 0; i < R - 1; ++i) fetch();
+  // The weight tiles are written by no earlier kernel: their first copies go out at once. (Asking
+  // the run's next tiles into L2 as well delays the activations behind them: 60 -> 66 us per layer.)
+  for (int i = 0; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride);
 
-  Fmt::before_wait(a, xfrag);  // tables that do not depend on earlier launches
+  Fmt::before_wait(a, tables);  // tables that do not depend on earlier launches
 
   // Warm L2 and the address translation with this CTA's slice of x. Only a hint: x may still be
   // written by the kernel before this one, its values are read after the wait below, through L2.
-  for (int r = warp; r < a.M; r += (int)(blockDim.x >> 5)) {
-    const char *row = reinterpret_cast<const char *>(a.x + (long long)r * a.K + (long long)ub0 * 256);
+  for (int m = warp; m < a.M; m += W) {
+    const char *row = reinterpret_cast<const char *>(a.x + (long long)m * a.K + (long long)ub0 * 256);
     for (int c = lane; c < uc * 4; c += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c * 128));
   }
 
@@ -449,177 +455,161 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
         if (!ok) *a.err = 2;  // give up: the result is wrong, the error word tells the host
       }
     }
+    __syncthreads();  // the other GPUs' rows have arrived, for every warp
   }
-  __syncthreads();  // the control block is set up for every warp; the other GPUs' rows have arrived
   ISHI_STAMP(2);
 
   // activations of the column range into fragment order (all warps)
-  Fmt::stage_x(a, xfrag, ub0, uc, [&]() { ISHI_STAMP(8); });
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+    Fmt::stage_x(a, a.x + (long long)(8 * b) * a.K, a.M - 8 * b, xfrag + b * a.xregion, ub0, uc);
   ISHI_STAMP(3);
-  __syncthreads();
+  __syncthreads();  // staged, and the control block is set up for every warp
   ISHI_STAMP(4);
   // shared-memory loads are plain asm the compiler may move; tie their addresses to the waits
-  const uint32_t xf = stage_acquire(xfrag);
+  const uint32_t xf = stage_acquire(xfrag), tb = stage_acquire(tables);
 
-  if (S > 1) cluster_wait_relaxed();
-  ISHI_STAMP(5);
-
-  int arrived = 0, waited = 0;  // cluster barrier generations this thread has arrived at / waited for
-  int gen = 0, gpos = 0;        // generation of inbox slots, position of the lane's panel in it
-  uint32_t c_slot = ring, c_phase = 0;
-  int c_idx = 0;
-  for (int i = 0; i < rounds; ++i, ++gpos) {
-    if (gpos == G) {
-      gpos = 0;
-      ++gen;
-      if (S > 1) {
-        // generation gen - 1 is finished here; generation gen reuses the inbox slots of gen - 2,
-        // which every leader has read once all warps of the cluster have finished gen - 2
-        if (arrived > waited) {
-          cluster_wait_relaxed();
-          ++waited;
-        }
-        cluster_arrive_relaxed();
-        ++arrived;
+  bool joined = S == 1;  // this warp has seen every CTA of the cluster arrive
+  uint32_t c_slot = ring, f_slot = ring + (uint32_t)(R - 1) * kStride;
+  const uint32_t ring_end = ring + (uint32_t)R * kStride;
+  int at = t0, u = t0 - q0 * uc;
+  for (int q = q0; at < t1; ++q) {
+    const int first = at, end = min(t1, (q + 1) * uc);
+    double acc[NB][4];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) acc[b][0] = acc[b][1] = acc[b][2] = acc[b][3] = 0.0;
+    for (; at < end; ++at, ++u) {
+      ISHI_CLOCK(c0);
+      // this tile has landed (all but the last R - 2 groups are complete), for every lane, and every
+      // lane is done with the tile before, whose slot is refilled
+      if (R == 2) cp_async_wait<0>();
+      else if (R == 3) cp_async_wait<1>();
+      else cp_async_wait<2>();
+      __syncwarp();
+      if (at == t0) ISHI_STAMP(6);
+      ISHI_CLOCK(c1);
+      fetch(f_slot);
+      float tile[NB][4];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) tile[b][0] = tile[b][1] = tile[b][2] = tile[b][3] = 0.f;
+      Fmt::template unit<MODE, NB>(tile, a, stage_acquire(c_slot), xf, tb, u, g, t, lane);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        values_ready(tile[b][0], tile[b][1], tile[b][2], tile[b][3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[b][i] += (double)tile[b][i];
       }
+      ISHI_CLOCK(c2);
+      ISHI_SPENT(16, c0, c1);
+      ISHI_SPENT(17, c1, c2);
+      f_slot = c_slot;
+      c_slot += kStride;
+      if (c_slot == ring_end) c_slot = ring;
     }
-    const int pi = wp + i * PP;  // the panel's index in the cluster's run
-    if (pi >= np || per == 0) continue;
-
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    {
-      int uq = wu;  // the unit's index in the column range
-      for (int qi = 0; qi < per; ++qi) {
-        ISHI_CLOCK(c0);
-        if (!mbar_wait_u32(wbar + 8u * c_idx, c_phase, abort_word)) *a.err = 1;  // this slot has landed
-        __syncwarp();  // every lane is done with the previous slot
-        if (i == 0 && qi == 0) ISHI_STAMP(6);
-        ISHI_CLOCK(c1);
-        fetch();                         // refill the previous slot
-        Fmt::template unit<MODE>(acc, a, stage_acquire(c_slot), xf, uq, g, t, lane);
-        values_ready(acc[0], acc[1], acc[2], acc[3]);
-        ISHI_CLOCK(c2);
-        ISHI_SPENT(16, c0, c1);
-        ISHI_SPENT(17, c1, c2);
-        uq += Wu;
-        c_slot += kStride;
-        if (++c_idx == R) {
-          c_idx = 0;
-          c_slot = ring;
-          c_phase ^= 1u;
-        }
-      }
-      if (MODE == 1) {
-        // single activation row: each lane holds partial dot products of rows g (acc[0]) and
-        // g + 8 (acc[2]) over its own k positions; add across the four lanes of a row
-        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
-        acc[2] += __shfl_xor_sync(0xffffffffu, acc[2], 1);
-        acc[2] += __shfl_xor_sync(0xffffffffu, acc[2], 2);
-        if (t != 0) acc[0] = acc[2] = 0.f;  // one copy per row enters the sums below (column m = 0)
-        acc[1] = acc[3] = 0.f;
-      }
+    u = 0;
+    if (MODE == 1) {
+      // single activation row: each lane holds partial dot products of rows g (acc[0]) and
+      // g + 8 (acc[2]) over its own k positions; add across the four lanes of a row
+      double *c = acc[0];
+      c[0] += __shfl_xor_sync(0xffffffffu, c[0], 1);
+      c[0] += __shfl_xor_sync(0xffffffffu, c[0], 2);
+      c[2] += __shfl_xor_sync(0xffffffffu, c[2], 1);
+      c[2] += __shfl_xor_sync(0xffffffffu, c[2], 2);
+      if (t != 0) c[0] = c[2] = 0.0;  // one copy per row enters the sums below (column m = 0)
+      c[1] = c[3] = 0.0;
     }
-    if (i == 0) ISHI_STAMP(7);
+    if (q == q0) ISHI_STAMP(7);
 
-    // park the partial tile; the warp of the lane that arrives last adds the lane's partials
     ISHI_CLOCK(c3);
-    float4 sum = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    bool last = true;
-    if (contributors > 1) {
-      const int rs = i & (kFragRed - 1);
-      const uint32_t slot = red + (uint32_t)((wp * kFragRed + rs) * Wu) * 512u;
-      if (i >= kFragRed && done[wp] < i - kFragRed + 1) {
-        // the slot still holds the partials of panel i - kFragRed of this lane
-        bool ok = false;
-        for (uint32_t spin = 0; spin < kWaitSpins && !ok; ++spin) {
-          ok = done[wp] >= i - kFragRed + 1;
-          if (!ok && *abort_word != 0) break;
-        }
-        if (!ok) {
-          *abort_word = 1;
-          *a.err = 1;
-        }
+    const int begin = q * uc;
+    if (first != begin || end != begin + uc) {
+      // The panel is shared with other warps: park the partial tile; the warp that arrives last adds
+      // the partials in warp order. The panel begins in run wa (parked in that warp's ring, which is
+      // drained: the panel's part is the last of the run; the plan leaves it kPark bytes) and ends in run wb (parked in the slots).
+      const int wa = (int)((((unsigned)begin + 1u) * We - 1u) / T), wb = (int)(((unsigned)(begin + uc) * We - 1u) / T);
+      const uint32_t mine = (warp == wa ? ring : red + (uint32_t)warp * kPark) + (uint32_t)lane * 16u;
+      __syncwarp();  // every lane is done with the last tile
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        sts128d(mine + b * 1024u, acc[b][0], acc[b][1]);
+        sts128d(mine + b * 1024u + 512u, acc[b][2], acc[b][3]);
       }
-      sts128(stage_acquire(slot) + (uint32_t)(wu * 32 + lane) * 16u, sum);
       __syncwarp();
       int old = 0;
       if (lane == 0) {
         __threadfence_block();
-        old = atomicAdd(cnt + wp * kFragRed + rs, 1);
+        old = atomicAdd(cnt + wa, 1);
       }
       old = __shfl_sync(0xffffffffu, old, 0);
-      last = old == contributors - 1;
-      if (last) {
-        __threadfence_block();
-        const uint32_t src = stage_acquire(slot) + (uint32_t)lane * 16u;
-        sum = lds128f(src);
-        for (int w = 1; w < contributors; ++w) {
-          const float4 o = lds128f(src + (uint32_t)w * 512u);
-          sum.x += o.x, sum.y += o.y, sum.z += o.z, sum.w += o.w;
-        }
-        values_ready(sum.x, sum.y, sum.z, sum.w);
-        __syncwarp();
-        if (lane == 0) {
-          cnt[wp * kFragRed + rs] = 0;
-          __threadfence_block();
-          done[wp] = i + 1;
+      if (old != wb - wa) continue;
+      __threadfence_block();
+      for (int w = wa; w <= wb; ++w) {
+        const uint32_t src = stage_acquire(w == wa ? rings + (uint32_t)(wa * R) * kStride : red + (uint32_t)w * kPark) + (uint32_t)lane * 16u;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const double2 lo = lds128d(src + b * 1024u), hi = lds128d(src + b * 1024u + 512u);
+          acc[b][0] = w == wa ? lo.x : acc[b][0] + lo.x, acc[b][1] = w == wa ? lo.y : acc[b][1] + lo.y;
+          acc[b][2] = w == wa ? hi.x : acc[b][2] + hi.x, acc[b][3] = w == wa ? hi.y : acc[b][3] + hi.y;
         }
       }
     }
+    float4 sum[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      constexpr double kUnit = Fmt::kUnit;  // a power of two: the decoder's unit of a tile's result
+      sum[b] = make_float4((float)(acc[b][0] * kUnit), (float)(acc[b][1] * kUnit), (float)(acc[b][2] * kUnit), (float)(acc[b][3] * kUnit));
+    }
     ISHI_CLOCK(c4);
     ISHI_SPENT(18, c3, c4);
-    if (!last) continue;
 
     if (S == 1) {
-      frag_write(a, pa + pi, lane, sum);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) frag_write(a, pa + q, lane, sum[b], 8 * b);
     } else {
-      // the CTA's partial panel goes to the panel's leader, rank pi % S
-      const int lead = pi - frag_div((unsigned)pi, a.inv_s) * S;
-      const int is = wp * 2 * G + (gen & 1) * G + gpos;  // inbox slot
-      const uint32_t bar = ctrl + (uint32_t)is * 8u;
-      const uint32_t box = inbox + (uint32_t)(is * S) * 512u + (uint32_t)lane * 16u;
-      if (lead == r) {
-        if (lane == 0) mbar_arrive_expect_tx(bars + is, (uint32_t)S * 512u);
-        __syncwarp();
-      }
-      st_async128(cluster_map(box + (uint32_t)r * 512u, (uint32_t)lead), sum, cluster_map(bar, (uint32_t)lead));
+      // the CTA's partial panel goes to the panel's leader, rank q % S, into inbox slot q / S
+      if (!joined) cluster_wait_relaxed(), joined = true;
+      const int slot = frag_div((unsigned)q, a.inv_s), lead = q - slot * S;
+      const uint32_t box = cluster_map(inbox + (uint32_t)(slot * S + r) * kPart + (uint32_t)lane * 16u, (uint32_t)lead);
+      const uint32_t bar = cluster_map(ctrl + kFragCtrlInbox + 8u * slot, (uint32_t)lead);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) st_async128(box + b * 512u, sum[b], bar);
       ISHI_CLOCK(c5);
       ISHI_SPENT(19, c4, c5);
-      if (lead == r) {
-        // a CTA leads only some of the panels that map to this slot, so the barrier's phase is
-        // counted here; the slot's next use is two generations away, behind a cluster barrier
-        const uint32_t parity = (uint32_t)uses[is] & 1u;
-        bool ok = mbar_try_wait_cluster(bar, parity);
-        for (uint32_t spin = 0; spin < kWaitSpins && !ok; ++spin) {
-          ok = mbar_try_wait_cluster(bar, parity);
-          if (!ok && *abort_word != 0) break;
-        }
-        if (!ok) {  // give up: y of this panel stays wrong, the error word tells the host
-          *abort_word = 1;
-          *a.err = 1;
-        } else {
-          const uint32_t src = stage_acquire(box);
-          float4 total = lds128f(src);
-          for (int q = 1; q < S; ++q) {
-            const float4 o = lds128f(src + (uint32_t)q * 512u);
-            total.x += o.x, total.y += o.y, total.z += o.z, total.w += o.w;
-          }
-          frag_write(a, pa + pi, lane, total);
-        }
-        __syncwarp();
-        if (lane == 0) uses[is] = (int)parity + 1;
-        ISHI_CLOCK(c6);
-        ISHI_SPENT(20, c5, c6);
-      }
     }
   }
   ISHI_STAMP(24);
   if (S > 1) {
-    // no CTA leaves while another may still send to it or read its barriers
-    if (arrived > waited) cluster_wait_relaxed();
-    cluster_arrive_relaxed();
-    cluster_wait_relaxed();
+    if (!joined) cluster_wait_relaxed();
+    for (int i = warp; i < led; i += W) {
+      const uint32_t bar = ctrl + kFragCtrlInbox + 8u * i;
+      bool ok = mbar_try_wait_cluster(bar, 0u);
+      for (uint32_t spin = 0; spin < kWaitSpins && !ok; ++spin) {
+        ok = mbar_try_wait_cluster(bar, 0u);
+        if (!ok && *abort_word != 0) break;
+      }
+      if (!ok) {  // give up: y of this panel stays wrong, the error word tells the host
+        *abort_word = 1;
+        *a.err = 1;
+        break;
+      }
+      const uint32_t src = stage_acquire(inbox) + (uint32_t)(i * S) * kPart + (uint32_t)lane * 16u;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        float4 total = lds128f(src + b * 512u);
+        for (int k = 1; k < S; ++k) {
+          const float4 o = lds128f(src + (uint32_t)k * kPart + b * 512u);
+          total.x += o.x, total.y += o.y, total.z += o.z, total.w += o.w;
+        }
+        frag_write(a, pa + i * S + r, lane, total, 8 * b);
+      }
+    }
+    // A CTA that received all it leads may leave: nobody sends to it any more. One that gave up stays
+    // until the others have left or given up too, since they may still send to it (a thread that
+    // has exited counts as arrived).
+    if (__shfl_sync(0xffffffffu, *abort_word, 0) != 0) {
+      cluster_arrive_relaxed();
+      cluster_wait_relaxed();
+    }
   }
   ISHI_STAMP(27);
   if (a.world > 0) {
@@ -642,7 +632,6 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
     }
   }
 }
-
 // waits (bounded) until every rank's arrival word has reached this rank's latest launch
 static __global__ void peer_wait_kernel(const unsigned *local_flags, int world, const unsigned *launch_no, int *err) {
   if ((int)threadIdx.x < world) {

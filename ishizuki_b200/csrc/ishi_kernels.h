@@ -14,17 +14,18 @@ namespace ishi {
 struct FragLaunch {
   int clusters, split, warps;  // grid = clusters * split CTAs of warps * 32 threads
   size_t smem;
-  int mode;    // 0: tensor cores, rows 1..8; 1: CUDA cores, one row
+  int mode;    // 0: tensor cores, rows 1..16; 1: CUDA cores, one row
   bool early;  // programmatic dependent launch
   cudaStream_t stream;
 };
 
 struct FragOps {
-  int tile_bytes, x_bytes, x_extra;  // bytes per tile; activation staging per unit of the column range, and per CTA
+  int tile_bytes;
+  int x_bytes, x_fixed, x_extra;  // a staged region of eight rows: bytes per unit of the column range, once; tables per CTA
   // raises the dynamic shared memory limit of every variant (once per device)
   cudaError_t (*configure)(int max_smem);
-  // how many clusters of `split` CTAs the device keeps resident, 0 if the launch is impossible
-  int (*max_clusters)(int split, int warps, size_t smem, int sm_count);
+  // how many clusters of `split` CTAs the device keeps resident, 0 if the launch is impossible; groups: of eight rows
+  int (*max_clusters)(int split, int warps, int groups, size_t smem, int sm_count);
   cudaError_t (*launch)(const FragLaunch &cfg, const FragArgs &args);
   // the one-time re-tiling into fragment order
   cudaError_t (*prepare)(const FragSrc &src, int units, uint8_t *dst, int grid, cudaStream_t stream);

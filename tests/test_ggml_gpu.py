@@ -209,6 +209,22 @@ def test_every_launch_plan_gives_the_same_product(plan, type_id, monkeypatch):
     lin.ctx.poll()
 
 
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("n,k", [(1, 256), (17, 256), (16, 2048), (40, 1280), (2600, 768), (5000, 1024)])
+def test_runs_of_tiles_that_share_panels(type_id, n, k):
+    """A CTA's tiles are dealt to its warps in equal runs that begin and end inside panels: fewer tiles
+    than warps, panels cut between two and many warps, runs that hold several panels; one and two
+    column groups of activation rows."""
+    rng = np.random.default_rng(n + k)
+    blocks = synth.ggml_blocks(rng, int(type_id), n, k)
+    lin = PackedLinear(ggml=GGUFBlocks(dev(blocks), type_id, (n, k)))
+    for m in (1, 8, 9, 16):
+        x = synth.activations(rng, m, k)
+        want32, _ = oracle.ggml_matmul(int(type_id), blocks, x, n)
+        assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
+    lin.ctx.poll()
+
+
 @pytest.mark.parametrize("type_id", OTHERS)
 @pytest.mark.parametrize("m", [1, 8, 16])
 def test_projection_of_the_other_block_formats(type_id, m):

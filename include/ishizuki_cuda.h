@@ -443,10 +443,9 @@ ishi_status ishi_exl3_rotate(ishi_ctx *ctx, const void *x, int x_dtype, int64_t 
  * A fragment of mma.sync m16n8k16 with n on the M side); no rotation. */
 ishi_status ishi_exl3_matvec(ishi_ctx *ctx, const ishi_exl3_desc *t, const void *x, int rows, float *y, void *stream);
 /* EXL3Kernels.apply (EXL3.swift:83-106): rotate x with the input scales (to fp16), multiply, rotate
- * the fp32 product with the output scales; y [rows, n] fp16, 1...16 rows (9...16 as two products,
- * as the reference does; its dense route above 16 rows is not part of this library: ISHI_E_SHAPE).
- * Uses scratch of the context, grown on demand by the first call of a larger shape (which then
- * allocates and must not be captured into a graph). */
+ * the fp32 product with the output scales, in one launch; y [rows, n] fp16, 1...16 rows (the
+ * reference's dense route above 16 rows is not part of this library: ISHI_E_SHAPE). Allocates
+ * nothing. */
 ishi_status ishi_exl3_apply(ishi_ctx *ctx, const ishi_exl3_desc *t, const void *x, int rows, void *y, void *stream);
 
 #ifdef __cplusplus

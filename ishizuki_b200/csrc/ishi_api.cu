@@ -96,9 +96,6 @@ struct ishi_ctx {
   void *pin_x = nullptr, *pin_y = nullptr;  // pinned staging for apply_host
   void *dev_x = nullptr, *dev_y = nullptr;
   size_t pin_x_bytes = 0, pin_y_bytes = 0;
-  __half *exl3_x = nullptr;  // ishi_exl3_apply: rotated activations [16][k] and fp32 products [16][n]
-  float *exl3_y = nullptr;
-  size_t exl3_x_cap = 0, exl3_y_cap = 0;
   // apply_host_batch: its two copy streams and the events that order them against the caller's stream
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   std::vector<cudaEvent_t> ev_in, ev_done;
@@ -805,8 +802,6 @@ void ishi_ctx_destroy(ishi_ctx *ctx) {
   if (ctx->pin_y) cudaFreeHost(ctx->pin_y);
   if (ctx->dev_x) cudaFree(ctx->dev_x);
   if (ctx->dev_y) cudaFree(ctx->dev_y);
-  if (ctx->exl3_x) cudaFree(ctx->exl3_x);
-  if (ctx->exl3_y) cudaFree(ctx->exl3_y);
   for (cudaEvent_t e : ctx->ev_in) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->ev_done) cudaEventDestroy(e);
   if (ctx->ev_begin) cudaEventDestroy(ctx->ev_begin);
@@ -1736,8 +1731,9 @@ ishi_status ishi_exl3_matvec(ishi_ctx *ctx, const ishi_exl3_desc *t, const void 
   if (reinterpret_cast<uintptr_t>(x) & 3u) return fail(ctx, ISHI_E_INVALID, "x must be 4-byte aligned");
   if (rows < 1 || rows > 8) return fail(ctx, ISHI_E_SHAPE, "rows %d outside 1...8", rows);
   ISHI_CUDA(ctx, cudaSetDevice(ctx->device));
-  ISHI_CUDA(ctx, launch_exl3_matvec(t->trellis_dev, (int)(t->k / 16), (int)(t->n / 16), t->words_per_tile, t->codebook,
-                                    static_cast<const __half *>(x), rows, y, ctx->sm_count, static_cast<cudaStream_t>(stream)));
+  ISHI_CUDA(ctx, launch_exl3_product(t->trellis_dev, (int)(t->k / 16), (int)(t->n / 16), t->words_per_tile, t->codebook,
+                                     static_cast<const __half *>(x), nullptr, nullptr, rows, y, ctx->err_dev, ctx->sm_count,
+                                     static_cast<cudaStream_t>(stream)));
   return ISHI_OK;
 }
 
@@ -1747,30 +1743,10 @@ ishi_status ishi_exl3_apply(ishi_ctx *ctx, const ishi_exl3_desc *t, const void *
   if (s != ISHI_OK) return s;
   if (!x || !y) return fail(ctx, ISHI_E_INVALID, "null pointer");
   if (rows < 1 || rows > 16) return fail(ctx, ISHI_E_SHAPE, "rows %d outside 1...16", rows);
-  std::lock_guard<std::mutex> g(ctx->lock);
   ISHI_CUDA(ctx, cudaSetDevice(ctx->device));
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t xb = (size_t)16 * t->k * sizeof(__half), yb = (size_t)16 * t->n * sizeof(float);
-  if (ctx->exl3_x_cap < xb) {
-    ISHI_CUDA(ctx, cudaStreamSynchronize(st));  // earlier calls may still read the smaller buffer
-    if (ctx->exl3_x) cudaFree(ctx->exl3_x);
-    ctx->exl3_x = nullptr, ctx->exl3_x_cap = 0;
-    ISHI_CUDA(ctx, cudaMalloc(&ctx->exl3_x, xb));
-    ctx->exl3_x_cap = xb;
-  }
-  if (ctx->exl3_y_cap < yb) {
-    ISHI_CUDA(ctx, cudaStreamSynchronize(st));
-    if (ctx->exl3_y) cudaFree(ctx->exl3_y);
-    ctx->exl3_y = nullptr, ctx->exl3_y_cap = 0;
-    ISHI_CUDA(ctx, cudaMalloc(&ctx->exl3_y, yb));
-    ctx->exl3_y_cap = yb;
-  }
-  ISHI_CUDA(ctx, launch_exl3_rotate(x, ISHI_DT_F16, rows, t->k, static_cast<const __half *>(t->input_scales_dev), 1, ctx->exl3_x,
-                                    ISHI_DT_F16, ctx->sm_count, st));
-  for (int r0 = 0; r0 < rows; r0 += 8)
-    ISHI_CUDA(ctx, launch_exl3_matvec(t->trellis_dev, (int)(t->k / 16), (int)(t->n / 16), t->words_per_tile, t->codebook,
-                                      ctx->exl3_x + (size_t)r0 * t->k, std::min(8, rows - r0), ctx->exl3_y + (size_t)r0 * t->n, ctx->sm_count, st));
-  ISHI_CUDA(ctx, launch_exl3_rotate(ctx->exl3_y, ISHI_DT_F32, rows, t->n, static_cast<const __half *>(t->output_scales_dev), 0, y,
-                                    ISHI_DT_F16, ctx->sm_count, st));
+  ISHI_CUDA(ctx, launch_exl3_product(t->trellis_dev, (int)(t->k / 16), (int)(t->n / 16), t->words_per_tile, t->codebook,
+                                     static_cast<const __half *>(x), static_cast<const __half *>(t->input_scales_dev),
+                                     static_cast<const __half *>(t->output_scales_dev), rows, y, ctx->err_dev, ctx->sm_count,
+                                     static_cast<cudaStream_t>(stream)));
   return ISHI_OK;
 }

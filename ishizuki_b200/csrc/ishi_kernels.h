@@ -59,8 +59,10 @@ cudaError_t launch_rms_norm(const void *x, int x_dtype, const void *w, int w_dty
 bool exl3_rate_supported(int words16, int codebook);
 cudaError_t launch_exl3_dequantize(const int16_t *trellis, int tiles_k, int tiles_n, int words16, int codebook, void *out,
                                    int out_dtype, int sm_count, cudaStream_t st);
-cudaError_t launch_exl3_matvec(const int16_t *trellis, int tiles_k, int tiles_n, int words16, int codebook, const __half *x,
-                               int rows, float *y, int sm_count, cudaStream_t st);
+// y [rows][n] = x [rows][k] . W for 1...16 rows; with su and sv the input and output rotations around
+// it and y fp16 (EXL3Kernels.apply), without them y fp32. err: raised by a cluster wait that gives up
+cudaError_t launch_exl3_product(const int16_t *trellis, int tiles_k, int tiles_n, int words16, int codebook, const __half *x,
+                                const __half *su, const __half *sv, int rows, void *y, int *err, int sm_count, cudaStream_t st);
 cudaError_t launch_exl3_rotate(const void *x, int x_dtype, long long rows, long long width, const __half *scales, int before,
                                void *y, int y_dtype, int sm_count, cudaStream_t st);
 

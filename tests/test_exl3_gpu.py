@@ -128,6 +128,26 @@ def test_projection_at_a_model_shape():
         assert np.abs(y - want).max() / np.abs(want).max() < 2e-3
 
 
+@pytest.mark.parametrize("k,n", [(128, 128), (384, 256), (1152, 1024), (6016, 640), (640, 19200), (47104, 128)])
+@pytest.mark.parametrize("words,codebook", [(24, 2), (64, 0), (64, 2), (80, 1), (128, 2)])
+def test_apply_at_the_edges_of_the_split(k, n, words, codebook):
+    """One k block, odd numbers of them, every K split up to a cluster of eight, more groups than
+    clusters at a time, inputs staged in several chunks; rows in one and two column groups, and
+    operands without 16-byte alignment. Against the three steps: rotate, expanded weight, rotate."""
+    rng = np.random.default_rng(k + n + words)
+    trellis = dev(random_trellis(rng, k, n, words))
+    su, sv = dev(rng.standard_normal(k).astype(np.float16)), dev(rng.standard_normal(n).astype(np.float16))
+    t = EXL3Tensor(trellis, su, sv, codebook)
+    w = EXL3Kernels.dequantize(t, torch.float32).double()
+    for rows in (1, 8, 9, 16):
+        pad = torch.zeros(rows * k + 1, dtype=torch.float16, device="cuda")
+        for x in (torch.randn(rows, k, device="cuda").half(), pad[1:].copy_(torch.randn(rows * k)).view(rows, k)):
+            y = EXL3Kernels.apply(x, t).double()
+            xr = EXL3Kernels.rotate(x, su, True, torch.float16).double()
+            want = EXL3Kernels.rotate((xr @ w).float(), sv, False, torch.float32).double()
+            assert float((y - want).abs().max() / want.abs().max()) < 1e-3
+
+
 def test_guards():
     rng = np.random.default_rng(1)
     ok = random_trellis(rng, 128, 128, 64)

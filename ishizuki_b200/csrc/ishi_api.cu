@@ -1315,15 +1315,18 @@ ishi_status ishi_projection_apply_host_batch(ishi_projection *const *ps, const v
   }
   // Three lanes: x copies run ahead on one stream, the products follow on the caller's stream as
   // their inputs land, the y copies trail on a third; the caller's stream ends behind all of them.
-  // The lanes hand over in chunks of kChunk entries, not entry by entry: an event between two
-  // product kernels would serialise them, inside a chunk they follow each other with programmatic
-  // dependent launch as in a plain sequence of applies.
-  constexpr int kChunk = 16;
+  // The lanes hand over in chunks, not entry by entry: an event between two product kernels
+  // serialises them (about 2.5 us), inside a chunk they follow each other with programmatic dependent
+  // launch as in a plain sequence of applies. The chunks are short at both ends, where one lane waits
+  // for another (1, 3, then sixteen at a time, then 3, 1): four layers of the 27B shape at eight
+  // rows, 16 entries, took 470 us as one chunk, 75 of them before the first product and 110 after the
+  // last, and take 318 us now (products alone 220).
   ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_begin, st));
   ISHI_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_in, ctx->ev_begin, 0));
   ISHI_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, ctx->ev_begin, 0));
-  for (int c0 = 0; c0 < count; c0 += kChunk) {
-    const int c1 = std::min(count, c0 + kChunk);
+  for (int c0 = 0, c1 = 0; c0 < count; c0 = c1) {
+    const int left = count - c0, want = c0 == 0 ? 1 : c0 < 4 ? 3 : 16;
+    c1 = c0 + (left > 4 ? std::min(want, left - 4) : left > 1 ? std::min(want, left - 1) : 1);
     for (int i = c0; i < c1; ++i) {
       const size_t xb = (size_t)rows * ps[i]->d.k * sizeof(__half);
       ISHI_CUDA(ctx, cudaMemcpyAsync(ps[i]->host_x, x_hosts[i], xb, cudaMemcpyHostToDevice, ctx->copy_in));

@@ -1,4 +1,4 @@
-// MLX affine group-quantized packs (4 or 2 bits, fp16 or bf16 scales) for the warp-level kernel.
+// MLX affine group-quantized packs (8, 4 or 2 bits, fp16 or bf16 scales) for the warp-level kernel.
 //
 // Layout of the source (reference: Sources/IshizukiKit/Core/VerifyMatmul.swift:282-287 and
 // Sources/IshizukiKit/Quantize/WeightedAffineQuantizer.swift:142-161): row n is K*bits/32
@@ -15,6 +15,7 @@
 // Fragment mapping (m16n8k16; lane g = lane / 4, t = lane % 4 holds weight rows g and g + 8): of
 // every four consecutive words ("quad" q) lane t owns word 4q + t of both rows. One word yields
 // the A registers of 8 / BITS ... k-steps: with mask m (the m-th code of each byte pair),
+//   8 bits: k-step q:            a0 = codes (0, 2), a2 = codes (1, 3) of the word
 //   4 bits: k-step (q, m), m < 2:  a0 = codes (m, m + 4), a2 = codes (m + 2, m + 6) of the word
 //   2 bits: k-step (q, m), m < 4:  a0 = codes (m, m + 8), a2 = codes (m + 4, m + 12)
 // and x is staged in exactly that order, scaled by 2^-(BITS * m).
@@ -30,13 +31,13 @@ namespace ishi {
 
 template <int BITS, int GS, bool BF16>
 struct FragAffine {
-  static_assert(BITS == 4 || BITS == 2, "4- and 2-bit codes");
+  static_assert(BITS == 8 || BITS == 4 || BITS == 2, "8-, 4- and 2-bit codes");
   static_assert(GS == 32 || GS == 64 || GS == 128, "group sizes of the reference");
-  static_assert(BITS == 4 || GS >= 64, "a 2-bit k-step spans 64 inputs");
+  static_assert(BITS != 2 || GS >= 64, "a 2-bit k-step spans 64 inputs");
   static constexpr int kGroups = 256 / GS;           // per unit
-  static constexpr int kQuads = 2 * BITS;            // word quads per unit: 8 (32 words) or 4 (16 words)
-  static constexpr int kMasks = 8 / BITS;            // k-steps per quad: 2 or 4
-  static constexpr int kQuadK = 256 / kQuads;        // inputs a quad covers: 32 or 64
+  static constexpr int kQuads = 2 * BITS;            // word quads per unit: 16 (64 words), 8 or 4
+  static constexpr int kMasks = 8 / BITS;            // k-steps per quad: 1, 2 or 4
+  static constexpr int kQuadK = 256 / kQuads;        // inputs a quad covers: 16, 32 or 64
   static constexpr int kHeader = BITS * 512;         // offset of the scales and biases
   static constexpr int kRowHeader = 4 * kGroups;     // bytes per row there
   static constexpr int kTileBytes = kHeader + 16 * kRowHeader;
@@ -112,7 +113,13 @@ struct FragAffine {
                               a.rot_signs ? a.rot_signs + (long long)(ub0 + (i >> 3)) * 256 + lane * 8 : nullptr, lane);
         const uint32_t base = xfrag + (uint32_t)(i >> 3) * kXBytes;
         // halves of v: x0 x1 | x2 x3 | x4 x5 | x6 x7
-        if (BITS == 4) {
+        if (BITS == 8) {
+          // the lane holds words 2l and 2l + 1: quad q = l / 2, t = 2 (l % 2) and t + 1, each (x0, x2), (x1, x3)
+          const int q = lane >> 1;
+          sts128u(base + (uint32_t)q * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + 2 * (lane & 1)) * 8),
+                  make_uint4(prmt(v[e].x, v[e].y, 0x5410u), prmt(v[e].x, v[e].y, 0x7632u), prmt(v[e].z, v[e].w, 0x5410u),
+                             prmt(v[e].z, v[e].w, 0x7632u)));
+        } else if (BITS == 4) {
           // the lane holds word l: quad q = l / 4, t = l % 4; k-step m pairs (x_m, x_m+4), (x_m+2, x_m+6)
           const int q = lane >> 2, t = lane & 3;
           const uint32_t dst = base + (uint32_t)(2 * q) * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + t) * 8);
@@ -295,7 +302,7 @@ struct FragAffine {
         const uint32_t xq = xl ^ (uint32_t)((q & 3) << 5);  // the quad's staging swizzle
 #pragma unroll
         for (int m = 0; m < kMasks; ++m) {
-          const uint32_t mask = (BITS == 4 ? 0x000f000fu : 0x00030003u) << (BITS * m);
+          const uint32_t mask = (BITS == 8 ? 0x00ff00ffu : BITS == 4 ? 0x000f000fu : 0x00030003u) << (BITS * m);
           const uint32_t a0 = x0 & mask, a1 = x1 & mask, a2 = y0 & mask, a3 = y1 & mask;
           const bool first = (q * kQuadK) % GS == 0 && m == 0;  // first k-step of a group
           if (MODE == 0) {

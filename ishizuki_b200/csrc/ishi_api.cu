@@ -35,6 +35,7 @@ const FragOps *frag_ops_iq1s();
 const FragOps *frag_ops_iq1m();
 const FragOps *frag_ops_ggml_a(int type);
 const FragOps *frag_ops_ggml_b(int type);
+const FragOps *frag_ops_affine8(int group_size, bool bf16);
 const FragOps *frag_ops_affine4(int group_size, bool bf16);
 const FragOps *frag_ops_affine2(int group_size, bool bf16);
 const RowOps *row_ops_ggml(int type);
@@ -430,6 +431,7 @@ const FragOps *frag_ops_for(const ishi_weight_desc &d) {
   }
   if (d.scale_dtype != ISHI_DT_F16 && d.scale_dtype != ISHI_DT_BF16) return nullptr;
   const bool bf16 = d.scale_dtype == ISHI_DT_BF16;
+  if (d.bits == 8) return frag_ops_affine8(d.group_size, bf16);
   if (d.bits == 4) return frag_ops_affine4(d.group_size, bf16);
   if (d.bits == 2) return frag_ops_affine2(d.group_size, bf16);
   return nullptr;
@@ -1052,6 +1054,9 @@ static ishi_status create_projection(ishi_ctx *ctx, const ishi_weight_desc *desc
     wb += part;
     n_total += b.n;
   }
+  // (8-bit packs are not stacked, an interface the callers know: they run on the warp-level kernel alone)
+  if (count > 1 && descs[0].kind == ISHI_KIND_AFFINE && descs[0].bits == 8)
+    return fail(ctx, ISHI_E_UNSUPPORTED, "8-bit packs cannot be stacked into one projection");
   if (gated && (count != 2 || descs[0].n != descs[1].n || (descs[0].n & 7)))
     return fail(ctx, ISHI_E_SHAPE, "a gated pair needs two weights of the same height, a multiple of 8");
   std::lock_guard<std::mutex> g(ctx->lock);

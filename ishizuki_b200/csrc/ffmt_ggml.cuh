@@ -46,9 +46,6 @@ struct FragGGML {
 
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 16u; }
 
-  // nothing to set up ahead of the dependency wait
-  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t) {}
-
   // Activations of the CTA's column range as they lie in x (rows past M as zeros). A warp task is
   // (unit, activation row): lane l loads and stores k = 8l .. 8l + 7. GGML blocks have no input rotation.
   static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {

@@ -20,10 +20,12 @@
 //
 // Fragment mapping as for IQ2_XS: a lane owns the sub-blocks (sixteen weights = two entries)
 // 4 j + t, j = 0..3, of rows g and g + 8. Both formats are tiled into one form, a word per sub-block
-// and row: index bytes of its two entries, their three high index bits (bits 16-18, 19-21), the
-// scale (bits 24-26), the entries' delta signs (bits 27, 28). Tile (16 rows x 256 k, 1056 bytes;
-// the blocks are 800 and 896): [2][lane][16 bytes] = for j = 2p, 2p + 1: the word of row g, of
-// row g + 8; then d of rows (g, g + 8) side by side.
+// and row, a half for each of its two entries: the index from bit 5 up, where a mask makes it a byte
+// offset into the grid, the delta's sign at bit 3 (one shift brings both to bits 15 and 31) and the
+// scale at bits 0 ... 2 of both halves. Tile (16 rows x 256 k, 1056 bytes; the blocks are 800 and 896):
+// [2][lane][16 bytes] = for j = 2p, 2p + 1: the word of row g, of row g + 8; then d of rows (g, g + 8)
+// side by side. The loop is bound by instruction issue: 17408 x 5120 at eight rows 17.4 us
+// with index bytes, high bits and scale in fields of their own, 16.3 us with this layout.
 //
 // Activations of a unit in shared memory: eight rows of 256 fp16 as they lie in x, the rows
 // umax * 512 + 16 bytes apart; behind all rows, per unit, the entry sums: [k-step][lane][hi hi | lo lo].
@@ -53,42 +55,31 @@ struct FragIQ1 {
   }
   static __device__ __forceinline__ uint32_t u16_at(const uint8_t *p) { return (uint32_t)p[0] | ((uint32_t)p[1] << 8); }
 
-  // byte `bi` of the word of sub-block sb of a block (see above)
-  static __device__ __forceinline__ uint8_t word_byte(const uint8_t *blk, int sb, int bi) {
-    const int ib = sb >> 1, l0 = 2 * (sb & 1);  // the 32-group, the first of the sub-block's two entries in it
+  // half e (entry e) of the word of sub-block sb of a block (see above)
+  static __device__ __forceinline__ uint16_t word_half(const uint8_t *blk, int sb, int e) {
+    const int ib = sb >> 1, l = 2 * (sb & 1) + e;  // the 32-group, the entry in it
     if (TYPE == 19) {
       const uint32_t qh = u16_at(blk + 34 + 2 * ib);
-      if (bi < 2) return blk[2 + 4 * ib + l0 + bi];
-      if (bi == 2) return (uint8_t)((qh >> (3 * l0)) & 63u);
-      return (uint8_t)(((qh >> 12) & 7u) | ((qh >> 15) << 3) | ((qh >> 15) << 4));
+      return (uint16_t)((((uint32_t)blk[2 + 4 * ib + l] | (((qh >> (3 * l)) & 7u) << 8)) << 5) | ((qh >> 15) << 3) | ((qh >> 12) & 7u));
     }
-    const uint32_t qhb = blk[32 + 2 * ib + (l0 >> 1)];  // low nibble: the first entry, high nibble: the second
-    if (bi < 2) return blk[4 * ib + l0 + bi];
-    if (bi == 2) return (uint8_t)((qhb & 7u) | (((qhb >> 4) & 7u) << 3));
+    const uint32_t nibble = ((uint32_t)blk[32 + 2 * ib + (l >> 1)] >> (4 * (l & 1))) & 15u;
     const uint32_t scale = (u16_at(blk + 48 + 2 * (ib >> 1)) >> (6 * (ib & 1) + 3 * (sb & 1))) & 7u;
-    return (uint8_t)(scale | (((qhb >> 3) & 1u) << 3) | (((qhb >> 7) & 1u) << 4));
-  }
-
-  static __device__ __forceinline__ uint8_t tile_byte(const FragSrc &s, long long p, int u, int b) {
-    if (b < kD) {
-      const int pc = b >> 9, lane = (b & 511) >> 4, i = b & 15;
-      const int g = lane >> 2, t = lane & 3, slot = i >> 2, bi = i & 3;
-      const long long row = p * kFragRows + g + 8 * (slot & 1);
-      if (row >= s.N) return 0;
-      return word_byte(block(s, row, u), 4 * (2 * pc + (slot >> 1)) + t, bi);
-    }
-    const int idx = b - kD;
-    const long long row = p * kFragRows + (idx >> 2) + 8 * ((idx >> 1) & 1);
-    if (row >= s.N) return 0;
-    const uint8_t *blk = block(s, row, u);
-    if (TYPE == 19) return blk[idx & 1];
-    const uint32_t s0 = u16_at(blk + 48), s1 = u16_at(blk + 50), s2 = u16_at(blk + 52), s3 = u16_at(blk + 54);
-    const uint32_t d = (s0 >> 12) | ((s1 >> 8) & 0x00f0u) | ((s2 >> 4) & 0x0f00u) | (s3 & 0xf000u);
-    return (uint8_t)(d >> (8 * (idx & 1)));
+    return (uint16_t)((((uint32_t)blk[4 * ib + l] | ((nibble & 7u) << 8)) << 5) | (nibble & 8u) | scale);
   }
 
   static __device__ __forceinline__ uint16_t tile_halfword(const FragSrc &s, long long p, int u, int hw) {
-    return (uint16_t)(tile_byte(s, p, u, 2 * hw) | ((uint32_t)tile_byte(s, p, u, 2 * hw + 1) << 8));
+    const int h = hw & 1;  // half of a word
+    if (hw < kD / 2) {
+      const int j = 2 * (hw >> 8) + ((hw >> 2) & 1), lane = (hw & 255) >> 3;
+      const long long row = p * kFragRows + (lane >> 2) + 8 * ((hw >> 1) & 1);
+      return row < s.N ? word_half(block(s, row, u), 4 * j + (lane & 3), h) : (uint16_t)0;
+    }
+    const long long row = p * kFragRows + ((hw - kD / 2) >> 1) + 8 * h;
+    if (row >= s.N) return 0;
+    const uint8_t *blk = block(s, row, u);
+    if (TYPE == 19) return (uint16_t)u16_at(blk);
+    const uint32_t s0 = u16_at(blk + 48), s1 = u16_at(blk + 50), s2 = u16_at(blk + 52), s3 = u16_at(blk + 54);
+    return (uint16_t)((s0 >> 12) | ((s1 >> 8) & 0x00f0u) | ((s2 >> 4) & 0x0f00u) | (s3 & 0xf000u));
   }
 
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 16u; }
@@ -97,13 +88,9 @@ struct FragIQ1 {
     return xfrag + (uint32_t)a.umax * 4096u + 128u + (uint32_t)u * 1024u;
   }
 
-  // the grid (each value + 128), set up ahead of the dependency wait; four consecutive threads
-  // store the four copies of an entry
-  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t tables) {
-    for (int i = threadIdx.x; i < 2048 * 4; i += blockDim.x) {
-      const uint64_t v = d_iq1s_grid[i >> 2] ^ 0x8080808080808080ull;
-      sts64(tables + (uint32_t)i * 8u, (uint32_t)v, (uint32_t)(v >> 32));
-    }
+  // word i of the grid: entry i / 8's eight values, each + 128, in four copies side by side
+  static __device__ __forceinline__ uint32_t table_word(int i) {
+    return (uint32_t)((d_iq1s_grid[i >> 3] ^ 0x8080808080808080ull) >> (32 * (i & 1)));
   }
 
   // Activations of the CTA's column range as they lie in x (rows past M as zeros), and per entry
@@ -146,10 +133,10 @@ struct FragIQ1 {
     }
   }
 
-  // eight weights as four A registers, value * (2 s + 1): the grid index (this lane's copy of the
-  // grid), scale = 2 s + 1 and offset = -1152 * (2 s + 1) in both halves
-  static __device__ __forceinline__ void entry(uint32_t (&r)[4], uint32_t index, uint32_t grid, __half2 scale, __half2 offset) {
-    const uint2 m = lds64(grid + index * 32u);
+  // eight weights as four A registers, value * (2 s + 1): address of the grid entry (this lane's
+  // copy), scale = 2 s + 1 and offset = -1152 * (2 s + 1) in both halves
+  static __device__ __forceinline__ void entry(uint32_t *r, uint32_t at, __half2 scale, __half2 offset) {
+    const uint2 m = lds64(at);
     const uint32_t bits[4] = {prmt(m.x, 0x64646464u, 0x4140u), prmt(m.x, 0x64646464u, 0x4342u), prmt(m.y, 0x64646464u, 0x4140u),
                               prmt(m.y, 0x64646464u, 0x4342u)};
 #pragma unroll
@@ -158,13 +145,23 @@ struct FragIQ1 {
       r[i] = *reinterpret_cast<const uint32_t *>(&v);
     }
   }
+  // a word's sixteen weights as eight A registers (`copy`: byte offset of this lane's copy of the
+  // grid), and its entries' +-(2 s + 1)
+  static __device__ __forceinline__ uint32_t sub_block(uint32_t (&r)[8], uint32_t w, uint32_t grid, uint32_t copy) {
+    const uint32_t bits = (w & 0x00070007u) | 0x64006400u;  // 1024 + s
+    const __half2 scale = __hfma2(*reinterpret_cast<const __half2 *>(&bits), __float2half2_rn(2.f), __float2half2_rn(-2047.f));
+    const __half2 offset = __hmul2(scale, __float2half2_rn(-1152.f));
+    entry(r, grid + ((w & 0xffe0u) | copy), scale, offset);
+    entry(r + 4, grid + (((w >> 16) & 0xffe0u) | copy), scale, offset);
+    return *reinterpret_cast<const uint32_t *>(&scale) ^ ((w << 12) & 0x80008000u);
+  }
 
   // One tile against the activations of its unit; acc is the warp's C fragment.
   template <int MODE, int NB>
   static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
                                               uint32_t tables, int uq, int g, int t, int lane) {
     const uint32_t R = row_stride(a);
-    const uint32_t grid = tables + (uint32_t)(lane & 3) * 8u;
+    const uint32_t copy = (uint32_t)(lane & 3) * 8u;
     const uint32_t xrow = xbase + (uint32_t)g * R + (uint32_t)uq * 512u + (uint32_t)t * 32u;
     float c[NB][4];
     uint32_t da[2][4];  // the A registers of the two k-steps over the entries: +-(2 s + 1)
@@ -174,30 +171,20 @@ struct FragIQ1 {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int j = 2 * pc + e;
-        const uint32_t q0 = e ? w.z : w.x, q1 = e ? w.w : w.y;  // the sub-block's word of row g, of row g + 8
-        uint32_t lo0[4], hi0[4], lo1[4], hi1[4];
-        const uint32_t b0 = ((q0 >> 24) & 7u) * 0x00020002u + 0x64016401u, b1 = ((q1 >> 24) & 7u) * 0x00020002u + 0x64016401u;
-        const __half2 s0 = __hsub2(*reinterpret_cast<const __half2 *>(&b0), __float2half2_rn(1024.f));
-        const __half2 s1 = __hsub2(*reinterpret_cast<const __half2 *>(&b1), __float2half2_rn(1024.f));
-        const __half2 o0 = __hmul2(s0, __float2half2_rn(-1152.f)), o1 = __hmul2(s1, __float2half2_rn(-1152.f));
-        entry(lo0, (q0 & 0xffu) | ((q0 >> 8) & 0x700u), grid, s0, o0);
-        entry(hi0, ((q0 >> 8) & 0xffu) | ((q0 >> 11) & 0x700u), grid, s0, o0);
-        entry(lo1, (q1 & 0xffu) | ((q1 >> 8) & 0x700u), grid, s1, o1);
-        entry(hi1, ((q1 >> 8) & 0xffu) | ((q1 >> 11) & 0x700u), grid, s1, o1);
-        // the two entries' +-(2 s + 1): the delta's sign bits 27 and 28 to bits 15 and 31
-        da[j >> 1][(j & 1) * 2] = *reinterpret_cast<const uint32_t *>(&s0) ^ (((q0 >> 12) & 0x8000u) | ((q0 << 3) & 0x80000000u));
-        da[j >> 1][(j & 1) * 2 + 1] = *reinterpret_cast<const uint32_t *>(&s1) ^ (((q1 >> 12) & 0x8000u) | ((q1 << 3) & 0x80000000u));
+        uint32_t r0[8], r1[8];  // sub-block 4 j + t of row g, of row g + 8
+        da[j >> 1][(j & 1) * 2] = sub_block(r0, e ? w.z : w.x, tables, copy);
+        da[j >> 1][(j & 1) * 2 + 1] = sub_block(r1, e ? w.w : w.y, tables, copy);
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
           const uint32_t xj = xrow + nb * a.xregion + (uint32_t)j * 128u;
           const uint4 x0 = lds128(xj), x1 = lds128(xj + 16u);
           if (j == 0)
-            mma16816_first(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
+            mma16816_first(c[nb], r0[0], r1[0], r0[1], r1[1], x0.x, x0.y);
           else
-            mma16816(c[nb], lo0[0], lo1[0], lo0[1], lo1[1], x0.x, x0.y);
-          mma16816(c[nb], lo0[2], lo1[2], lo0[3], lo1[3], x0.z, x0.w);
-          mma16816(c[nb], hi0[0], hi1[0], hi0[1], hi1[1], x1.x, x1.y);
-          mma16816(c[nb], hi0[2], hi1[2], hi0[3], hi1[3], x1.z, x1.w);
+            mma16816(c[nb], r0[0], r1[0], r0[1], r1[1], x0.x, x0.y);
+          mma16816(c[nb], r0[2], r1[2], r0[3], r1[3], x0.z, x0.w);
+          mma16816(c[nb], r0[4], r1[4], r0[5], r1[5], x1.x, x1.y);
+          mma16816(c[nb], r0[6], r1[6], r0[7], r1[7], x1.z, x1.w);
         }
       }
     }

@@ -65,13 +65,11 @@ struct FragIQ4XS {
     return (uint16_t)(tile_byte(s, p, u, 2 * hw) | ((uint32_t)tile_byte(s, p, u, 2 * hw + 1) << 8));
   }
 
-  // the pair table, filled ahead of the dependency wait: it depends on no earlier launch
-  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t tables) {
-    for (int i = threadIdx.x; i < 256 * 32; i += blockDim.x) {
-      const int e = i >> 5;  // consecutive threads store one entry's 32 copies: consecutive banks
-      const __half2 pair = __halves2half2(__int2half_rn((int)d_kvalues_iq4nl[e & 15]), __int2half_rn((int)d_kvalues_iq4nl[e >> 4]));
-      sts32(tables + (uint32_t)i * 4u, *reinterpret_cast<const uint32_t *>(&pair));
-    }
+  // word i of the pair table: byte i / 32's two values as fp16, a copy per lane
+  static __device__ __forceinline__ uint32_t table_word(int i) {
+    const int e = i >> 5;
+    const __half2 pair = __halves2half2(__int2half_rn((int)d_kvalues_iq4nl[e & 15]), __int2half_rn((int)d_kvalues_iq4nl[e >> 4]));
+    return *reinterpret_cast<const uint32_t *>(&pair);
   }
 
   // Activations of the CTA's column range into fragment order. A warp task is (unit, activation

@@ -66,9 +66,6 @@ struct FragQ2K {
     return (uint16_t)(tile_byte(s, p, u, 2 * hw) | ((uint32_t)tile_byte(s, p, u, 2 * hw + 1) << 8));
   }
 
-  // nothing to set up ahead of the dependency wait
-  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t) {}
-
   // Activations of the CTA's column range into fragment order. A warp task is (unit, activation
   // row r): lane l loads k = 8l .. 8l + 7: half n = l / 16, shift j = (l / 4) % 4, h = (l % 4) / 2,
   // the weights l % 16 = 8 (l % 2) ... + 7 of sub-block is = 8 n + 2 j + h, i.e. what lanes

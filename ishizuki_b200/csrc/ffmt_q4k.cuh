@@ -103,9 +103,6 @@ struct FragQ4K {
   // every sub-block for the minimum term. Q4_K has no input rotation.
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
-  // nothing to set up ahead of the dependency wait
-  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t) {}
-
   static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const uint32_t R = row_stride(a), sums = xfrag + 8u * R;

@@ -14,23 +14,23 @@
 // MMA whose k index runs over the groups, against the group sums of x.
 //
 // A 6-bit value masked in place at bits 0..5 of each half of a register is the bit pattern of the
-// fp16 number q * 2^-24; at bits 4..9 it is q * 2^-20 (both subnormal, hence linear in q). The tile
-// stores the nibbles and the bit pairs where those masks find them:
-//   a pair of k-steps (2i, 2i + 1) takes, per lane, one nibble word per weight row (X1: row g,
-//   X2: row g + 8) and one word H of sixteen bit pairs. With Y = X >> 8, the k-step 2i uses
-//   (X1, X2, Y1, Y2) & 0x000f000f as its four A registers and the k-step 2i + 1 uses the same words
-//   & 0x00f000f0 (sixteen times too large; its scale is divided by 16). The high bits come from H
-//   rotated right by 0, 2, 8 and 10: each rotation lines one pair of fields up with mask
-//   0x00300030 (first k-step) and another with 0x03000300 (second k-step), so a register costs two
-//   bit operations: (X & m) | (rot(H) & c).
+// fp16 number q * 2^-24; at bits 4..9 it is q * 2^-20 (both subnormal, hence linear in q). A pair of
+// k-steps (2i, 2i + 1) takes eight A registers per lane, sixteen values, and they lie in three words:
+// each half of a word has one value at bits 4..9 (a register for one mask), one at bits 10..15 (a shift
+// and a mask) and four bits below; the low nibbles of the first k-step's row g are those of words 0
+// and 1, their high bit pairs bits 0..1 and 2..3 of word 2. That is fifteen bit operations for eight
+// registers, where nibbles and bit pairs in words of their own take twenty-one. The row whose values
+// lie at bits 0..5 has its own sums, in units of 2^-24; all others are sixteen times as large.
+// The loop is bound by the integer pipe and by memory in equal parts: 17408 x 5120 at eight
+// rows 19.1 -> 16.7 us, 587 -> 498 warp instructions a tile; 248320 x 5120 213 -> 182 us, 5.7 TB/s.
 // Inside a k-step the lane t holds the weights 4t .. 4t + 3 of the group: slots (2t, 2t + 1) are
 // 4t, 4t + 1 and slots (2t + 8, 2t + 9) are 4t + 2, 4t + 3; the activations are staged in the same
 // order, so that a lane reads the B registers of two k-steps with one 16-byte load.
 //
-// Tile (16 rows x 256 k, 3360 bytes = 16 * 210): nibble words [4][lane][X1 X2 | X1' X2'] @0,
-// bit-pair words [4][lane][H H'] @2048, per row the sixteen scales @3072 in the order
-// (2t, 2t + 1, 2t + 8, 2t + 9) for t = 0..3 (a lane's A registers of the group-sum MMA are then one
-// word), and d of rows (g, g + 8) side by side @3328.
+// Tile (16 rows x 256 k, 3360 bytes = 16 * 210): [6][lane][16 bytes] = the lane's words 3 i + w of
+// pair i, four at a time; per row the sixteen scales + 128 @3072 in the order (2t, 2t + 1, 2t + 8,
+// 2t + 9) for t = 0..3 (a lane's A registers of the group-sum MMA are then one word), and d of rows
+// (g, g + 8) side by side @3328.
 #pragma once
 #include "ishi_fragstream.cuh"
 
@@ -58,62 +58,35 @@ struct FragQ6K {
     return s.w[seg] + local * s.w_row_bytes + (long long)u * 210;
   }
 
-  static __device__ __forceinline__ uint8_t tile_byte(const FragSrc &s, long long p, int u, int b) {
-    if (b < 2048) {
-      const int pp = b >> 9, lane = (b & 511) >> 4, i = b & 15;
-      const int g = lane >> 2, t = lane & 3, w = i >> 2, bi = i & 3;
-      const long long row = p * kFragRows + g + 8 * (w & 1);
-      if (row >= s.N) return 0;
-      const uint8_t *blk = block(s, row, u);
-      const int pi = 2 * pp + (w >> 1);
-      uint32_t out = 0;
-      for (int e = 0; e < 2; ++e) {
-        const int n = 2 * bi + e;  // nibble of the word
-        const int ks = 2 * pi + (n & 1), kk = 4 * t + 2 * ((n >> 1) & 1) + (n >> 2);
-        out |= (code(blk, 16 * ks + kk) & 15u) << (4 * e);
-      }
-      return (uint8_t)out;
-    }
-    if (b < 3072) {
-      const int idx = b - 2048, pp = idx >> 8, lane = (idx & 255) >> 3, i = idx & 7;
-      const int g = lane >> 2, t = lane & 3, pi = 2 * pp + (i >> 2), bi = i & 3;
-      uint32_t out = 0;
-      for (int e = 0; e < 4; ++e) {
-        const int pos = 8 * bi + 2 * e;  // bit position of the field in H
-        // which register's half the field feeds: rotation r lines positions 4 + r, 20 + r (first
-        // k-step) and 8 + r, 24 + r (second) up with the masks; r = 0, 2 serve row g (X, Y), 8, 10 row g + 8
-        int second, y, x2, half;
-        const int q = pos & 15;  // position modulo the halves
-        if (q == 4 || q == 6) second = 0, x2 = 0, y = q == 6, half = pos >> 4;
-        else if (q == 8 || q == 10) second = 1, x2 = 0, y = q == 10, half = pos >> 4;
-        else if (q == 12 || q == 14) second = 0, x2 = 1, y = q == 14, half = pos >> 4;
-        else second = 1, x2 = 1, y = q == 2, half = 1 - (pos >> 4);  // positions 16, 18 | 0, 2: rotated across the halves
-        const long long row = p * kFragRows + g + 8 * x2;
-        if (row >= s.N) continue;
-        const int ks = 2 * pi + second, kk = 4 * t + 2 * y + half;
-        out |= (code(block(s, row, u), 16 * ks + kk) >> 4) << (2 * e);
-      }
-      return (uint8_t)out;
-    }
-    if (b < 3328) {
-      const int idx = b - 3072, j = idx & 15;
-      const long long row = p * kFragRows + (idx >> 4);
-      if (row >= s.N) return 0;
-      const int ks = 2 * (j >> 2) + (j & 1) + 8 * ((j >> 1) & 1);
-      return block(s, row, u)[192 + ks];
-    }
-    const int idx = b - 3328;
-    const long long row = p * kFragRows + (idx >> 2) + 8 * ((idx >> 1) & 1);
-    if (row >= s.N) return 0;
-    return block(s, row, u)[208 + (idx & 1)];
-  }
-
   static __device__ __forceinline__ uint16_t tile_halfword(const FragSrc &s, long long p, int u, int hw) {
-    return (uint16_t)(tile_byte(s, p, u, 2 * hw) | ((uint32_t)tile_byte(s, p, u, 2 * hw + 1) << 8));
+    const int h = hw & 1;  // half of a word
+    if (hw < 1536) {
+      const int lane = (hw & 255) >> 3, word = 4 * (hw >> 8) + ((hw & 7) >> 1), pi = word / 3, w = word - 3 * pi;
+      const int g = lane >> 2, t = lane & 3;
+      // value of k-step 2 pi + second, row g or g + 8, slots (2t, 2t + 1) or (2t + 8, 2t + 9), half h
+      auto value = [&](int second, int below, int y) -> uint32_t {
+        const long long row = p * kFragRows + g + 8 * below;
+        return row < s.N ? code(block(s, row, u), 16 * (2 * pi + second) + 4 * t + 2 * y + h) : 0u;
+      };
+      const uint32_t a0 = value(0, 0, 0), a2 = value(0, 0, 1);
+      uint32_t out;
+      if (w == 0) out = (a0 & 15u) | (value(0, 1, 0) << 4) | (value(0, 1, 1) << 10);
+      else if (w == 1) out = (a2 & 15u) | (value(1, 0, 0) << 4) | (value(1, 1, 0) << 10);
+      else out = (a0 >> 4) | ((a2 >> 4) << 2) | (value(1, 0, 1) << 4) | (value(1, 1, 1) << 10);
+      return (uint16_t)out;
+    }
+    if (hw < 1664) {
+      const int row16 = (hw - 1536) >> 3, pair = (hw - 1536) & 7;  // scales 2 (pair / 2) + 8 (pair % 2) and the next
+      const long long row = p * kFragRows + row16;
+      if (row >= s.N) return 0;
+      const uint8_t *sc = block(s, row, u) + 192 + 2 * (pair >> 1) + 8 * (pair & 1);
+      return (uint16_t)(((uint32_t)sc[0] | ((uint32_t)sc[1] << 8)) ^ 0x8080u);
+    }
+    const long long row = p * kFragRows + ((hw - 1664) >> 1) + 8 * h;
+    if (row >= s.N) return 0;
+    const uint8_t *blk = block(s, row, u);
+    return (uint16_t)((uint32_t)blk[208] | ((uint32_t)blk[209] << 8));
   }
-
-  // nothing to set up ahead of the dependency wait
-  static __device__ __forceinline__ void before_wait(const FragArgs &, uint32_t) {}
 
   // Activations of the CTA's column range into fragment order. A warp task is (unit, activation
   // row r): lane l loads k = 8l .. 8l + 7, half of group l / 2, i.e. what lanes t = 2(l & 1) and
@@ -163,12 +136,13 @@ struct FragQ6K {
     }
   }
 
+  // byte `byte` of a word of scales + 128 as the scale: the low mantissa bits of 2^23
   static __device__ __forceinline__ float scale_of(uint32_t word, int byte) {
-    return (float)(int)(int8_t)(word >> (8 * byte));
+    return __uint_as_float(prmt(word, 0x4b000000u, 0x7650u + (uint32_t)byte)) - 8388736.f;
   }
-  // two int8 of a word (already xor 0x80 per byte) as a half2: the bits of 1024 + 128 + b, minus 1152
-  static __device__ __forceinline__ uint32_t scale_pair(uint32_t biased, uint32_t selector) {
-    const uint32_t bits = prmt(biased, 0x64646464u, selector);
+  // two of its bytes as a half2: the low mantissa bits of 1024
+  static __device__ __forceinline__ uint32_t scale_pair(uint32_t word, uint32_t selector) {
+    const uint32_t bits = prmt(word, 0x64646464u, selector);
     const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&bits), __float2half2_rn(1152.f));
     return *reinterpret_cast<const uint32_t *>(&v);
   }
@@ -181,43 +155,43 @@ struct FragQ6K {
     const uint4 h0 = lds128(tile + 3072u + (uint32_t)g * 16u), h1 = lds128(tile + 3072u + (uint32_t)(g + 8) * 16u);
     const uint32_t hw0[4] = {h0.x, h0.y, h0.z, h0.w}, hw1[4] = {h1.x, h1.y, h1.z, h1.w};
     const uint32_t lane_off = (uint32_t)g * 64u + (uint32_t)t * 16u;
-    float su[NB][4];
+    float su[NB][2], sv[NB][4];  // first k-steps of row g; all others, sixteen times as large
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = su[nb][2] = su[nb][3] = 0.f;
+    for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = sv[nb][0] = sv[nb][1] = sv[nb][2] = sv[nb][3] = 0.f;
+    uint32_t qw[12];  // the words of four pairs
 #pragma unroll
-    for (int pp = 0; pp < 4; ++pp) {
-      const uint4 q = lds128(tile + (uint32_t)pp * 512u + (uint32_t)lane * 16u);
-      const uint2 hh = lds64(tile + 2048u + (uint32_t)pp * 256u + (uint32_t)lane * 8u);
+    for (int pi = 0; pi < 8; ++pi) {
+      if ((pi & 3) == 0) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int pi = 2 * pp + e;
-        const uint32_t x1 = e ? q.z : q.x, x2 = e ? q.w : q.y, h = e ? hh.y : hh.x;
-        const uint32_t y1 = x1 >> 8, y2 = x2 >> 8;
-        const uint32_t r2 = __funnelshift_r(h, h, 2), r8 = __funnelshift_r(h, h, 8), r10 = __funnelshift_r(h, h, 10);
-        const uint32_t a0 = (x1 & 0x000f000fu) | (h & 0x00300030u), a1 = (x2 & 0x000f000fu) | (r8 & 0x00300030u);
-        const uint32_t a2 = (y1 & 0x000f000fu) | (r2 & 0x00300030u), a3 = (y2 & 0x000f000fu) | (r10 & 0x00300030u);
-        const uint32_t e0 = (x1 & 0x00f000f0u) | (h & 0x03000300u), e1 = (x2 & 0x00f000f0u) | (r8 & 0x03000300u);
-        const uint32_t e2 = (y1 & 0x00f000f0u) | (r2 & 0x03000300u), e3 = (y2 & 0x00f000f0u) | (r10 & 0x03000300u);
-        // scales of groups 2 pi and 2 pi + 1: word pi % 4 of the row's sixteen, bytes 2 (pi / 4) and + 1
-        const float s00 = scale_of(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1) * 0.0625f;
-        const float s10 = scale_of(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1) * 0.0625f;
-#pragma unroll
-        for (int nb = 0; nb < NB; ++nb) {
-          const uint4 b = lds128(xu + nb * a.xregion + (uint32_t)pi * 512u + (lane_off ^ (uint32_t)(pi << 6)));
-          float c0[4], c1[4];
-          mma16816_first(c0, a0, a1, a2, a3, b.x, b.y);
-          mma16816_first(c1, e0, e1, e2, e3, b.z, b.w);
-          su[nb][0] = fmaf(s00, c0[0], su[nb][0]), su[nb][1] = fmaf(s00, c0[1], su[nb][1]);
-          su[nb][2] = fmaf(s10, c0[2], su[nb][2]), su[nb][3] = fmaf(s10, c0[3], su[nb][3]);
-          su[nb][0] = fmaf(s01, c1[0], su[nb][0]), su[nb][1] = fmaf(s01, c1[1], su[nb][1]);
-          su[nb][2] = fmaf(s11, c1[2], su[nb][2]), su[nb][3] = fmaf(s11, c1[3], su[nb][3]);
+        for (int i = 0; i < 3; ++i) {
+          const uint4 q = lds128(tile + (uint32_t)(3 * (pi >> 2) + i) * 512u + (uint32_t)lane * 16u);
+          qw[4 * i] = q.x, qw[4 * i + 1] = q.y, qw[4 * i + 2] = q.z, qw[4 * i + 3] = q.w;
         }
+      }
+      const uint32_t w0 = qw[3 * (pi & 3)], w1 = qw[3 * (pi & 3) + 1], w2 = qw[3 * (pi & 3) + 2];
+      const uint32_t a0 = (w0 & 0x000f000fu) | ((w2 << 4) & 0x00300030u), a2 = (w1 & 0x000f000fu) | ((w2 << 2) & 0x00300030u);
+      const uint32_t a1 = w0 & 0x03f003f0u, a3 = (w0 >> 6) & 0x03f003f0u;
+      const uint32_t e0 = w1 & 0x03f003f0u, e1 = (w1 >> 6) & 0x03f003f0u;
+      const uint32_t e2 = w2 & 0x03f003f0u, e3 = (w2 >> 6) & 0x03f003f0u;
+      // scales of groups 2 pi and 2 pi + 1: word pi % 4 of the row's sixteen, bytes 2 (pi / 4) and + 1
+      const float s00 = scale_of(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1);
+      const float s10 = scale_of(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1);
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) {
+        const uint4 b = lds128(xu + nb * a.xregion + (uint32_t)pi * 512u + (lane_off ^ (uint32_t)(pi << 6)));
+        float c0[4], c1[4];
+        mma16816_first(c0, a0, a1, a2, a3, b.x, b.y);
+        mma16816_first(c1, e0, e1, e2, e3, b.z, b.w);
+        su[nb][0] = fmaf(s00, c0[0], su[nb][0]), su[nb][1] = fmaf(s00, c0[1], su[nb][1]);
+        sv[nb][2] = fmaf(s10, c0[2], sv[nb][2]), sv[nb][3] = fmaf(s10, c0[3], sv[nb][3]);
+        sv[nb][0] = fmaf(s01, c1[0], sv[nb][0]), sv[nb][1] = fmaf(s01, c1[1], sv[nb][1]);
+        sv[nb][2] = fmaf(s11, c1[2], sv[nb][2]), sv[nb][3] = fmaf(s11, c1[3], sv[nb][3]);
       }
     }
     // sum_g scale_g * (sum of x over group g): the MMA over groups; this lane's slots are groups
     // 2t, 2t + 1, 2t + 8, 2t + 9, the word t of each row's scales
-    const uint32_t w0 = (t == 0 ? h0.x : t == 1 ? h0.y : t == 2 ? h0.z : h0.w) ^ 0x80808080u;
-    const uint32_t w1 = (t == 0 ? h1.x : t == 1 ? h1.y : t == 2 ? h1.z : h1.w) ^ 0x80808080u;
+    const uint32_t w0 = (t == 0 ? h0.x : t == 1 ? h0.y : t == 2 ? h0.z : h0.w);
+    const uint32_t w1 = (t == 0 ? h1.x : t == 1 ? h1.y : t == 2 ? h1.z : h1.w);
     const uint32_t a0 = scale_pair(w0, 0x4140u), a1 = scale_pair(w1, 0x4140u);
     const uint32_t a2 = scale_pair(w0, 0x4342u), a3 = scale_pair(w1, 0x4342u);
     const uint32_t dd = lds32(tile + 3328u + (uint32_t)g * 4u);
@@ -229,10 +203,10 @@ struct FragQ6K {
       float cm[4];
       mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
       mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);
-      acc[nb][0] = fmaf(d0, su[nb][0], fmaf(dm0, cm[0], acc[nb][0]));
-      acc[nb][1] = fmaf(d0, su[nb][1], fmaf(dm0, cm[1], acc[nb][1]));
-      acc[nb][2] = fmaf(d1, su[nb][2], fmaf(dm1, cm[2], acc[nb][2]));
-      acc[nb][3] = fmaf(d1, su[nb][3], fmaf(dm1, cm[3], acc[nb][3]));
+      acc[nb][0] = fmaf(d0, fmaf(sv[nb][0], 0.0625f, su[nb][0]), fmaf(dm0, cm[0], acc[nb][0]));
+      acc[nb][1] = fmaf(d0, fmaf(sv[nb][1], 0.0625f, su[nb][1]), fmaf(dm0, cm[1], acc[nb][1]));
+      acc[nb][2] = fmaf(d1 * 0.0625f, sv[nb][2], fmaf(dm1, cm[2], acc[nb][2]));
+      acc[nb][3] = fmaf(d1 * 0.0625f, sv[nb][3], fmaf(dm1, cm[3], acc[nb][3]));
     }
   }
 };

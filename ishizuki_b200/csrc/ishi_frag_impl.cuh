@@ -29,6 +29,17 @@ struct FragOpsOf {
             const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
             if (e != cudaSuccess) return e;
           }
+    if constexpr (Fmt::kExtraBytes > 0) {
+      // on a stream of its own: other threads may be using the default stream
+      cudaStream_t st = nullptr;
+      cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+      if (e != cudaSuccess) return e;
+      fill_table_kernel<Fmt><<<32, 256, 0, st>>>();
+      e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      cudaStreamDestroy(st);
+      return e;
+    }
     return cudaSuccess;
   }
 

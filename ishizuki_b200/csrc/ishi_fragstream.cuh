@@ -350,6 +350,18 @@ __device__ __forceinline__ void st_async128(uint32_t addr, float4 v, uint32_t mb
                : "memory");
 }
 
+// A decoder's shared-memory tables (kExtraBytes, a multiple of 16), laid out once per device from
+// Fmt::table_word; every CTA copies them from here, a few 16-byte async copies per thread that land
+// while it waits for the launch before. Building them in place, lookups and conversions ahead of the
+// activations, cost a launch 0.8 us more (IQ4_XS, 17408 x 5120).
+template <class Fmt>
+__device__ __align__(16) uint8_t frag_table[Fmt::kExtraBytes ? Fmt::kExtraBytes : 16];
+template <class Fmt>
+__global__ void fill_table_kernel() {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Fmt::kExtraBytes / 4; i += gridDim.x * blockDim.x)
+    reinterpret_cast<uint32_t *>(frag_table<Fmt>)[i] = Fmt::table_word(i);
+}
+
 // MODE 0: tensor-core (up to eight rows per column group); MODE 1: CUDA-core FMA for a single row.
 // MAXW: most warps of a block. NB: column groups of eight activation rows, 1 or 2.
 template <class Fmt, int MODE, int MAXW, int NB>
@@ -407,6 +419,11 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   // barriers: every CTA arrives here, and a warp waits before its first partial panel.
   if (S > 1) cluster_arrive_relaxed();  // the init fence above is what the peers need; nothing else to publish yet
 
+  if (Fmt::kExtraBytes) {
+    for (int i = threadIdx.x * 16; i < Fmt::kExtraBytes; i += blockDim.x * 16) cp_async16(tables + i, frag_table<Fmt> + i);
+    cp_async_commit();
+  }
+
   // This warp's run of tiles. The fetch cursor runs R - 1 tiles ahead of the compute cursor: a tile is
   // fetched into the slot of the tile decoded last. One commit group per tile, empty past the end.
   int f_left = t1 - t0, f_u = t0 - q0 * uc;
@@ -427,8 +444,6 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   // The weight tiles are written by no earlier kernel: their first copies go out at once. (Asking
   // the run's next tiles into L2 as well delays the activations behind them: 60 -> 66 us per layer.)
   for (int i = 0; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride);
-
-  Fmt::before_wait(a, tables);  // tables that do not depend on earlier launches
 
   // Warm L2 and the address translation with this CTA's slice of x. Only a hint: x may still be
   // written by the kernel before this one, its values are read after the wait below, through L2.
@@ -464,6 +479,11 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   for (int b = 0; b < NB; ++b)
     Fmt::stage_x(a, a.x + (long long)(8 * b) * a.K, a.M - 8 * b, xfrag + b * a.xregion, ub0, uc);
   ISHI_STAMP(3);
+  if (Fmt::kExtraBytes) {  // the tables have landed: all groups but the R - 1 tiles' behind them
+    if (R == 2) cp_async_wait<1>();
+    else if (R == 3) cp_async_wait<2>();
+    else cp_async_wait<3>();
+  }
   __syncthreads();  // staged, and the control block is set up for every warp
   ISHI_STAMP(4);
   // shared-memory loads are plain asm the compiler may move; tie their addresses to the waits

@@ -22,7 +22,7 @@ struct FragLaunch {
 struct FragOps {
   int tile_bytes;
   int x_bytes, x_fixed, x_extra;  // a staged region of eight rows: bytes per unit of the column range, once; tables per CTA
-  // raises the dynamic shared memory limit of every variant (once per device)
+  // raises the dynamic shared memory limit of every variant and lays out the decoder's tables (once per device; synchronises)
   cudaError_t (*configure)(int max_smem);
   // how many clusters of `split` CTAs the device keeps resident, 0 if the launch is impossible; groups: of eight rows
   int (*max_clusters)(int split, int warps, int groups, size_t smem, int sm_count);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <array>
 #include <cstdarg>
 #include <cstdio>
@@ -120,6 +121,7 @@ struct ishi_projection {
   Workspace ws;          // this projection's own scratch and tiled weight: apply never allocates
   __half *xr = nullptr;  // rotated activations [16][k] when the pack is rotated
   __half *host_x = nullptr, *host_y = nullptr;  // device staging of apply_host_async: [16][k], [16][n]
+  unsigned long long host_batch = 0;            // the last (part of a) host batch it was in
   int64_t weight_bytes = 0;
 };
 
@@ -590,7 +592,7 @@ bool single_row_on_cuda_cores(const ishi_ctx *ctx) {
 // rows 1...16 through the warp-level kernel; gemv picks the CUDA-core variant for a single row
 ishi_status run_frag(ishi_ctx *ctx, const FragPlans &plans, const Workspace &ws, const ishi_weight_desc &d, const void *x,
                      int rows, void *y, long long ldy, int flags, bool gemv, bool early, bool rotate, cudaStream_t st,
-                     const PeerOut *peers = nullptr, bool gated = false) {
+                     const PeerOut *peers = nullptr, bool gated = false, bool release_late = false) {
   const bool whole = rows <= 8 || plans.many.ok;  // one launch, or pieces of eight rows
   for (int r0 = 0; r0 < rows; r0 += whole ? 16 : 8) {
     const FragPlan &pl = whole && rows > 8 ? plans.many : plans.few;
@@ -620,6 +622,7 @@ ishi_status run_frag(ishi_ctx *ctx, const FragPlans &plans, const Workspace &ws,
     a.rot_block = rotate ? d.hadamard_block : 0;
     a.rot_signs = rotate ? static_cast<const float *>(d.signs_dev) : nullptr;
     a.swiglu = gated ? 1 : 0;
+    a.release_late = release_late ? 1 : 0;
 #ifdef ISHI_TRACE
     a.trace = g_trace;
 #endif
@@ -1286,6 +1289,119 @@ static ishi_status ensure_host_staging(ishi_projection *p) {
   return ISHI_OK;
 }
 
+static std::atomic<unsigned long long> g_host_batches{0};
+
+// the address under which kernels reach `bytes` bytes at p, or null: not mapped page-locked memory, or
+// not 16-byte aligned
+static void *mapped_address(const void *p, size_t bytes) {
+  cudaPointerAttributes first, last;
+  if (!aligned16(p) || cudaPointerGetAttributes(&first, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&last, static_cast<const uint8_t *>(p) + bytes - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
+      static_cast<uint8_t *>(first.devicePointer) + bytes - 1 != last.devicePointer)
+    return nullptr;
+  return first.devicePointer;
+}
+
+// the y copies of entries [c0, c1) behind what is on the caller's stream now
+static ishi_status host_batch_out(ishi_ctx *ctx, ishi_projection *const *ps, int rows, void *const *y_hosts, int c0, int c1,
+                                  cudaStream_t st) {
+  ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_done[c0], st));
+  ISHI_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, ctx->ev_done[c0], 0));
+  for (int i = c0; i < c1; ++i) {
+    const size_t yb = (size_t)rows * out_rows(ps[i]) * sizeof(__half);
+    ISHI_CUDA(ctx, cudaMemcpyAsync(y_hosts[i], ps[i]->host_y, yb, cudaMemcpyDeviceToHost, ctx->copy_out));
+  }
+  return ISHI_OK;
+}
+
+// The leading entries of a list without repeats whose products are the warp-level kernel's and whose
+// inputs kernels can reach: one chain of programmatic launches, in groups of products with a kernel
+// ahead of each that copies the group's inputs in while the last product of the group before runs, and
+// behind each the y copies on the copy stream. *done: entries enqueued.
+// The copying kernel does not wait for that product, and need not: the product releases it only when
+// everything before has completed (release_late), the last use of the inputs' staging included.
+// A group takes as many inputs as cross the bus meanwhile; the last groups are short (3, 1), their y
+// copies stand at the end. Four layers of the 27B shape at eight rows, 16 entries: 315 us with both
+// directions on the copy engines, 269 this way (products alone 228).
+static ishi_status host_batch_chain(ishi_ctx *ctx, ishi_projection *const *ps, const void *const *x_hosts, int rows,
+                                    void *const *y_hosts, int count, cudaStream_t st, int *done) {
+  const bool early = getenv("ISHI_NO_EARLY_LAUNCH") == nullptr, rotation = getenv("ISHI_NO_FUSED_ROTATION") == nullptr;
+  HostCopies in;
+  // the next group: entries whose inputs add up to `budget` bytes, at least one
+  auto take = [&](int first, long long budget) {
+    const int left = count - first, most = left > 4 ? left - 4 : left > 1 ? left - 1 : left;
+    in.wait = first == 0;
+    for (in.count = 0; in.count < std::min(kHostGroup, most); ++in.count) {
+      const ishi_projection *p = ps[first + in.count];
+      if (!p->frag.few.ok || (p->d.hadamard_block != 0 && !(rotation && rotates_in_kernel(p)))) return;
+      const unsigned bytes = (unsigned)(rows * p->d.k * sizeof(__half));
+      if (in.count > 0 && bytes > budget) return;
+      budget -= bytes;
+      in.src[in.count] = mapped_address(x_hosts[first + in.count], bytes);
+      in.dst[in.count] = p->host_x;
+      in.bytes[in.count] = bytes;
+      if (!in.src[in.count]) return;
+    }
+  };
+  int c0 = 0;
+  for (take(0, 0); in.count > 0;) {
+    ISHI_CUDA(ctx, launch_host_copies(in, st));
+    if (c0 > 0) {
+      ishi_status s = host_batch_out(ctx, ps, rows, y_hosts, *done, c0, st);
+      if (s != ISHI_OK) return s;
+    }
+    *done = c0;
+    const int c1 = c0 + in.count;
+    for (int i = c0; i < c1; ++i) {
+      const ishi_projection *p = ps[i];
+      ishi_status s = run_frag(ctx, p->frag, p->ws, p->d, p->host_x, rows, p->host_y, out_rows(p), 0, single_row_on_cuda_cores(ctx),
+                               early, p->d.hadamard_block != 0, st, nullptr, p->gated, i + 1 == c1);
+      if (s != ISHI_OK) return s;
+    }
+    // the last product takes about 4 us and its tiles at 5.5 TB/s, the bus moves 40 GB/s
+    take(c1, 160000 + (long long)(ps[c1 - 1]->frag.few.tiles_bytes / 140));
+    c0 = c1;
+  }
+  if (c0 == 0) return ISHI_OK;
+  ishi_status s = host_batch_out(ctx, ps, rows, y_hosts, *done, c0, st);
+  *done = c0;
+  return s;
+}
+
+// A list without repeats through the copy engines: x copies run ahead on one stream, the products follow
+// on the caller's stream as their inputs land, the y copies trail on a third. The lanes hand over in
+// chunks, not entry by entry: an event between two product kernels serialises them (about 2.5 us),
+// inside a chunk they follow each other with programmatic dependent launch as in a plain sequence of
+// applies. The chunks are short at both ends, where one lane waits for another (1, 3, then sixteen at a
+// time, then 3, 1): four layers of the 27B shape at eight rows, 16 entries, took 470 us as one chunk
+// and take 315 us in these.
+static ishi_status host_batch_lanes(ishi_ctx *ctx, ishi_projection *const *ps, const void *const *x_hosts, int rows,
+                                    void *const *y_hosts, int count, cudaStream_t st) {
+  ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_begin, st));
+  ISHI_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_in, ctx->ev_begin, 0));
+  for (int c0 = 0, c1 = 0; c0 < count; c0 = c1) {
+    const int left = count - c0, want = c0 == 0 ? 1 : c0 < 4 ? 3 : 16;
+    c1 = c0 + (left > 4 ? std::min(want, left - 4) : left > 1 ? std::min(want, left - 1) : 1);
+    for (int i = c0; i < c1; ++i) {
+      const size_t xb = (size_t)rows * ps[i]->d.k * sizeof(__half);
+      ISHI_CUDA(ctx, cudaMemcpyAsync(ps[i]->host_x, x_hosts[i], xb, cudaMemcpyHostToDevice, ctx->copy_in));
+    }
+    ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_in[c0], ctx->copy_in));
+    ISHI_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_in[c0], 0));
+    for (int i = c0; i < c1; ++i) {
+      ishi_status s = ishi_projection_apply(ps[i], ps[i]->host_x, rows, ps[i]->host_y, out_rows(ps[i]), 0, st);
+      if (s != ISHI_OK) return s;
+    }
+    ishi_status s = host_batch_out(ctx, ps, rows, y_hosts, c0, c1, st);
+    if (s != ISHI_OK) return s;
+  }
+  return ISHI_OK;
+}
+
 ishi_status ishi_projection_apply_host_batch(ishi_projection *const *ps, const void *const *x_hosts, int rows,
                                              void *const *y_hosts, int count, void *stream) {
   if (!ps || count < 1 || !ps[0]) return ISHI_E_INVALID;
@@ -1318,39 +1434,20 @@ ishi_status ishi_projection_apply_host_batch(ishi_projection *const *ps, const v
     ishi_status s = ensure_host_staging(ps[i]);
     if (s != ISHI_OK) return s;
   }
-  // Three lanes: x copies run ahead on one stream, the products follow on the caller's stream as
-  // their inputs land, the y copies trail on a third; the caller's stream ends behind all of them.
-  // The lanes hand over in chunks, not entry by entry: an event between two product kernels
-  // serialises them (about 2.5 us), inside a chunk they follow each other with programmatic dependent
-  // launch as in a plain sequence of applies. The chunks are short at both ends, where one lane waits
-  // for another (1, 3, then sixteen at a time, then 3, 1): four layers of the 27B shape at eight
-  // rows, 16 entries, took 470 us as one chunk, 75 of them before the first product and 110 after the
-  // last, and take 318 us now (products alone 220).
-  ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_begin, st));
-  ISHI_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_in, ctx->ev_begin, 0));
-  ISHI_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, ctx->ev_begin, 0));
-  for (int c0 = 0, c1 = 0; c0 < count; c0 = c1) {
-    const int left = count - c0, want = c0 == 0 ? 1 : c0 < 4 ? 3 : 16;
-    c1 = c0 + (left > 4 ? std::min(want, left - 4) : left > 1 ? std::min(want, left - 1) : 1);
-    for (int i = c0; i < c1; ++i) {
-      const size_t xb = (size_t)rows * ps[i]->d.k * sizeof(__half);
-      ISHI_CUDA(ctx, cudaMemcpyAsync(ps[i]->host_x, x_hosts[i], xb, cudaMemcpyHostToDevice, ctx->copy_in));
-    }
-    ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_in[c0], ctx->copy_in));
-    ISHI_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_in[c0], 0));
-    for (int i = c0; i < c1; ++i) {
-      ishi_status s = ishi_projection_apply(ps[i], ps[i]->host_x, rows, ps[i]->host_y, out_rows(ps[i]), 0, stream);
-      if (s != ISHI_OK) return s;
-    }
-    ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_done[c0], st));
-    ISHI_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, ctx->ev_done[c0], 0));
-    for (int i = c0; i < c1; ++i) {
-      const size_t yb = (size_t)rows * out_rows(ps[i]) * sizeof(__half);
-      ISHI_CUDA(ctx, cudaMemcpyAsync(y_hosts[i], ps[i]->host_y, yb, cudaMemcpyDeviceToHost, ctx->copy_out));
-    }
+  // A projection's staging serves one entry at a time: a list that names one again is cut there, the
+  // copies of the part before are waited for.
+  while (count > 0) {
+    const unsigned long long mark = ++g_host_batches;
+    int whole = 0, done = 0;
+    for (; whole < count && ps[whole]->host_batch != mark; ++whole) ps[whole]->host_batch = mark;
+    ishi_status s = host_batch_chain(ctx, ps, x_hosts, rows, y_hosts, whole, st, &done);
+    if (s == ISHI_OK && done < whole)
+      s = host_batch_lanes(ctx, ps + done, x_hosts + done, rows, y_hosts + done, whole - done, st);
+    if (s != ISHI_OK) return s;
+    ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_end, ctx->copy_out));
+    ISHI_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_end, 0));
+    ps += whole, x_hosts += whole, y_hosts += whole, count -= whole;
   }
-  ISHI_CUDA(ctx, cudaEventRecord(ctx->ev_end, ctx->copy_out));
-  ISHI_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_end, 0));
   return ISHI_OK;
 }
 

@@ -85,6 +85,9 @@ struct FragArgs {
   // Gated pair (the weight was tiled with FragSrc::pair_rows): rows g and g + 8 of a panel are the
   // gate and the up row of output row 8 p + g, and the epilogue writes silu(gate) * up, N / 2 rows
   int swiglu;
+  // The next kernel of the stream may start at once (0) or only when the launch before this one has
+  // completed (1): a kernel that uses what that launch wrote without waiting for this one (HostCopies)
+  int release_late;
   // Output exchange between the GPUs of an N-sharded projection (world = 0: none). Every rank holds
   // the whole output as [rows of all shards][8 or 16] fp16 at the same place of its exchange buffer; this
   // launch computes rows row_offset ... row_offset + N - 1 and stores them into every rank's copy
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
 
   ISHI_STAMP(0);
   // Let the next kernel on the stream start its own prologue as SMs fall free.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!a.release_late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (threadIdx.x < 32) {  // the control block
     for (int i = threadIdx.x; i < led; i += 32) {
@@ -455,6 +458,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   // x may be the output of the kernel before this one and y may still be read by it: wait for the
   // earlier kernels (returns at once unless this kernel was launched early).
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (a.release_late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   ISHI_STAMP(1);
   unsigned previous_launch = 0;
   if (a.world > 0) {

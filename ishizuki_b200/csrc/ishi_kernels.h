@@ -54,6 +54,17 @@ long long rms_norm_max_width();
 cudaError_t launch_rms_norm(const void *x, int x_dtype, const void *w, int w_dtype, long long rows, long long width, float eps,
                             __half *y, cudaStream_t st);
 
+// Copies of mapped page-locked host memory to the device; pointers and sizes multiples of 16 bytes.
+// wait: only when the launches before have completed, else ahead of the kernel's dependency wait.
+constexpr int kHostGroup = 8;
+struct HostCopies {
+  const void *src[kHostGroup];
+  void *dst[kHostGroup];
+  unsigned bytes[kHostGroup];
+  int count, wait;
+};
+cudaError_t launch_host_copies(const HostCopies &copies, cudaStream_t st);
+
 // ---- EXL3 trellis-coded weights (ishi_exl3.cu) ---------------------------------------------------
 // words16: int16 words per 16 x 16 tile (16 * bits); codebook: 0 3INST, 1 MCG, 2 MUL1; dtypes: 0 fp16, 2 fp32
 bool exl3_rate_supported(int words16, int codebook);

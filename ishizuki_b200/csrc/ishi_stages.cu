@@ -75,6 +75,61 @@ cudaError_t launch_as(const void *x, const void *w, long long rows, long long wi
 
 }  // namespace
 
+namespace {
+
+// The inputs of a host batch, a kernel between two products that copies those of the next few. The copy
+// engine takes 4.7 us a copy on top of the bytes and an event between two products, which idles the
+// SMs for 2.5 us; this kernel is a link of the chain of programmatic launches and runs beside the
+// product before it, whose CTAs leave 4096 registers and 1 KB of shared memory of an SM free: a CTA
+// of this kernel. The copies are one range of 16-byte pieces over all CTAs: one after the other, each
+// would add the bus's 2 us of latency. 32 CTAs keep 128 KB on the way; 16 are slower by 8 % of a
+// whole batch, more gain nothing. (Outputs stay with the copy engine: written to the host by a
+// kernel, they hold up the product's loads, 45 us in a batch of 16 entries.)
+constexpr int kCopyThreads = 128, kCopyBlocks = 32;
+
+__global__ void __launch_bounds__(kCopyThreads, 16) host_copy_kernel(const HostCopies c) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (c.wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+  constexpr int kStep = kCopyThreads * kCopyBlocks, kBatch = 2;
+  int job = 0, base = 0;  // the job the next piece lies in, its first piece
+  auto piece = [&](int i) {  // moves on to piece i; false past the end
+    while (job < c.count && i >= base + (int)(c.bytes[job] / 16u)) base += (int)(c.bytes[job++] / 16u);
+    return job < c.count;
+  };
+  for (int i0 = (int)(blockIdx.x * kCopyThreads + threadIdx.x); piece(i0); i0 += kStep * kBatch) {
+    uint4 v[kBatch], *dst[kBatch];
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e) {
+      const int i = i0 + e * kStep;
+      dst[e] = nullptr;
+      if (piece(i)) {
+        dst[e] = static_cast<uint4 *>(c.dst[job]) + (i - base);
+        v[e] = __ldcv(static_cast<const uint4 *>(c.src[job]) + (i - base));
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e)
+      if (dst[e]) *dst[e] = v[e];
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the chain: whoever waits for this kernel waits for all before it
+}
+
+}  // namespace
+
+cudaError_t launch_host_copies(const HostCopies &copies, cudaStream_t st) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(kCopyBlocks);
+  cfg.blockDim = dim3(kCopyThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, host_copy_kernel, copies);
+}
+
 long long rms_norm_max_width() { return 256ll * kNormPer; }
 
 // dtypes: 0 fp16, 1 bf16, 2 fp32

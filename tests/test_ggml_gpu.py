@@ -9,7 +9,7 @@ import torch
 
 from ishizuki_b200 import synth
 from ishizuki_b200 import _lib
-from ishizuki_b200.interface import (BonsaiRuntime, Context, FusedLinear, GGMLKernels, GGMLType, GGUFBlocks, IshizukiError,
+from ishizuki_b200.interface import (BonsaiRuntime, Context, FusedLinear, GGMLKernels, GGMLType, GGUFBlocks, HostBatch, IshizukiError,
                                      PackedLinear, _ptr, _stream)
 from oracle import oracle
 
@@ -181,6 +181,30 @@ def test_host_buffer_entry_points_agree():
         y2 = np.empty((x.shape[0], n), dtype=np.float16)
         lin.apply_host(x, y2)
         assert np.array_equal(y2.view(np.uint16), w.numpy().view(np.uint16))
+
+
+@pytest.mark.parametrize("rows", [1, 8, 13])
+def test_host_batch_entries(rows):
+    """A host batch gives the device path's results: ragged heights, a projection twice in a row and
+    again later, pageable buffers in the middle, one entry alone, more small entries than one copy
+    kernel takes; new inputs on every run."""
+    rng = np.random.default_rng(6)
+    shapes = [(1003, 512), (2048, 4096)] + [(37 + i, 256) for i in range(11)]
+    lins = [PackedLinear(ggml=GGUFBlocks(dev(synth.q4k_blocks(rng, n, k)), GGMLType.q4K, (n, k))) for n, k in shapes]
+    for order, pageable in (([0, 1, 1, 0, 2, 0, 1, 2], None), ([1, 0, 2, 1, 0], 2), ([0], None), (list(range(2, 13)) + [0, 1], None)):
+        xs = [torch.empty((rows, shapes[i][1]), dtype=torch.float16) for i in order]
+        ys = [torch.empty((rows, shapes[i][0]), dtype=torch.float16) for i in order]
+        for e in range(len(order)):
+            if e != pageable:
+                xs[e], ys[e] = xs[e].pin_memory(), ys[e].pin_memory()
+        batch = HostBatch([lins[i] for i in order], xs, ys)
+        for _ in range(3):
+            for i, x in zip(order, xs):
+                x.copy_(torch.from_numpy(synth.activations(rng, rows, shapes[i][1])))
+            batch.run()
+            torch.cuda.current_stream().synchronize()
+            for i, x, y in zip(order, xs, ys):
+                assert torch.equal(y, lins[i](x.cuda()).cpu())
 
 
 @pytest.mark.parametrize("type_id", STREAMED)

@@ -9,8 +9,8 @@ import torch
 
 from ishizuki_b200 import synth
 from ishizuki_b200 import _lib
-from ishizuki_b200.interface import (BonsaiRuntime, Context, FusedLinear, GGMLKernels, GGMLType, GGUFBlocks, HostBatch, IshizukiError,
-                                     PackedLinear, _ptr, _stream)
+from ishizuki_b200.interface import (BonsaiRuntime, Context, FusedLinear, GGMLKernels, GGMLType, GGUFBlocks, HostBatch,
+                                     IshizukiError, PackedLinear, _ptr, _stream)
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu

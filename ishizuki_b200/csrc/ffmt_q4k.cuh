@@ -34,8 +34,8 @@
 // and dmin of every row.
 //
 // Activations of a unit in shared memory: eight rows of 256 fp16 as they lie in x, 576 bytes
-// apart (rows g and g + 1 then sit 64 bytes apart modulo the 128 bytes of a bank sweep), copied by
-// the bulk copy engine; then the sub-block sums of x for the minimum term.
+// apart (rows g and g + 1 then sit 64 bytes apart modulo the 128 bytes of a bank sweep); then the
+// sub-block sums of x for the minimum term.
 #pragma once
 #include "ishi_fragstream.cuh"
 

@@ -44,13 +44,16 @@ struct FragQ6K {
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
 
-  // the 6-bit code of weight k of a block
-  static __device__ __forceinline__ uint32_t code(const uint8_t *blk, int k) {
+  // the low four and the high two bits of weight k of a block
+  static __device__ __forceinline__ uint32_t low4(const uint8_t *blk, int k) {
     const int n = k >> 7, c = (k >> 5) & 3, l = k & 31;
-    const uint32_t lo = blk[64 * n + 32 * (c & 1) + l];
-    const uint32_t hi = blk[128 + 32 * n + l];
-    return ((c >= 2 ? lo >> 4 : lo) & 15u) | (((hi >> (2 * c)) & 3u) << 4);
+    return ((uint32_t)blk[64 * n + 32 * (c & 1) + l] >> (c >= 2 ? 4 : 0)) & 15u;
   }
+  static __device__ __forceinline__ uint32_t high2(const uint8_t *blk, int k) {
+    const int n = k >> 7, c = (k >> 5) & 3, l = k & 31;
+    return ((uint32_t)blk[128 + 32 * n + l] >> (2 * c)) & 3u;
+  }
+  static __device__ __forceinline__ uint32_t code(const uint8_t *blk, int k) { return low4(blk, k) | (high2(blk, k) << 4); }
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {
     long long local;
@@ -63,16 +66,21 @@ struct FragQ6K {
     if (hw < 1536) {
       const int lane = (hw & 255) >> 3, word = 4 * (hw >> 8) + ((hw & 7) >> 1), pi = word / 3, w = word - 3 * pi;
       const int g = lane >> 2, t = lane & 3;
-      // value of k-step 2 pi + second, row g or g + 8, slots (2t, 2t + 1) or (2t + 8, 2t + 9), half h
-      auto value = [&](int second, int below, int y) -> uint32_t {
-        const long long row = p * kFragRows + g + 8 * below;
-        return row < s.N ? code(block(s, row, u), 16 * (2 * pi + second) + 4 * t + 2 * y + h) : 0u;
-      };
-      const uint32_t a0 = value(0, 0, 0), a2 = value(0, 0, 1);
-      uint32_t out;
-      if (w == 0) out = (a0 & 15u) | (value(0, 1, 0) << 4) | (value(0, 1, 1) << 10);
-      else if (w == 1) out = (a2 & 15u) | (value(1, 0, 0) << 4) | (value(1, 1, 0) << 10);
-      else out = (a0 >> 4) | ((a2 >> 4) << 2) | (value(1, 0, 1) << 4) | (value(1, 1, 1) << 10);
+      const long long row = p * kFragRows + g;
+      const uint8_t *top = row < s.N ? block(s, row, u) : nullptr, *low = row + 8 < s.N ? block(s, row + 8, u) : nullptr;
+      // weights of k-steps 2 pi (k0) and 2 pi + 1, slots (2t, 2t + 1); two further on: slots (2t + 8, 2t + 9)
+      const int k0 = 32 * pi + 4 * t + h, k1 = k0 + 16;
+      uint32_t out = 0;
+      if (w == 0) {
+        if (top) out = low4(top, k0);
+        if (low) out |= (code(low, k0) << 4) | (code(low, k0 + 2) << 10);
+      } else if (w == 1) {
+        if (top) out = low4(top, k0 + 2) | (code(top, k1) << 4);
+        if (low) out |= code(low, k1) << 10;
+      } else {
+        if (top) out = high2(top, k0) | (high2(top, k0 + 2) << 2) | (code(top, k1 + 2) << 4);
+        if (low) out |= code(low, k1 + 2) << 10;
+      }
       return (uint16_t)out;
     }
     if (hw < 1664) {

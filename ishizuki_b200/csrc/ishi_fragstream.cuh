@@ -1,4 +1,4 @@
-// The warp-level verify-matmul kernel: y[m, n] = sum_k x[m, k] * w[n, k] for 1..8 activation rows
+// The warp-level verify-matmul kernel: y[m, n] = sum_k x[m, k] * w[n, k] for 1..16 activation rows
 // on mma.sync (m16n8k16, weights on the M side, activation rows on the N side), with a CUDA-core
 // variant for a single row.
 //
@@ -12,8 +12,8 @@
 // tile is 16 output rows x 256 k (one unit), stored as [16-byte piece][lane] so that every
 // warp-wide 128-bit access is one contiguous 512-byte run, followed by a small per-row section
 // (block scales). Lane (g = lane / 4, t = lane % 4) owns weight rows g and g + 8 of the tile and,
-// in every k-step, the four k positions the format's decoder assigns to t. Same bytes as the raw
-// weight, different order.
+// in every k-step, the four k positions the format's decoder assigns to t. The raw weight's bits in
+// another order (a few formats take some bytes more).
 //
 // Work. K is cut into S column ranges and the kernel is launched as thread-block clusters of S
 // CTAs (S = 1: no cluster): CTA r of a cluster stages the activations of column range r into shared

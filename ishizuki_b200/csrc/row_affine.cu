@@ -1,5 +1,5 @@
-// The tcgen05 kernel for the MLX affine packs the warp-level kernel does not take (8-bit, 2-bit
-// group 32, fp32 scales).
+// The tcgen05 kernel for the MLX affine packs the warp-level kernel does not take (2-bit group 32,
+// fp32 scales) and for inputs too wide for its shared memory.
 #include "ishi_row_impl.cuh"
 #include "rfmt_affine.cuh"
 

@@ -495,7 +495,8 @@ def hadamardRotate(x: torch.Tensor, block: int, signs: torch.Tensor | None) -> t
 def rmsNorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:  # noqa: N802
     """MLXFast.rmsNorm(x, weight:, eps:) ahead of a projection (TextModel.swift:151-161): fp32 or
     fp16 rows in, fp16 out."""
-    return _calls.rms_norm(Context.of(x).address, x, weight, eps)
+    ctx = Context.of(x)  # (the first context loads _calls)
+    return _calls.rms_norm(ctx.address, x, weight, eps)
 
 
 class EXL3Tensor:
@@ -564,7 +565,8 @@ class EXL3Kernels:
     @staticmethod
     def apply(x: torch.Tensor, t: EXL3Tensor) -> torch.Tensor:
         """rotate -> product -> rotate, 1...16 fp16 rows."""
-        return _calls.exl3_apply(Context.of(x).address, t.trellis, t.inputScales, t.outputScales, t.codebook, x)
+        ctx = Context.of(x)
+        return _calls.exl3_apply(ctx.address, t.trellis, t.inputScales, t.outputScales, t.codebook, x)
 
 
 class EXL3Linear:

@@ -26,35 +26,67 @@ __device__ __forceinline__ float to_float<__half>(__half v) { return __half2floa
 template <>
 __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// one CTA of 256 threads per row; the row stays in registers between the two passes (width <= 256 * kPer)
-constexpr int kNormPer = 32;
-template <class XT, class WT>
-__global__ void __launch_bounds__(256) rms_norm_kernel(const XT *__restrict__ x, const WT *__restrict__ w, long long width, float eps,
-                                                       __half *__restrict__ y) {
-  __shared__ float part[8];
+// One CTA of 1024 threads per row, eight values each in 16-byte loads; the row stays in registers
+// between the two passes. Bound by latency alone (a row is 10-20 KB): x and w are on their way together
+// as soon as the launch before is done, w already hinted into L2 (its values are read after the wait, they
+// may be that launch's as well), and the rest is one barrier. Two decoder layers of the 27B shape, four
+// norms, in Q4_K at eight rows: 119.9 us with 256 threads reading value by value and w after the sum,
+// 114.1 this way.
+constexpr int kNormThreads = 1024, kNormPer = 8;
+
+template <class T>
+__device__ __forceinline__ void load8(const T *p, float (&v)[kNormPer]) {
+  uint4 raw[sizeof(T) / 2];
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(T) / 2); ++i) raw[i] = reinterpret_cast<const uint4 *>(p)[i];
+  const T *t = reinterpret_cast<const T *>(raw);
+#pragma unroll
+  for (int i = 0; i < kNormPer; ++i) v[i] = to_float(t[i]);
+}
+
+// WIDE: width a multiple of eight, all pointers 16-byte aligned; else value by value
+template <class XT, class WT, bool WIDE>
+__global__ void __launch_bounds__(kNormThreads) rms_norm_kernel(const XT *__restrict__ x, const WT *__restrict__ w, long long width, float eps,
+                                                                __half *__restrict__ y) {
+  __shared__ float part[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int i0 = (int)threadIdx.x * kNormPer, n = (int)min((long long)kNormPer, width - i0);
+  if (n > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + i0));
   asm volatile("griddepcontrol.wait;" ::: "memory");  // x may be the output of the launch before
   const XT *row = x + (long long)blockIdx.x * width;
-  float v[kNormPer];
+  float v[kNormPer] = {}, f[kNormPer] = {};
+  if (WIDE) {
+    if (n > 0) load8(row + i0, v), load8(w + i0, f);
+  } else {
+#pragma unroll
+    for (int j = 0; j < kNormPer; ++j)
+      if (j < n) v[j] = to_float(row[i0 + j]), f[j] = to_float(w[i0 + j]);
+  }
   float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < kNormPer; ++j) {
-    const long long i = (long long)j * 256 + threadIdx.x;
-    v[j] = i < width ? to_float(row[i]) : 0.f;
-    ss = fmaf(v[j], v[j], ss);
-  }
+  for (int j = 0; j < kNormPer; ++j) ss = fmaf(v[j], v[j], ss);
 #pragma unroll
   for (int d = 16; d; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
   __syncthreads();
-  float total = 0.f;
+  float total = part[threadIdx.x & 31];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) total += part[i];
+  for (int d = 16; d; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
   const float r = rsqrtf(total / (float)width + eps);
+  __half *out = y + (long long)blockIdx.x * width + i0;
+  __half h[kNormPer];
 #pragma unroll
-  for (int j = 0; j < kNormPer; ++j) {
-    const long long i = (long long)j * 256 + threadIdx.x;
-    if (i < width) y[(long long)blockIdx.x * width + i] = __float2half_rn(v[j] * r * to_float(w[i]));
+  for (int j = 0; j < kNormPer; ++j) h[j] = __float2half_rn(v[j] * r * f[j]);
+  if (WIDE) {
+    if (n > 0) {
+      uint4 o;
+      memcpy(&o, h, sizeof(o));
+      *reinterpret_cast<uint4 *>(out) = o;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kNormPer; ++j)
+      if (j < n) out[j] = h[j];
   }
 }
 
@@ -63,14 +95,16 @@ cudaError_t launch_as(const void *x, const void *w, long long rows, long long wi
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)rows);
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(kNormThreads);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, rms_norm_kernel<XT, WT>, static_cast<const XT *>(x), static_cast<const WT *>(w), width, eps, y);
+  const bool wide = width % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;
+  return cudaLaunchKernelEx(&cfg, wide ? rms_norm_kernel<XT, WT, true> : rms_norm_kernel<XT, WT, false>, static_cast<const XT *>(x),
+                            static_cast<const WT *>(w), width, eps, y);
 }
 
 }  // namespace
@@ -130,7 +164,7 @@ cudaError_t launch_host_copies(const HostCopies &copies, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, host_copy_kernel, copies);
 }
 
-long long rms_norm_max_width() { return 256ll * kNormPer; }
+long long rms_norm_max_width() { return (long long)kNormThreads * kNormPer; }
 
 // dtypes: 0 fp16, 1 bf16, 2 fp32
 cudaError_t launch_rms_norm(const void *x, int x_dtype, const void *w, int w_dtype, long long rows, long long width, float eps,

@@ -30,6 +30,20 @@ def test_rms_norm_matches_the_oracle(rows, width, xdt, wdt):
     assert (got.view(np.uint16) != want.view(np.uint16)).mean() < 0.01
 
 
+@pytest.mark.parametrize("rows,width,shift", [(3, 203, 0), (1, 7, 0), (2, 4099, 0), (2, 8191, 0), (2, 512, 1)])
+def test_rms_norm_value_by_value(rows, width, shift):
+    """Widths that are no multiple of eight and rows off a 16-byte boundary."""
+    rng = np.random.default_rng(width)
+    x = (rng.standard_normal((rows, width)) * 3).astype(np.float32)
+    w = (1 + 0.1 * rng.standard_normal(width)).astype(np.float32)
+    flat = torch.zeros(rows * width + shift, device="cuda")
+    flat[shift:] = dev(x).reshape(-1)
+    got = rmsNorm(flat[shift:].view(rows, width), dev(w), 1e-6).cpu().numpy()
+    want = oracle.rms_norm(x, w, 1e-6)
+    diff = np.abs(got.astype(np.float32) - want.astype(np.float32))
+    assert np.all(diff <= np.abs(want.astype(np.float32)) * 2.0 ** -10 + 1e-7)
+
+
 def test_norm_then_stacked_projection_in_one_graph():
     """rmsNorm -> q+k+v as consecutive dependent launches, captured and replayed: the product of the
     normalised rows, against the oracle's."""

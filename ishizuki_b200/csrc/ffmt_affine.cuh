@@ -82,81 +82,64 @@ struct FragAffine {
   // row): lane l loads the eight values k = 8l .. 8l + 7. The fragment of k-step st = kMasks * q + m
   // sits at st * 256 + ((g ^ (q & 3)) * 4 + t) * 8: the xor spreads a store's quads over the banks,
   // and a k-step's 32 lanes still read one 256-byte run.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
     if (BITS == 2 && GS == 128 && a.rot_block == 128 && !a.rot_signs) {
-      stage_x_rot128(a, x, M, xfrag, ub0, uc);
+      stage_x_rot128(a, m, xfrag, ub0, uc);
       return;
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int tasks = uc * 8;
-    constexpr int kBatch = 8;
-    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
-      uint4 v[kBatch];
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < M)
-          v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
-      }
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        if (i >= tasks) break;
-        const int g = i & 7;
-        if (a.rot_block)
-          v[e] = frag_rotate8(v[e], a.rot_block,
-                              a.rot_signs ? a.rot_signs + (long long)(ub0 + (i >> 3)) * 256 + lane * 8 : nullptr, lane);
-        const uint32_t base = xfrag + (uint32_t)(i >> 3) * kXBytes;
-        // halves of v: x0 x1 | x2 x3 | x4 x5 | x6 x7
-        if (BITS == 8) {
-          // the lane holds words 2l and 2l + 1: quad q = l / 2, t = 2 (l % 2) and t + 1, each (x0, x2), (x1, x3)
-          const int q = lane >> 1;
-          sts128u(base + (uint32_t)q * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + 2 * (lane & 1)) * 8),
-                  make_uint4(prmt(v[e].x, v[e].y, 0x5410u), prmt(v[e].x, v[e].y, 0x7632u), prmt(v[e].z, v[e].w, 0x5410u),
-                             prmt(v[e].z, v[e].w, 0x7632u)));
-        } else if (BITS == 4) {
-          // the lane holds word l: quad q = l / 4, t = l % 4; k-step m pairs (x_m, x_m+4), (x_m+2, x_m+6)
-          const int q = lane >> 2, t = lane & 3;
-          const uint32_t dst = base + (uint32_t)(2 * q) * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + t) * 8);
-          sts64(dst, prmt(v[e].x, v[e].z, 0x5410u), prmt(v[e].y, v[e].w, 0x5410u));
-          sts64(dst + 256u, scale_down<4>(prmt(v[e].x, v[e].z, 0x7632u)), scale_down<4>(prmt(v[e].y, v[e].w, 0x7632u)));
+    const int lane = threadIdx.x & 31;
+    frag_stage_rows(a, m, ub0, uc, [&](int u, int g, uint4 v) {
+      if (a.rot_block)
+        v = frag_rotate8(v, a.rot_block,
+                            a.rot_signs ? a.rot_signs + (long long)(ub0 + u) * 256 + lane * 8 : nullptr, lane);
+      const uint32_t base = xfrag + (uint32_t)u * kXBytes;
+      // halves of v: x0 x1 | x2 x3 | x4 x5 | x6 x7
+      if (BITS == 8) {
+        // the lane holds words 2l and 2l + 1: quad q = l / 2, t = 2 (l % 2) and t + 1, each (x0, x2), (x1, x3)
+        const int q = lane >> 1;
+        sts128u(base + (uint32_t)q * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + 2 * (lane & 1)) * 8),
+                make_uint4(prmt(v.x, v.y, 0x5410u), prmt(v.x, v.y, 0x7632u), prmt(v.z, v.w, 0x5410u),
+                           prmt(v.z, v.w, 0x7632u)));
+      } else if (BITS == 4) {
+        // the lane holds word l: quad q = l / 4, t = l % 4; k-step m pairs (x_m, x_m+4), (x_m+2, x_m+6)
+        const int q = lane >> 2, t = lane & 3;
+        const uint32_t dst = base + (uint32_t)(2 * q) * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + t) * 8);
+        sts64(dst, prmt(v.x, v.z, 0x5410u), prmt(v.y, v.w, 0x5410u));
+        sts64(dst + 256u, scale_down<4>(prmt(v.x, v.z, 0x7632u)), scale_down<4>(prmt(v.y, v.w, 0x7632u)));
+      } else {
+        // the lane holds half of word l / 2 (codes 0..7 when l is even, 8..15 when odd): quad
+        // q = l / 8, t = (l / 2) % 4. k-step m pairs (x_m, x_m+8), (x_m+4, x_m+12): the even lane
+        // builds m = 0, 1 and the odd lane m = 2, 3, each with the other's half of the word.
+        const uint32_t ox = __shfl_xor_sync(0xffffffffu, v.x, 1), oy = __shfl_xor_sync(0xffffffffu, v.y, 1);
+        const uint32_t oz = __shfl_xor_sync(0xffffffffu, v.z, 1), ow = __shfl_xor_sync(0xffffffffu, v.w, 1);
+        const bool odd = lane & 1;
+        // lo = codes 0..7 of the word, hi = codes 8..15
+        const uint32_t lx = odd ? ox : v.x, ly = odd ? oy : v.y, lz = odd ? oz : v.z, lw = odd ? ow : v.w;
+        const uint32_t hx = odd ? v.x : ox, hy = odd ? v.y : oy, hz = odd ? v.z : oz, hw = odd ? v.w : ow;
+        const int q = lane >> 3, t = (lane >> 1) & 3;
+        const uint32_t dst = base + (uint32_t)(4 * q + (odd ? 2 : 0)) * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + t) * 8);
+        // m = 0 / 2: (lo_m, hi_m), (lo_m+4, hi_m+4) with lo_0 = lx.lo, lo_2 = ly.lo, lo_4 = lz.lo, lo_6 = lw.lo
+        const uint32_t ea = odd ? ly : lx, eb = odd ? hy : hx, ec = odd ? lw : lz, ed = odd ? hw : hz;
+        if (odd) {
+          sts64(dst, scale_down<4>(prmt(ea, eb, 0x5410u)), scale_down<4>(prmt(ec, ed, 0x5410u)));
+          sts64(dst + 256u, scale_down<6>(prmt(ea, eb, 0x7632u)), scale_down<6>(prmt(ec, ed, 0x7632u)));
         } else {
-          // the lane holds half of word l / 2 (codes 0..7 when l is even, 8..15 when odd): quad
-          // q = l / 8, t = (l / 2) % 4. k-step m pairs (x_m, x_m+8), (x_m+4, x_m+12): the even lane
-          // builds m = 0, 1 and the odd lane m = 2, 3, each with the other's half of the word.
-          const uint32_t ox = __shfl_xor_sync(0xffffffffu, v[e].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[e].y, 1);
-          const uint32_t oz = __shfl_xor_sync(0xffffffffu, v[e].z, 1), ow = __shfl_xor_sync(0xffffffffu, v[e].w, 1);
-          const bool odd = lane & 1;
-          // lo = codes 0..7 of the word, hi = codes 8..15
-          const uint32_t lx = odd ? ox : v[e].x, ly = odd ? oy : v[e].y, lz = odd ? oz : v[e].z, lw = odd ? ow : v[e].w;
-          const uint32_t hx = odd ? v[e].x : ox, hy = odd ? v[e].y : oy, hz = odd ? v[e].z : oz, hw = odd ? v[e].w : ow;
-          const int q = lane >> 3, t = (lane >> 1) & 3;
-          const uint32_t dst = base + (uint32_t)(4 * q + (odd ? 2 : 0)) * 256u + (uint32_t)(((g ^ (q & 3)) * 4 + t) * 8);
-          // m = 0 / 2: (lo_m, hi_m), (lo_m+4, hi_m+4) with lo_0 = lx.lo, lo_2 = ly.lo, lo_4 = lz.lo, lo_6 = lw.lo
-          const uint32_t ea = odd ? ly : lx, eb = odd ? hy : hx, ec = odd ? lw : lz, ed = odd ? hw : hz;
-          if (odd) {
-            sts64(dst, scale_down<4>(prmt(ea, eb, 0x5410u)), scale_down<4>(prmt(ec, ed, 0x5410u)));
-            sts64(dst + 256u, scale_down<6>(prmt(ea, eb, 0x7632u)), scale_down<6>(prmt(ec, ed, 0x7632u)));
-          } else {
-            sts64(dst, prmt(ea, eb, 0x5410u), prmt(ec, ed, 0x5410u));
-            sts64(dst + 256u, scale_down<2>(prmt(ea, eb, 0x7632u)), scale_down<2>(prmt(ec, ed, 0x7632u)));
-          }
+          sts64(dst, prmt(ea, eb, 0x5410u), prmt(ec, ed, 0x5410u));
+          sts64(dst + 256u, scale_down<2>(prmt(ea, eb, 0x7632u)), scale_down<2>(prmt(ec, ed, 0x7632u)));
         }
-        // fp32 sums of x over the groups (GS / 8 lanes each) in the codes' unit, for the bias term
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].y));
-        const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].z));
-        const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].w));
-        float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-#pragma unroll
-        for (int d = 1; d < GS / 8; d *= 2) s += __shfl_xor_sync(0xffffffffu, s, d);
-        if ((lane & (GS / 8 - 1)) == 0)
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kSums + (uint32_t)((lane / (GS / 8)) * 8 + g) * 4u), "f"(s * (1.f / 16777216.f))
-                       : "memory");
       }
-    }
+      // fp32 sums of x over the groups (GS / 8 lanes each) in the codes' unit, for the bias term
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
+      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
+      float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+#pragma unroll
+      for (int d = 1; d < GS / 8; d *= 2) s += __shfl_xor_sync(0xffffffffu, s, d);
+      if ((lane & (GS / 8 - 1)) == 0)
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kSums + (uint32_t)((lane / (GS / 8)) * 8 + g) * 4u), "f"(s * (1.f / 16777216.f))
+                     : "memory");
+    });
   }
 
   // +1 or -1 in fp16 by the parity of v
@@ -180,10 +163,9 @@ struct FragAffine {
   // to fp32 rounding. Lane (g, t) ends up with the values k' = 16 (4 h + t) + g and + 8 of each
   // block: the codes g and g + 8 of the block's word 4 h + t, which are one B register of the
   // product's k-step (quad 2 block + h, mask g % 4), low register when g < 4.
-  static __device__ __forceinline__ void stage_x_rot128(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
+  static __device__ __forceinline__ void stage_x_rot128(const FragArgs &a, const FragRows &rows, uint32_t xfrag, int ub0, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int tasks = uc * 8;
     constexpr int kBatch = 8;
     const uint32_t h8 = sign_half(g & (2 * t)) | (sign_half(g & (2 * t + 1)) << 16);
     uint32_t h16[2][2];
@@ -197,15 +179,16 @@ struct FragAffine {
     const uint32_t down1 = (uint32_t)(15 - 2 * m) << 10;  // 2^-(2 m) in fp16
     const uint32_t down = down1 | (down1 << 16);
     const float scale = 1.0f / sqrtf(128.f);
-    const uint32_t *xl = reinterpret_cast<const uint32_t *>(x + (long long)ub0 * 256) + lane;
-    const long long row_words = a.K >> 1;
+    const uint32_t *xl = reinterpret_cast<const uint32_t *>(rows.x + (long long)ub0 * 256) + lane;
+    const int tasks = uc * rows.staged;
     for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
       uint32_t v[kBatch][4];  // [block * 2 + half]
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
-        const bool live = i < tasks && (i & 7) < M;
-        const uint32_t *src = xl + (long long)(i & 7) * row_words + (i >> 3) * 128;
+        const int2 task = rows.task(i);
+        const bool live = i < tasks && task.y < rows.live;
+        const uint32_t *src = xl + (long long)task.y * (a.K >> 1) + task.x * 128;
 #pragma unroll
         for (int c = 0; c < 4; ++c) v[e][c] = live ? __ldg(src + 32 * c) : 0u;
       }
@@ -213,8 +196,9 @@ struct FragAffine {
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
         if (i >= tasks) break;
-        const int r = i & 7;
-        const uint32_t base = xfrag + (uint32_t)(i >> 3) * kXBytes;
+        const int2 task = rows.task(i);
+        const int r = task.y;
+        const uint32_t base = xfrag + (uint32_t)task.x * kXBytes;
         uint32_t zh[4], zl[4];  // stage 2's A registers: (block 0, half 0), (block 1, half 0), (block 0, half 1), (block 1, half 1)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

@@ -97,40 +97,23 @@ struct FragIQ1 {
   // (the eight values of one lane) their sum as fp16 high and low parts, where the MMA over the
   // entries reads them: entry E = 2 (4 j + t) + e is slot 2t + e + 8 (j % 2) of k-step j / 2, i.e.
   // register j % 2, half e, of lane (r, t). No rotation here.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+    const int lane = threadIdx.x & 31;
     const uint32_t R = row_stride(a);
-    const int tasks = uc * 8;
-    constexpr int kBatch = 8;
-    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
     const int sb = lane >> 1, j = sb >> 2, t = sb & 3;
     const uint32_t slot = (uint32_t)((j >> 1) * 512 + t * 16 + (j & 1) * 4 + (lane & 1) * 2);
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
-      uint4 v[kBatch];
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < M)
-          v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
-      }
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        if (i >= tasks) break;
-        const int r = i & 7, u = i >> 3;
-        sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v[e]);
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].y));
-        const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].z));
-        const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].w));
-        const float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-        const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-        const uint32_t at = sums_of(a, xfrag, u) + (uint32_t)r * 64u + slot;
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
-      }
-    }
+    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+      sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
+      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
+      const float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+      const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+      const uint32_t at = sums_of(a, xfrag, u) + (uint32_t)r * 64u + slot;
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
+    });
   }
 
   // eight weights as four A registers, value * (2 s + 1): address of the grid entry (this lane's

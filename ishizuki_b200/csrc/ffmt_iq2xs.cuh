@@ -165,28 +165,12 @@ struct FragIQ2 {
   // Activations of the CTA's column range as they lie in x (rows past M as zeros).
   // A warp task is (unit, activation row): lane l loads and stores k = 8l .. 8l + 7.
   // IQ2_XS has no rotation.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+    const int lane = threadIdx.x & 31;
     const uint32_t R = row_stride(a);
-    const int tasks = uc * 8;
-    constexpr int kBatch = 8;
-    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
-      uint4 v[kBatch];
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < M)
-          v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
-      }
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        if (i >= tasks) break;
-        sts128u(xfrag + (uint32_t)(i & 7) * R + (uint32_t)(i >> 3) * 512u + (uint32_t)lane * 16u, v[e]);
-      }
-    }
+    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+      sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
+    });
   }
 
   // 2 s + 1 of scale nibble j, in both halves, from the nibbles of a row in both halves: the nibble

@@ -93,8 +93,8 @@ struct FragIQ3 {
   }
 
   // the activations as for IQ2_XS: the rows as they lie in x
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
-    FragIQ2<17>::stage_x(a, x, M, xfrag, ub0, uc);
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+    FragIQ2<17>::stage_x(a, m, xfrag, ub0, uc);
   }
 
   // a sub-block's sixteen weights (two words) as eight A registers; `copy`: byte offset of this lane's copy

@@ -80,41 +80,24 @@ struct FragIQ4XS {
   // ks = 2 ib + s and quad row r lie at ks * 256 + ((r ^ (ks % 8)) * 4 + t) * 8; the xor spreads the
   // stores over the banks, a warp's read of one k-step is still one 256-byte run.
   // No rotation here.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int tasks = uc * 8;
-    constexpr int kBatch = 8;
-    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+    const int lane = threadIdx.x & 31;
     const int ib = lane >> 2, r4 = lane & 3;
     const bool second = r4 >= 2;
     const int t = second ? 2 * (r4 - 2) + 1 : 2 * r4;
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
-      uint4 v[kBatch];
+    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+      const uint32_t base = xfrag + (uint32_t)u * kXBytes;
+      const uint32_t got0 = __shfl_xor_sync(0xffffffffu, second ? v.x : v.z, 2);
+      const uint32_t got1 = __shfl_xor_sync(0xffffffffu, second ? v.y : v.w, 2);
+      const uint32_t lo0 = second ? got0 : v.x, lo1 = second ? got1 : v.y;
+      const uint32_t hi0 = second ? v.z : got0, hi1 = second ? v.w : got1;
 #pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < M)
-          v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
+      for (int s = 0; s < 2; ++s) {
+        const int ks = 2 * ib + s;
+        const uint32_t lo = s ? lo1 : lo0, hi = s ? hi1 : hi0;
+        sts64(base + (uint32_t)ks * 256u + (uint32_t)(((r ^ (ks & 7)) * 4 + t) * 8), prmt(lo, hi, 0x5410u), prmt(lo, hi, 0x7632u));
       }
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        if (i >= tasks) break;
-        const int r = i & 7;
-        const uint32_t base = xfrag + (uint32_t)(i >> 3) * kXBytes;
-        const uint32_t got0 = __shfl_xor_sync(0xffffffffu, second ? v[e].x : v[e].z, 2);
-        const uint32_t got1 = __shfl_xor_sync(0xffffffffu, second ? v[e].y : v[e].w, 2);
-        const uint32_t lo0 = second ? got0 : v[e].x, lo1 = second ? got1 : v[e].y;
-        const uint32_t hi0 = second ? v[e].z : got0, hi1 = second ? v[e].w : got1;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const int ks = 2 * ib + s;
-          const uint32_t lo = s ? lo1 : lo0, hi = s ? hi1 : hi0;
-          sts64(base + (uint32_t)ks * 256u + (uint32_t)(((r ^ (ks & 7)) * 4 + t) * 8), prmt(lo, hi, 0x5410u), prmt(lo, hi, 0x7632u));
-        }
-      }
-    }
+    });
   }
 
   // the value pair of byte `byte` of word w

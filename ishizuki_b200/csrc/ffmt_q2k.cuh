@@ -73,56 +73,39 @@ struct FragQ2K {
   // is * 256 + ((r ^ (is % 8)) * 4 + t) * 8 (the xor spreads the stores over the banks, a warp's read
   // of one k-step is still one 256-byte run). Then the sub-block sums of the undivided values
   // (fp16 hi + lo) for the MMA over sub-blocks. No rotation here.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int tasks = uc * 8;
-    constexpr int kBatch = 8;
-    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+    const int lane = threadIdx.x & 31;
     const int j = (lane >> 2) & 3;
     const int is = 8 * (lane >> 4) + 2 * j + ((lane & 3) >> 1);
     const uint32_t down1 = (uint32_t)(15 - 2 * j) << 10;  // 4^-j in fp16
     const uint32_t down = down1 | (down1 << 16);
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
-      uint4 v[kBatch];
+    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+      const uint32_t base = xfrag + (uint32_t)u * kXBytes;
+      const __half2 dn = *reinterpret_cast<const __half2 *>(&down);
+      // (x0 x2), (x1 x3) for t = 2 (l % 2); (x4 x6), (x5 x7) for t + 1
+      uint32_t w[4] = {prmt(v.x, v.y, 0x5410u), prmt(v.x, v.y, 0x7632u), prmt(v.z, v.w, 0x5410u),
+                       prmt(v.z, v.w, 0x7632u)};
 #pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < M)
-          v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
+      for (int q = 0; q < 4; ++q) {
+        const __half2 h = __hmul2(*reinterpret_cast<const __half2 *>(&w[q]), dn);
+        w[q] = *reinterpret_cast<const uint32_t *>(&h);
       }
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        if (i >= tasks) break;
-        const int r = i & 7;
-        const uint32_t base = xfrag + (uint32_t)(i >> 3) * kXBytes;
-        const __half2 dn = *reinterpret_cast<const __half2 *>(&down);
-        // (x0 x2), (x1 x3) for t = 2 (l % 2); (x4 x6), (x5 x7) for t + 1
-        uint32_t w[4] = {prmt(v[e].x, v[e].y, 0x5410u), prmt(v[e].x, v[e].y, 0x7632u), prmt(v[e].z, v[e].w, 0x5410u),
-                         prmt(v[e].z, v[e].w, 0x7632u)};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const __half2 h = __hmul2(*reinterpret_cast<const __half2 *>(&w[q]), dn);
-          w[q] = *reinterpret_cast<const uint32_t *>(&h);
-        }
-        sts128u(base + (uint32_t)is * 256u + (uint32_t)(((r ^ (is & 7)) * 4 + 2 * (lane & 1)) * 8), make_uint4(w[0], w[1], w[2], w[3]));
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].y));
-        const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].z));
-        const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].w));
-        float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-        s += __shfl_xor_sync(0xffffffffu, s, 1);  // the sub-block's sixteen values
-        if ((lane & 1) == 0) {
-          const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-          // sub-block is is slot is of the MMA over sub-blocks: lane t' = (is % 8) / 2 of quad r holds
-          // it in register is / 8, half is % 2
-          const uint32_t at = base + kXSums + (uint32_t)((r * 4 + ((is & 7) >> 1)) * 16 + (is >> 3) * 4 + (is & 1) * 2);
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
-        }
+      sts128u(base + (uint32_t)is * 256u + (uint32_t)(((r ^ (is & 7)) * 4 + 2 * (lane & 1)) * 8), make_uint4(w[0], w[1], w[2], w[3]));
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
+      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
+      float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+      s += __shfl_xor_sync(0xffffffffu, s, 1);  // the sub-block's sixteen values
+      if ((lane & 1) == 0) {
+        const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+        // sub-block is is slot is of the MMA over sub-blocks: lane t' = (is % 8) / 2 of quad r holds
+        // it in register is / 8, half is % 2
+        const uint32_t at = base + kXSums + (uint32_t)((r * 4 + ((is & 7) >> 1)) * 16 + (is >> 3) * 4 + (is & 1) * 2);
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
       }
-    }
+    });
   }
 
   // 8388608 + byte `byte` of word w, as a float

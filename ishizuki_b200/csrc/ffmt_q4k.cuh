@@ -103,48 +103,32 @@ struct FragQ4K {
   // every sub-block for the minimum term. Q4_K has no input rotation.
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+    const int lane = threadIdx.x & 31;
     const uint32_t R = row_stride(a), sums = xfrag + 8u * R;
-    const int tasks = uc * 8, jj = lane >> 3;
-    constexpr int kBatch = 8;
-    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
-      uint4 v[kBatch];
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < M)
-          v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
+    const int jj = lane >> 3;
+    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+      sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
+      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
+      float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      const float o = __shfl_xor_sync(0xffffffffu, s, 4);
+      const uint32_t base = sums + (uint32_t)u * kSumBytes;
+      if ((lane & 7) == 0) {
+        // sub-blocks 2t' and 2t' + 1 (t' = lane / 8) of activation row r, as fp16 hi + lo: the B
+        // fragment of the minimum-term MMA, whose k index runs over sub-blocks
+        const __half h0 = __float2half_rn(s), h1 = __float2half_rn(o);
+        const __half l0 = __float2half_rn(s - __half2float(h0)), l1 = __float2half_rn(o - __half2float(h1));
+        sts64(base + (uint32_t)(r * 4 + jj) * 8u, (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
+              (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16));
       }
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        if (i >= tasks) break;
-        const int r = i & 7, u = i >> 3;
-        sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v[e]);
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].y));
-        const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].z));
-        const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].w));
-        float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        const float o = __shfl_xor_sync(0xffffffffu, s, 4);
-        const uint32_t base = sums + (uint32_t)u * kSumBytes;
-        if ((lane & 7) == 0) {
-          // sub-blocks 2t' and 2t' + 1 (t' = lane / 8) of activation row r, as fp16 hi + lo: the B
-          // fragment of the minimum-term MMA, whose k index runs over sub-blocks
-          const __half h0 = __float2half_rn(s), h1 = __float2half_rn(o);
-          const __half l0 = __float2half_rn(s - __half2float(h0)), l1 = __float2half_rn(o - __half2float(h1));
-          sts64(base + (uint32_t)(r * 4 + jj) * 8u, (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
-                (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16));
-        }
-        if (r == 0 && (lane & 3) == 0)  // fp32 sums of activation row 0 (the single-row kernel's minimum term)
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + 256u + (uint32_t)(lane >> 2) * 4u), "f"(s) : "memory");
-      }
-    }
+      if (r == 0 && (lane & 3) == 0)  // fp32 sums of activation row 0 (the single-row kernel's minimum term)
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + 256u + (uint32_t)(lane >> 2) * 4u), "f"(s) : "memory");
+    });
   }
 
   static __device__ __forceinline__ float half_lo(uint32_t pair) { return __half2float(__ushort_as_half((unsigned short)(pair & 0xffffu))); }

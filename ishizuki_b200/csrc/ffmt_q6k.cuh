@@ -102,46 +102,29 @@ struct FragQ6K {
   // i * 512 + ((r ^ i) * 4 + t) * 16 (+ 8 for the odd k-step); the xor spreads the stores over the
   // banks and a warp's read of one pair is still one 512-byte run. Then the group sums (fp16 hi +
   // lo) for the MMA over groups.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const __half *x, int M, uint32_t xfrag, int ub0, int uc) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int tasks = uc * 8;
-    constexpr int kBatch = 8;
-    const __half *xl = x + (long long)ub0 * 256 + lane * 8;
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
-      uint4 v[kBatch];
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        v[e] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < tasks && (i & 7) < M)
-          v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)(i & 7) * a.K + (i >> 3) * 256));
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+    const int lane = threadIdx.x & 31;
+    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+      const uint32_t base = xfrag + (uint32_t)u * kXBytes;
+      const int pi = lane >> 2, ks = lane >> 1;
+      const uint32_t dst = base + (uint32_t)pi * 512u + (uint32_t)(((r ^ pi) * 4 + 2 * (lane & 1)) * 16 + (ks & 1) * 8);
+      sts64(dst, v.x, v.y);
+      sts64(dst + 16u, v.z, v.w);
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
+      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
+      float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+      s += __shfl_xor_sync(0xffffffffu, s, 1);  // the group's sixteen values
+      if ((lane & 1) == 0) {
+        const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+        // group ks is slot ks of the MMA over groups: lane t' = (ks % 8) / 2 of quad r holds it in
+        // register ks / 8, half ks % 2
+        const uint32_t at = base + kXSums + (uint32_t)((r * 4 + ((ks & 7) >> 1)) * 16 + (ks >> 3) * 4 + (ks & 1) * 2);
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
       }
-#pragma unroll
-      for (int e = 0; e < kBatch; ++e) {
-        const int i = i0 + e * nw;
-        if (i >= tasks) break;
-        const int r = i & 7, u = i >> 3;
-        const uint32_t base = xfrag + (uint32_t)u * kXBytes;
-        const int pi = lane >> 2, ks = lane >> 1;
-        const uint32_t dst = base + (uint32_t)pi * 512u + (uint32_t)(((r ^ pi) * 4 + 2 * (lane & 1)) * 16 + (ks & 1) * 8);
-        sts64(dst, v[e].x, v[e].y);
-        sts64(dst + 16u, v[e].z, v[e].w);
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].y));
-        const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].z));
-        const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v[e].w));
-        float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-        s += __shfl_xor_sync(0xffffffffu, s, 1);  // the group's sixteen values
-        if ((lane & 1) == 0) {
-          const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-          // group ks is slot ks of the MMA over groups: lane t' = (ks % 8) / 2 of quad r holds it in
-          // register ks / 8, half ks % 2
-          const uint32_t at = base + kXSums + (uint32_t)((r * 4 + ((ks & 7) >> 1)) * 16 + (ks >> 3) * 4 + (ks & 1) * 2);
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
-        }
-      }
-    }
+    });
   }
 
   // byte `byte` of a word of scales + 128 as the scale: the low mantissa bits of 2^23

@@ -9,15 +9,17 @@ namespace ishi {
 
 template <class Fmt>
 struct FragOpsOf {
-  // the variant that serves a launch: column groups of eight rows, CUDA cores or not, block size.
+  // the variant that serves a launch: column groups of eight rows, CUDA cores or not, block size, a
+  // single row of no exchange (which stores all eight columns).
   // Two column groups keep twice the accumulators: at most kFragFewWarps warps.
-  static const void *kernel(int groups, int mode, int warps) {
+  static const void *kernel(int groups, int mode, int warps, bool one) {
     const bool few = warps <= kFragFewWarps;
     if (groups == 2) return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 2> : nullptr;
     if constexpr (Fmt::kRowMode) {
       // (a format without a CUDA-core variant for one activation row runs that row through the MMA path)
       if (mode == 1) return few ? (const void *)frag_kernel<Fmt, 1, kFragFewWarps, 1> : (const void *)frag_kernel<Fmt, 1, kFragMaxWarps, 1>;
     }
+    if (one) return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 1, true> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1, true>;
     return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 1> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1>;
   }
 
@@ -25,10 +27,11 @@ struct FragOpsOf {
     for (int groups = 1; groups <= 2; ++groups)
       for (int mode = 0; mode < 2; ++mode)
         for (int warps : {kFragFewWarps, kFragMaxWarps})
-          if (const void *k = kernel(groups, mode, warps)) {
-            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-            if (e != cudaSuccess) return e;
-          }
+          for (bool one : {false, true})
+            if (const void *k = kernel(groups, mode, warps, one)) {
+              const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+              if (e != cudaSuccess) return e;
+            }
     if constexpr (Fmt::kExtraBytes > 0) {
       // on a stream of its own: other threads may be using the default stream
       cudaStream_t st = nullptr;
@@ -61,7 +64,7 @@ struct FragOpsOf {
     cudaLaunchAttribute at[2];
     fill(&cfg, at, sm_count, split, warps, smem);
     int n = 0;
-    const void *k = kernel(groups, 0, warps);
+    const void *k = kernel(groups, 0, warps, false);
     const cudaError_t e = k ? cudaOccupancyMaxActiveClusters(&n, k, &cfg) : cudaErrorInvalidValue;
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -82,7 +85,7 @@ struct FragOpsOf {
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = l.early ? 2 : 1;
     void *params[1] = {const_cast<FragArgs *>(&args)};
-    return cudaLaunchKernelExC(&cfg, kernel(args.M > 8 ? 2 : 1, l.mode, l.warps), params);
+    return cudaLaunchKernelExC(&cfg, kernel(args.M > 8 ? 2 : 1, l.mode, l.warps, args.M == 1 && args.world == 0), params);
   }
 
   static cudaError_t prepare(const FragSrc &src, int units, uint8_t *dst, int grid, cudaStream_t stream) {

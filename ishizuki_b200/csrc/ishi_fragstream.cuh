@@ -353,6 +353,43 @@ __device__ __forceinline__ void st_async128(uint32_t addr, float4 v, uint32_t mb
                : "memory");
 }
 
+// The activation rows of a group of eight: `live` rows of x; `staged`, 8 or 1, is known when the kernel is
+// compiled. Staged rows past the live ones are zeros. In the single-row variant the other seven are
+// whatever the shared memory holds: a row is a column of every MMA from there to y, and columns of no
+// row are not written.
+struct FragRows {
+  const __half *x;
+  int live, staged;
+  // task i of the staging: (unit, row)
+  __device__ __forceinline__ int2 task(int i) const { return staged == 1 ? make_int2(i, 0) : make_int2(i >> 3, i & 7); }
+};
+
+// Staging, a warp task per (unit, row): put(unit, row, v) with the values k = 8l .. 8l + 7 of lane l. All
+// loads of up to eight tasks go out before the first is used: the staging costs one L2 latency.
+template <class Put>
+__device__ __forceinline__ void frag_stage_rows(const FragArgs &a, const FragRows &m, int ub0, int uc, Put put) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, tasks = uc * m.staged;
+  constexpr int kBatch = 8;
+  const __half *xl = m.x + (long long)ub0 * 256 + lane * 8;
+  for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
+    uint4 v[kBatch];
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e) {
+      const int i = i0 + e * nw;
+      const int2 t = m.task(i);
+      v[e] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < tasks && t.y < m.live) v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)t.y * a.K + t.x * 256));
+    }
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e) {
+      const int i = i0 + e * nw;
+      if (i >= tasks) break;
+      const int2 t = m.task(i);
+      put(t.x, t.y, v[e]);
+    }
+  }
+}
+
 // A decoder's shared-memory tables (kExtraBytes, a multiple of 16), laid out once per device from
 // Fmt::table_word; every CTA copies them from here, a few 16-byte async copies per thread that land
 // while it waits for the launch before. Building them in place, lookups and conversions ahead of the
@@ -366,10 +403,14 @@ __global__ void fill_table_kernel() {
 }
 
 // MODE 0: tensor-core (up to eight rows per column group); MODE 1: CUDA-core FMA for a single row.
-// MAXW: most warps of a block. NB: column groups of eight activation rows, 1 or 2.
-template <class Fmt, int MODE, int MAXW, int NB>
+// MAXW: most warps of a block. NB: column groups of eight activation rows, 1 or 2. ONE: a single activation
+// row on the tensor cores, which stages that row alone (17408 x 5120: 0.6 us less in affine 4-bit, 1.5 us
+// in ternary, whose staging rotates; a variant of its own because the choice inside one kernel costs
+// eight rows 0.5 us).
+template <class Fmt, int MODE, int MAXW, int NB, bool ONE = false>
 __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   static_assert(MODE == 0 || NB == 1, "the CUDA-core variant takes one row");
+  static_assert(!ONE || (MODE == 0 && NB == 1), "one row is one column group");
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kTile = Fmt::kTileBytes;
   constexpr uint32_t kStride = (uint32_t)((kTile + 15) & ~15), kPart = NB * 512u, kPark = NB * 1024u;  // bytes of a partial tile in fp32, fp64
@@ -481,7 +522,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   // activations of the column range into fragment order (all warps)
 #pragma unroll
   for (int b = 0; b < NB; ++b)
-    Fmt::stage_x(a, a.x + (long long)(8 * b) * a.K, a.M - 8 * b, xfrag + b * a.xregion, ub0, uc);
+    Fmt::stage_x(a, FragRows{a.x + (long long)(8 * b) * a.K, ONE ? 1 : a.M - 8 * b, ONE ? 1 : 8}, xfrag + b * a.xregion, ub0, uc);
   ISHI_STAMP(3);
   if (Fmt::kExtraBytes) {  // the tables have landed: all groups but the R - 1 tiles' behind them
     if (R == 2) cp_async_wait<1>();

@@ -354,12 +354,14 @@ __device__ __forceinline__ void st_async128(uint32_t addr, float4 v, uint32_t mb
 }
 
 // The activation rows of a group of eight: `live` rows of x; `staged`, 8 or 1, is known when the kernel is
-// compiled. Staged rows past the live ones are zeros. In the single-row variant the other seven are
+// compiled. Staged rows past the live ones are zeros, in the single-row variant the other seven are
 // whatever the shared memory holds: a row is a column of every MMA from there to y, and columns of no
-// row are not written.
+// row are not written. Staging that is dear (the rotation on the tensor cores) leaves out the rows from
+// `stored` on; it is eight where an output exchange stores all columns. (Plain staging loses by the
+// extra branch: 1-3 % of a launch.)
 struct FragRows {
   const __half *x;
-  int live, staged;
+  int live, stored, staged;
   // task i of the staging: (unit, row)
   __device__ __forceinline__ int2 task(int i) const { return staged == 1 ? make_int2(i, 0) : make_int2(i >> 3, i & 7); }
 };
@@ -522,7 +524,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   // activations of the column range into fragment order (all warps)
 #pragma unroll
   for (int b = 0; b < NB; ++b)
-    Fmt::stage_x(a, FragRows{a.x + (long long)(8 * b) * a.K, ONE ? 1 : a.M - 8 * b, ONE ? 1 : 8}, xfrag + b * a.xregion, ub0, uc);
+    Fmt::stage_x(a, FragRows{a.x + (long long)(8 * b) * a.K, ONE ? 1 : a.M - 8 * b, ONE ? 1 : a.world > 0 ? 8 : a.M - 8 * b, ONE ? 1 : 8}, xfrag + b * a.xregion, ub0, uc);
   ISHI_STAMP(3);
   if (Fmt::kExtraBytes) {  // the tables have landed: all groups but the R - 1 tiles' behind them
     if (R == 2) cp_async_wait<1>();

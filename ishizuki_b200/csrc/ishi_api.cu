@@ -465,7 +465,7 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
   c.P = (int)((d.n + kFragRows - 1) / kFragRows);
   c.S = s, c.W = w, c.NB = groups;
   c.tile_bytes = ops->tile_bytes;
-  if (s < 1 || s > kFragMaxSplit || s > c.units || w < 1 || w > (groups == 2 ? kFragFewWarps : kFragMaxWarps)) return false;
+  if (s < 1 || s > kFragMaxSplit || s > c.units || w < 1 || w > (groups == 2 ? ops->many_warps : kFragMaxWarps)) return false;
   // the kernel divides by multiplication, exact while (clusters + 1) * P < 2^32 / clusters
   if ((long long)c.P * (ctx->sm_count + 1) * ctx->sm_count >= (1ll << 32)) return false;
   c.umax = (c.units + s - 1) / s;

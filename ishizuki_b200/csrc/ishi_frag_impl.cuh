@@ -11,10 +11,10 @@ template <class Fmt>
 struct FragOpsOf {
   // the variant that serves a launch: column groups of eight rows, CUDA cores or not, block size, a
   // single row of no exchange (which stores all eight columns).
-  // Two column groups keep twice the accumulators: at most kFragFewWarps warps.
+  // Two column groups keep twice the accumulators and activations: at most Fmt::kManyWarps warps.
   static const void *kernel(int groups, int mode, int warps, bool one) {
     const bool few = warps <= kFragFewWarps;
-    if (groups == 2) return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 2> : nullptr;
+    if (groups == 2) return warps <= Fmt::kManyWarps ? (const void *)frag_kernel<Fmt, 0, Fmt::kManyWarps, 2> : nullptr;
     if constexpr (Fmt::kRowMode) {
       // (a format without a CUDA-core variant for one activation row runs that row through the MMA path)
       if (mode == 1) return few ? (const void *)frag_kernel<Fmt, 1, kFragFewWarps, 1> : (const void *)frag_kernel<Fmt, 1, kFragMaxWarps, 1>;
@@ -26,7 +26,7 @@ struct FragOpsOf {
   static cudaError_t configure(int max_smem) {
     for (int groups = 1; groups <= 2; ++groups)
       for (int mode = 0; mode < 2; ++mode)
-        for (int warps : {kFragFewWarps, kFragMaxWarps})
+        for (int warps : {Fmt::kManyWarps, kFragFewWarps, kFragMaxWarps})
           for (bool one : {false, true})
             if (const void *k = kernel(groups, mode, warps, one)) {
               const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
@@ -94,7 +94,7 @@ struct FragOpsOf {
   }
 
   static constexpr FragOps ops() {
-    return FragOps{Fmt::kTileBytes, Fmt::kXBytes, Fmt::kXFixed, Fmt::kExtraBytes, &configure, &max_clusters, &launch, &prepare};
+    return FragOps{Fmt::kTileBytes, Fmt::kXBytes, Fmt::kXFixed, Fmt::kExtraBytes, Fmt::kManyWarps, &configure, &max_clusters, &launch, &prepare};
   }
 };
 

@@ -22,6 +22,7 @@ struct FragLaunch {
 struct FragOps {
   int tile_bytes;
   int x_bytes, x_fixed, x_extra;  // a staged region of eight rows: bytes per unit of the column range, once; tables per CTA
+  int many_warps;  // most warps of a launch of nine to sixteen rows
   // raises the dynamic shared memory limit of every variant and lays out the decoder's tables (once per device; synchronises)
   cudaError_t (*configure)(int max_smem);
   // how many clusters of `split` CTAs the device keeps resident, 0 if the launch is impossible; groups: of eight rows

@@ -249,6 +249,23 @@ def test_runs_of_tiles_that_share_panels(type_id, n, k):
     lin.ctx.poll()
 
 
+@pytest.mark.parametrize("warps", [4, 16, 20])
+@pytest.mark.parametrize("type_id", TYPES)
+def test_largest_block_of_a_launch_of_nine_to_sixteen_rows(type_id, warps, monkeypatch):
+    """Formats differ in the most warps of a block that takes nine to sixteen rows; past it, and past shared
+    memory, the rows go in pieces of eight."""
+    rng = np.random.default_rng(int(type_id) * 7 + warps)
+    n, k = 1000, 2048
+    blocks = synth.ggml_blocks(rng, int(type_id), n, k)
+    monkeypatch.setenv("ISHI_FRAG_PLAN", f"2,4,{warps},2")  # one range of columns per CTA: `warps` warps
+    lin = PackedLinear(ggml=GGUFBlocks(dev(blocks), type_id, (n, k)))
+    for m in (9, 16):
+        x = synth.activations(rng, m, k)
+        want32, _ = oracle.ggml_matmul(int(type_id), blocks, x, n)
+        assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
+    lin.ctx.poll()
+
+
 @pytest.mark.parametrize("type_id", OTHERS)
 @pytest.mark.parametrize("m", [1, 8, 16])
 def test_projection_of_the_other_block_formats(type_id, m):

@@ -45,6 +45,7 @@ struct FragAffine {
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
+  static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
   // most warps at nine to sixteen rows: a 2-bit pack without rotated inputs gains nothing from the registers
   static constexpr int kManyWarps = BITS == 2 && !BF16 ? 20 : 16;
   static constexpr int kXBytes = 4096 + (32 * kGroups > 128 ? 32 * kGroups : 128), kXFixed = 0;  // per unit of a staged region

@@ -32,6 +32,7 @@ struct FragGGML {
   static constexpr double kUnit = 1.0;  // unit of the tile results
   static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;     // one activation row runs through the MMA path as well
+  static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
   static constexpr int kManyWarps = 20;       // most warps at nine to sixteen rows
 
   static __device__ __forceinline__ uint8_t tile_byte(const FragSrc &s, long long p, int u, int b) {

@@ -47,6 +47,7 @@ struct FragIQ1 {
   static constexpr double kUnit = 1.0;  // unit of the tile results
   static constexpr int kExtraBytes = 2048 * 32;  // the grid, four copies interleaved
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
+  static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
   static constexpr int kManyWarps = 16;  // most warps at nine to sixteen rows
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {

@@ -75,6 +75,7 @@ struct FragIQ2 {
   static constexpr double kUnit = 0.125;         // tile results come in units of 1/8
   static constexpr int kExtraBytes = kEntries * kCopies * 16;  // the grid as fp16, its copies interleaved
   static constexpr bool kRowMode = false;        // one activation row runs through the MMA path as well
+  static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
   static constexpr int kManyWarps = kWide ? 20 : 16;  // most warps at nine to sixteen rows
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {

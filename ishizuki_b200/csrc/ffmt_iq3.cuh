@@ -43,6 +43,7 @@ struct FragIQ3 {
   static constexpr double kUnit = kNine ? 1.0 : 0.25;  // unit of the tile results
   static constexpr int kExtraBytes = kEntries * 128;  // the grid as fp16, sixteen copies interleaved
   static constexpr bool kRowMode = false;  // one activation row runs through the MMA path as well
+  static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
   static constexpr int kManyWarps = 16;  // most warps at nine to sixteen rows
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {

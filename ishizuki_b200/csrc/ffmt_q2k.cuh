@@ -34,6 +34,7 @@ struct FragQ2K {
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;       // one activation row runs through the MMA path as well
+  static constexpr int kFewWarps = 16;  // most warps of the smaller block size at up to eight rows
   static constexpr int kManyWarps = 20;  // most warps at nine to sixteen rows
 
   static __device__ __forceinline__ const uint8_t *block(const FragSrc &s, long long row, int u) {

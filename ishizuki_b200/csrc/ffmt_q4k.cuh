@@ -46,6 +46,7 @@ struct FragQ4K {
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
+  static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
   static constexpr int kManyWarps = 16;  // most warps at nine to sixteen rows
   static constexpr int kSumBytes = 384;  // per unit: sub-block sums as fp16 hi / lo pairs, [lane][8 bytes], then
                                          // the fp32 sub-block sums of row 0 (single-row kernel) @256

@@ -43,6 +43,7 @@ struct FragQ6K {
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
+  static constexpr int kFewWarps = 16;  // most warps of the smaller block size at up to eight rows
   static constexpr int kManyWarps = 20;  // most warps at nine to sixteen rows
 
   // the low four and the high two bits of weight k of a block

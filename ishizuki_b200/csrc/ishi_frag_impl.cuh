@@ -13,20 +13,20 @@ struct FragOpsOf {
   // single row of no exchange (which stores all eight columns).
   // Two column groups keep twice the accumulators and activations: at most Fmt::kManyWarps warps.
   static const void *kernel(int groups, int mode, int warps, bool one) {
-    const bool few = warps <= kFragFewWarps;
+    const bool few = warps <= Fmt::kFewWarps;
     if (groups == 2) return warps <= Fmt::kManyWarps ? (const void *)frag_kernel<Fmt, 0, Fmt::kManyWarps, 2> : nullptr;
     if constexpr (Fmt::kRowMode) {
       // (a format without a CUDA-core variant for one activation row runs that row through the MMA path)
-      if (mode == 1) return few ? (const void *)frag_kernel<Fmt, 1, kFragFewWarps, 1> : (const void *)frag_kernel<Fmt, 1, kFragMaxWarps, 1>;
+      if (mode == 1) return few ? (const void *)frag_kernel<Fmt, 1, Fmt::kFewWarps, 1> : (const void *)frag_kernel<Fmt, 1, kFragMaxWarps, 1>;
     }
-    if (one) return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 1, true> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1, true>;
-    return few ? (const void *)frag_kernel<Fmt, 0, kFragFewWarps, 1> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1>;
+    if (one) return few ? (const void *)frag_kernel<Fmt, 0, Fmt::kFewWarps, 1, true> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1, true>;
+    return few ? (const void *)frag_kernel<Fmt, 0, Fmt::kFewWarps, 1> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1>;
   }
 
   static cudaError_t configure(int max_smem) {
     for (int groups = 1; groups <= 2; ++groups)
       for (int mode = 0; mode < 2; ++mode)
-        for (int warps : {Fmt::kManyWarps, kFragFewWarps, kFragMaxWarps})
+        for (int warps : {Fmt::kManyWarps, Fmt::kFewWarps, kFragMaxWarps})
           for (bool one : {false, true})
             if (const void *k = kernel(groups, mode, warps, one)) {
               const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);

@@ -19,10 +19,17 @@
 // each half of a word has one value at bits 4..9 (a register for one mask), one at bits 10..15 (a shift
 // and a mask) and four bits below; the low nibbles of the first k-step's row g are those of words 0
 // and 1, their high bit pairs bits 0..1 and 2..3 of word 2. That is fifteen bit operations for eight
-// registers, where nibbles and bit pairs in words of their own take twenty-one. The row whose values
-// lie at bits 0..5 has its own sums, in units of 2^-24; all others are sixteen times as large.
+// registers, where nibbles and bit pairs in words of their own take twenty-one. The first k-step's
+// registers all hold q * 2^-24 (row g's put together at bits 0..5, row g + 8's shifted there from bits
+// 10..15), the second's q * 2^-20. A k-step has one unit for both rows because the MMA's rounding
+// depends on it (codes of the larger unit lose fewer low bits of a product), and both rows add up their
+// k-steps in the same order: a weight row's product must not depend on which half of a panel it
+// lies in, or a gated pair and the same two weights stacked differ.
 // The loop is bound by the integer pipe and by memory in equal parts: 17408 x 5120 at eight
-// rows 19.1 -> 16.7 us, 587 -> 498 warp instructions a tile; 248320 x 5120 213 -> 182 us, 5.7 TB/s.
+// rows 19.1 -> 16.9 us; 248320 x 5120 at eight rows 213 -> 175 us in short runs, 5.9 TB/s (a loop of
+// seconds runs into the power cap: 219). Row g + 8's first k-steps in the larger unit and row g's with sums
+// of their own took as long at eight rows, 23.4 instead of 24.4 us at sixteen rows of 17408 x 5120, but
+// 112 of 65536 products of a weight turned by eight rows changed.
 // Inside a k-step the lane t holds the weights 4t .. 4t + 3 of the group: slots (2t, 2t + 1) are
 // 4t, 4t + 1 and slots (2t + 8, 2t + 9) are 4t + 2, 4t + 3; the activations are staged in the same
 // order, so that a lane reads the B registers of two k-steps with one 16-byte load.
@@ -74,11 +81,11 @@ struct FragQ6K {
       const int k0 = 32 * pi + 4 * t + h, k1 = k0 + 16;
       uint32_t out = 0;
       if (w == 0) {
-        if (top) out = low4(top, k0);
-        if (low) out |= (code(low, k0) << 4) | (code(low, k0 + 2) << 10);
+        if (top) out = low4(top, k0) | (code(top, k1) << 4);
+        if (low) out |= code(low, k0) << 10;
       } else if (w == 1) {
-        if (top) out = low4(top, k0 + 2) | (code(top, k1) << 4);
-        if (low) out |= code(low, k1) << 10;
+        if (top) out = low4(top, k0 + 2);
+        if (low) out |= (code(low, k1) << 4) | (code(low, k0 + 2) << 10);
       } else {
         if (top) out = high2(top, k0) | (high2(top, k0 + 2) << 2) | (code(top, k1 + 2) << 4);
         if (low) out |= code(low, k1 + 2) << 10;
@@ -129,9 +136,12 @@ struct FragQ6K {
     });
   }
 
-  // byte `byte` of a word of scales + 128 as the scale: the low mantissa bits of 2^23
+  // byte `byte` of a word of scales + 128 as the scale: the low mantissa bits of 2^23; SIXTEEN: as sixteen
+  // times the scale, the low mantissa bits of 2^27
+  template <bool SIXTEEN = false>
   static __device__ __forceinline__ float scale_of(uint32_t word, int byte) {
-    return __uint_as_float(prmt(word, 0x4b000000u, 0x7650u + (uint32_t)byte)) - 8388736.f;
+    return __uint_as_float(prmt(word, SIXTEEN ? 0x4d000000u : 0x4b000000u, 0x7650u + (uint32_t)byte)) -
+           (SIXTEEN ? 16.f * 8388736.f : 8388736.f);
   }
   // two of its bytes as a half2: the low mantissa bits of 1024
   static __device__ __forceinline__ uint32_t scale_pair(uint32_t word, uint32_t selector) {
@@ -148,9 +158,15 @@ struct FragQ6K {
     const uint4 h0 = lds128(tile + 3072u + (uint32_t)g * 16u), h1 = lds128(tile + 3072u + (uint32_t)(g + 8) * 16u);
     const uint32_t hw0[4] = {h0.x, h0.y, h0.z, h0.w}, hw1[4] = {h1.x, h1.y, h1.z, h1.w};
     const uint32_t lane_off = (uint32_t)g * 64u + (uint32_t)t * 16u;
-    float su[NB][2], sv[NB][4];  // first k-steps of row g; all others, sixteen times as large
+    // The first k-steps of the pairs are added up in su, the second, sixteen times as large, in sv. Two column
+    // groups have no registers for both (20 warps spill; 16 warps lose as much): sixteen times the first k-steps'
+    // scales, one sum.
+    constexpr bool kOneSum = NB == 2;
+    float su[NB][4], sv[NB][4];
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = sv[nb][0] = sv[nb][1] = sv[nb][2] = sv[nb][3] = 0.f;
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) su[nb][i] = sv[nb][i] = 0.f;
     uint32_t qw[12];  // the words of four pairs
 #pragma unroll
     for (int pi = 0; pi < 8; ++pi) {
@@ -163,22 +179,23 @@ struct FragQ6K {
       }
       const uint32_t w0 = qw[3 * (pi & 3)], w1 = qw[3 * (pi & 3) + 1], w2 = qw[3 * (pi & 3) + 2];
       const uint32_t a0 = (w0 & 0x000f000fu) | ((w2 << 4) & 0x00300030u), a2 = (w1 & 0x000f000fu) | ((w2 << 2) & 0x00300030u);
-      const uint32_t a1 = w0 & 0x03f003f0u, a3 = (w0 >> 6) & 0x03f003f0u;
-      const uint32_t e0 = w1 & 0x03f003f0u, e1 = (w1 >> 6) & 0x03f003f0u;
+      const uint32_t a1 = (w0 >> 10) & 0x003f003fu, a3 = (w1 >> 10) & 0x003f003fu;
+      const uint32_t e0 = w0 & 0x03f003f0u, e1 = w1 & 0x03f003f0u;
       const uint32_t e2 = w2 & 0x03f003f0u, e3 = (w2 >> 6) & 0x03f003f0u;
       // scales of groups 2 pi and 2 pi + 1: word pi % 4 of the row's sixteen, bytes 2 (pi / 4) and + 1
-      const float s00 = scale_of(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1);
-      const float s10 = scale_of(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1);
+      const float s00 = scale_of<kOneSum>(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1);
+      const float s10 = scale_of<kOneSum>(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1);
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
         const uint4 b = lds128(xu + nb * a.xregion + (uint32_t)pi * 512u + (lane_off ^ (uint32_t)(pi << 6)));
         float c0[4], c1[4];
         mma16816_first(c0, a0, a1, a2, a3, b.x, b.y);
         mma16816_first(c1, e0, e1, e2, e3, b.z, b.w);
+        float(&sw)[4] = kOneSum ? su[nb] : sv[nb];
         su[nb][0] = fmaf(s00, c0[0], su[nb][0]), su[nb][1] = fmaf(s00, c0[1], su[nb][1]);
-        sv[nb][2] = fmaf(s10, c0[2], sv[nb][2]), sv[nb][3] = fmaf(s10, c0[3], sv[nb][3]);
-        sv[nb][0] = fmaf(s01, c1[0], sv[nb][0]), sv[nb][1] = fmaf(s01, c1[1], sv[nb][1]);
-        sv[nb][2] = fmaf(s11, c1[2], sv[nb][2]), sv[nb][3] = fmaf(s11, c1[3], sv[nb][3]);
+        su[nb][2] = fmaf(s10, c0[2], su[nb][2]), su[nb][3] = fmaf(s10, c0[3], su[nb][3]);
+        sw[0] = fmaf(s01, c1[0], sw[0]), sw[1] = fmaf(s01, c1[1], sw[1]);
+        sw[2] = fmaf(s11, c1[2], sw[2]), sw[3] = fmaf(s11, c1[3], sw[3]);
       }
     }
     // sum_g scale_g * (sum of x over group g): the MMA over groups; this lane's slots are groups
@@ -196,10 +213,11 @@ struct FragQ6K {
       float cm[4];
       mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
       mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);
-      acc[nb][0] = fmaf(d0, fmaf(sv[nb][0], 0.0625f, su[nb][0]), fmaf(dm0, cm[0], acc[nb][0]));
-      acc[nb][1] = fmaf(d0, fmaf(sv[nb][1], 0.0625f, su[nb][1]), fmaf(dm0, cm[1], acc[nb][1]));
-      acc[nb][2] = fmaf(d1 * 0.0625f, sv[nb][2], fmaf(dm1, cm[2], acc[nb][2]));
-      acc[nb][3] = fmaf(d1 * 0.0625f, sv[nb][3], fmaf(dm1, cm[3], acc[nb][3]));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float sum = kOneSum ? su[nb][i] * 0.0625f : fmaf(sv[nb][i], 0.0625f, su[nb][i]);
+        acc[nb][i] = fmaf(i < 2 ? d0 : d1, sum, fmaf(i < 2 ? dm0 : dm1, cm[i], acc[nb][i]));
+      }
     }
   }
 };

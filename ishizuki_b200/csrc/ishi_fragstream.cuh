@@ -62,7 +62,7 @@ constexpr int kFragRows = 16;
 // where the decoder does not use the registers and the smaller tiles want warps. 16 rows, 17408 x 5120
 // and 5120 x 17408, 20 -> 16 warps: IQ1_S 25.7 / 31.3 -> 23.6 / 29.5 us, affine 8-bit 23.2 / 26.2 -> 21.3
 // / 24.7, affine 4-bit in groups of 32 22.9 / 27.0 -> 21.6 / 25.5, IQ4_XS 23.6 / 26.4 -> 22.8 / 25.9, IQ2_XS,
-// Q4_K, ternary and the other affine 4-bit 1 to 2 % less; Q6_K 23.2 / 28.0 -> 24.0 / 28.9, Q2_K 21.2 / 24.3
+// Q4_K, ternary and the other affine 4-bit 1 to 2 % less; Q6_K 24.4 / 28.8 -> 24.3 / 29.9, Q2_K 21.2 / 24.3
 // -> 21.6 / 26.0, affine 2-bit 19.4 / 21.7 -> 19.5 / 22.4, IQ2_S the same: these stay at 20.
 constexpr int kFragMaxWarps = ISHI_FRAG_MAX_WARPS;
 constexpr int kFragMaxRing = 4;   // most tiles per warp-private ring (FragArgs::ring of them are used:

@@ -381,6 +381,23 @@ def test_a_projection_under_another_ones_plan_gives_the_same_bits():
         b.set_plan((2, 25, 8, 3))  # more warps than a block holds: not a plan of this projection
 
 
+@pytest.mark.parametrize("type_id", TYPES)
+def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(type_id):
+    """A panel is sixteen weight rows, a lane works on row g of its upper and of its lower eight. The same
+    weight turned by eight rows moves every row to the other half: the same products bit for bit under
+    the same plan. (A gated pair lies in halves in which the two weights stacked do not.)"""
+    rng = np.random.default_rng(int(type_id) + 900)
+    n, k = 2048, 5120
+    blocks = synth.ggml_blocks(rng, int(type_id), n, k).reshape(n, -1)
+    here = PackedLinear(ggml=GGUFBlocks(dev(blocks.reshape(-1)), type_id, (n, k)))
+    there = PackedLinear(ggml=GGUFBlocks(dev(np.roll(blocks, 8, axis=0).reshape(-1)), type_id, (n, k)))
+    there.set_plan(here.plan)
+    for m in (1, 8, 16):
+        x = dev(synth.activations(rng, m, k))
+        assert torch.equal(there(x), torch.roll(here(x), 8, 1))
+    here.ctx.poll()
+
+
 @pytest.mark.parametrize("type_id", [GGMLType.q4K, GGMLType.q6K])
 def test_rotated_input_ahead_of_a_gguf_projection(type_id):
     """A GGUF projection with a rotation block: the input goes through the stand-alone rotation

@@ -253,6 +253,13 @@ struct FragAffine {
   static __device__ __forceinline__ float half_lo(uint32_t pair) { return __half2float(__ushort_as_half((unsigned short)(pair & 0xffffu))); }
   static __device__ __forceinline__ float half_hi(uint32_t pair) { return __half2float(__ushort_as_half((unsigned short)(pair >> 16))); }
 
+  // acc += scale * codes + bias * xs, its roundings spelled out: left to the compiler, which of the two products
+  // goes into the fused multiply-add differs between the rows of a lane, and a weight row's product with
+  // its half of a panel
+  static __device__ __forceinline__ void add_group(float &acc, float scale, float codes, float bias, float xs) {
+    acc = __fadd_rn(acc, __fmaf_rn(scale, codes, __fmul_rn(bias, xs)));
+  }
+
   // One tile against the activations of its unit. acc: the warp's C fragment (MODE 0) or this
   // lane's partial dot products of rows g (acc[0]) and g + 8 (acc[2]) (MODE 1).
   template <int MODE, int NB>
@@ -322,16 +329,16 @@ struct FragAffine {
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb) {
               const float2 xs = lds64f(xu + nb * a.xregion + kSums + (uint32_t)(grp * 8 + 2 * t) * 4u);
-              acc[nb][0] += s0 * part[nb][0] + b0 * xs.x;
-              acc[nb][1] += s0 * part[nb][1] + b0 * xs.y;
-              acc[nb][2] += s1 * part[nb][2] + b1 * xs.x;
-              acc[nb][3] += s1 * part[nb][3] + b1 * xs.y;
+              add_group(acc[nb][0], s0, part[nb][0], b0, xs.x);
+              add_group(acc[nb][1], s0, part[nb][1], b0, xs.y);
+              add_group(acc[nb][2], s1, part[nb][2], b1, xs.x);
+              add_group(acc[nb][3], s1, part[nb][3], b1, xs.y);
             }
           } else {
             // the bias term enters once per row: lane t = 0 adds it
             const float xs = t == 0 ? lds32f(xu + kSums + (uint32_t)(grp * 8) * 4u) : 0.f;
-            acc[0][0] += s0 * part[0][0] + b0 * xs;
-            acc[0][2] += s1 * part[0][2] + b1 * xs;
+            add_group(acc[0][0], s0, part[0][0], b0, xs);
+            add_group(acc[0][2], s1, part[0][2], b1, xs);
           }
         }
       }

@@ -176,3 +176,27 @@ def test_rotation_inside_the_product_kernel(block, signed):
         want32, _ = oracle.affine_matmul(w, s, b, 4, 64, xr)
         assert rel_err(y.cpu().numpy(), want32) < TOL
     lin.ctx.poll()
+
+
+@pytest.mark.parametrize("bits,gs", [(2, 64), (2, 128), (4, 32), (4, 64), (4, 128), (8, 32), (8, 64), (8, 128)])
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(bits, gs, dtype):
+    """The same pack turned by eight rows, half a panel of the kernel: the same products bit for bit under
+    the same plan, on tensor cores in one and two column groups and, a single row, on CUDA cores."""
+    from ishizuki_b200 import _lib
+    from ishizuki_b200.interface import BonsaiRuntime
+
+    rng = np.random.default_rng(bits * 1000 + gs)
+    n, k = 2048, 5120
+    w, s, b, sd, bd, bf16 = make_pack(rng, n, k, bits, gs, dtype)
+    here = PackedLinear(dev(w), sd, bd, None, 0, groupSize=gs, bits=bits)
+    there = PackedLinear(dev(np.roll(w, 8, axis=0)), torch.roll(sd, 8, 0), torch.roll(bd, 8, 0), None, 0, groupSize=gs, bits=bits)
+    there.set_plan(here.plan)
+    for rows, route in ((1, _lib.ROUTE_AUTO), (1, _lib.ROUTE_GEMV), (8, _lib.ROUTE_AUTO), (16, _lib.ROUTE_AUTO)):
+        x = dev(synth.activations(rng, rows, k))
+        BonsaiRuntime.route = route
+        try:
+            assert torch.equal(there(x), torch.roll(here(x), 8, 1)), (rows, route)
+        finally:
+            BonsaiRuntime.route = _lib.ROUTE_AUTO
+    here.ctx.poll()

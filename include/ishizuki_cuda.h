@@ -192,7 +192,8 @@ ishi_status ishi_projection_apply_host_async(ishi_projection *p, const void *x_h
  * caller's stream ends behind all of them, so one cudaStreamSynchronize(stream) completes the whole
  * list. Page-locked inputs (16-byte aligned) are read by a kernel between the products, other
  * buffers go through the copy engines in chunks of entries. The projections must share a context and
- * are independent of each other (none reads another's output). */
+ * are independent of each other (none reads another's output). The first call allocates the device
+ * staging of all projections that have none yet in one piece, freed with the last of them. */
 ishi_status ishi_projection_apply_host_batch(ishi_projection *const *projections,
                                              const void *const *x_hosts, int rows,
                                              void *const *y_hosts, int count, void *stream);

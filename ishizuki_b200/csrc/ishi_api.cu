@@ -958,91 +958,102 @@ ishi_status ishi_verify_matmul(ishi_ctx *ctx, const void *x, int rows, const voi
 
 // ---- projection: the PackedLinear counterpart ---------------------------------------------------
 
-// The tile layout does not depend on the launch plan, so the plan can be chosen by measurement:
-// the planner's best candidates run a few times on the projection's own tiles (activations of
-// zeros, eight or sixteen rows) and the fastest stays.
-static void tune_frag_plan(ishi_ctx *ctx, ishi_projection *p, int groups, std::vector<FragPlan> *candidates) {
-  constexpr size_t kTuned = 16;
-  constexpr int kLaunches = 4;
-  FragPlan *plan = groups == 2 ? &p->frag.many : &p->frag.few;
-  if (candidates->size() < 2) return;
-  // a shape measured before on this context keeps its plan (all layers of a model then agree)
-  const auto key = std::make_tuple((const void *)plan->ops, (long long)p->d.n, (long long)p->d.k, groups);
-  const auto known = ctx->tuned.find(key);
-  if (known != ctx->tuned.end()) {
-    for (const FragPlan &c : *candidates)
-      if (c.S == known->second[0] && c.W == known->second[1] && c.ring == known->second[2]) {
-        *plan = c;
-        return;
+// The tile layout does not depend on the launch plan, so the plans of both launches (up to eight rows, and nine
+// to sixteen) can be chosen by measurement: the planner's best candidates run a few times on the
+// projection's own tiles (activations of zeros, eight or sixteen rows) and the fastest stays.
+// What the measurement costs counts, since the first projection of every shape pays for it: one pair of buffers
+// for both launches, one wait per pass, and no more candidates and launches than the choice needs (create
+// for 17408 x 5120, Q4_K 8.0 -> 4.6 ms, Q6_K 9.7 -> 5.6, against sixteen candidates, four launches and sixteen,
+// a wait per candidate; 512 x 1024 2.0 -> 1.1). Over ten shapes of five formats the choice stays within
+// 3 % (8 % on 4096 x 4096) of the best plan as before; with one launch per candidate in the first pass it
+// is up to 30 % behind.
+static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragPlan> *few, std::vector<FragPlan> *many) {
+  constexpr size_t kTuned[2] = {12, 10}, kFinalists = 4;
+  constexpr int kLaunches = 3, kFinalLaunches = 8;
+  constexpr float kBehind = 1.15f;  // a candidate this far behind in the first pass is no finalist
+  typedef std::pair<float, const FragPlan *> Timed;
+  const size_t x_bytes = (size_t)16 * p->d.k * sizeof(__half), y_bytes = (size_t)16 * p->d.n * sizeof(__half);
+  uint8_t *buffer = nullptr;  // x, then y
+  cudaEvent_t marks[2 * kTuned[0]] = {nullptr};
+  for (int groups = 1; groups <= 2; ++groups) {
+    std::vector<FragPlan> *candidates = groups == 2 ? many : few;
+    FragPlan *plan = groups == 2 ? &p->frag.many : &p->frag.few;
+    if (candidates->size() < 2) continue;
+    // a shape measured before on this context keeps its plan (all layers of a model then agree)
+    const auto key = std::make_tuple((const void *)plan->ops, (long long)p->d.n, (long long)p->d.k, groups);
+    const auto known = ctx->tuned.find(key);
+    if (known != ctx->tuned.end()) {
+      const FragPlan *same = nullptr;
+      for (const FragPlan &c : *candidates)
+        if (c.S == known->second[0] && c.W == known->second[1] && c.ring == known->second[2]) same = &c;
+      if (same) {
+        *plan = *same;
+        continue;
       }
-  }
-  std::sort(candidates->begin(), candidates->end(), [](const FragPlan &a, const FragPlan &b) { return a.cost < b.cost; });
-  if (candidates->size() > kTuned) candidates->resize(kTuned);
-  const int rows = 8 * groups;
-  __half *x = nullptr, *y = nullptr;
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  bool ok = cudaMalloc(&x, (size_t)rows * p->d.k * sizeof(__half)) == cudaSuccess &&
-            cudaMalloc(&y, (size_t)rows * p->d.n * sizeof(__half)) == cudaSuccess &&
-            cudaMemset(x, 0, (size_t)rows * p->d.k * sizeof(__half)) == cudaSuccess && cudaEventCreate(&e0) == cudaSuccess &&
-            cudaEventCreate(&e1) == cudaSuccess;
-  // one timing: a warm-up launch, then `launches` back to back between two events
-  auto time_plan = [&](const FragPlan &c, int launches, float *ms_per_launch) {
-    FragPlans both;
-    both.few = both.many = c;
-    auto launch = [&] { return run_frag(ctx, both, p->ws, p->d, x, rows, y, p->d.n, 0, false, true, false, 0) == ISHI_OK; };
-    bool fine = launch();
-    if (fine) fine = cudaEventRecord(e0, 0) == cudaSuccess;
-    for (int r = 0; fine && r < launches; ++r) fine = launch();
-    if (fine) fine = cudaEventRecord(e1, 0) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess;
-    float ms = 0.f;
-    if (fine) fine = cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess;
-    *ms_per_launch = ms / launches;
-    return fine;
-  };
-  // first pass over all candidates, then the best few again with more launches (the first pass
-  // alone picks among near-equal plans by noise)
-  constexpr size_t kFinalists = 4;
-  std::vector<std::pair<float, const FragPlan *>> timed;
-  for (size_t i = 0; ok && i < candidates->size(); ++i) {
-    float ms = 0.f;
-    ok = time_plan((*candidates)[i], kLaunches, &ms);
-    if (ok) timed.push_back({ms, &(*candidates)[i]});
-  }
-  std::sort(timed.begin(), timed.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
-  float best_ms = 0.f;
-  const FragPlan *best = nullptr;
-  std::vector<std::pair<float, const FragPlan *>> finals;
-  for (size_t i = 0; ok && i < timed.size() && i < kFinalists; ++i) {
-    float ms = 0.f;
-    ok = time_plan(*timed[i].second, 4 * kLaunches, &ms);
-    if (ok) finals.push_back({ms, timed[i].second});
-    if (ok && (!best || ms < best_ms)) best = timed[i].second, best_ms = ms;
-  }
-  // Near-equal finalists: the smaller cluster wins. The timing repeats one launch, where the SMs
-  // fall free in the pattern the next launch's clusters need; between launches of different shapes
-  // a large cluster waits longer for its SMs of one GPC, which this timing does not see (measured
-  // on the benchmark's stack: 3 % per layer between K splits of 4 and 5 that time within 2 %).
-  const char *tie_env = getenv("ISHI_TUNE_TIE");
-  const float tie = tie_env ? (float)atof(tie_env) * 0.01f : 0.03f;
-  if (ok && best)
-    for (const auto &f : finals)
-      if (f.first <= best_ms * (1.f + tie) && f.second->S < best->S) best = f.second;
-  if (ok && best) {
+    }
+    bool ok = true;
+    if (!buffer) {
+      ok = cudaMalloc(&buffer, x_bytes + y_bytes) == cudaSuccess && cudaMemsetAsync(buffer, 0, x_bytes, 0) == cudaSuccess;
+      for (cudaEvent_t &e : marks) ok = ok && cudaEventCreate(&e) == cudaSuccess;
+    }
+    const int rows = 8 * groups;
+    // One timing of every plan in the list, fastest first: a warm-up launch, then `launches` back to back between
+    // two events; the host waits once, behind the last plan
+    auto time_plans = [&](std::vector<Timed> *plans, int launches) {
+      auto launch = [&](const FragPlan &c) {
+        FragPlans both;
+        both.few = both.many = c;
+        return run_frag(ctx, both, p->ws, p->d, buffer, rows, buffer + x_bytes, p->d.n, 0, false, true, false, 0) == ISHI_OK;
+      };
+      for (size_t i = 0; ok && i < plans->size(); ++i) {
+        const FragPlan &c = *(*plans)[i].second;
+        ok = launch(c) && cudaEventRecord(marks[2 * i], 0) == cudaSuccess;
+        for (int r = 0; ok && r < launches; ++r) ok = launch(c);
+        ok = ok && cudaEventRecord(marks[2 * i + 1], 0) == cudaSuccess;
+      }
+      ok = ok && cudaEventSynchronize(marks[2 * plans->size() - 1]) == cudaSuccess;
+      for (size_t i = 0; ok && i < plans->size(); ++i) {
+        float ms = 0.f;
+        ok = cudaEventElapsedTime(&ms, marks[2 * i], marks[2 * i + 1]) == cudaSuccess;
+        (*plans)[i].first = ms / launches;
+      }
+      if (ok) std::sort(plans->begin(), plans->end(), [](const Timed &a, const Timed &b) { return a.first < b.first; });
+    };
+    // a first pass over all candidates, then the best few again with more launches (the first pass
+    // alone picks among near-equal plans by noise)
+    std::sort(candidates->begin(), candidates->end(), [](const FragPlan &a, const FragPlan &b) { return a.cost < b.cost; });
+    if (candidates->size() > kTuned[groups - 1]) candidates->resize(kTuned[groups - 1]);
+    std::vector<Timed> timed, finals;
+    for (const FragPlan &c : *candidates) timed.push_back({0.f, &c});
+    if (ok) time_plans(&timed, kLaunches);
+    for (const Timed &t : timed)
+      if (ok && finals.size() < kFinalists && t.first <= timed[0].first * kBehind) finals.push_back(t);
+    if (ok) time_plans(&finals, kFinalLaunches);
+    if (!ok) {
+      cudaGetLastError();  // keep the estimate's choice
+      continue;
+    }
+    // Near-equal finalists: the smaller cluster wins. The timing repeats one launch, where the SMs
+    // fall free in the pattern the next launch's clusters need; between launches of different shapes
+    // a large cluster waits longer for its SMs of one GPC, which this timing does not see (measured
+    // on the benchmark's stack: 3 % per layer between K splits of 4 and 5 that time within 2 %).
+    const FragPlan *best = finals[0].second;
+    const char *tie_env = getenv("ISHI_TUNE_TIE");
+    const float tie = tie_env ? (float)atof(tie_env) * 0.01f : 0.03f;
+    for (const Timed &f : finals)
+      if (f.first <= finals[0].first * (1.f + tie) && f.second->S < best->S) best = f.second;
     *plan = *best;
     ctx->tuned[key] = {best->S, best->W, best->ring};
     if (getenv("ISHI_DEBUG_PLAN")) {
       fprintf(stderr, "ishi plan n=%lld k=%lld rows<=%d measured: split %d, %d clusters, %d warps, ring %d: %.2f us;", (long long)p->d.n,
-              (long long)p->d.k, rows, best->S, best->NC, best->W, best->ring, best_ms * 1e3f);
+              (long long)p->d.k, rows, best->S, best->NC, best->W, best->ring, finals[0].first * 1e3f);
       for (const auto &c : timed) fprintf(stderr, " %d/%d/%d:%.1f", c.second->S, c.second->W, c.second->ring, c.first * 1e3f);
       fprintf(stderr, "\n");
     }
-  } else {
-    cudaGetLastError();  // keep the estimate's choice
   }
-  if (e0) cudaEventDestroy(e0);
-  if (e1) cudaEventDestroy(e1);
-  if (x) cudaFree(x);
-  if (y) cudaFree(y);
+  for (cudaEvent_t e : marks)
+    if (e) cudaEventDestroy(e);
+  if (buffer) cudaFree(buffer);
 }
 
 static ishi_status create_projection(ishi_ctx *ctx, const ishi_weight_desc *descs, int count, bool gated,
@@ -1087,10 +1098,7 @@ static ishi_status create_projection(ishi_ctx *ctx, const ishi_weight_desc *desc
     make_frag_plan(ctx, p->d, 2, &p->frag.many, &many);
     s = ensure_workspace(ctx, &p->ws, 0, 0, p->frag.few.tiles_bytes, 0);
     if (s == ISHI_OK) s = tile_weight_frag(ctx, p->frag.few, descs, count, n_total, p->ws.tiles, 0, gated);
-    if (s == ISHI_OK && !getenv("ISHI_NO_AUTOTUNE") && !getenv("ISHI_FRAG_PLAN")) {
-      tune_frag_plan(ctx, p, 1, &few);
-      tune_frag_plan(ctx, p, 2, &many);
-    }
+    if (s == ISHI_OK && !getenv("ISHI_NO_AUTOTUNE") && !getenv("ISHI_FRAG_PLAN")) tune_frag_plans(ctx, p, &few, &many);
   } else if (count > 1) {
     delete p;
     return fail(ctx, ISHI_E_UNSUPPORTED, "only the warp-level kernel's formats can be stacked into one projection");

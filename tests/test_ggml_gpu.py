@@ -3,6 +3,8 @@
 Mirrors Tests/IshizukiKitTests/GGMLKernelTests.swift: the decode is held to the reference bit
 for bit, and the fused products are compared with "expand the weight and multiply".
 """
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -406,6 +408,31 @@ def test_stacked_affine_packs():
     for piece, (w, s, b) in zip(fused.split(y), packs):
         want32, _ = oracle.affine_matmul(w, s, b, 4, 64, x)
         assert rel_err(piece.cpu().numpy(), want32) < TOL
+
+
+def test_measuring_the_plans_of_a_new_shape_costs_no_more_than_their_choice_needs():
+    """The first projection of a shape measures the plans of both its launches: in all about eighty
+    launches of each, not the 150 that repeated timings of every candidate take."""
+    rng = np.random.default_rng(4)
+    k, spent = 5120, []
+    blocks = dev(synth.q6k_blocks(rng, 17456, k))
+
+    def seconds(work):
+        torch.cuda.synchronize()
+        begin = time.perf_counter()
+        work()
+        torch.cuda.synchronize()
+        return time.perf_counter() - begin
+
+    for n in (17408, 17424, 17440, 17456):  # the shortest of four: allocations vary
+        made = []
+        weight = GGUFBlocks(blocks[: n * k // 256 * 210], GGMLType.q6K, (n, k))
+        first = seconds(lambda: made.append(PackedLinear(ggml=weight)))
+        again = min(seconds(lambda: made.append(PackedLinear(ggml=weight))) for _ in range(3))
+        xs = [torch.zeros((m, k), dtype=torch.float16, device="cuda") for m in (8, 16)]
+        launches = min(seconds(lambda: [made[0](x) for x in xs for _ in range(50)]) for _ in range(3)) / 50
+        spent.append((first - again) / launches)
+    assert min(spent) < 150, spent
 
 
 def test_a_projection_under_another_ones_plan_gives_the_same_bits():

@@ -187,6 +187,10 @@ PyObject *gather(PyObject *, PyObject *const *a, Py_ssize_t n) {
   const int type = (int)PyLong_AsLong(a[3]);
   const int64_t per_row = PyLong_AsLongLong(a[4]), width = PyLong_AsLongLong(a[5]);
   if (PyErr_Occurred()) return nullptr;
+  if (per_row == 0) {  // an input width of 0: the division below would end the process
+    PyErr_SetString(PyExc_ZeroDivisionError, "a table row of no bytes");
+    return nullptr;
+  }
   at::ScalarType st;
   if (!output_type(a[6], &st)) return nullptr;
   ids = ids.to(at::kInt).contiguous();

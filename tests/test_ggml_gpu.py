@@ -617,6 +617,12 @@ def test_gather_decodes_the_requested_rows(type_id):
     assert GGMLKernels.gather(torch.tensor([1]).cuda(), dev(blocks), type_id, 100) is None
 
 
+def test_gather_of_rows_without_width_is_an_exception():
+    blocks, ids = torch.zeros(144, dtype=torch.uint8, device="cuda"), torch.tensor([0], device="cuda")
+    with pytest.raises(ZeroDivisionError):
+        GGMLKernels.gather(ids, blocks, GGMLType.q4K, 0)
+
+
 @pytest.mark.parametrize("type_id", [GGMLType.q4K, GGMLType.q6K, GGMLType.iq4Xs])
 @pytest.mark.parametrize("m", [1, 8, 16])
 def test_head_argmax_matches_argmax_of_the_logits(type_id, m):

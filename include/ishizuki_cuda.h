@@ -112,7 +112,7 @@ ishi_status ishi_ctx_set_route(ishi_ctx *ctx, int route, int crossover_rows);
 /* PackedLinear.init + VerifyMatmul.warm (Hadamard.swift:51-86, VerifyMatmul.swift:40-61):
  * validates the weight, allocates the projection's own memory, copies the weight into it in tiled
  * order and fixes the launch plan for its shape: for the warp-level kernel's formats by timing the
- * best dozen candidate plans on the tiled weight (1 to 5 ms for the first projection of a shape, later
+ * best ten candidate plans on the tiled weight (1 to 5 ms for the first projection of a shape, later
  * ones of the context take over its plan; ISHI_NO_AUTOTUNE=1 in the environment keeps the estimate's choice). Synchronises the device. */
 ishi_status ishi_projection_create(ishi_ctx *ctx, const ishi_weight_desc *desc,
                                    ishi_projection **out);

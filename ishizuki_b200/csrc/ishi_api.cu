@@ -963,13 +963,14 @@ ishi_status ishi_verify_matmul(ishi_ctx *ctx, const void *x, int rows, const voi
 // projection's own tiles (activations of zeros, eight or sixteen rows) and the fastest stays.
 // What the measurement costs counts, since the first projection of every shape pays for it: one pair of buffers
 // for both launches, one wait per pass, and no more candidates and launches than the choice needs (create
-// for 17408 x 5120, Q4_K 8.0 -> 4.6 ms, Q6_K 9.7 -> 5.6, against sixteen candidates, four launches and sixteen,
-// a wait per candidate; 512 x 1024 2.0 -> 1.1). Over ten shapes of five formats the choice stays within
-// 3 % (8 % on 4096 x 4096) of the best plan as before; with one launch per candidate in the first pass it
-// is up to 30 % behind.
+// for 17408 x 5120, Q4_K 8.0 -> 4.7 ms, Q6_K 9.7 -> 5.5, against sixteen candidates of each, four launches and
+// sixteen, a wait per candidate; 512 x 1024 2.0 -> 1.1). Over eleven shapes of six formats, twenty times each, the
+// choice is the one of the longer measurement, within 3.5 % of the best plan at eight rows. One launch per
+// candidate in the first pass is up to 30 % behind; with eight final launches at eight rows the events'
+// share lets more plans tie, and the choice varies from run to run.
 static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragPlan> *few, std::vector<FragPlan> *many) {
-  constexpr size_t kTuned[2] = {12, 10}, kFinalists = 4;
-  constexpr int kLaunches = 3, kFinalLaunches = 8;
+  constexpr size_t kTuned[2] = {10, 8}, kFinalists = 4;
+  constexpr int kLaunches = 3, kFinalLaunches[2] = {16, 8};
   constexpr float kBehind = 1.15f;  // a candidate this far behind in the first pass is no finalist
   typedef std::pair<float, const FragPlan *> Timed;
   const size_t x_bytes = (size_t)16 * p->d.k * sizeof(__half), y_bytes = (size_t)16 * p->d.n * sizeof(__half);
@@ -1028,7 +1029,7 @@ static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragP
     if (ok) time_plans(&timed, kLaunches);
     for (const Timed &t : timed)
       if (ok && finals.size() < kFinalists && t.first <= timed[0].first * kBehind) finals.push_back(t);
-    if (ok) time_plans(&finals, kFinalLaunches);
+    if (ok) time_plans(&finals, kFinalLaunches[groups - 1]);
     if (!ok) {
       cudaGetLastError();  // keep the estimate's choice
       continue;

@@ -177,15 +177,6 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-// 4 bytes into another CTA's shared memory; the bytes count as completed on that CTA's mbarrier
-// when they have landed, so the reader needs no fence: it waits for the barrier's phase
-__device__ __forceinline__ void st_async32(uint32_t addr, float v, uint32_t mbar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v),
-               "r"(mbar)
-               : "memory");
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // arrival without the release fence, which would wait for every copy and store in flight; the
 // data that crosses CTAs here is published by mbarriers instead
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }

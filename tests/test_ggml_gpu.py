@@ -596,7 +596,7 @@ def test_stacking_guards():
         FusedLinear([a, b])  # different input widths
     packs = [synth.affine_pack(rng, 64, 512, 8, 64, np.float16) for _ in range(2)]
     with pytest.raises(IshizukiError) as err:
-        FusedLinear([(dev(w), dev(sc), dev(b)) for w, sc, b in packs], groupSize=64, bits=8)  # 8-bit packs run on the tcgen05 kernel: cannot be stacked
+        FusedLinear([(dev(w), dev(sc), dev(b)) for w, sc, b in packs], groupSize=64, bits=8)  # 8-bit packs are not stacked (an interface the callers know)
     assert err.value.status == _lib.E_UNSUPPORTED
 
 

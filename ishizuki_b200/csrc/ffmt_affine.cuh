@@ -201,7 +201,7 @@ struct FragAffine {
         if (i >= tasks) break;
         const int2 task = rows.task(i);
         const int r = task.y;
-        if (r >= rows.stored) continue;  // 27B layers in ternary at four rows: 102 -> 97 us
+        if (r >= rows.stored) continue;  // two 27B layers in ternary at four rows: 106.2 -> 102.3 us
         const uint32_t base = xfrag + (uint32_t)task.x * kXBytes;
         uint32_t zh[4], zl[4];  // stage 2's A registers: (block 0, half 0), (block 1, half 0), (block 0, half 1), (block 1, half 1)
 #pragma unroll

@@ -24,8 +24,9 @@
 // offset into the grid, the delta's sign at bit 3 (one shift brings both to bits 15 and 31) and the
 // scale at bits 0 ... 2 of both halves. Tile (16 rows x 256 k, 1056 bytes; the blocks are 800 and 896):
 // [2][lane][16 bytes] = for j = 2p, 2p + 1: the word of row g, of row g + 8; then d of rows (g, g + 8)
-// side by side. The loop is bound by instruction issue: 17408 x 5120 at eight rows 17.4 us
-// with index bytes, high bits and scale in fields of their own, 16.3 us with this layout.
+// side by side. The loop is bound by instruction issue: 17408 x 5120 at eight rows, one weight repeated
+// out of L2, 17.4 us with index bytes, high bits and scale in fields of their own, 16.5 us with this
+// layout (17.9 us with weights of their own in HBM).
 //
 // Activations of a unit in shared memory: eight rows of 256 fp16 as they lie in x, the rows
 // umax * 512 + 16 bytes apart; behind all rows, per unit, the entry sums: [k-step][lane][hi hi | lo lo].

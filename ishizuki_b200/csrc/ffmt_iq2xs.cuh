@@ -18,8 +18,9 @@
 // integer) and its two signs by one shift, which brings its sign pair to bits 15 and 31, and a
 // mask-and-xor. With the scale inside the fragments a whole tile accumulates in one MMA chain; d / 8
 // remains for fp32. A 17408 x 5120 projection
-// of eight rows took 18.7 us and 587 warp instructions a tile with index and seven sign bits packed
-// as the block has them and the parity recomputed, 14.9 us and 458 with this layout.
+// of eight rows, one weight repeated out of L2, took 18.7 us and 587 warp instructions a tile with index and
+// seven sign bits packed as the block has them and the parity recomputed, 14.9 us and 473 with this layout
+// (16.0 us with weights of their own in HBM).
 //
 // Fragment mapping (m16n8k16; lane g = lane / 4, t = lane % 4 holds weight rows g and g + 8): a
 // lane owns the sub-blocks (sixteen weights = two u16 = one scale) 4 j + t, j = 0..3, of both rows.

@@ -21,9 +21,10 @@
 // second in its high half, from bit 7 up, where a mask makes it a byte offset into the grid. The bits
 // below hold the signs, register r's pair at p and p + 16 (p = 3 ... 6 in a first word, 2, 4, 5, 6 in a
 // second), and in both halves the scale s: its low three bits at 0 ... 2 of the first word, the fourth
-// at bit 3 of the second. The loop is bound by instruction issue: 17408 x 5120 at eight rows took
-// 19.2 us and 640 warp instructions a tile with index bytes, ninth bits, signs and scales in words of
-// their own (1824 bytes), 16.3 us and 519 with this layout.
+// at bit 3 of the second. The loop is bound by instruction issue: 17408 x 5120 at eight rows, one
+// weight repeated out of L2, took 19.2 us and 640 warp instructions a tile with index bytes, ninth bits,
+// signs and scales in words of their own (1824 bytes), 16.5 us and 519 with this layout (17.7 us with
+// weights of their own in HBM).
 #pragma once
 #include "ffmt_iq2xs.cuh"
 

@@ -30,8 +30,10 @@ __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { retu
 // between the two passes. Bound by latency alone (a row is 10-20 KB): x and w are on their way together
 // as soon as the launch before is done, w already hinted into L2 (its values are read after the wait, they
 // may be that launch's as well), and the rest is one barrier. Two decoder layers of the 27B shape, four
-// norms, in Q4_K at eight rows: 119.9 us with 256 threads reading value by value and w after the sum,
-// 114.1 this way.
+// norms, in Q4_K: 122.8 us at eight rows and 112.3 at one with 256 threads reading value by value and w
+// after the sum, 117.2 and 106.3 this way. The squares add up in another order than with 256 threads,
+// which moves a row's factor by its last bit now and then: of 4.1 million values at eight widths 260
+// are not the 64-bit result rounded, 288 before.
 constexpr int kNormThreads = 1024, kNormPer = 8;
 
 template <class T>

@@ -13,26 +13,24 @@
 // every k-step's accumulator takes its (exact, fp32) scale afterwards; the second sum is one more
 // MMA whose k index runs over the groups, against the group sums of x.
 //
-// A 6-bit value masked in place at bits 0..5 of each half of a register is the bit pattern of the
-// fp16 number q * 2^-24; at bits 4..9 it is q * 2^-20 (both subnormal, hence linear in q). A pair of
-// k-steps (2i, 2i + 1) takes eight A registers per lane, sixteen values, and they lie in three words:
-// each half of a word has one value at bits 4..9 (a register for one mask), one at bits 10..15 (a shift
-// and a mask) and four bits below; the low nibbles of the first k-step's row g are those of words 0
-// and 1, their high bit pairs bits 0..1 and 2..3 of word 2. That is fifteen bit operations for eight
-// registers, where nibbles and bit pairs in words of their own take twenty-one. The first k-step's
-// registers all hold q * 2^-24 (row g's put together at bits 0..5, row g + 8's shifted there from bits
-// 10..15), the second's q * 2^-20. A k-step has one unit for both rows because the MMA's rounding
-// depends on it (codes of the larger unit lose fewer low bits of a product), and both rows add up their
-// k-steps in the same order: a weight row's product must not depend on which half of a panel it
-// lies in, or a gated pair and the same two weights stacked differ.
-// The loop is bound by the integer pipe and by memory in equal parts: 17408 x 5120 at eight
-// rows 19.1 -> 16.9 us; 248320 x 5120 at eight rows 213 -> 175 us in short runs, 5.9 TB/s (a loop of
-// seconds runs into the power cap: 219). Row g + 8's first k-steps in the larger unit and row g's with sums
-// of their own took as long at eight rows, 23.4 instead of 24.4 us at sixteen rows of 17408 x 5120, but
-// 112 of 65536 products of a weight turned by eight rows changed. Of 393216 products (8192 x 5120) 683 are
-// not the 64-bit result rounded to fp16: 617 then, 750 with one sum for both k-steps. All codes at 2^-20
-// would make it 522, and take two more shifts a pair: 17.3 us (the 2-norm of the error, 2.0703e-4, is
-// fp16's own and the same in all four).
+// A 6-bit value at bits 4..9 of each half of a register is the bit pattern of the fp16 number
+// q * 2^-20 (subnormal, hence linear in q). A pair of k-steps (2i, 2i + 1) takes eight A registers per
+// lane, sixteen values, and they lie in three words: each half of a word has one value at bits 4..9 (a
+// register for one mask), one at bits 10..15 (a shift and a mask) and four bits below; the low nibbles of
+// the first k-step's row g are those of words 0 and 1, their high bit pairs bits 0..1 and 2..3 of word 2.
+// These two are put together at bits 0..5, q * 2^-24, and multiplied by sixteen as half2. That is
+// fifteen bit operations and two multiplies for eight registers, where nibbles and bit pairs in words of
+// their own take twenty-one.
+// All registers hold one unit, and both rows of a lane add up their k-steps in the same order, because a
+// weight row's product must not depend on which half of a panel it lies in (or a gated pair and the same
+// two weights stacked differ) and the MMA's rounding depends on the unit: codes at bits 0..5 lose more
+// low bits of a product. With row g's first k-steps left at 2^-24 and in sums of their own 112 of 65536
+// products of a weight turned by eight rows changed. Of 393216 products (8192 x 5120) 522 are not the
+// 64-bit result rounded to fp16, 617 with that, 683 with both rows' first k-steps at 2^-24, 750 with one
+// sum besides. The half2 multiplies cost 1 to 2 %, shifts in their place 2 %.
+// The loop is bound by the integer pipe and by memory in equal parts: 17408 x 5120 at eight rows 19.1
+// -> 17.1 us (23.5 at sixteen); 248320 x 5120 at eight rows 213 -> 177 us in short runs, 5.9 TB/s (a
+// loop of seconds runs into the power cap: 219).
 // Inside a k-step the lane t holds the weights 4t .. 4t + 3 of the group: slots (2t, 2t + 1) are
 // 4t, 4t + 1 and slots (2t + 8, 2t + 9) are 4t + 2, 4t + 3; the activations are staged in the same
 // order, so that a lane reads the B registers of two k-steps with one 16-byte load.
@@ -54,7 +52,7 @@ struct FragQ6K {
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 16;  // most warps of the smaller block size at up to eight rows
-  static constexpr int kManyWarps = 20;  // most warps at nine to sixteen rows
+  static constexpr int kManyWarps = 16;  // most warps at nine to sixteen rows
 
   // the low four and the high two bits of weight k of a block
   static __device__ __forceinline__ uint32_t low4(const uint8_t *blk, int k) {
@@ -139,12 +137,14 @@ struct FragQ6K {
     });
   }
 
-  // byte `byte` of a word of scales + 128 as the scale: the low mantissa bits of 2^23; SIXTEEN: as sixteen
-  // times the scale, the low mantissa bits of 2^27
-  template <bool SIXTEEN = false>
+  // byte `byte` of a word of scales + 128 as the scale: the low mantissa bits of 2^23
   static __device__ __forceinline__ float scale_of(uint32_t word, int byte) {
-    return __uint_as_float(prmt(word, SIXTEEN ? 0x4d000000u : 0x4b000000u, 0x7650u + (uint32_t)byte)) -
-           (SIXTEEN ? 16.f * 8388736.f : 8388736.f);
+    return __uint_as_float(prmt(word, 0x4b000000u, 0x7650u + (uint32_t)byte)) - 8388736.f;
+  }
+  // both halves times sixteen, exact
+  static __device__ __forceinline__ uint32_t times16(uint32_t v) {
+    const __half2 r = __hmul2(*reinterpret_cast<const __half2 *>(&v), __float2half2_rn(16.f));
+    return *reinterpret_cast<const uint32_t *>(&r);
   }
   // two of its bytes as a half2: the low mantissa bits of 1024
   static __device__ __forceinline__ uint32_t scale_pair(uint32_t word, uint32_t selector) {
@@ -161,9 +161,8 @@ struct FragQ6K {
     const uint4 h0 = lds128(tile + 3072u + (uint32_t)g * 16u), h1 = lds128(tile + 3072u + (uint32_t)(g + 8) * 16u);
     const uint32_t hw0[4] = {h0.x, h0.y, h0.z, h0.w}, hw1[4] = {h1.x, h1.y, h1.z, h1.w};
     const uint32_t lane_off = (uint32_t)g * 64u + (uint32_t)t * 16u;
-    // The first k-steps of the pairs are added up in su, the second, sixteen times as large, in sv. Two column
-    // groups have no registers for both (20 warps spill; 16 warps lose as much): sixteen times the first k-steps'
-    // scales, one sum.
+    // The first k-steps of the pairs are added up in su, the second in sv: shorter chains. Two column groups
+    // have too few registers for both (sixteen rows: 2 % slower than with one sum).
     constexpr bool kOneSum = NB == 2;
     float su[NB][4], sv[NB][4];
 #pragma unroll
@@ -181,13 +180,13 @@ struct FragQ6K {
         }
       }
       const uint32_t w0 = qw[3 * (pi & 3)], w1 = qw[3 * (pi & 3) + 1], w2 = qw[3 * (pi & 3) + 2];
-      const uint32_t a0 = (w0 & 0x000f000fu) | ((w2 << 4) & 0x00300030u), a2 = (w1 & 0x000f000fu) | ((w2 << 2) & 0x00300030u);
-      const uint32_t a1 = (w0 >> 10) & 0x003f003fu, a3 = (w1 >> 10) & 0x003f003fu;
+      const uint32_t a0 = times16((w0 & 0x000f000fu) | ((w2 << 4) & 0x00300030u)), a2 = times16((w1 & 0x000f000fu) | ((w2 << 2) & 0x00300030u));
+      const uint32_t a1 = (w0 >> 6) & 0x03f003f0u, a3 = (w1 >> 6) & 0x03f003f0u;
       const uint32_t e0 = w0 & 0x03f003f0u, e1 = w1 & 0x03f003f0u;
       const uint32_t e2 = w2 & 0x03f003f0u, e3 = (w2 >> 6) & 0x03f003f0u;
       // scales of groups 2 pi and 2 pi + 1: word pi % 4 of the row's sixteen, bytes 2 (pi / 4) and + 1
-      const float s00 = scale_of<kOneSum>(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1);
-      const float s10 = scale_of<kOneSum>(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1);
+      const float s00 = scale_of(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1);
+      const float s10 = scale_of(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1);
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
         const uint4 b = lds128(xu + nb * a.xregion + (uint32_t)pi * 512u + (lane_off ^ (uint32_t)(pi << 6)));
@@ -209,7 +208,7 @@ struct FragQ6K {
     const uint32_t a2 = scale_pair(w0, 0x4342u), a3 = scale_pair(w1, 0x4342u);
     const uint32_t dd = lds32(tile + 3328u + (uint32_t)g * 4u);
     const float d0 = half_bits_to_float(dd & 0xffffu), d1 = half_bits_to_float(dd >> 16);
-    const float dm0 = d0 * (-32.f / 16777216.f), dm1 = d1 * (-32.f / 16777216.f);
+    const float dl0 = d0 * 0.0625f, dl1 = d1 * 0.0625f, dm0 = d0 * (-32.f / 16777216.f), dm1 = d1 * (-32.f / 16777216.f);
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
       const uint4 bs = lds128(xu + nb * a.xregion + kXSums + (uint32_t)lane * 16u);
@@ -218,8 +217,8 @@ struct FragQ6K {
       mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float sum = kOneSum ? su[nb][i] * 0.0625f : fmaf(sv[nb][i], 0.0625f, su[nb][i]);
-        acc[nb][i] = fmaf(i < 2 ? d0 : d1, sum, fmaf(i < 2 ? dm0 : dm1, cm[i], acc[nb][i]));
+        const float sum = kOneSum ? su[nb][i] : su[nb][i] + sv[nb][i];
+        acc[nb][i] = fmaf(i < 2 ? dl0 : dl1, sum, fmaf(i < 2 ? dm0 : dm1, cm[i], acc[nb][i]));
       }
     }
   }

@@ -56,13 +56,13 @@ constexpr int kFragRows = 16;
 // At up to eight rows the kernel is compiled for two block sizes: up to Fmt::kFewWarps warps, and up to
 // kFragMaxWarps with 80 registers per thread. The smaller one is 20 warps with 96 registers (the decoders'
 // loads then run further ahead of their use), or 16 with 128 in Q2_K and Q6_K (17408 x 5120, eight rows:
-// Q2_K 16.4 -> 15.4 us, Q6_K 17.0 -> 16.8; one row 15.7 -> 14.9, 16.6 -> 16.3). The other formats gain nothing
+// Q2_K 16.4 -> 15.4 us, Q6_K 17.0 -> 16.8 when it was chosen; one row 15.7 -> 14.9, 16.6 -> 16.3). The other formats gain nothing
 // by that, and the affine packs lose 2 to 5 % with their 20-warp plans. With two column
 // groups it is one block size per format, Fmt::kManyWarps: 16 warps with 128 registers, or 20 with 96
 // where the decoder does not use the registers and the smaller tiles want warps. 16 rows, 17408 x 5120
 // and 5120 x 17408, 20 -> 16 warps: IQ1_S 25.7 / 31.3 -> 23.6 / 29.5 us, affine 8-bit 23.2 / 26.2 -> 21.3
 // / 24.7, affine 4-bit in groups of 32 22.9 / 27.0 -> 21.6 / 25.5, IQ4_XS 23.6 / 26.4 -> 22.8 / 25.9, IQ2_XS,
-// Q4_K, ternary and the other affine 4-bit 1 to 2 % less; Q6_K 24.4 / 28.8 -> 24.3 / 29.9, Q2_K 21.2 / 24.3
+// Q4_K, ternary and the other affine 4-bit 1 to 2 % less, Q6_K 24.2 / 29.6 -> 23.8 / 28.4; Q2_K 21.2 / 24.3
 // -> 21.6 / 26.0, affine 2-bit 19.4 / 21.7 -> 19.5 / 22.4, IQ2_S the same: these stay at 20.
 constexpr int kFragMaxWarps = ISHI_FRAG_MAX_WARPS;
 constexpr int kFragMaxRing = 4;   // most tiles per warp-private ring (FragArgs::ring of them are used:

@@ -85,13 +85,14 @@ struct FragAffine {
   // row): lane l loads the eight values k = 8l .. 8l + 7. The fragment of k-step st = kMasks * q + m
   // sits at st * 256 + ((g ^ (q & 3)) * 4 + t) * 8: the xor spreads a store's quads over the banks,
   // and a k-step's 32 lanes still read one 256-byte run.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     if (BITS == 2 && GS == 128 && a.rot_block == 128 && !a.rot_signs) {
-      stage_x_rot128(a, m, xfrag, ub0, uc);
+      stage_x_rot128(a, m, xfrag, ub0, uc, then);
       return;
     }
     const int lane = threadIdx.x & 31;
-    frag_stage_rows(a, m, ub0, uc, [&](int u, int g, uint4 v) {
+    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int g, uint4 v) {
       if (a.rot_block)
         v = frag_rotate8(v, a.rot_block,
                             a.rot_signs ? a.rot_signs + (long long)(ub0 + u) * 256 + lane * 8 : nullptr, lane);
@@ -166,7 +167,8 @@ struct FragAffine {
   // to fp32 rounding. Lane (g, t) ends up with the values k' = 16 (4 h + t) + g and + 8 of each
   // block: the codes g and g + 8 of the block's word 4 h + t, which are one B register of the
   // product's k-step (quad 2 block + h, mask g % 4), low register when g < 4.
-  static __device__ __forceinline__ void stage_x_rot128(const FragArgs &a, const FragRows &rows, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x_rot128(const FragArgs &a, const FragRows &rows, uint32_t xfrag, int ub0, int uc, Then then) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     constexpr int kBatch = 8;
@@ -184,7 +186,8 @@ struct FragAffine {
     const float scale = 1.0f / sqrtf(128.f);
     const uint32_t *xl = reinterpret_cast<const uint32_t *>(rows.x + (long long)ub0 * 256) + lane;
     const int tasks = uc * rows.staged;
-    for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
+    int i0 = warp;
+    do {
       uint32_t v[kBatch][4];  // [block * 2 + half]
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
@@ -195,6 +198,7 @@ struct FragAffine {
 #pragma unroll
         for (int c = 0; c < 4; ++c) v[e][c] = live ? __ldg(src + 32 * c) : 0u;
       }
+      if (i0 == warp) then();
 #pragma unroll
       for (int e = 0; e < kBatch; ++e) {
         const int i = i0 + e * nw;
@@ -243,7 +247,8 @@ struct FragAffine {
         if ((lane & 15) == 0)
           asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kSums + (uint32_t)((lane >> 4) * 8 + r) * 4u), "f"(keep * (1.f / 16777216.f)) : "memory");
       }
-    }
+      i0 += nw * kBatch;
+    } while (i0 < tasks);
   }
 
   static __device__ __forceinline__ float param(uint32_t pair, int hi) {

@@ -100,12 +100,13 @@ struct FragIQ1 {
   // (the eight values of one lane) their sum as fp16 high and low parts, where the MMA over the
   // entries reads them: entry E = 2 (4 j + t) + e is slot 2t + e + 8 (j % 2) of k-step j / 2, i.e.
   // register j % 2, half e, of lane (r, t). No rotation here.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
     const uint32_t R = row_stride(a);
     const int sb = lane >> 1, j = sb >> 2, t = sb & 3;
     const uint32_t slot = (uint32_t)((j >> 1) * 512 + t * 16 + (j & 1) * 4 + (lane & 1) * 2);
-    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
       sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
       const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
       const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));

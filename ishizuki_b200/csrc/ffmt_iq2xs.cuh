@@ -168,10 +168,11 @@ struct FragIQ2 {
   // Activations of the CTA's column range as they lie in x (rows past M as zeros).
   // A warp task is (unit, activation row): lane l loads and stores k = 8l .. 8l + 7.
   // IQ2_XS has no rotation.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
     const uint32_t R = row_stride(a);
-    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
       sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
     });
   }

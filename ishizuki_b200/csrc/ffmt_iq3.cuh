@@ -96,8 +96,9 @@ struct FragIQ3 {
   }
 
   // the activations as for IQ2_XS: the rows as they lie in x
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
-    FragIQ2<17>::stage_x(a, m, xfrag, ub0, uc);
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
+    FragIQ2<17>::stage_x(a, m, xfrag, ub0, uc, then);
   }
 
   // a sub-block's sixteen weights (two words) as eight A registers; `copy`: byte offset of this lane's copy

@@ -82,12 +82,13 @@ struct FragIQ4XS {
   // ks = 2 ib + s and quad row r lie at ks * 256 + ((r ^ (ks % 8)) * 4 + t) * 8; the xor spreads the
   // stores over the banks, a warp's read of one k-step is still one 256-byte run.
   // No rotation here.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
     const int ib = lane >> 2, r4 = lane & 3;
     const bool second = r4 >= 2;
     const int t = second ? 2 * (r4 - 2) + 1 : 2 * r4;
-    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
       const uint32_t base = xfrag + (uint32_t)u * kXBytes;
       const uint32_t got0 = __shfl_xor_sync(0xffffffffu, second ? v.x : v.z, 2);
       const uint32_t got1 = __shfl_xor_sync(0xffffffffu, second ? v.y : v.w, 2);

@@ -75,13 +75,14 @@ struct FragQ2K {
   // is * 256 + ((r ^ (is % 8)) * 4 + t) * 8 (the xor spreads the stores over the banks, a warp's read
   // of one k-step is still one 256-byte run). Then the sub-block sums of the undivided values
   // (fp16 hi + lo) for the MMA over sub-blocks. No rotation here.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
     const int j = (lane >> 2) & 3;
     const int is = 8 * (lane >> 4) + 2 * j + ((lane & 3) >> 1);
     const uint32_t down1 = (uint32_t)(15 - 2 * j) << 10;  // 4^-j in fp16
     const uint32_t down = down1 | (down1 << 16);
-    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
       const uint32_t base = xfrag + (uint32_t)u * kXBytes;
       const __half2 dn = *reinterpret_cast<const __half2 *>(&down);
       // (x0 x2), (x1 x3) for t = 2 (l % 2); (x4 x6), (x5 x7) for t + 1

@@ -105,11 +105,12 @@ struct FragQ4K {
   // every sub-block for the minimum term. Q4_K has no input rotation.
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
     const uint32_t R = row_stride(a), sums = xfrag + 8u * R;
     const int jj = lane >> 3;
-    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
       sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
       const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
       const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));

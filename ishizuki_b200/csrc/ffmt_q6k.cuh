@@ -112,9 +112,10 @@ struct FragQ6K {
   // i * 512 + ((r ^ i) * 4 + t) * 16 (+ 8 for the odd k-step); the xor spreads the stores over the
   // banks and a warp's read of one pair is still one 512-byte run. Then the group sums (fp16 hi +
   // lo) for the MMA over groups.
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc) {
+  template <class Then>
+  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
-    frag_stage_rows(a, m, ub0, uc, [&](int u, int r, uint4 v) {
+    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
       const uint32_t base = xfrag + (uint32_t)u * kXBytes;
       const int pi = lane >> 2, ks = lane >> 1;
       const uint32_t dst = base + (uint32_t)pi * 512u + (uint32_t)(((r ^ pi) * 4 + 2 * (lane & 1)) * 16 + (ks & 1) * 8);

@@ -481,7 +481,8 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
   // shared memory depends on the clusters (fewer of them lead more panels each), which depend on it
   for (int tries = 0; tries < 3; ++tries) {
     const int panels = (c.P + c.NC - 1) / c.NC;
-    if ((long long)panels * c.umax * (kFragMaxWarps + 1) >= (1ll << 31)) return false;
+    // (T * w * W, T * units in the kernel)
+    if ((long long)panels * c.umax * std::max(kFragMaxWarps * kFragMaxWarps, c.umax) >= (1ll << 32)) return false;
     c.led = s > 1 ? (panels + s - 1) / s : 0;
     bool fits = false;
     for (int r = ring ? ring : kFragMaxRing; r >= (ring ? ring : 2) && !fits; --r) {
@@ -596,6 +597,12 @@ bool single_row_on_cuda_cores(const ishi_ctx *ctx) {
   return ctx->crossover_rows > 1;
 }
 
+// Tiles per warp asked for ahead of the dependency wait, about 64 KB per CTA. They travel ahead of the activations: a
+// CTA that starts as the launch before it ends waits that much longer for x (4096 x 4096, affine 4-bit, eight
+// launches: 43.6 us up to 64 KB, 45.7 from 96 KB on; two 27B layers in Q4_K at eight rows 112.9 at 48 and 64 KB, 113.8 at one tile and
+// 96 KB, 116.3 with the whole ring; ternary 98.8 at one tile, 97.4 from 64 KB on). The rest of the ring follows the loads of x.
+int tiles_ahead(const FragPlan &pl) { return std::max(1, std::min(pl.ring - 1, (64 << 10) / (pl.W * pl.tile_bytes))); }
+
 // rows 1...16 through the warp-level kernel; gemv picks the CUDA-core variant for a single row
 ishi_status run_frag(ishi_ctx *ctx, const FragPlans &plans, const Workspace &ws, const ishi_weight_desc &d, const void *x,
                      int rows, void *y, long long ldy, int flags, bool gemv, bool early, bool rotate, cudaStream_t st,
@@ -618,10 +625,14 @@ ishi_status run_frag(ishi_ctx *ctx, const FragPlans &plans, const Workspace &ws,
     a.P = pl.P;
     a.NC = pl.NC;
     a.ring = pl.ring;
+    a.ahead = tiles_ahead(pl);
     a.led = pl.led;
     a.xregion = pl.xregion;
     a.inv_s = frag_inverse(pl.S);
     a.inv_nc = frag_inverse(pl.NC);
+    a.inv_w = frag_inverse(pl.W);
+    a.inv_u = frag_inverse(pl.umax);
+    a.inv_u1 = frag_inverse(pl.umax - 1);
     a.umax = pl.umax;
     a.group_size = d.group_size;
     a.scale_dtype = d.scale_dtype;

@@ -79,9 +79,10 @@ struct FragArgs {
   int M, N, K;
   int units, S, P, NC;  // NC clusters of S CTAs
   int ring;             // tiles per warp-private ring, 2 ... kFragMaxRing
+  int ahead;            // of them, tiles asked for before the dependency wait, 1 ... ring - 1
   int led;              // most panels a CTA leads (S > 1)
-  // ceil(2^32 / d) for d = S, NC, or 0 for d = 1: see frag_div()
-  unsigned inv_s, inv_nc;
+  // ceil(2^32 / d) for d = S, NC, warps, umax, umax - 1, or 0 for d = 1: see frag_div()
+  unsigned inv_s, inv_nc, inv_w, inv_u, inv_u1;
   int umax;             // most units in a column range
   uint32_t xregion;     // bytes of one staged region: umax * Fmt::kXBytes + Fmt::kXFixed
   int group_size, scale_dtype;
@@ -166,6 +167,13 @@ __device__ __forceinline__ double2 lds128d(uint32_t addr) {
   asm("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr));
   return v;
 }
+// One more arrival at a counter in shared memory: returns the arrivals before it. Releases what the warp's lanes
+// stored (the caller's __syncwarp orders them ahead of it) and acquires what those who arrived before released.
+__device__ __forceinline__ int count_in(uint32_t addr) {
+  int old;
+  asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], 1;" : "=r"(old) : "r"(addr) : "memory");
+  return old;
+}
 __device__ __forceinline__ float lds32f(uint32_t addr) {
   float v;
   asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
@@ -195,7 +203,7 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
 
 // n / d through inv = ceil(2^32 / d), exact for n * d < 2^32; inv = 0 stands for d = 1
 __device__ __forceinline__ int frag_div(unsigned n, unsigned inv) { return inv ? (int)__umulhi(n, inv) : (int)n; }
-__host__ inline unsigned frag_inverse(int d) { return d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
+__host__ inline unsigned frag_inverse(int d) { return d <= 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
 
 __host__ __device__ inline int frag_column_begin(int c, int units, int S) { return (c * units) / S; }
 __host__ __device__ inline int frag_ring_stride(int tile_bytes) { return (tile_bytes + 15) & ~15; }
@@ -365,13 +373,15 @@ struct FragRows {
 };
 
 // Staging, a warp task per (unit, row): put(unit, row, v) with the values k = 8l .. 8l + 7 of lane l. All
-// loads of up to eight tasks go out before the first is used: the staging costs one L2 latency.
-template <class Put>
-__device__ __forceinline__ void frag_stage_rows(const FragArgs &a, const FragRows &m, int ub0, int uc, Put put) {
+// loads of up to eight tasks go out before the first is used: the staging costs one L2 latency. then() runs
+// once, behind the first loads.
+template <class Then, class Put>
+__device__ __forceinline__ void frag_stage_rows(const FragArgs &a, const FragRows &m, int ub0, int uc, Then then, Put put) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, tasks = uc * m.staged;
   constexpr int kBatch = 8;
   const __half *xl = m.x + (long long)ub0 * 256 + lane * 8;
-  for (int i0 = warp; i0 < tasks; i0 += nw * kBatch) {
+  int i0 = warp;
+  do {
     uint4 v[kBatch];
 #pragma unroll
     for (int e = 0; e < kBatch; ++e) {
@@ -380,6 +390,7 @@ __device__ __forceinline__ void frag_stage_rows(const FragArgs &a, const FragRow
       v[e] = make_uint4(0u, 0u, 0u, 0u);
       if (i < tasks && t.y < m.live) v[e] = __ldg(reinterpret_cast<const uint4 *>(xl + (long long)t.y * a.K + t.x * 256));
     }
+    if (i0 == warp) then();
 #pragma unroll
     for (int e = 0; e < kBatch; ++e) {
       const int i = i0 + e * nw;
@@ -387,7 +398,8 @@ __device__ __forceinline__ void frag_stage_rows(const FragArgs &a, const FragRow
       const int2 t = m.task(i);
       put(t.x, t.y, v[e]);
     }
-  }
+    i0 += nw * kBatch;
+  } while (i0 < tasks);
 }
 
 // A decoder's shared-memory tables (kExtraBytes, a multiple of 16), laid out once per device from
@@ -438,11 +450,12 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   const int pa = frag_div((unsigned)cid * (unsigned)a.P, a.inv_nc);
   const int np = frag_div((unsigned)(cid + 1) * (unsigned)a.P, a.inv_nc) - pa;
   const int led = S > 1 ? frag_div((unsigned)(np - 1 - r + S), a.inv_s) : 0;  // panels this CTA leads: r, r + S, ...
-  // the CTA's tiles, and this warp's run of them
-  const unsigned T = (unsigned)(np * uc), We = min((unsigned)W, T);
-  const int t0 = (unsigned)warp < We ? (int)(T * (unsigned)warp / We) : (int)T;
-  const int t1 = (unsigned)warp < We ? (int)(T * (unsigned)(warp + 1) / We) : (int)T;
-  const int q0 = (int)((unsigned)t0 / (unsigned)uc);  // the run's first panel
+  // the CTA's tiles, and this warp's run of them: tiles T w / W ... T (w + 1) / W - 1, or tile w where there are
+  // fewer tiles than warps (no division: three of them held up the first copies by 0.2 us)
+  const unsigned T = (unsigned)(np * uc);
+  auto run_begin = [&](unsigned w) { return T >= (unsigned)W ? frag_div(T * w, a.inv_w) : (int)min(w, T); };
+  const int t0 = run_begin((unsigned)warp), t1 = run_begin((unsigned)warp + 1u);
+  const int q0 = frag_div((unsigned)t0, uc == a.umax ? a.inv_u : a.inv_u1);  // the run's first panel
 
   ISHI_STAMP(0);
   // Let the next kernel on the stream start its own prologue as SMs fall free.
@@ -485,16 +498,17 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
     --f_left;
     cp_async_commit();
   };
-  // The weight tiles are written by no earlier kernel: their first copies go out at once. (Asking
-  // the run's next tiles into L2 as well delays the activations behind them: 60 -> 66 us per layer.)
-  for (int i = 0; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride);
-
   // Warm L2 and the address translation with this CTA's slice of x. Only a hint: x may still be
   // written by the kernel before this one, its values are read after the wait below, through L2.
   for (int m = warp; m < a.M; m += W) {
     const char *row = reinterpret_cast<const char *>(a.x + (long long)m * a.K + (long long)ub0 * 256);
     for (int c = lane; c < uc * 4; c += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c * 128));
   }
+
+  // The weight tiles are written by no earlier kernel: the first copies go out at once, no more of them than leave
+  // the way free for the activations (a.ahead; the rest of the ring follows the loads of x). Asking the
+  // run's next tiles into L2 as well delays the activations too: 60 -> 66 us per layer.
+  for (int i = 0; i < a.ahead; ++i) fetch(ring + (uint32_t)i * kStride);
 
   // x may be the output of the kernel before this one and y may still be read by it: wait for the
   // earlier kernels (returns at once unless this kernel was launched early).
@@ -522,7 +536,8 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   // activations of the column range into fragment order (all warps)
 #pragma unroll
   for (int b = 0; b < NB; ++b)
-    Fmt::stage_x(a, FragRows{a.x + (long long)(8 * b) * a.K, ONE ? 1 : a.M - 8 * b, ONE ? 1 : a.world > 0 ? 8 : a.M - 8 * b, ONE ? 1 : 8}, xfrag + b * a.xregion, ub0, uc);
+    Fmt::stage_x(a, FragRows{a.x + (long long)(8 * b) * a.K, ONE ? 1 : a.M - 8 * b, ONE ? 1 : a.world > 0 ? 8 : a.M - 8 * b, ONE ? 1 : 8}, xfrag + b * a.xregion, ub0, uc,
+                 [&] { if (b == 0) for (int i = a.ahead; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride); });
   ISHI_STAMP(3);
   if (Fmt::kExtraBytes) {  // the tables have landed: all groups but the R - 1 tiles' behind them
     if (R == 2) cp_async_wait<1>();
@@ -591,7 +606,10 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
       // The panel is shared with other warps: park the partial tile; the warp that arrives last adds
       // the partials in warp order. The panel begins in run wa (parked in that warp's ring, which is
       // drained: the panel's part is the last of the run; the plan leaves it kPark bytes) and ends in run wb (parked in the slots).
-      const int wa = (int)((((unsigned)begin + 1u) * We - 1u) / T), wb = (int)(((unsigned)(begin + uc) * We - 1u) / T);
+      const int begun = run_begin((unsigned)lane);  // lane w: where run w begins
+      const unsigned runs = (1u << W) - 1u;
+      const int wa = __popc(__ballot_sync(0xffffffffu, begun <= begin) & runs) - 1;
+      const int wb = __popc(__ballot_sync(0xffffffffu, begun < begin + uc) & runs) - 1;
       const uint32_t mine = (warp == wa ? ring : red + (uint32_t)warp * kPark) + (uint32_t)lane * 16u;
       __syncwarp();  // every lane is done with the last tile
 #pragma unroll
@@ -601,13 +619,10 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
       }
       __syncwarp();
       int old = 0;
-      if (lane == 0) {
-        __threadfence_block();
-        old = atomicAdd(cnt + wa, 1);
-      }
+      if (lane == 0) old = count_in(ctrl + 4u * (uint32_t)wa);
+      __syncwarp();
       old = __shfl_sync(0xffffffffu, old, 0);
       if (old != wb - wa) continue;
-      __threadfence_block();
       for (int w = wa; w <= wb; ++w) {
         const uint32_t src = stage_acquire(w == wa ? rings + (uint32_t)(wa * R) * kStride : red + (uint32_t)w * kPark) + (uint32_t)lane * 16u;
 #pragma unroll

@@ -43,6 +43,7 @@ struct FragAffine {
   static constexpr int kTileBytes = kHeader + 16 * kRowHeader;
   static constexpr int kSums = 4096;                 // offset of the group sums of x: [group][activation row] fp32
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
+  static constexpr bool kRows = false, kRowSums = false;  // staged in fragment order
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

@@ -30,6 +30,7 @@ struct FragGGML {
   static constexpr int kTileBytes = 16 * kBlock;
   static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 16;  // a staged region: per unit eight rows of 512 bytes; the rows' skews
   static constexpr double kUnit = 1.0;  // unit of the tile results
+  static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
   static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;     // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
@@ -47,17 +48,6 @@ struct FragGGML {
   }
 
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 16u; }
-
-  // Activations of the CTA's column range as they lie in x (rows past M as zeros). A warp task is
-  // (unit, activation row): lane l loads and stores k = 8l .. 8l + 7. GGML blocks have no input rotation.
-  template <class Then>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t R = row_stride(a);
-    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
-      sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
-    });
-  }
 
   // eight decoded weights as four A registers (fp16 pairs)
   static __device__ __forceinline__ void pack(uint32_t (&r)[4], const float (&w)[8]) {

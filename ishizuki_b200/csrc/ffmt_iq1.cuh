@@ -46,6 +46,7 @@ struct FragIQ1 {
   // a staged region: per unit eight rows of 512 bytes and the entry sums; the rows' 16-byte skews
   static constexpr int kXBytes = 8 * 512 + 1024, kXFixed = 8 * 16;
   static constexpr double kUnit = 1.0;  // unit of the tile results
+  static constexpr bool kRows = false, kRowSums = false;  // staged by loads and stores: the entry sums come from the registers (a pass over copied rows: 0.4 us a launch more)
   static constexpr int kExtraBytes = 2048 * 32;  // the grid, four copies interleaved
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

@@ -74,6 +74,7 @@ struct FragIQ2 {
   static constexpr int kTileBytes = kD + 32;
   static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 16;    // a staged region: per unit eight rows of 512 bytes; the rows' skews
   static constexpr double kUnit = 0.125;         // tile results come in units of 1/8
+  static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
   static constexpr int kExtraBytes = kEntries * kCopies * 16;  // the grid as fp16, its copies interleaved
   static constexpr bool kRowMode = false;        // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
@@ -163,18 +164,6 @@ struct FragIQ2 {
     }
     const __half2 h = __halves2half2(__int2half_rn((int)m0), __int2half_rn((int)m1));
     return *reinterpret_cast<const uint32_t *>(&h);
-  }
-
-  // Activations of the CTA's column range as they lie in x (rows past M as zeros).
-  // A warp task is (unit, activation row): lane l loads and stores k = 8l .. 8l + 7.
-  // IQ2_XS has no rotation.
-  template <class Then>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t R = row_stride(a);
-    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
-      sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
-    });
   }
 
   // 2 s + 1 of scale nibble j, in both halves, from the nibbles of a row in both halves: the nibble

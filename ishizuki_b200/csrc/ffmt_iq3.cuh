@@ -42,6 +42,7 @@ struct FragIQ3 {
   static constexpr uint32_t kMask = (uint32_t)(kEntries - 1) << 7;
   static constexpr int kXBytes = FragIQ2<17>::kXBytes, kXFixed = FragIQ2<17>::kXFixed;
   static constexpr double kUnit = kNine ? 1.0 : 0.25;  // unit of the tile results
+  static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
   static constexpr int kExtraBytes = kEntries * 128;  // the grid as fp16, sixteen copies interleaved
   static constexpr bool kRowMode = false;  // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
@@ -93,12 +94,6 @@ struct FragIQ3 {
     const uint32_t bytes = (kNine ? d_iq3s_grid[i >> 5] : d_iq3xxs_grid[i >> 5]) >> (16 * (i & 1));
     const __half2 h = __halves2half2(__int2half_rn((int)(bytes & 0xffu)), __int2half_rn((int)((bytes >> 8) & 0xffu)));
     return *reinterpret_cast<const uint32_t *>(&h);
-  }
-
-  // the activations as for IQ2_XS: the rows as they lie in x
-  template <class Then>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
-    FragIQ2<17>::stage_x(a, m, xfrag, ub0, uc, then);
   }
 
   // a sub-block's sixteen weights (two words) as eight A registers; `copy`: byte offset of this lane's copy

@@ -28,6 +28,7 @@ struct FragIQ4XS {
   static constexpr int kTileBytes = 2048 + 128 + 32;
   static constexpr int kXBytes = 4096, kXFixed = 0;   // a staged region: per unit sixteen k-steps of 256 bytes
   static constexpr double kUnit = 1.0;  // unit of the tile results
+  static constexpr bool kRows = false, kRowSums = false;  // staged in fragment order
   static constexpr int kExtraBytes = 256 * 128;       // the pair table: entry e of lane l's copy at e * 128 + l * 4
   static constexpr bool kRowMode = false;             // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

@@ -44,6 +44,7 @@ namespace ishi {
 struct FragQ4K {
   static constexpr int kTileBytes = 2048 + 16 * 16 + 16 * 4;
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
+  static constexpr bool kRows = true, kRowSums = true;  // the activations as they lie in x
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
@@ -100,11 +101,42 @@ struct FragQ4K {
     return (uint16_t)(tile_byte(s, p, u, 2 * hw) | ((uint32_t)tile_byte(s, p, u, 2 * hw + 1) << 8));
   }
 
-  // Activations of the CTA's column range. A warp task is (unit, activation row): lane l loads
-  // k = 8l .. 8l + 7 of it, stores them as they lie in x (rows past M as zeros) and the warp adds up
-  // every sub-block for the minimum term. Q4_K has no input rotation.
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
+  // Sub-block sums of x for the minimum term, a warp task per unit. The sixteen bytes of lane l are part of
+  // sub-block l / 4: as B registers (column l / 4, any k) two MMAs with a weight of ones give the row's eight
+  // sums, the same in every row of C, and lane (g, t) keeps sub-blocks 2t and 2t + 1 of activation row g. (One accumulator per row, not
+  // a matrix that picks the row: 0 * inf would reach the other rows.)
+  static __device__ __forceinline__ void row_sums(const FragArgs &a, uint32_t xfrag, int rows, int uc) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, g = lane >> 2;
+    const uint32_t R = row_stride(a), x = stage_acquire(xfrag);
+    constexpr uint32_t kOnes = 0x3c003c00u;
+    for (int u = warp; u < uc; u += nw) {
+      float s0 = 0.f, s1 = 0.f;
+      for (int r0 = 0; r0 < rows; r0 += 4) {  // (rows past the live ones: whatever is there, for columns of no row)
+        uint4 v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = lds128(x + (uint32_t)(r0 + e) * R + (uint32_t)u * 512u + (uint32_t)lane * 16u);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float c[4];
+          mma16816_first(c, kOnes, kOnes, kOnes, kOnes, v[e].x, v[e].y);
+          mma16816(c, kOnes, kOnes, kOnes, kOnes, v[e].z, v[e].w);
+          if (g == r0 + e) s0 = c[0], s1 = c[1];
+        }
+      }
+      // as fp16 hi + lo: the B fragment of the minimum-term MMA, whose k index runs over sub-blocks
+      const __half h0 = __float2half_rn(s0), h1 = __float2half_rn(s1);
+      const __half l0 = __float2half_rn(s0 - __half2float(h0)), l1 = __float2half_rn(s1 - __half2float(h1));
+      const uint32_t base = x + 8u * R + (uint32_t)u * kSumBytes;
+      sts64(base + (uint32_t)lane * 8u, (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
+            (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16));
+      if (g == 0)  // fp32 sums of activation row 0 (the single-row kernel's minimum term)
+        sts64(base + 256u + (uint32_t)lane * 8u, __float_as_uint(s0), __float_as_uint(s1));
+    }
+  }
+
+  // The same for a single activation row, stored and added up on its way from x: a warp task is (unit, row).
   template <class Then>
   static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
@@ -129,8 +161,6 @@ struct FragQ4K {
         sts64(base + (uint32_t)(r * 4 + jj) * 8u, (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
               (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16));
       }
-      if (r == 0 && (lane & 3) == 0)  // fp32 sums of activation row 0 (the single-row kernel's minimum term)
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + 256u + (uint32_t)(lane >> 2) * 4u), "f"(s) : "memory");
     });
   }
 

@@ -49,6 +49,7 @@ struct FragQ6K {
   static constexpr int kXSums = 4096;             // after the activations: [lane][hi hi | lo lo] group sums
   static constexpr int kXBytes = kXSums + 512, kXFixed = 0;  // per unit of a staged region
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
+  static constexpr bool kRows = false, kRowSums = false;  // staged in fragment order
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 16;  // most warps of the smaller block size at up to eight rows

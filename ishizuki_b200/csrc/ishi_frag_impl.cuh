@@ -19,7 +19,8 @@ struct FragOpsOf {
       // (a format without a CUDA-core variant for one activation row runs that row through the MMA path)
       if (mode == 1) return few ? (const void *)frag_kernel<Fmt, 1, Fmt::kFewWarps, 1> : (const void *)frag_kernel<Fmt, 1, kFragMaxWarps, 1>;
     }
-    if (one) return few ? (const void *)frag_kernel<Fmt, 0, Fmt::kFewWarps, 1, true> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1, true>;
+    if constexpr (!Fmt::kRows || Fmt::kRowSums)  // (copying one row as it lies in x needs no variant)
+      if (one) return few ? (const void *)frag_kernel<Fmt, 0, Fmt::kFewWarps, 1, true> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1, true>;
     return few ? (const void *)frag_kernel<Fmt, 0, Fmt::kFewWarps, 1> : (const void *)frag_kernel<Fmt, 0, kFragMaxWarps, 1>;
   }
 

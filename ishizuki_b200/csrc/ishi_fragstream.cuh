@@ -211,8 +211,8 @@ __host__ __device__ inline int frag_ring_stride(int tile_bytes) { return (tile_b
 // shared memory of one CTA, in order: the staged activations (a region per group of eight rows),
 // the format's tables, the warps' partial-tile slots, the inbox for the partial panels of the
 // cluster's CTAs, a control block, the warps' rings
-// control block: arrival counters [warp] @0, abort @96, inbox mbarriers [led] @128
-constexpr uint32_t kFragCtrlAbort = 96, kFragCtrlInbox = 128;
+// control block: arrival counters [warp] @0, abort @96, the activations' mbarrier @104, inbox mbarriers [led] @128
+constexpr uint32_t kFragCtrlAbort = 96, kFragCtrlX = 104, kFragCtrlInbox = 128;
 static_assert(4 * kFragMaxWarps <= (int)kFragCtrlAbort, "control block");
 __host__ __device__ inline uint32_t frag_ctrl_bytes(int led) { return (kFragCtrlInbox + 8u * (uint32_t)led + 127u) & ~127u; }
 // x: the staged regions and the format's tables; led: most panels a CTA leads; NB: groups of eight rows
@@ -402,6 +402,28 @@ __device__ __forceinline__ void frag_stage_rows(const FragArgs &a, const FragRow
   } while (i0 < tasks);
 }
 
+// The activations of a decoder that reads them as they lie in x (Fmt::kRows): a bulk copy per row, asked for by
+// one warp, all counted on `bar`. No thread's load or store is in the way: alone on the GPU 80 KB are there 1500
+// cycles after the request where loads and stores by all warps take 2200 to 2500 (10 KB: 720 against 1150). Launches over weights
+// from HBM, in us: Q4_K at eight rows 34816 x 5120 21.5 -> 20.5, 8192 x 5120 unsplit 9.15 -> 8.17, 5120 x 17408 14.55 -> 14.2; IQ2_XS
+// 8192 x 5120 11.6 -> 11.2 at sixteen rows, 8.87 -> 8.71 at eight; IQ3_S 5120 x 17408 18.1 -> 17.5.
+// An exchange stores all eight columns: there the rows past the live ones are zeros. Elsewhere they are whatever
+// the shared memory holds, columns of no row.
+template <int NB>
+__device__ __forceinline__ void frag_copy_rows(const FragArgs &a, uint32_t xfrag, uint32_t stride, uint32_t bar, int ub0, int uc) {
+  auto row_at = [&](int m) { return xfrag + (uint32_t)(m >> 3) * a.xregion + (uint32_t)(m & 7) * stride; };
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) mbar_arrive_expect_tx_u32(bar, (uint32_t)(a.M * uc) * 512u);
+    __syncwarp();
+    if (a.world > 0) asm volatile("fence.proxy.async;" ::: "memory");  // rows that other GPUs stored, seen by plain loads
+    if ((int)threadIdx.x < a.M)
+      bulk_g2s_u32(row_at((int)threadIdx.x), a.x + (long long)threadIdx.x * a.K + (long long)ub0 * 256, (uint32_t)uc * 512u, bar);
+  }
+  if (a.world > 0)
+    for (int m = a.M; m < 8 * NB; ++m)
+      for (int i = (int)threadIdx.x; i < uc * 32; i += (int)blockDim.x) sts128u(row_at(m) + 16u * (uint32_t)i, make_uint4(0u, 0u, 0u, 0u));
+}
+
 // A decoder's shared-memory tables (kExtraBytes, a multiple of 16), laid out once per device from
 // Fmt::table_word; every CTA copies them from here, a few 16-byte async copies per thread that land
 // while it waits for the launch before. Building them in place, lookups and conversions ahead of the
@@ -423,6 +445,8 @@ template <class Fmt, int MODE, int MAXW, int NB, bool ONE = false>
 __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   static_assert(MODE == 0 || NB == 1, "the CUDA-core variant takes one row");
   static_assert(!ONE || (MODE == 0 && NB == 1), "one row is one column group");
+  // a single row whose sums the decoder needs is staged by loads and stores, the sums on the way
+  constexpr bool kCopied = Fmt::kRows && !(ONE && Fmt::kRowSums);
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kTile = Fmt::kTileBytes;
   constexpr uint32_t kStride = (uint32_t)((kTile + 15) & ~15), kPart = NB * 512u, kPark = NB * 1024u;  // bytes of a partial tile in fp32, fp64
@@ -468,7 +492,10 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
       mbar_arrive_expect_tx_u32(ctrl + kFragCtrlInbox + 8u * i, (uint32_t)S * kPart);
     }
     if ((int)threadIdx.x < W) cnt[threadIdx.x] = 0;
-    if (threadIdx.x == 0) *abort_word = 0;
+    if (threadIdx.x == 0) {
+      *abort_word = 0;
+      if (kCopied) mbar_init_u32(ctrl + kFragCtrlX, 1);
+    }
     mbar_fence_init();
     __syncwarp();
   }
@@ -533,18 +560,34 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   }
   ISHI_STAMP(2);
 
-  // activations of the column range into fragment order (all warps)
+  auto rest = [&] {  // the ring's other tiles, behind the activations
+    for (int i = a.ahead; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride);
+  };
+  if constexpr (kCopied) {
+    frag_copy_rows<NB>(a, xfrag, Fmt::row_stride(a), ctrl + kFragCtrlX, ub0, uc);
+    rest();
+  } else {
+    // activations of the column range into fragment order (all warps)
 #pragma unroll
-  for (int b = 0; b < NB; ++b)
-    Fmt::stage_x(a, FragRows{a.x + (long long)(8 * b) * a.K, ONE ? 1 : a.M - 8 * b, ONE ? 1 : a.world > 0 ? 8 : a.M - 8 * b, ONE ? 1 : 8}, xfrag + b * a.xregion, ub0, uc,
-                 [&] { if (b == 0) for (int i = a.ahead; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride); });
+    for (int b = 0; b < NB; ++b)
+      Fmt::stage_x(a, FragRows{a.x + (long long)(8 * b) * a.K, ONE ? 1 : a.M - 8 * b, ONE ? 1 : a.world > 0 ? 8 : a.M - 8 * b, ONE ? 1 : 8}, xfrag + b * a.xregion, ub0, uc,
+                   [&] { if (b == 0) rest(); });
+  }
   ISHI_STAMP(3);
   if (Fmt::kExtraBytes) {  // the tables have landed: all groups but the R - 1 tiles' behind them
     if (R == 2) cp_async_wait<1>();
     else if (R == 3) cp_async_wait<2>();
     else cp_async_wait<3>();
   }
-  __syncthreads();  // staged, and the control block is set up for every warp
+  __syncthreads();  // staged, the tables there, and the control block set up for every warp
+  if constexpr (kCopied) {
+    if (!mbar_wait_u32(ctrl + kFragCtrlX, 0u, abort_word)) *a.err = 1;  // (y stays wrong, the error word tells the host)
+    if constexpr (Fmt::kRowSums) {
+#pragma unroll
+      for (int b = 0; b < NB; ++b) Fmt::row_sums(a, xfrag + b * a.xregion, min(a.M - 8 * b, 8), uc);
+      __syncthreads();
+    }
+  }
   ISHI_STAMP(4);
   // shared-memory loads are plain asm the compiler may move; tie their addresses to the waits
   const uint32_t xf = stage_acquire(xfrag), tb = stage_acquire(tables);

@@ -147,8 +147,8 @@ int64_t ishi_projection_weight_bytes(const ishi_projection *p);
  * (VerifyMatmul.swift:19-26), whose table was tuned for Apple M1 (ishi_reference_minimum_rows). */
 int ishi_projection_crossover_rows(const ishi_projection *p);
 /* The launch plan create settled on, for the warp-level kernel's formats: {K split = cluster size,
- * a, b: a * b warps per CTA, tiles per warp ring | the launch of 9...16 rows << 8} (zeros for the
- * other kernels), and a way to impose one: the order in which partial sums are added follows the
+ * a, b: a * b warps per CTA, tiles per warp ring | the launch of 9...16 rows << 8 | that of one row << 21} (zeros
+ * for the other kernels; without the last part one row runs as two to eight do), and a way to impose one: the order in which partial sums are added follows the
  * plan, so two projections of the same weight agree bit for bit only under the same plan (the tiled
  * copy does not depend on it). set_plan accepts what ishi_projection_plan of a projection of the
  * same shape returned. */

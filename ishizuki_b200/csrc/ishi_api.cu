@@ -76,11 +76,13 @@ struct FragPlan {
   int lane_warps = 1;  // W as ishi_projection_plan reports it: lane_warps * (W / lane_warps)
   uint32_t xregion = 0;
   size_t smem = 0, tiles_bytes = 0;
-  double cost = 0;
+  double cost = 0, staging = 0;  // the estimate in microseconds; of it, the activations of all rows
 };
-// one for up to eight rows, one for nine to sixteen (not ok: such a call runs as two launches of the first)
+// one for two to eight rows, one for nine to sixteen (not ok: such a call runs as two launches of the first), one
+// for a single row: without eight rows to stage and read, fewer column ranges are the faster ones (4096 x 4096, affine 4-bit, one row:
+// split 4 / 16 warps 5.25 us, unsplit / 12 warps 4.63; at eight rows 5.3 and 5.7)
 struct FragPlans {
-  FragPlan few, many;
+  FragPlan few, many, one;
 };
 
 // One allocation with the device staging of several projections, freed with the last of them.
@@ -459,8 +461,14 @@ int max_frag_clusters(ishi_ctx *ctx, const FragOps *ops, int s, int warps, int g
   return n;
 }
 
+// Tiles per warp in the ring: no more than keep the warps fed, since every tile asked for at the start goes
+// ahead of something. Deeper rings fitted nearly everywhere and were slower in 40 of 48 measured (format, shape, rows): Q4_K 5120 x 6144 at
+// eight rows 2 ranges / 12 warps, ring 4 -> 3: 7.57 -> 7.07 us; ternary 34816 x 5120 2 / 20, 4 -> 2: 17.66 -> 17.14;
+// IQ4_XS 5120 x 6144 4 / 12, 4 -> 2: 9.13 -> 8.76.
+int ring_for(int groups, int s, int w) { return groups == 2 || w > 16 || (w > 12 && s > 1) ? 2 : 3; }
+
 // The plan with K split s (= cluster size) and w warps per CTA, or false if it does not fit. ring:
-// tiles per warp, 0 for the deepest ring that fits.
+// tiles per warp, 0 for ring_for()'s, or less where that does not fit.
 bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int w, int ring, FragPlan *out) {
   const FragOps *ops = frag_ops_for(d);
   if (!ops) return false;
@@ -485,7 +493,7 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
     if ((long long)panels * c.umax * std::max(kFragMaxWarps * kFragMaxWarps, c.umax) >= (1ll << 32)) return false;
     c.led = s > 1 ? (panels + s - 1) / s : 0;
     bool fits = false;
-    for (int r = ring ? ring : kFragMaxRing; r >= (ring ? ring : 2) && !fits; --r) {
+    for (int r = ring ? ring : ring_for(groups, s, w); r >= (ring ? ring : 2) && !fits; --r) {
       if (r * frag_ring_stride(c.tile_bytes) < groups * 1024) break;  // a drained ring holds a partial tile
       c.ring = r;
       c.smem = frag_smem_bytes((size_t)groups * c.xregion + ops->x_extra, w, c.led, s, groups, c.tile_bytes, r);
@@ -499,7 +507,8 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
       // Estimate in microseconds: the warps' runs of tiles, a tile every 0.075 us of an SM that is
       // full of warps or one per 0.9 us and warp in one that is not; staging; the hand-over in a cluster.
       const double run = (double)((panels * c.umax + w - 1) / w);
-      c.cost = run * std::max(0.9, 0.075 * w) * (groups == 2 ? 1.3 : 1.0) + 0.05 * c.umax * groups + (s > 1 ? 0.5 + 0.05 * s : 0.0);
+      c.staging = 0.05 * c.umax * groups;
+      c.cost = run * std::max(0.9, 0.075 * w) * (groups == 2 ? 1.3 : 1.0) + c.staging + (s > 1 ? 0.5 + 0.05 * s : 0.0);
       c.tiles_bytes = (size_t)c.P * c.units * c.tile_bytes;
       c.ok = true;
       *out = c;
@@ -539,6 +548,7 @@ bool make_frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, FragPl
 // Both launches of a weight; false: the warp-level kernel does not take it.
 bool make_frag_plans(ishi_ctx *ctx, const ishi_weight_desc &d, FragPlans *pl) {
   if (!make_frag_plan(ctx, d, 1, &pl->few)) return false;
+  pl->one = pl->few;
   make_frag_plan(ctx, d, 2, &pl->many);
   return true;
 }
@@ -609,7 +619,7 @@ ishi_status run_frag(ishi_ctx *ctx, const FragPlans &plans, const Workspace &ws,
                      const PeerOut *peers = nullptr, bool gated = false, bool release_late = false) {
   const bool whole = rows <= 8 || plans.many.ok;  // one launch, or pieces of eight rows
   for (int r0 = 0; r0 < rows; r0 += whole ? 16 : 8) {
-    const FragPlan &pl = whole && rows > 8 ? plans.many : plans.few;
+    const FragPlan &pl = whole && rows > 8 ? plans.many : rows == 1 ? plans.one : plans.few;
     FragArgs a;
     memset(&a, 0, sizeof(a));
     a.tiles = ws.tiles;
@@ -969,30 +979,33 @@ ishi_status ishi_verify_matmul(ishi_ctx *ctx, const void *x, int rows, const voi
 
 // ---- projection: the PackedLinear counterpart ---------------------------------------------------
 
-// The tile layout does not depend on the launch plan, so the plans of both launches (up to eight rows, and nine
-// to sixteen) can be chosen by measurement: the planner's best candidates run a few times on the
-// projection's own tiles (activations of zeros, eight or sixteen rows) and the fastest stays.
+// The tile layout does not depend on the launch plan, so the plans of the three launches (two to eight rows, nine to
+// sixteen, one) can be chosen by measurement: the planner's best candidates run a few times on the
+// projection's own tiles (activations of zeros) and the fastest stays.
 // What the measurement costs counts, since the first projection of every shape pays for it: one pair of buffers
-// for both launches, one wait per pass, and no more candidates and launches than the choice needs (create
-// for 17408 x 5120, Q4_K 8.0 -> 4.7 ms, Q6_K 9.7 -> 5.5, against sixteen candidates of each, four launches and
-// sixteen, a wait per candidate; 512 x 1024 2.0 -> 1.1). Over eleven shapes of six formats, twenty times each, the
-// choice is the one of the longer measurement, within 3.5 % of the best plan at eight rows. One launch per
-// candidate in the first pass is up to 30 % behind; with eight final launches at eight rows the events'
-// share lets more plans tie, and the choice varies from run to run.
+// for all launches, one wait per pass, and no more candidates and launches than the choice needs (create
+// for 17408 x 5120, Q4_K 4.3 ms, Q6_K 5.4, 4096 x 4096 affine 4-bit 2.8; ten, eight and eight candidates, four finalists and up to sixteen
+// launches of each 5.7, 7.5 and 3.5). Over sixteen (format, shape) pairs, eight times each, against all 72 plans of one to
+// eight ranges, 12 to 24 warps, rings of two to four, timed on weights from HBM: the choice is the best one or within 3 % of it in
+// 47 of 48, at most 10 % behind (Q4_K 5120 x 17408, one row, two of eight times). One launch per
+// candidate in the first pass is up to 30 % behind. Copies of the tiles that exceed L2, so that the weight comes from HBM as in use,
+// chose no better and cost 1 ms.
 static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragPlan> *few, std::vector<FragPlan> *many) {
-  constexpr size_t kTuned[2] = {10, 8}, kFinalists = 4;
-  constexpr int kLaunches = 3, kFinalLaunches[2] = {16, 8};
+  constexpr int kRows[3] = {8, 16, 1};
+  constexpr size_t kTuned[3] = {8, 7, 6}, kFinalists = 3;
+  constexpr int kLaunches = 3, kFinalLaunches[3] = {12, 8, 8};
   constexpr float kBehind = 1.15f;  // a candidate this far behind in the first pass is no finalist
   typedef std::pair<float, const FragPlan *> Timed;
   const size_t x_bytes = (size_t)16 * p->d.k * sizeof(__half), y_bytes = (size_t)16 * p->d.n * sizeof(__half);
   uint8_t *buffer = nullptr;  // x, then y
   cudaEvent_t marks[2 * kTuned[0]] = {nullptr};
-  for (int groups = 1; groups <= 2; ++groups) {
-    std::vector<FragPlan> *candidates = groups == 2 ? many : few;
-    FragPlan *plan = groups == 2 ? &p->frag.many : &p->frag.few;
+  for (int kind = 0; kind < 3; ++kind) {
+    const int rows = kRows[kind];
+    std::vector<FragPlan> *candidates = rows == 16 ? many : few;
+    FragPlan *plan = rows == 16 ? &p->frag.many : rows == 1 ? &p->frag.one : &p->frag.few;
     if (candidates->size() < 2) continue;
     // a shape measured before on this context keeps its plan (all layers of a model then agree)
-    const auto key = std::make_tuple((const void *)plan->ops, (long long)p->d.n, (long long)p->d.k, groups);
+    const auto key = std::make_tuple((const void *)plan->ops, (long long)p->d.n, (long long)p->d.k, rows);
     const auto known = ctx->tuned.find(key);
     if (known != ctx->tuned.end()) {
       const FragPlan *same = nullptr;
@@ -1008,13 +1021,12 @@ static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragP
       ok = cudaMalloc(&buffer, x_bytes + y_bytes) == cudaSuccess && cudaMemsetAsync(buffer, 0, x_bytes, 0) == cudaSuccess;
       for (cudaEvent_t &e : marks) ok = ok && cudaEventCreate(&e) == cudaSuccess;
     }
-    const int rows = 8 * groups;
     // One timing of every plan in the list, fastest first: a warm-up launch, then `launches` back to back between
     // two events; the host waits once, behind the last plan
     auto time_plans = [&](std::vector<Timed> *plans, int launches) {
       auto launch = [&](const FragPlan &c) {
         FragPlans both;
-        both.few = both.many = c;
+        both.few = both.many = both.one = c;
         return run_frag(ctx, both, p->ws, p->d, buffer, rows, buffer + x_bytes, p->d.n, 0, false, true, false, 0) == ISHI_OK;
       };
       for (size_t i = 0; ok && i < plans->size(); ++i) {
@@ -1033,14 +1045,14 @@ static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragP
     };
     // a first pass over all candidates, then the best few again with more launches (the first pass
     // alone picks among near-equal plans by noise)
-    std::sort(candidates->begin(), candidates->end(), [](const FragPlan &a, const FragPlan &b) { return a.cost < b.cost; });
-    if (candidates->size() > kTuned[groups - 1]) candidates->resize(kTuned[groups - 1]);
     std::vector<Timed> timed, finals;
-    for (const FragPlan &c : *candidates) timed.push_back({0.f, &c});
+    for (const FragPlan &c : *candidates) timed.push_back({(float)(c.cost - (rows == 1 ? c.staging : 0.0)), &c});
+    std::sort(timed.begin(), timed.end(), [](const Timed &a, const Timed &b) { return a.first < b.first; });
+    if (timed.size() > kTuned[kind]) timed.resize(kTuned[kind]);
     if (ok) time_plans(&timed, kLaunches);
     for (const Timed &t : timed)
       if (ok && finals.size() < kFinalists && t.first <= timed[0].first * kBehind) finals.push_back(t);
-    if (ok) time_plans(&finals, kFinalLaunches[groups - 1]);
+    if (ok) time_plans(&finals, kFinalLaunches[kind]);
     if (!ok) {
       cudaGetLastError();  // keep the estimate's choice
       continue;
@@ -1057,7 +1069,7 @@ static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragP
     *plan = *best;
     ctx->tuned[key] = {best->S, best->W, best->ring};
     if (getenv("ISHI_DEBUG_PLAN")) {
-      fprintf(stderr, "ishi plan n=%lld k=%lld rows<=%d measured: split %d, %d clusters, %d warps, ring %d: %.2f us;", (long long)p->d.n,
+      fprintf(stderr, "ishi plan n=%lld k=%lld rows %d measured: split %d, %d clusters, %d warps, ring %d: %.2f us;", (long long)p->d.n,
               (long long)p->d.k, rows, best->S, best->NC, best->W, best->ring, finals[0].first * 1e3f);
       for (const auto &c : timed) fprintf(stderr, " %d/%d/%d:%.1f", c.second->S, c.second->W, c.second->ring, c.first * 1e3f);
       fprintf(stderr, "\n");
@@ -1107,6 +1119,7 @@ static ishi_status create_projection(ishi_ctx *ctx, const ishi_weight_desc *desc
   // again afterwards.
   std::vector<FragPlan> few, many;
   if (make_frag_plan(ctx, p->d, 1, &p->frag.few, &few)) {
+    p->frag.one = p->frag.few;
     make_frag_plan(ctx, p->d, 2, &p->frag.many, &many);
     s = ensure_workspace(ctx, &p->ws, 0, 0, p->frag.few.tiles_bytes, 0);
     if (s == ISHI_OK) s = tile_weight_frag(ctx, p->frag.few, descs, count, n_total, p->ws.tiles, 0, gated);
@@ -1189,10 +1202,10 @@ int ishi_projection_crossover_rows(const ishi_projection *p) {
 ishi_status ishi_projection_plan(const ishi_projection *p, int plan[4]) {
   if (!p || !plan) return ISHI_E_INVALID;
   plan[0] = plan[1] = plan[2] = plan[3] = 0;
-  const FragPlan &f = p->frag.few, &m = p->frag.many;
+  const FragPlan &f = p->frag.few, &m = p->frag.many, &o = p->frag.one;
   if (f.ok) {
     plan[0] = f.S, plan[1] = f.lane_warps, plan[2] = f.W / f.lane_warps;
-    plan[3] = f.ring | (m.ok ? m.ring << 8 | m.S << 12 | m.W << 16 : 0);
+    plan[3] = f.ring | (m.ok ? m.ring << 8 | m.S << 12 | m.W << 16 : 0) | o.W << 21 | (o.S - 1) << 26 | (o.ring - 1) << 29;
   }
   return ISHI_OK;
 }
@@ -1202,14 +1215,16 @@ ishi_status ishi_projection_set_plan(ishi_projection *p, const int plan[4]) {
   ishi_ctx *ctx = p->ctx;
   if (!p->frag.few.ok) return fail(ctx, ISHI_E_UNSUPPORTED, "this projection's kernel has one launch plan only");
   std::lock_guard<std::mutex> g(ctx->lock);
-  const int many = plan[3] >> 8;
+  const int many = (plan[3] >> 8) & 0x1fff, one = plan[3] >> 21;  // (0: the launch of two to eight rows' plan)
   FragPlans both;
   bool fine = plan[1] > 0 && plan[2] > 0 && plan[1] <= kFragMaxWarps && plan[2] <= kFragMaxWarps &&
               frag_plan(ctx, p->d, 1, plan[0], plan[1] * plan[2], plan[3] & 255, &both.few);
   if (fine && many > 0) fine = frag_plan(ctx, p->d, 2, (many >> 4) & 15, many >> 8, many & 15, &both.many);
+  if (fine && one > 0) fine = frag_plan(ctx, p->d, 1, ((one >> 5) & 7) + 1, one & 31, (one >> 8) + 1, &both.one);
   if (!fine)
     return fail(ctx, ISHI_E_INVALID, "plan %d,%d,%d,%d is not among this projection's launch plans", plan[0], plan[1], plan[2], plan[3]);
   both.few.lane_warps = plan[1];
+  if (one == 0) both.one = both.few;
   if (many == 0) make_frag_plan(ctx, p->d, 2, &both.many);
   p->frag = both;
   return ISHI_OK;

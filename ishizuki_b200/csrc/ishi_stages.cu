@@ -26,59 +26,85 @@ __device__ __forceinline__ float to_float<__half>(__half v) { return __half2floa
 template <>
 __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// One CTA of 1024 threads per row, eight values each in 16-byte loads; the row stays in registers
-// between the two passes. Bound by latency alone (a row is 10-20 KB): x and w are on their way together
-// as soon as the launch before is done, w already hinted into L2 (its values are read after the wait, they
-// may be that launch's as well), and the rest is one barrier. Two decoder layers of the 27B shape, four
-// norms, in Q4_K: 122.8 us at eight rows and 112.3 at one with 256 threads reading value by value and w
-// after the sum, 117.2 and 106.3 this way. The squares add up in another order than with 256 threads,
-// which moves a row's factor by its last bit now and then: of 4.1 million values at eight widths 260
-// are not the 64-bit result rounded, 288 before.
-constexpr int kNormThreads = 1024, kNormPer = 8;
+// A row is a cluster of CTAs of 128 threads, eight values per thread in 16-byte loads, held in registers between the
+// two passes. Bound by latency alone (a row is 10-20 KB): x and w are hinted into L2 ahead of the wait
+// (hints only: either may be the output of the launch before), the rest is one exchange of the warps' sums through
+// distributed shared memory and one cluster barrier. The CTAs are as small as the product kernel's leave room for (4096
+// registers, 1280 bytes of shared memory of an SM), so they sit beside the products: one CTA of 1024 threads per row kept
+// its SM from the product behind it, whose CTA there started 3 us and was ready 1.2 us after the others.
+// FIGURES
+// Sums: a warp's 256 squares, then the warps' sums, each by a butterfly, whatever the number of CTAs.
+constexpr int kNormThreads = 128, kNormPer = 8, kNormWarps = 32;  // threads of a CTA, values of one, most warps of a row
 
 template <class T>
-__device__ __forceinline__ void load8(const T *p, float (&v)[kNormPer]) {
+__device__ __forceinline__ void load8_raw(const T *p, T (&v)[kNormPer]) {
   uint4 raw[sizeof(T) / 2];
 #pragma unroll
   for (int i = 0; i < (int)(sizeof(T) / 2); ++i) raw[i] = reinterpret_cast<const uint4 *>(p)[i];
-  const T *t = reinterpret_cast<const T *>(raw);
+  memcpy(v, raw, sizeof(v));
+}
+template <class T>
+__device__ __forceinline__ void load8(const T *p, float (&v)[kNormPer]) {
+  T t[kNormPer];
+  load8_raw(p, t);
 #pragma unroll
   for (int i = 0; i < kNormPer; ++i) v[i] = to_float(t[i]);
 }
 
 // WIDE: width a multiple of eight, all pointers 16-byte aligned; else value by value
 template <class XT, class WT, bool WIDE>
-__global__ void __launch_bounds__(kNormThreads) rms_norm_kernel(const XT *__restrict__ x, const WT *__restrict__ w, long long width, float eps,
-                                                                __half *__restrict__ y) {
-  __shared__ float part[32];
+__global__ void __launch_bounds__(kNormThreads, 16) rms_norm_kernel(const XT *__restrict__ x, const WT *__restrict__ w, long long width, float eps,
+                                                                    int ctas, __half *__restrict__ y) {
+  __shared__ float part[kNormWarps];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int i0 = (int)threadIdx.x * kNormPer, n = (int)min((long long)kNormPer, width - i0);
-  if (n > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + i0));
+  const int r = (int)(blockIdx.x / (unsigned)ctas), c = (int)blockIdx.x - r * ctas, lane = (int)threadIdx.x & 31;
+  const int i0 = (c * kNormThreads + (int)threadIdx.x) * kNormPer, n = (int)min((long long)kNormPer, width - i0);
+  const XT *row = x + (long long)r * width;
+  if (n > 0) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(w + i0));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(row + i0));
+  }
+  if (threadIdx.x < kNormWarps) part[threadIdx.x] = 0.f;  // (of warps that the row does not have)
+  // the CTAs of the row run and their sums are cleared (waited for ahead of the first sum)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");  // x may be the output of the launch before
-  const XT *row = x + (long long)blockIdx.x * width;
-  float v[kNormPer] = {}, f[kNormPer] = {};
+  float v[kNormPer] = {};
   if (WIDE) {
-    if (n > 0) load8(row + i0, v), load8(w + i0, f);
+    if (n > 0) load8(row + i0, v);
   } else {
 #pragma unroll
     for (int j = 0; j < kNormPer; ++j)
-      if (j < n) v[j] = to_float(row[i0 + j]), f[j] = to_float(w[i0 + j]);
+      if (j < n) v[j] = to_float(row[i0 + j]);
+  }
+  WT f[kNormPer];
+  if (WIDE) {
+    if (n > 0) load8_raw(w + i0, f);
+  } else {
+#pragma unroll
+    for (int j = 0; j < kNormPer; ++j)
+      if (j < n) f[j] = w[i0 + j];
   }
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < kNormPer; ++j) ss = fmaf(v[j], v[j], ss);
 #pragma unroll
   for (int d = 16; d; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  float total = part[threadIdx.x & 31];
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (lane < ctas) {  // to every CTA of the row
+    uint32_t at = (uint32_t)__cvta_generic_to_shared(part + c * (kNormThreads / 32) + ((int)threadIdx.x >> 5));
+    asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(at) : "r"(lane));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(ss) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  float total = part[lane];
 #pragma unroll
   for (int d = 16; d; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
-  const float r = rsqrtf(total / (float)width + eps);
-  __half *out = y + (long long)blockIdx.x * width + i0;
+  const float s = rsqrtf(total / (float)width + eps);
+  __half *out = y + (long long)r * width + i0;
   __half h[kNormPer];
 #pragma unroll
-  for (int j = 0; j < kNormPer; ++j) h[j] = __float2half_rn(v[j] * r * f[j]);
+  for (int j = 0; j < kNormPer; ++j) h[j] = __float2half_rn(v[j] * s * to_float(f[j]));
   if (WIDE) {
     if (n > 0) {
       uint4 o;
@@ -96,17 +122,21 @@ template <class XT, class WT>
 cudaError_t launch_as(const void *x, const void *w, long long rows, long long width, float eps, __half *y, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)rows);
+  const int ctas = (int)((width + kNormThreads * kNormPer - 1) / (kNormThreads * kNormPer));  // at most 8: rms_norm_max_width()
+  cfg.gridDim = dim3((unsigned)(rows * ctas));
   cfg.blockDim = dim3(kNormThreads);
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)ctas;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const bool wide = width % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;
   return cudaLaunchKernelEx(&cfg, wide ? rms_norm_kernel<XT, WT, true> : rms_norm_kernel<XT, WT, false>, static_cast<const XT *>(x),
-                            static_cast<const WT *>(w), width, eps, y);
+                            static_cast<const WT *>(w), width, eps, ctas, y);
 }
 
 }  // namespace
@@ -166,7 +196,7 @@ cudaError_t launch_host_copies(const HostCopies &copies, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, host_copy_kernel, copies);
 }
 
-long long rms_norm_max_width() { return (long long)kNormThreads * kNormPer; }
+long long rms_norm_max_width() { return (long long)kNormWarps * 32 * kNormPer; }
 
 // dtypes: 0 fp16, 1 bf16, 2 fp32
 cudaError_t launch_rms_norm(const void *x, int x_dtype, const void *w, int w_dtype, long long rows, long long width, float eps,

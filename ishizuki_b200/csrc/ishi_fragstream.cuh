@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   static_assert(MODE == 0 || NB == 1, "the CUDA-core variant takes one row");
   static_assert(!ONE || (MODE == 0 && NB == 1), "one row is one column group");
   // a single row whose sums the decoder needs is staged by loads and stores, the sums on the way
-  constexpr bool kCopied = Fmt::kRows && !(ONE && Fmt::kRowSums);
+  constexpr bool kCopied = Fmt::kRows && !(ONE && Fmt::kRowSums), kStaged = !Fmt::kRows || Fmt::kRowSums;
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kTile = Fmt::kTileBytes;
   constexpr uint32_t kStride = (uint32_t)((kTile + 15) & ~15), kPart = NB * 512u, kPark = NB * 1024u;  // bytes of a partial tile in fp32, fp64
@@ -563,10 +563,11 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   auto rest = [&] {  // the ring's other tiles, behind the activations
     for (int i = a.ahead; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride);
   };
-  if constexpr (kCopied) {
-    frag_copy_rows<NB>(a, xfrag, Fmt::row_stride(a), ctrl + kFragCtrlX, ub0, uc);
+  const bool copied = kCopied && a.rot_block == 0;
+  if (copied) {
+    if constexpr (kCopied) frag_copy_rows<NB>(a, xfrag, Fmt::row_stride(a), ctrl + kFragCtrlX, ub0, uc);
     rest();
-  } else {
+  } else if constexpr (kStaged) {
     // activations of the column range into fragment order (all warps)
 #pragma unroll
     for (int b = 0; b < NB; ++b)
@@ -580,13 +581,11 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
     else cp_async_wait<3>();
   }
   __syncthreads();  // staged, the tables there, and the control block set up for every warp
-  if constexpr (kCopied) {
-    if (!mbar_wait_u32(ctrl + kFragCtrlX, 0u, abort_word)) *a.err = 1;  // (y stays wrong, the error word tells the host)
-    if constexpr (Fmt::kRowSums) {
+  if (copied && !mbar_wait_u32(ctrl + kFragCtrlX, 0u, abort_word)) *a.err = 1;  // (y stays wrong, the error word tells the host)
+  if constexpr (kCopied && Fmt::kRowSums) {
 #pragma unroll
-      for (int b = 0; b < NB; ++b) Fmt::row_sums(a, xfrag + b * a.xregion, min(a.M - 8 * b, 8), uc);
-      __syncthreads();
-    }
+    for (int b = 0; b < NB; ++b) Fmt::row_sums(a, xfrag + b * a.xregion, min(a.M - 8 * b, 8), uc);
+    __syncthreads();
   }
   ISHI_STAMP(4);
   // shared-memory loads are plain asm the compiler may move; tie their addresses to the waits

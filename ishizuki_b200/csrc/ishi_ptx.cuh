@@ -187,6 +187,23 @@ __device__ __forceinline__ void mma16816_first(float (&c)[4], uint32_t a0, uint3
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// D(16x8, f32) += A(16x8 or 16x4, tf32, row) * B(tf32, col). Thread (g, t) holds a0 = A[g][t], a1 = A[g+8][t],
+// a2 = A[g][t+4], a3 = A[g+8][t+4], b0 = B[t][g], b1 = B[t+4][g]; the operands' low 13 bits are not read.
+__device__ __forceinline__ void mma1688_tf32(float (&c)[4], float a0, float a1, float a2, float a3, uint32_t b0, uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma1684_tf32(float (&c)[4], float a0, float a1, uint32_t b0) {
+  asm(
+      "mma.sync.aligned.m16n8k4.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(b0));
+}
+
 // c += float(a) * float(b) with fp16 operands and an fp32 accumulator, one rounding.
 __device__ __forceinline__ void fma_f32_f16(float &c, uint16_t a, uint16_t b) {
   asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(c) : "h"(a), "h"(b));

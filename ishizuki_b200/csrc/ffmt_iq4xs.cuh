@@ -6,14 +6,14 @@
 //   bytes qs[16 ib + j]: weight j takes the low nibble, weight j + 16 the high nibble, as indices
 //   into the sixteen non-uniform values kvalues_iq4nl; w = d * (ls - 32) * value.
 //
-// A byte is two weights, 16 apart: exactly one A register (an fp16 pair), looked up whole in a
-// 256-entry table of value pairs in shared memory (one copy per lane, so that the 32 lookups of a
-// warp never meet in a bank). The k order inside the MMA follows the bytes: in k-step s (0, 1) of
-// sub-block ib the lane t uses bytes 4t + 2s and 4t + 2s + 1 of the sub-block, i.e. the MMA's k
-// columns (2t, 2t + 1) are the weights (4t + 2s, 4t + 2s + 16) and (2t + 8, 2t + 9) the weights
-// (4t + 2s + 1, 4t + 2s + 17); the activations are staged in the same order. A lane thus owns the
-// 32-bit word t of every sub-block of its two rows. The table values are small integers, exact in
-// fp16; a sub-block's two k-steps accumulate in fp32 inside the MMA and take the integer ls - 32
+// The tile holds the nibbles in the weights' order: a byte is two neighbours, exactly one A register (an fp16
+// pair), looked up whole in a 256-entry table of value pairs in shared memory (one copy per lane, so that the 32
+// lookups of a warp never meet in a bank). Lane t owns weights 8t ... 8t + 7 of every sub-block of its two rows, a 32-bit word: in
+// k-step s (0, 1) its bytes 2s and 2s + 1 are the MMA's k columns (2t, 2t + 1) and (2t + 8, 2t + 9). The activations of both k-steps
+// are then 16 bytes of x as it lies in memory: copied, not staged, and one load (with bytes as the block has them, two
+// weights 16 apart, x was staged in that order by shuffles and read in two; over weights from HBM, best plans, 17408 x 5120 at sixteen / eight / one row
+// 22.8 / 16.1 / 15.5 -> 21.9 / 15.0 / 14.9 us, 5120 x 17408 at eight 18.6 -> 16.8, 4096 x 4096 6.21 -> 5.78). The table values are small
+// integers, exact in fp16; a sub-block's two k-steps accumulate in fp32 inside the MMA and take the integer ls - 32
 // afterwards, the block's d at the end of the tile.
 //
 // Tile (16 rows x 256 k, 2208 bytes): words [4][lane][row g: sub-blocks 2j, 2j + 1; row g + 8: the
@@ -26,9 +26,9 @@ namespace ishi {
 
 struct FragIQ4XS {
   static constexpr int kTileBytes = 2048 + 128 + 32;
-  static constexpr int kXBytes = 4096, kXFixed = 0;   // a staged region: per unit sixteen k-steps of 256 bytes
+  static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 64;  // a staged region: per unit eight rows of 512 bytes; the rows' skews
   static constexpr double kUnit = 1.0;  // unit of the tile results
-  static constexpr bool kRows = false, kRowSums = false;  // staged in fragment order
+  static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
   static constexpr int kExtraBytes = 256 * 128;       // the pair table: entry e of lane l's copy at e * 128 + l * 4
   static constexpr bool kRowMode = false;             // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
@@ -47,7 +47,9 @@ struct FragIQ4XS {
       const long long row = p * kFragRows + g + 8 * (wi >> 1);
       if (row >= s.N) return 0;
       const int sb = 2 * j + (wi & 1);
-      return block(s, row, u)[8 + 16 * sb + 4 * t + bi];
+      // weights 8 t + 2 bi and the next: the low or the high nibbles of two bytes
+      const uint8_t *q = block(s, row, u) + 8 + 16 * sb + 8 * (t & 1) + 2 * bi;
+      return (uint8_t)(t < 2 ? (q[0] & 15) | (q[1] << 4) : (q[0] >> 4) | (q[1] & 0xf0));
     }
     if (b < 2176) {
       const int idx = b - 2048, sb = idx & 7;
@@ -75,34 +77,7 @@ struct FragIQ4XS {
     return *reinterpret_cast<const uint32_t *>(&pair);
   }
 
-  // Activations of the CTA's column range into fragment order. A warp task is (unit, activation
-  // row r): lane l loads k = 8l .. 8l + 7, a quarter of sub-block l / 4: the low-nibble weights
-  // 8 (l % 4) ... + 7 when l % 4 < 2, else the high-nibble weights 16 + 8 (l % 4 - 2) ... + 7. Lanes
-  // l and l ^ 2 hold the two halves of the same eight pairs: they swap four values each, the first
-  // builds the pairs of t = 2 (l % 4), the second those of t + 1. The B registers of k-step
-  // ks = 2 ib + s and quad row r lie at ks * 256 + ((r ^ (ks % 8)) * 4 + t) * 8; the xor spreads the
-  // stores over the banks, a warp's read of one k-step is still one 256-byte run.
-  // No rotation here.
-  template <class Then>
-  static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
-    const int lane = threadIdx.x & 31;
-    const int ib = lane >> 2, r4 = lane & 3;
-    const bool second = r4 >= 2;
-    const int t = second ? 2 * (r4 - 2) + 1 : 2 * r4;
-    frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
-      const uint32_t base = xfrag + (uint32_t)u * kXBytes;
-      const uint32_t got0 = __shfl_xor_sync(0xffffffffu, second ? v.x : v.z, 2);
-      const uint32_t got1 = __shfl_xor_sync(0xffffffffu, second ? v.y : v.w, 2);
-      const uint32_t lo0 = second ? got0 : v.x, lo1 = second ? got1 : v.y;
-      const uint32_t hi0 = second ? v.z : got0, hi1 = second ? v.w : got1;
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const int ks = 2 * ib + s;
-        const uint32_t lo = s ? lo1 : lo0, hi = s ? hi1 : hi0;
-        sts64(base + (uint32_t)ks * 256u + (uint32_t)(((r ^ (ks & 7)) * 4 + t) * 8), prmt(lo, hi, 0x5410u), prmt(lo, hi, 0x7632u));
-      }
-    });
-  }
+  static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
   // the value pair of byte `byte` of word w
   static __device__ __forceinline__ uint32_t pair_of(uint32_t w, int byte, uint32_t table) {
@@ -117,13 +92,12 @@ struct FragIQ4XS {
   template <int MODE, int NB>
   static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
                                               uint32_t tables, int uq, int g, int t, int lane) {
-    const uint32_t xu = xbase + (uint32_t)uq * kXBytes;
+    const uint32_t xrow = xbase + (uint32_t)g * row_stride(a) + (uint32_t)uq * 512u + (uint32_t)t * 16u;
     const uint32_t table = tables + (uint32_t)lane * 4u;
     const uint2 sc0 = lds64(tile + 2048u + (uint32_t)g * 8u), sc1 = lds64(tile + 2048u + (uint32_t)(g + 8) * 8u);
     float su[NB][4];  // sum over the sub-blocks of (ls - 32) * (sum of value * x), d follows at the end
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = su[nb][2] = su[nb][3] = 0.f;
-    const uint32_t xl = xu + (uint32_t)t * 8u;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint4 q = lds128(tile + (uint32_t)j * 512u + (uint32_t)lane * 16u);
@@ -132,16 +106,17 @@ struct FragIQ4XS {
         const int sb = 2 * j + e;
         const uint32_t w0 = e ? q.y : q.x, w1 = e ? q.w : q.z;
         float part[NB][4];
+        uint4 x[NB];
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) x[nb] = lds128(xrow + nb * a.xregion + (uint32_t)sb * 64u);
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
-          const int ks = 2 * sb + s;
           const uint32_t a0 = pair_of(w0, 2 * s, table), a2 = pair_of(w0, 2 * s + 1, table);
           const uint32_t a1 = pair_of(w1, 2 * s, table), a3 = pair_of(w1, 2 * s + 1, table);
 #pragma unroll
           for (int nb = 0; nb < NB; ++nb) {
-            const uint2 b = lds64(xl + nb * a.xregion + (uint32_t)ks * 256u + (uint32_t)((g ^ (ks & 7)) * 32));
-            if (s == 0) mma16816_first(part[nb], a0, a1, a2, a3, b.x, b.y);
-            else mma16816(part[nb], a0, a1, a2, a3, b.x, b.y);
+            if (s == 0) mma16816_first(part[nb], a0, a1, a2, a3, x[nb].x, x[nb].y);
+            else mma16816(part[nb], a0, a1, a2, a3, x[nb].z, x[nb].w);
           }
         }
         const float f0 = byte_float(sb < 4 ? sc0.x : sc0.y, sb & 3) - 8388640.f;  // ls - 32, exact

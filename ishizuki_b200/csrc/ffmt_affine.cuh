@@ -64,6 +64,8 @@ struct FragAffine {
   // the packs that are rotated on the tensor cores all by loads and stores: both ways in one kernel take registers from the loop
   // (34816 x 5120, ternary, eight rows: 17.5 us against 17.1).
   static constexpr bool kRows = !(BITS == 2 && GS == 128), kRowSums = kRows;
+  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
+  static constexpr bool kSumsLater = true;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
@@ -161,37 +163,38 @@ struct FragAffine {
     }
   }
 
-  // After the copies: a warp task per unit. The sums by MMAs with a weight of ones, as in ffmt_q4k.cuh: lane (g, t) gets those of
+  // After the copies: a warp task per unit and four rows. The sums by MMAs with a weight of ones, as in ffmt_q4k.cuh: lane (g, t) gets those of
   // inputs 64 t ... + 31 and + 32 ... + 63 of activation row g.
   static __device__ __forceinline__ void row_sums(const FragArgs &a, uint32_t xfrag, int rows, int uc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t R = row_stride(a), x = stage_acquire(xfrag);
     constexpr uint32_t kOnes = 0x3c003c00u;
-    for (int u = warp; u < uc; u += nw) {
+    const FragPass pass(rows, uc);
+    for (int i = warp; i < pass.tasks; i += nw) {
+      const int u = pass.unit(i), r0 = pass.row(i);
       float s0 = 0.f, s1 = 0.f;
-      for (int r0 = 0; r0 < rows; r0 += 4) {  // (rows past the live ones: whatever is there, for columns of no row)
-        uint4 v[4];
+      uint4 v[4];  // (rows past the live ones: whatever is there, for columns of no row)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = lds128(x + (uint32_t)(r0 + e) * R + (uint32_t)u * 512u + (uint32_t)lane * 16u);
+      for (int e = 0; e < 4; ++e) v[e] = lds128(x + (uint32_t)(r0 + e) * R + (uint32_t)u * 512u + (uint32_t)lane * 16u);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t at = x + (uint32_t)(r0 + e) * R + (uint32_t)u * 512u + (uint32_t)lane * 16u;
-          const uint4 w = arranged(v[e], lane);
-          if (BITS == 4) sts64(at + 8u, w.z, w.w);
-          if (BITS == 2) sts128u(at, w);
-          float c[4];
-          mma16816_first(c, kOnes, kOnes, kOnes, kOnes, v[e].x, v[e].y);
-          mma16816(c, kOnes, kOnes, kOnes, kOnes, v[e].z, v[e].w);
-          if (g == r0 + e) s0 = c[0], s1 = c[1];
-        }
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t at = x + (uint32_t)(r0 + e) * R + (uint32_t)u * 512u + (uint32_t)lane * 16u;
+        const uint4 w = arranged(v[e], lane);
+        if (BITS == 4) sts64(at + 8u, w.z, w.w);
+        if (BITS == 2) sts128u(at, w);
+        float c[4];
+        mma16816_first(c, kOnes, kOnes, kOnes, kOnes, v[e].x, v[e].y);
+        mma16816(c, kOnes, kOnes, kOnes, kOnes, v[e].z, v[e].w);
+        if (g == r0 + e) s0 = c[0], s1 = c[1];
       }
+      if (GS == 128) s0 += s1, s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+      if ((g & 4) != r0) continue;
       const uint32_t base = sums_of(a, x, u);
       if (GS == 32) {
         store_sum(base, g, 2 * t, s0), store_sum(base, g, 2 * t + 1, s1);
       } else {
-        float s = s0 + s1;
-        if (GS == 128) s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if (GS == 64 || !(t & 1)) store_sum(base, g, GS == 64 ? t : t >> 1, s);
+        if (GS == 64) s0 += s1;
+        if (GS == 64 || !(t & 1)) store_sum(base, g, GS == 64 ? t : t >> 1, s0);
       }
     }
   }

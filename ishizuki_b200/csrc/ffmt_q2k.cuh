@@ -13,15 +13,16 @@
 //
 // A 2-bit code masked in place at bits 2j, 2j + 1 of each half of a register is the bit pattern of
 // the fp16 number q * 4^j * 2^-24 (subnormal, hence linear in q); the activations of shift j are
-// staged divided by 4^j (exact unless |x| is tiny). A lane t owns, per weight row, the 32-bit word
-// of code bytes 32 n + 16 h + 4t .. + 3 (h = l / 16): masked at shift j it gives the weights
-// l % 16 = 4t, 4t + 2 of sub-block 8 n + 2 j + h, shifted right by 8 and masked the weights 4t + 1,
-// 4t + 3: the MMA's k columns (2t, 2t + 1) and (2t + 8, 2t + 9); the activations are staged in that order.
+// divided by 4^j (exact unless |x| is tiny). A lane t owns, per weight row, the 32-bit word
+// of code bytes 32 n + 16 h + 4t + {0, 2, 1, 3} (h = l / 16): masked at shift j it gives the weights
+// l % 16 = 4t, 4t + 1 of sub-block 8 n + 2 j + h, shifted right by 8 and masked the weights 4t + 2,
+// 4t + 3: the MMA's k columns (2t, 2t + 1) and (2t + 8, 2t + 9). The activations are copied as they lie in x and divided and put
+// in the order of one 16-byte load per two sub-blocks in place (frag_rows_by_16()). Over weights from HBM, best plans,
+// 17408 x 5120 at sixteen / four / one row 21.9 / 14.3 / 13.8 -> 20.1 / 13.95 / 13.4 us, 4096 x 4096 at sixteen 8.3 -> 7.8.
 //
 // Tile (16 rows x 256 k, 1344 bytes = 16 * 84): code words [2][lane][row g: h = 0, 1; row g + 8:
-// h = 0, 1] @0, per row the sixteen scale bytes @1024 in the order (2t, 2t + 1, 2t + 8, 2t + 9) for
-// t = 0..3 (a lane's A registers of the MMA over sub-blocks are then one word), d of rows
-// (g, g + 8) side by side @1280, dmin the same @1312.
+// h = 0, 1] @0, per row the sixteen scale bytes @1024 (a lane's A registers of the MMA over sub-blocks, 4t .. 4t + 3, are
+// one word), d of rows (g, g + 8) side by side @1280, dmin the same @1312.
 #pragma once
 #include "ishi_fragstream.cuh"
 
@@ -29,10 +30,13 @@ namespace ishi {
 
 struct FragQ2K {
   static constexpr int kTileBytes = 16 * 84;
-  static constexpr int kXSums = 4096;           // after the activations: [lane][hi hi | lo lo] sub-block sums
-  static constexpr int kXBytes = kXSums + 512, kXFixed = 0;  // per unit of a staged region
+  static constexpr int kSumBytes = 512;         // per unit: [lane][hi hi | lo lo] sub-block sums
+  static constexpr int kXBytes = 8 * 512 + kSumBytes, kXFixed = 8 * 64;  // a staged region: per unit eight rows and the sums; the rows' skews
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
-  static constexpr bool kRows = false, kRowSums = false;  // staged in fragment order
+  static constexpr bool kRows = true, kRowSums = true;  // the activations as they lie in x, then put in order and added up
+  // five to eight rows by loads and stores, which arrange and add up on the way (4096 x 4096 at eight rows, copied: 5.66 us against 5.45)
+  static constexpr int kCopyRows = 4;
+  static constexpr bool kSumsLater = false;
   static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;       // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 16;  // most warps of the smaller block size at up to eight rows
@@ -50,14 +54,14 @@ struct FragQ2K {
       const int g = lane >> 2, t = lane & 3, wi = i >> 2, bi = i & 3;
       const long long row = p * kFragRows + g + 8 * (wi >> 1);
       if (row >= s.N) return 0;
-      return block(s, row, u)[16 + 32 * n + 16 * (wi & 1) + 4 * t + bi];
+      const int k = bi == 1 ? 2 : bi == 2 ? 1 : bi;
+      return block(s, row, u)[16 + 32 * n + 16 * (wi & 1) + 4 * t + k];
     }
     if (b < 1280) {
       const int idx = b - 1024, pos = idx & 15;
       const long long row = p * kFragRows + (idx >> 4);
       if (row >= s.N) return 0;
-      const int is = 2 * (pos >> 2) + (pos & 1) + 8 * ((pos >> 1) & 1);
-      return block(s, row, u)[is];
+      return block(s, row, u)[pos];
     }
     const int idx = (b - 1280) & 31;
     const long long row = p * kFragRows + (idx >> 2) + 8 * ((idx >> 1) & 1);
@@ -69,46 +73,19 @@ struct FragQ2K {
     return (uint16_t)(tile_byte(s, p, u, 2 * hw) | ((uint32_t)tile_byte(s, p, u, 2 * hw + 1) << 8));
   }
 
-  // Activations of the CTA's column range into fragment order. A warp task is (unit, activation
-  // row r): lane l loads k = 8l .. 8l + 7: half n = l / 16, shift j = (l / 4) % 4, h = (l % 4) / 2,
-  // the weights l % 16 = 8 (l % 2) ... + 7 of sub-block is = 8 n + 2 j + h, i.e. what lanes
-  // t = 2 (l % 2) and t + 1 of quad r multiply in k-step is; stored divided by 4^j at
-  // is * 256 + ((r ^ (is % 8)) * 4 + t) * 8 (the xor spreads the stores over the banks, a warp's read
-  // of one k-step is still one 256-byte run). Then the sub-block sums of the undivided values
-  // (fp16 hi + lo) for the MMA over sub-blocks. No rotation here.
+  static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
+  // 4^-j in both halves for lane l's values k = 8l .. 8l + 7 of a unit
+  static __device__ __forceinline__ uint32_t factor() { return (uint32_t)(15 - 2 * ((threadIdx.x >> 2) & 3)) * 0x04000400u; }
+
+  static __device__ __forceinline__ void row_sums(const FragArgs &a, uint32_t xfrag, int rows, int uc) {
+    frag_rows_by_16<true>(xfrag, row_stride(a), xfrag + 8u * row_stride(a), kSumBytes, rows, uc, factor());
+  }
+  // Rows on their way from x. A warp task is (unit, row): lane l loads k = 8l .. 8l + 7.
   template <class Then>
   static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
-    const int lane = threadIdx.x & 31;
-    const int j = (lane >> 2) & 3;
-    const int is = 8 * (lane >> 4) + 2 * j + ((lane & 3) >> 1);
-    const uint32_t down1 = (uint32_t)(15 - 2 * j) << 10;  // 4^-j in fp16
-    const uint32_t down = down1 | (down1 << 16);
+    const uint32_t R = row_stride(a), f = factor();
     frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
-      const uint32_t base = xfrag + (uint32_t)u * kXBytes;
-      const __half2 dn = *reinterpret_cast<const __half2 *>(&down);
-      // (x0 x2), (x1 x3) for t = 2 (l % 2); (x4 x6), (x5 x7) for t + 1
-      uint32_t w[4] = {prmt(v.x, v.y, 0x5410u), prmt(v.x, v.y, 0x7632u), prmt(v.z, v.w, 0x5410u),
-                       prmt(v.z, v.w, 0x7632u)};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const __half2 h = __hmul2(*reinterpret_cast<const __half2 *>(&w[q]), dn);
-        w[q] = *reinterpret_cast<const uint32_t *>(&h);
-      }
-      sts128u(base + (uint32_t)is * 256u + (uint32_t)(((r ^ (is & 7)) * 4 + 2 * (lane & 1)) * 8), make_uint4(w[0], w[1], w[2], w[3]));
-      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
-      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
-      float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-      s += __shfl_xor_sync(0xffffffffu, s, 1);  // the sub-block's sixteen values
-      if ((lane & 1) == 0) {
-        const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-        // sub-block is is slot is of the MMA over sub-blocks: lane t' = (is % 8) / 2 of quad r holds
-        // it in register is / 8, half is % 2
-        const uint32_t at = base + kXSums + (uint32_t)((r * 4 + ((is & 7) >> 1)) * 16 + (is >> 3) * 4 + (is & 1) * 2);
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
-      }
+      frag_put_by_16<true>(xfrag + (uint32_t)r * R + (uint32_t)u * 512u, xfrag + 8u * R + (uint32_t)(u * kSumBytes), r, v, f);
     });
   }
 
@@ -120,33 +97,34 @@ struct FragQ2K {
   template <int MODE, int NB>
   static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
                                               uint32_t tables, int uq, int g, int t, int lane) {
-    const uint32_t xu = xbase + (uint32_t)uq * kXBytes;
+    const uint32_t R = row_stride(a), xrow = xbase + (uint32_t)g * R + (uint32_t)uq * 512u + (uint32_t)t * 16u;
+    const uint32_t sums = xbase + 8u * R + (uint32_t)(uq * kSumBytes) + (uint32_t)lane * 16u;
     const uint4 h0 = lds128(tile + 1024u + (uint32_t)g * 16u), h1 = lds128(tile + 1024u + (uint32_t)(g + 8) * 16u);
-    // the scales (low nibbles), word tw = sub-blocks (2 tw, 2 tw + 1, 2 tw + 8, 2 tw + 9)
+    // the scales (low nibbles)
     const uint32_t sl0[4] = {h0.x & 0x0f0f0f0fu, h0.y & 0x0f0f0f0fu, h0.z & 0x0f0f0f0fu, h0.w & 0x0f0f0f0fu};
     const uint32_t sl1[4] = {h1.x & 0x0f0f0f0fu, h1.y & 0x0f0f0f0fu, h1.z & 0x0f0f0f0fu, h1.w & 0x0f0f0f0fu};
-    const uint32_t xl = xu + (uint32_t)t * 8u;
     float su[NB][4];
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) su[nb][0] = su[nb][1] = su[nb][2] = su[nb][3] = 0.f;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const uint4 q = lds128(tile + (uint32_t)n * 512u + (uint32_t)lane * 16u);
+      const uint32_t y[4] = {q.x >> 8, q.y >> 8, q.z >> 8, q.w >> 8};
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t w0 = h ? q.y : q.x, w1 = h ? q.w : q.z;
-        const uint32_t y0 = w0 >> 8, y1 = w1 >> 8;
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t mask = 0x00030003u << (2 * j);
+        uint4 b[NB];  // both sub-blocks' activations
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int nb = 0; nb < NB; ++nb) b[nb] = lds128(xrow + nb * a.xregion + (uint32_t)(4 * n + j) * 64u);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
           const int is = 8 * n + 2 * j + h;
-          const uint32_t mask = 0x00030003u << (2 * j);
-          const int tw = (is & 7) >> 1, e = (is & 1) + 2 * (is >> 3);
-          const float f0 = byte_float(sl0[tw], e) - 8388608.f, f1 = byte_float(sl1[tw], e) - 8388608.f;
+          const uint32_t w0 = h ? q.y : q.x, w1 = h ? q.w : q.z, y0 = h ? y[1] : y[0], y1 = h ? y[3] : y[2];
+          const float f0 = byte_float(sl0[is >> 2], is & 3) - 8388608.f, f1 = byte_float(sl1[is >> 2], is & 3) - 8388608.f;
 #pragma unroll
           for (int nb = 0; nb < NB; ++nb) {
-            const uint2 b = lds64(xl + nb * a.xregion + (uint32_t)is * 256u + (uint32_t)((g ^ (is & 7)) * 32));
             float part[4];
-            mma16816_first(part, w0 & mask, w1 & mask, y0 & mask, y1 & mask, b.x, b.y);
+            mma16816_first(part, w0 & mask, w1 & mask, y0 & mask, y1 & mask, h ? b[nb].z : b[nb].x, h ? b[nb].w : b[nb].y);
             su[nb][0] = fmaf(f0, part[0], su[nb][0]), su[nb][1] = fmaf(f0, part[1], su[nb][1]);
             su[nb][2] = fmaf(f1, part[2], su[nb][2]), su[nb][3] = fmaf(f1, part[3], su[nb][3]);
           }
@@ -154,7 +132,7 @@ struct FragQ2K {
       }
     }
     // sum_is min_is * (sum of x over sub-block is): the MMA over sub-blocks; this lane's slots are
-    // sub-blocks 2t, 2t + 1, 2t + 8, 2t + 9, the word t of each row's sixteen bytes, high nibbles
+    // sub-blocks 4t .. 4t + 3, the word t of each row's sixteen bytes, high nibbles
     const uint32_t m0 = ((t == 0 ? h0.x : t == 1 ? h0.y : t == 2 ? h0.z : h0.w) >> 4) & 0x0f0f0f0fu;
     const uint32_t m1 = ((t == 0 ? h1.x : t == 1 ? h1.y : t == 2 ? h1.z : h1.w) >> 4) & 0x0f0f0f0fu;
     // (a byte as the low bits of an fp16 is the subnormal number m * 2^-24, as the codes are)
@@ -165,7 +143,7 @@ struct FragQ2K {
     const float n0 = -half_bits_to_float(mm & 0xffffu), n1 = -half_bits_to_float(mm >> 16);
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
-      const uint4 bs = lds128(xu + nb * a.xregion + kXSums + (uint32_t)lane * 16u);
+      const uint4 bs = lds128(sums + nb * a.xregion);
       float cm[4];
       mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
       mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);

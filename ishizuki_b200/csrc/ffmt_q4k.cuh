@@ -45,6 +45,8 @@ struct FragQ4K {
   static constexpr int kTileBytes = 2048 + 16 * 16 + 16 * 4;
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr bool kRows = true, kRowSums = true;  // the activations as they lie in x
+  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
+  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows
@@ -103,7 +105,7 @@ struct FragQ4K {
 
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
-  // Sub-block sums of x for the minimum term, a warp task per unit. The sixteen bytes of lane l are part of
+  // Sub-block sums of x for the minimum term, a warp task per unit and four rows. The sixteen bytes of lane l are part of
   // sub-block l / 4: as B registers (column l / 4, any k) two MMAs with a weight of ones give the row's eight
   // sums, the same in every row of C, and lane (g, t) keeps sub-blocks 2t and 2t + 1 of activation row g. (One accumulator per row, not
   // a matrix that picks the row: 0 * inf would reach the other rows.)
@@ -111,20 +113,21 @@ struct FragQ4K {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, g = lane >> 2;
     const uint32_t R = row_stride(a), x = stage_acquire(xfrag);
     constexpr uint32_t kOnes = 0x3c003c00u;
-    for (int u = warp; u < uc; u += nw) {
+    const FragPass pass(rows, uc);
+    for (int i = warp; i < pass.tasks; i += nw) {
+      const int u = pass.unit(i), r0 = pass.row(i);
       float s0 = 0.f, s1 = 0.f;
-      for (int r0 = 0; r0 < rows; r0 += 4) {  // (rows past the live ones: whatever is there, for columns of no row)
-        uint4 v[4];
+      uint4 v[4];  // (rows past the live ones: whatever is there, for columns of no row)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = lds128(x + (uint32_t)(r0 + e) * R + (uint32_t)u * 512u + (uint32_t)lane * 16u);
+      for (int e = 0; e < 4; ++e) v[e] = lds128(x + (uint32_t)(r0 + e) * R + (uint32_t)u * 512u + (uint32_t)lane * 16u);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float c[4];
-          mma16816_first(c, kOnes, kOnes, kOnes, kOnes, v[e].x, v[e].y);
-          mma16816(c, kOnes, kOnes, kOnes, kOnes, v[e].z, v[e].w);
-          if (g == r0 + e) s0 = c[0], s1 = c[1];
-        }
+      for (int e = 0; e < 4; ++e) {
+        float c[4];
+        mma16816_first(c, kOnes, kOnes, kOnes, kOnes, v[e].x, v[e].y);
+        mma16816(c, kOnes, kOnes, kOnes, kOnes, v[e].z, v[e].w);
+        if (g == r0 + e) s0 = c[0], s1 = c[1];
       }
+      if ((g & 4) != r0) continue;
       // as fp16 hi + lo: the B fragment of the minimum-term MMA, whose k index runs over sub-blocks
       const __half h0 = __float2half_rn(s0), h1 = __float2half_rn(s1);
       const __half l0 = __float2half_rn(s0 - __half2float(h0)), l1 = __float2half_rn(s1 - __half2float(h1));

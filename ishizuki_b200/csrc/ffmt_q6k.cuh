@@ -32,13 +32,13 @@
 // -> 17.1 us (23.5 at sixteen); 248320 x 5120 at eight rows 213 -> 177 us in short runs, 5.9 TB/s (a
 // loop of seconds runs into the power cap: 219).
 // Inside a k-step the lane t holds the weights 4t .. 4t + 3 of the group: slots (2t, 2t + 1) are
-// 4t, 4t + 1 and slots (2t + 8, 2t + 9) are 4t + 2, 4t + 3; the activations are staged in the same
-// order, so that a lane reads the B registers of two k-steps with one 16-byte load.
+// 4t, 4t + 1 and slots (2t + 8, 2t + 9) are 4t + 2, 4t + 3; the activations are copied as they lie in x and put in that
+// order in place (frag_rows_by_16()), so that a lane reads the B registers of two k-steps with one 16-byte load. Over weights
+// from HBM, best plans, 17408 x 5120 at four / one row 16.5 / 16.1 -> 16.3 / 15.2 us, 5120 x 17408 18.6 / 17.5 -> 18.1 / 16.9.
 //
 // Tile (16 rows x 256 k, 3360 bytes = 16 * 210): [6][lane][16 bytes] = the lane's words 3 i + w of
-// pair i, four at a time; per row the sixteen scales + 128 @3072 in the order (2t, 2t + 1, 2t + 8,
-// 2t + 9) for t = 0..3 (a lane's A registers of the group-sum MMA are then one word), and d of rows
-// (g, g + 8) side by side @3328.
+// pair i, four at a time; per row the sixteen scales + 128 @3072 (a lane's A registers of the group-sum MMA, groups 4t .. 4t + 3,
+// are one word), and d of rows (g, g + 8) side by side @3328.
 #pragma once
 #include "ishi_fragstream.cuh"
 
@@ -46,10 +46,13 @@ namespace ishi {
 
 struct FragQ6K {
   static constexpr int kTileBytes = 16 * 210;
-  static constexpr int kXSums = 4096;             // after the activations: [lane][hi hi | lo lo] group sums
-  static constexpr int kXBytes = kXSums + 512, kXFixed = 0;  // per unit of a staged region
+  static constexpr int kSumBytes = 512;           // per unit: [lane][hi hi | lo lo] group sums
+  static constexpr int kXBytes = 8 * 512 + kSumBytes, kXFixed = 8 * 64;  // a staged region: per unit eight rows and the sums; the rows' skews
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
-  static constexpr bool kRows = false, kRowSums = false;  // staged in fragment order
+  static constexpr bool kRows = true, kRowSums = true;  // the activations as they lie in x, then put in order and added up
+  // five to eight rows by loads and stores, which arrange and add up on the way (4096 x 4096 at eight rows, copied: 6.6 us against 6.35)
+  static constexpr int kCopyRows = 4;
+  static constexpr bool kSumsLater = false;
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 16;  // most warps of the smaller block size at up to eight rows
@@ -95,10 +98,10 @@ struct FragQ6K {
       return (uint16_t)out;
     }
     if (hw < 1664) {
-      const int row16 = (hw - 1536) >> 3, pair = (hw - 1536) & 7;  // scales 2 (pair / 2) + 8 (pair % 2) and the next
+      const int row16 = (hw - 1536) >> 3, pair = (hw - 1536) & 7;
       const long long row = p * kFragRows + row16;
       if (row >= s.N) return 0;
-      const uint8_t *sc = block(s, row, u) + 192 + 2 * (pair >> 1) + 8 * (pair & 1);
+      const uint8_t *sc = block(s, row, u) + 192 + 2 * pair;
       return (uint16_t)(((uint32_t)sc[0] | ((uint32_t)sc[1] << 8)) ^ 0x8080u);
     }
     const long long row = p * kFragRows + ((hw - 1664) >> 1) + 8 * h;
@@ -107,35 +110,17 @@ struct FragQ6K {
     return (uint16_t)((uint32_t)blk[208] | ((uint32_t)blk[209] << 8));
   }
 
-  // Activations of the CTA's column range into fragment order. A warp task is (unit, activation
-  // row r): lane l loads k = 8l .. 8l + 7, half of group l / 2, i.e. what lanes t = 2(l & 1) and
-  // t + 1 of quad r multiply in k-step l / 2. The pair of k-steps i = l / 4 lies at
-  // i * 512 + ((r ^ i) * 4 + t) * 16 (+ 8 for the odd k-step); the xor spreads the stores over the
-  // banks and a warp's read of one pair is still one 512-byte run. Then the group sums (fp16 hi +
-  // lo) for the MMA over groups.
+  static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
+
+  static __device__ __forceinline__ void row_sums(const FragArgs &a, uint32_t xfrag, int rows, int uc) {
+    frag_rows_by_16<false>(xfrag, row_stride(a), xfrag + 8u * row_stride(a), kSumBytes, rows, uc, 0u);
+  }
+  // Rows on their way from x. A warp task is (unit, row): lane l loads k = 8l .. 8l + 7.
   template <class Then>
   static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
-    const int lane = threadIdx.x & 31;
+    const uint32_t R = row_stride(a);
     frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
-      const uint32_t base = xfrag + (uint32_t)u * kXBytes;
-      const int pi = lane >> 2, ks = lane >> 1;
-      const uint32_t dst = base + (uint32_t)pi * 512u + (uint32_t)(((r ^ pi) * 4 + 2 * (lane & 1)) * 16 + (ks & 1) * 8);
-      sts64(dst, v.x, v.y);
-      sts64(dst + 16u, v.z, v.w);
-      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
-      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
-      float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-      s += __shfl_xor_sync(0xffffffffu, s, 1);  // the group's sixteen values
-      if ((lane & 1) == 0) {
-        const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-        // group ks is slot ks of the MMA over groups: lane t' = (ks % 8) / 2 of quad r holds it in
-        // register ks / 8, half ks % 2
-        const uint32_t at = base + kXSums + (uint32_t)((r * 4 + ((ks & 7) >> 1)) * 16 + (ks >> 3) * 4 + (ks & 1) * 2);
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
-      }
+      frag_put_by_16<false>(xfrag + (uint32_t)r * R + (uint32_t)u * 512u, xfrag + 8u * R + (uint32_t)(u * kSumBytes), r, v, 0u);
     });
   }
 
@@ -159,10 +144,10 @@ struct FragQ6K {
   template <int MODE, int NB>
   static __device__ __forceinline__ void unit(float (&acc)[NB][4], const FragArgs &a, uint32_t tile, uint32_t xbase,
                                               uint32_t tables, int uq, int g, int t, int lane) {
-    const uint32_t xu = xbase + (uint32_t)uq * kXBytes;
+    const uint32_t R = row_stride(a), xrow = xbase + (uint32_t)g * R + (uint32_t)uq * 512u + (uint32_t)t * 16u;
+    const uint32_t sums = xbase + 8u * R + (uint32_t)(uq * kSumBytes) + (uint32_t)lane * 16u;
     const uint4 h0 = lds128(tile + 3072u + (uint32_t)g * 16u), h1 = lds128(tile + 3072u + (uint32_t)(g + 8) * 16u);
     const uint32_t hw0[4] = {h0.x, h0.y, h0.z, h0.w}, hw1[4] = {h1.x, h1.y, h1.z, h1.w};
-    const uint32_t lane_off = (uint32_t)g * 64u + (uint32_t)t * 16u;
     // The first k-steps of the pairs are added up in su, the second in sv: shorter chains. Two column groups
     // have too few registers for both (sixteen rows: 2 % slower than with one sum).
     constexpr bool kOneSum = NB == 2;
@@ -186,12 +171,12 @@ struct FragQ6K {
       const uint32_t a1 = (w0 >> 6) & 0x03f003f0u, a3 = (w1 >> 6) & 0x03f003f0u;
       const uint32_t e0 = w0 & 0x03f003f0u, e1 = w1 & 0x03f003f0u;
       const uint32_t e2 = w2 & 0x03f003f0u, e3 = (w2 >> 6) & 0x03f003f0u;
-      // scales of groups 2 pi and 2 pi + 1: word pi % 4 of the row's sixteen, bytes 2 (pi / 4) and + 1
-      const float s00 = scale_of(hw0[pi & 3], 2 * (pi >> 2)), s01 = scale_of(hw0[pi & 3], 2 * (pi >> 2) + 1);
-      const float s10 = scale_of(hw1[pi & 3], 2 * (pi >> 2)), s11 = scale_of(hw1[pi & 3], 2 * (pi >> 2) + 1);
+      // scales of groups 2 pi and 2 pi + 1
+      const float s00 = scale_of(hw0[pi >> 1], 2 * (pi & 1)), s01 = scale_of(hw0[pi >> 1], 2 * (pi & 1) + 1);
+      const float s10 = scale_of(hw1[pi >> 1], 2 * (pi & 1)), s11 = scale_of(hw1[pi >> 1], 2 * (pi & 1) + 1);
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
-        const uint4 b = lds128(xu + nb * a.xregion + (uint32_t)pi * 512u + (lane_off ^ (uint32_t)(pi << 6)));
+        const uint4 b = lds128(xrow + nb * a.xregion + (uint32_t)pi * 64u);
         float c0[4], c1[4];
         mma16816_first(c0, a0, a1, a2, a3, b.x, b.y);
         mma16816_first(c1, e0, e1, e2, e3, b.z, b.w);
@@ -203,7 +188,7 @@ struct FragQ6K {
       }
     }
     // sum_g scale_g * (sum of x over group g): the MMA over groups; this lane's slots are groups
-    // 2t, 2t + 1, 2t + 8, 2t + 9, the word t of each row's scales
+    // 4t .. 4t + 3, the word t of each row's scales
     const uint32_t w0 = (t == 0 ? h0.x : t == 1 ? h0.y : t == 2 ? h0.z : h0.w);
     const uint32_t w1 = (t == 0 ? h1.x : t == 1 ? h1.y : t == 2 ? h1.z : h1.w);
     const uint32_t a0 = scale_pair(w0, 0x4140u), a1 = scale_pair(w1, 0x4140u);
@@ -213,7 +198,7 @@ struct FragQ6K {
     const float dl0 = d0 * 0.0625f, dl1 = d1 * 0.0625f, dm0 = d0 * (-32.f / 16777216.f), dm1 = d1 * (-32.f / 16777216.f);
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
-      const uint4 bs = lds128(xu + nb * a.xregion + kXSums + (uint32_t)lane * 16u);
+      const uint4 bs = lds128(sums + nb * a.xregion);
       float cm[4];
       mma16816_first(cm, a0, a1, a2, a3, bs.x, bs.y);
       mma16816(cm, a0, a1, a2, a3, bs.z, bs.w);

@@ -424,6 +424,84 @@ __device__ __forceinline__ void frag_copy_rows(const FragArgs &a, uint32_t xfrag
       for (int i = (int)threadIdx.x; i < uc * 32; i += (int)blockDim.x) sts128u(row_at(m) + 16u * (uint32_t)i, make_uint4(0u, 0u, 0u, 0u));
 }
 
+// Decoders with a scale per sixteen weights (Q2_K, Q6_K) multiply a group per k-step, and a lane's four values of a group
+// are 8 bytes of x. Each 64 bytes of a row (two k-steps) are put in the order that makes its 8 bytes of both one 16-byte
+// load: lane t's at 16 t. Where lane l's values k = 8l .. 8l + 7 of a unit go inside a row, the last four 16 bytes further on:
+__device__ __forceinline__ uint32_t frag_pair_slot(int lane) { return (uint32_t)((lane >> 2) * 64 + (lane & 1) * 32 + (lane & 2) * 4); }
+__device__ __forceinline__ uint32_t frag_times(uint32_t v, uint32_t f) {
+  const __half2 r = __hmul2(*reinterpret_cast<const __half2 *>(&v), *reinterpret_cast<const __half2 *>(&f));
+  return *reinterpret_cast<const uint32_t *>(&r);
+}
+// The group sums of x as fp16 high and low parts, the B registers of the MMA over the sixteen groups, whose slots of lane t are groups
+// 4t .. 4t + 3: [lane (row, t)][hi hi lo lo].
+__device__ __forceinline__ void frag_store_sums16(uint32_t sums, int lane, const float (&s)[4]) {
+  uint32_t hi[4], lo[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half h = __float2half_rn(s[i]), l = __float2half_rn(s[i] - __half2float(h));
+    hi[i] = __half_as_ushort(h), lo[i] = __half_as_ushort(l);
+  }
+  sts128u(sums + (uint32_t)lane * 16u, make_uint4(hi[0] | (hi[1] << 16), hi[2] | (hi[3] << 16), lo[0] | (lo[1] << 16), lo[2] | (lo[3] << 16)));
+}
+// A pass over copied rows has a warp task per unit and four rows: task i of `halves` (one or two) per unit
+struct FragPass {
+  int tasks, halves;
+  __device__ __forceinline__ FragPass(int rows, int uc) : tasks(uc * (rows > 4 ? 2 : 1)), halves(rows > 4 ? 2 : 1) {}
+  __device__ __forceinline__ int unit(int i) const { return halves == 2 ? i >> 1 : i; }
+  __device__ __forceinline__ int row(int i) const { return halves == 2 ? (i & 1) * 4 : 0; }  // the first of the four
+};
+// Both, in place, for the copied rows of a column range. The sums by MMAs whose weight is one for the first
+// group of a column's 32 values in rows 0-7 and for the second in rows 8-15. SCALED: the values times `factor` (both halves), the sums without.
+template <bool SCALED>
+__device__ __forceinline__ void frag_rows_by_16(uint32_t xfrag, uint32_t R, uint32_t sums, uint32_t sum_bytes, int rows, int uc, uint32_t factor) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, g = lane >> 2;
+  const uint32_t x = stage_acquire(xfrag), first = lane & 2 ? 0u : 0x3c003c00u, second = lane & 2 ? 0x3c003c00u : 0u;
+  const FragPass pass(rows, uc);
+  for (int i = warp; i < pass.tasks; i += nw) {
+    const int u = pass.unit(i), r0 = pass.row(i);
+    const uint32_t at = x + (uint32_t)r0 * R + (uint32_t)u * 512u;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    uint4 v[4];  // (rows past the live ones: whatever is there, for columns of no row)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = lds128(at + (uint32_t)e * R + (uint32_t)lane * 16u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float c[4];
+      mma16816_first(c, first, second, first, second, v[e].x, v[e].y);
+      mma16816(c, first, second, first, second, v[e].z, v[e].w);
+      if (g == r0 + e) s[0] = c[0], s[1] = c[2], s[2] = c[1], s[3] = c[3];
+    }
+    __syncwarp();  // every lane has its values of the four rows (the MMAs took them all)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t to = at + (uint32_t)e * R + frag_pair_slot(lane);
+      sts64(to, SCALED ? frag_times(v[e].x, factor) : v[e].x, SCALED ? frag_times(v[e].y, factor) : v[e].y);
+      sts64(to + 16u, SCALED ? frag_times(v[e].z, factor) : v[e].z, SCALED ? frag_times(v[e].w, factor) : v[e].w);
+    }
+    if ((g & 4) == r0) frag_store_sums16(sums + (uint32_t)u * sum_bytes, lane, s);
+  }
+}
+// The same for rows that are stored and added up on their way from x: lane l's values v of the unit whose row begins at `row`.
+template <bool SCALED>
+__device__ __forceinline__ void frag_put_by_16(uint32_t row, uint32_t sums, int r, uint4 v, uint32_t factor) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t to = row + frag_pair_slot(lane);
+  sts64(to, SCALED ? frag_times(v.x, factor) : v.x, SCALED ? frag_times(v.y, factor) : v.y);
+  sts64(to + 16u, SCALED ? frag_times(v.z, factor) : v.z, SCALED ? frag_times(v.w, factor) : v.w);
+  const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+  const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+  const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
+  const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
+  float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+  s += __shfl_xor_sync(0xffffffffu, s, 1);  // the group's sixteen values
+  if ((lane & 1) == 0) {
+    const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+    const uint32_t at = sums + (uint32_t)((r * 4 + (lane >> 3)) * 16 + (lane & 6));
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
+  }
+}
+
 // A decoder's shared-memory tables (kExtraBytes, a multiple of 16), laid out once per device from
 // Fmt::table_word; every CTA copies them from here, a few 16-byte async copies per thread that land
 // while it waits for the launch before. Building them in place, lookups and conversions ahead of the
@@ -563,7 +641,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   auto rest = [&] {  // the ring's other tiles, behind the activations
     for (int i = a.ahead; i < R - 1; ++i) fetch(ring + (uint32_t)i * kStride);
   };
-  const bool copied = kCopied && a.rot_block == 0;
+  const bool copied = kCopied && a.rot_block == 0 && (NB == 2 || a.M <= Fmt::kCopyRows);
   if (copied) {
     if constexpr (kCopied) frag_copy_rows<NB>(a, xfrag, Fmt::row_stride(a), ctrl + kFragCtrlX, ub0, uc);
     rest();
@@ -583,9 +661,11 @@ __global__ void __launch_bounds__(MAXW * 32, 1) frag_kernel(const FragArgs a) {
   __syncthreads();  // staged, the tables there, and the control block set up for every warp
   if (copied && !mbar_wait_u32(ctrl + kFragCtrlX, 0u, abort_word)) *a.err = 1;  // (y stays wrong, the error word tells the host)
   if constexpr (kCopied && Fmt::kRowSums) {
+    if (copied || Fmt::kSumsLater) {
 #pragma unroll
-    for (int b = 0; b < NB; ++b) Fmt::row_sums(a, xfrag + b * a.xregion, min(a.M - 8 * b, 8), uc);
-    __syncthreads();
+      for (int b = 0; b < NB; ++b) Fmt::row_sums(a, xfrag + b * a.xregion, a.world > 0 ? 8 : min(a.M - 8 * b, 8), uc);
+      __syncthreads();
+    }
   }
   ISHI_STAMP(4);
   // shared-memory loads are plain asm the compiler may move; tie their addresses to the waits

@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) ggml_expand_kernel(const in
   constexpr int kBytes = ggml_type_bytes(TYPE), kTable = ggml_table_bytes(TYPE);
   __shared__ __align__(16) uint8_t s_blocks[kExpandWarps][kExpandSlot<TYPE>];
   __shared__ __align__(16) uint8_t s_table[kTable ? kTable : 16];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t table = smem_u32(s_table);
   if (kTable) {
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) ggml_expand_kernel(const in
     __syncthreads();
     table = stage_acquire(table);
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // ids and blocks may be the launch before's, and y read by it
   const uint32_t slot = smem_u32(s_blocks[warp]);
   const bool wide = (reinterpret_cast<uintptr_t>(y) & (8 * sizeof(OT) - 1)) == 0;
   const int chunk = 1 << chunk_log;
@@ -310,8 +312,19 @@ static cudaError_t launch_expand(int type, const int *ids, long long rows, const
   return with_type(type, [&](auto t) {
     constexpr int T = decltype(t)::value;
     auto launch = [&](auto *y) {
-      ggml_expand_kernel<T, std::remove_pointer_t<decltype(y)>, ROWS>
-          <<<(unsigned)grid, kExpandWarps * 32, 0, st>>>(ids, rows, blocks, table_rows, per_row, chunk_log, y);
+      // may start while the launch before it ends, and waits for that one itself: 2048 rows of 5120 in Q4_K 8.2 -> 7.0 us
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof(cfg));
+      cfg.gridDim = dim3((unsigned)grid);
+      cfg.blockDim = dim3(kExpandWarps * 32);
+      cfg.stream = st;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      cudaLaunchKernelEx(&cfg, ggml_expand_kernel<T, std::remove_pointer_t<decltype(y)>, ROWS>, ids, rows, blocks, table_rows, per_row,
+                         chunk_log, y);
     };
     if (out_dtype == 0) launch(static_cast<__half *>(out));
     else if (out_dtype == 1) launch(static_cast<__nv_bfloat16 *>(out));

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) exl3_dequantize_kernel(const uint32_t *__
 // 34.6 and, past eight rows, two products 65. Issue in 73 % of the cycles, the IMAD pipe 56 %.
 //
 // The trellis is the caller's own memory: nothing of it is read before the launches ahead have
-// finished (griddepcontrol.wait).
+// finished (griddepcontrol.wait), its first slices are only hinted into L2.
 constexpr int kExl3Warps = 32, kExl3Phases = 16, kExl3Cols = 4;
 constexpr int kExl3OutStride = 132;  // floats between rows of the k phases' sums: conflict-free stores
 struct Exl3Args {
@@ -343,7 +343,6 @@ __global__ void __launch_bounds__(kExl3Warps * 32, 1) exl3_product_kernel(const 
   }
   __syncwarp();
   if (S > 1) cluster_arrive_relaxed();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // this warp's slices: k tiles 8 kb0 + phase + 16 i
   const long long step = (a.N / 16) * kExl3Phases * (long long)kTileBytes;
@@ -365,6 +364,12 @@ __global__ void __launch_bounds__(kExl3Warps * 32, 1) exl3_product_kernel(const 
     --f_left;
     cp_async_commit();
   };
+  // The first slices into L2 while the launch before this one ends: hints, no value is read before the wait (two gate
+  // projections of 17408 x 5120 at eight rows 55.4 -> 54.9 us)
+  constexpr int kLines = (kSlice + 127) / 128;
+  for (int i = lane; i < min(f_left, R - 2) * kLines; i += 32)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(f_src + (i / kLines) * step + (i % kLines) * 128));
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int i = 0; i < R - 2; ++i) fetch(ring + (uint32_t)(i * kSlice));
 
   float acc[NB][kExl3Cols][4];

@@ -540,6 +540,10 @@ bool make_frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, FragPl
       if (all) all->push_back(c);
       if (!best.ok || c.cost < best.cost) best = c;
     }
+  // inputs so wide that the activations leave no room for four warps
+  for (int s = 1; !best.ok && s <= kFragMaxSplit && s <= units; ++s)
+    for (int w : {2, 1})
+      if (!best.ok) frag_plan(ctx, d, groups, s, w, 2, &best);
   if (!best.ok) return false;
   *pl = best;
   return true;

@@ -200,3 +200,45 @@ def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(bits, gs, dtype):
         finally:
             BonsaiRuntime.route = _lib.ROUTE_AUTO
     here.ctx.poll()
+
+
+@pytest.mark.parametrize("bits,gs", [(8, 32), (8, 64), (4, 32), (4, 64), (4, 128), (2, 64), (2, 128)])
+def test_an_infinite_activation_stays_in_its_row(bits, gs):
+    """The group sums of x come from MMAs over several rows at once, the bias term from their pieces in tf32: an infinity or
+    a NaN in one activation row must not reach the others, whose products keep their bits; a large finite row keeps its value."""
+    rng = np.random.default_rng(bits * 100 + gs)
+    n, k = 200, 1536
+    w, s, b, sd, bd, bf16 = make_pack(rng, n, k, bits, gs, "f16")
+    lin = PackedLinear(dev(w), sd, bd, groupSize=gs, bits=bits)
+    for m, bad in ((3, 1), (8, 6), (16, 11)):
+        x = (rng.standard_normal((m, k)) * 2).astype(np.float16)
+        want = lin(dev(x))
+        for value in (np.inf, np.nan):
+            worse = x.copy()
+            worse[bad, 777] = value
+            got = lin(dev(worse))
+            others = [r for r in range(m) if r != bad]
+            assert torch.equal(got[others], want[others])
+            assert not torch.isfinite(got[bad]).any()
+        large = x.copy()
+        large[bad] = 1000.0 * np.sign(large[bad])  # group sums beyond fp16
+        large[bad, :gs] = 2000.0
+        want32, _ = oracle.affine_matmul(w, s, b, bits, gs, large, bf16=bf16)
+        fits = np.abs(want32[bad]) < 6e4  # (fp16 outputs end at 65504)
+        assert rel_err(lin(dev(large)).float().cpu().numpy()[bad][fits], want32[bad][fits]) < TOL
+    lin.ctx.poll()
+
+
+@pytest.mark.parametrize("bits,gs,units", [(8, 64, 44), (4, 64, 48), (4, 128, 48), (2, 128, 50)])
+def test_the_widest_inputs_of_the_warp_level_kernel(bits, gs, units):
+    """Eight column ranges of as many units as shared memory has ever taken: the activations leave room for a few warps only."""
+    rng = np.random.default_rng(bits * 100 + gs + 1)
+    n, k = 24, units * 8 * 256
+    w, s, b, sd, bd, bf16 = make_pack(rng, n, k, bits, gs, "f16")
+    lin = PackedLinear(dev(w), sd, bd, groupSize=gs, bits=bits)
+    assert lin.plan[0] > 0
+    for m in (1, 8, 9):
+        x = (rng.standard_normal((m, k)) * 2).astype(np.float16)
+        want32, _ = oracle.affine_matmul(w, s, b, bits, gs, x, bf16=bf16)
+        assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
+    lin.ctx.poll()

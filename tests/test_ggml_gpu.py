@@ -469,6 +469,86 @@ def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(type_id):
     here.ctx.poll()
 
 
+@pytest.mark.parametrize("type_id", TYPES)
+def test_an_infinite_activation_stays_in_its_row(type_id):
+    """The sums of x that the decoders need come from MMAs over several rows at once: an infinity or a NaN in one
+    activation row must not reach the others, whose products keep their bits."""
+    rng = np.random.default_rng(int(type_id) + 70)
+    n, k = 200, 1536
+    lin = PackedLinear(ggml=GGUFBlocks(dev(synth.ggml_blocks(rng, int(type_id), n, k)), type_id, (n, k)))
+    for m, bad in ((3, 1), (8, 6), (16, 11)):
+        x = dev(synth.activations(rng, m, k))
+        want = lin(x)
+        for value in (float("inf"), float("nan")):
+            worse = x.clone()
+            worse[bad, 777] = value
+            got = lin(worse)
+            others = [r for r in range(m) if r != bad]
+            assert torch.equal(got[others], want[others])
+            assert not torch.isfinite(got[bad]).any()
+    lin.ctx.poll()
+
+
+@pytest.mark.parametrize("type_id", [GGMLType.q4K, GGMLType.iq3S])
+def test_the_plan_of_a_single_row(type_id):
+    """The plan's upper bits hold the launch of one row; without them one row runs as two to eight do."""
+    rng = np.random.default_rng(int(type_id) + 71)
+    n, k = 1000, 4096
+    blocks = synth.ggml_blocks(rng, int(type_id), n, k)
+    lin = PackedLinear(ggml=GGUFBlocks(dev(blocks), type_id, (n, k)))
+    x = synth.activations(rng, 1, k)
+    want32, _ = oracle.ggml_matmul(int(type_id), blocks, x, n)
+    split, a, b, rest = lin.plan
+    ring, many = rest & 255, rest & 0x1fff00
+    for one in (0, 1 | 3 << 5 | 1 << 8, 12 | 0 << 5 | 2 << 8, 20 | 7 << 5 | 1 << 8):  # none; split 4, a warp, ring 2; split 1, 12, 3; split 8, 20, 2
+        lin.set_plan((split, a, b, ring | many | one << 21))
+        assert lin.plan[3] >> 21 == (one or (a * b) | (split - 1) << 5 | (ring - 1) << 8)
+        assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
+    with pytest.raises(IshizukiError):
+        lin.set_plan((split, a, b, ring | many | (25 | 1 << 8) << 21))  # more warps than a block holds
+    lin.ctx.poll()
+
+
+@pytest.mark.parametrize("type_id,units", [(GGMLType.q2K, 46), (GGMLType.q6K, 42), (GGMLType.iq4Xs, 42), (GGMLType.iq2Xs, 35)])
+def test_the_widest_inputs_of_the_warp_level_kernel(type_id, units):
+    """Eight column ranges of as many units as shared memory has ever taken: the activations leave room for a few warps only."""
+    rng = np.random.default_rng(int(type_id) + 72)
+    n, k = 24, units * 8 * 256
+    blocks = synth.ggml_blocks(rng, int(type_id), n, k)
+    lin = PackedLinear(ggml=GGUFBlocks(dev(blocks), type_id, (n, k)))
+    assert lin.plan[0] > 0
+    for m in (1, 8, 9):
+        x = synth.activations(rng, m, k)
+        want32, _ = oracle.ggml_matmul(int(type_id), blocks, x, n)
+        assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
+    lin.ctx.poll()
+
+
+def test_a_chain_of_early_launches_reads_what_the_one_before_wrote():
+    """gather, norm, projection and gather again without a wait between them, each starting while the one before ends and reading
+    or writing over its arrays: the same bits as with a wait after every call."""
+    from ishizuki_b200.interface import rmsNorm
+    rng = np.random.default_rng(73)
+    n, k, rows = 5000, 2048, 8
+    blocks = dev(synth.q4k_blocks(rng, n, k))
+    lin = PackedLinear(ggml=GGUFBlocks(blocks, GGMLType.q4K, (n, k)))
+    w = torch.ones(k, dtype=torch.float16, device="cuda")
+
+    def chain(steps, wait):
+        ids, out = torch.arange(rows, dtype=torch.int32, device="cuda"), []
+        for _ in range(steps):
+            for call in (lambda v: GGMLKernels.gather(v, blocks, GGMLType.q4K, k, dtype=torch.float32),
+                         lambda v: rmsNorm(v, w, 1e-6), lin, lambda v: v.argmax(1).to(torch.int32)):
+                ids = call(ids)
+                out.append(ids)
+                if wait:
+                    torch.cuda.synchronize()
+        return out
+
+    for a, b in zip(chain(20, False), chain(20, True)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("type_id", [GGMLType.q4K, GGMLType.q6K])
 def test_rotated_input_ahead_of_a_gguf_projection(type_id):
     """A GGUF projection with a rotation block: the input goes through the stand-alone rotation

@@ -30,6 +30,18 @@ def test_rms_norm_matches_the_oracle(rows, width, xdt, wdt):
     assert (got.view(np.uint16) != want.view(np.uint16)).mean() < 0.01
 
 
+@pytest.mark.parametrize("rows,width", [(2, 8), (1, 256), (2, 1023), (3, 1024), (2, 1025), (2, 1032), (1, 2048), (5, 7168), (2, 7176), (1, 8185), (600, 1280)])
+def test_rms_norm_at_the_edges_of_a_rows_thread_blocks(rows, width):
+    """A row is one to eight thread blocks of 1024 values that exchange their warps' sums."""
+    rng = np.random.default_rng(width)
+    x = (rng.standard_normal((rows, width)) * 3).astype(np.float32)
+    w = (1 + 0.1 * rng.standard_normal(width)).astype(np.float16)
+    got = rmsNorm(dev(x), dev(w), 1e-6).cpu().numpy()
+    want = oracle.rms_norm(x, w, 1e-6)
+    diff = np.abs(got.astype(np.float32) - want.astype(np.float32))
+    assert np.all(diff <= np.abs(want.astype(np.float32)) * 2.0 ** -10 + 1e-7)  # as above
+
+
 @pytest.mark.parametrize("rows,width,shift", [(3, 203, 0), (1, 7, 0), (2, 4099, 0), (2, 8191, 0), (2, 512, 1)])
 def test_rms_norm_value_by_value(rows, width, shift):
     """Widths that are no multiple of eight and rows off a 16-byte boundary."""

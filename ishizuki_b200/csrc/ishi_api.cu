@@ -468,7 +468,7 @@ int max_frag_clusters(ishi_ctx *ctx, const FragOps *ops, int s, int warps, int g
 int ring_for(int groups, int s, int w) { return groups == 2 || w > 16 || (w > 12 && s > 1) ? 2 : 3; }
 
 // The plan with K split s (= cluster size) and w warps per CTA, or false if it does not fit. ring:
-// tiles per warp, 0 for ring_for()'s, or less where that does not fit.
+// tiles per warp (two at least: one is read while the next is filled), 0 for ring_for()'s, or less where that does not fit.
 bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int w, int ring, FragPlan *out) {
   const FragOps *ops = frag_ops_for(d);
   if (!ops) return false;
@@ -480,7 +480,7 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
   c.P = (int)((d.n + kFragRows - 1) / kFragRows);
   c.S = s, c.W = w, c.NB = groups;
   c.tile_bytes = ops->tile_bytes;
-  if (s < 1 || s > kFragMaxSplit || s > c.units || w < 1 || w > (groups == 2 ? ops->many_warps : kFragMaxWarps)) return false;
+  if (ring == 1 || s < 1 || s > kFragMaxSplit || s > c.units || w < 1 || w > (groups == 2 ? ops->many_warps : kFragMaxWarps)) return false;
   // the kernel divides by multiplication, exact while (clusters + 1) * P < 2^32 / clusters
   if ((long long)c.P * (ctx->sm_count + 1) * ctx->sm_count >= (1ll << 32)) return false;
   c.umax = (c.units + s - 1) / s;
@@ -1209,7 +1209,8 @@ ishi_status ishi_projection_plan(const ishi_projection *p, int plan[4]) {
   const FragPlan &f = p->frag.few, &m = p->frag.many, &o = p->frag.one;
   if (f.ok) {
     plan[0] = f.S, plan[1] = f.lane_warps, plan[2] = f.W / f.lane_warps;
-    plan[3] = f.ring | (m.ok ? m.ring << 8 | m.S << 12 | m.W << 16 : 0) | o.W << 21 | (o.S - 1) << 26 | (o.ring - 1) << 29;
+    plan[3] = (int)((unsigned)f.ring | (m.ok ? (unsigned)(m.ring << 8 | m.S << 12 | m.W << 16) : 0u) |
+                    (unsigned)(o.W | (o.S - 1) << 5 | (o.ring - 1) << 8) << 21);
   }
   return ISHI_OK;
 }
@@ -1219,7 +1220,8 @@ ishi_status ishi_projection_set_plan(ishi_projection *p, const int plan[4]) {
   ishi_ctx *ctx = p->ctx;
   if (!p->frag.few.ok) return fail(ctx, ISHI_E_UNSUPPORTED, "this projection's kernel has one launch plan only");
   std::lock_guard<std::mutex> g(ctx->lock);
-  const int many = (plan[3] >> 8) & 0x1fff, one = plan[3] >> 21;  // (0: the launch of two to eight rows' plan)
+  const int many = (plan[3] >> 8) & 0x1fff;
+  const int one = (int)((unsigned)plan[3] >> 21);  // (0: the launch of two to eight rows' plan)
   FragPlans both;
   bool fine = plan[1] > 0 && plan[2] > 0 && plan[1] <= kFragMaxWarps && plan[2] <= kFragMaxWarps &&
               frag_plan(ctx, p->d, 1, plan[0], plan[1] * plan[2], plan[3] & 255, &both.few);

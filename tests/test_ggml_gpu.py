@@ -504,8 +504,13 @@ def test_the_plan_of_a_single_row(type_id):
         lin.set_plan((split, a, b, ring | many | one << 21))
         assert lin.plan[3] >> 21 == (one or (a * b) | (split - 1) << 5 | (ring - 1) << 8)
         assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
-    with pytest.raises(IshizukiError):
-        lin.set_plan((split, a, b, ring | many | (25 | 1 << 8) << 21))  # more warps than a block holds
+    top = ring | many | (4 | 6 << 8) << 21  # a ring of seven tiles has the top bit
+    lin.set_plan((split, a, b, top - (1 << 32)))
+    assert lin.plan[3] == top - (1 << 32)
+    assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
+    for word in (ring | many | (25 | 1 << 8) << 21, ring | many | 4 << 21, 1 | many):  # more warps than a block holds; rings of one tile
+        with pytest.raises(IshizukiError):
+            lin.set_plan((split, a, b, word))
     lin.ctx.poll()
 
 

@@ -112,7 +112,7 @@ ishi_status ishi_ctx_set_route(ishi_ctx *ctx, int route, int crossover_rows);
 /* PackedLinear.init + VerifyMatmul.warm (Hadamard.swift:51-86, VerifyMatmul.swift:40-61):
  * validates the weight, allocates the projection's own memory, copies the weight into it in tiled
  * order and fixes the launch plan for its shape: for the warp-level kernel's formats by timing the
- * best ten candidate plans on the tiled weight (1 to 5 ms for the first projection of a shape, later
+ * best eight candidate plans on the tiled weight (1 to 6 ms for the first projection of a shape, later
  * ones of the context take over its plan; ISHI_NO_AUTOTUNE=1 in the environment keeps the estimate's choice). Synchronises the device. */
 ishi_status ishi_projection_create(ishi_ctx *ctx, const ishi_weight_desc *desc,
                                    ishi_projection **out);
@@ -148,10 +148,12 @@ int64_t ishi_projection_weight_bytes(const ishi_projection *p);
 int ishi_projection_crossover_rows(const ishi_projection *p);
 /* The launch plan create settled on, for the warp-level kernel's formats: {K split = cluster size,
  * a, b: a * b warps per CTA, tiles per warp ring | the launch of 9...16 rows << 8 | that of one row << 21} (zeros
- * for the other kernels; without the last part one row runs as two to eight do), and a way to impose one: the order in which partial sums are added follows the
+ * for the other kernels), and a way to impose one. The order in which partial sums are added follows the
  * plan, so two projections of the same weight agree bit for bit only under the same plan (the tiled
- * copy does not depend on it). set_plan accepts what ishi_projection_plan of a projection of the
- * same shape returned. */
+ * copy does not depend on it). create runs one row as it runs two to eight: a row's product has the
+ * same bits in all calls of up to eight rows. An imposed plan may give one row a launch of its own
+ * (without that part it runs as two to eight do), whose products can then differ in the last bit.
+ * set_plan accepts what ishi_projection_plan of a projection of the same shape returned. */
 ishi_status ishi_projection_plan(const ishi_projection *p, int plan[4]);
 ishi_status ishi_projection_set_plan(ishi_projection *p, const int plan[4]);
 

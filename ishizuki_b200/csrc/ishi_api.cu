@@ -76,11 +76,12 @@ struct FragPlan {
   int lane_warps = 1;  // W as ishi_projection_plan reports it: lane_warps * (W / lane_warps)
   uint32_t xregion = 0;
   size_t smem = 0, tiles_bytes = 0;
-  double cost = 0, staging = 0;  // the estimate in microseconds; of it, the activations of all rows
+  double cost = 0;  // the estimate in microseconds
 };
-// one for two to eight rows, one for nine to sixteen (not ok: such a call runs as two launches of the first), one
-// for a single row: without eight rows to stage and read, fewer column ranges are the faster ones (4096 x 4096, affine 4-bit, one row:
-// split 4 / 16 warps 5.25 us, unsplit / 12 warps 4.63; at eight rows 5.3 and 5.7)
+// one for up to eight rows, one for nine to sixteen (not ok: such a call runs as two launches of the first). A single row
+// has the first one's as well, unless set_plan gives it another: a row's product then has the same bits in a call of one row and of eight,
+// which plain decoding and the verify step of a draft rely on. (Fewer column ranges would be faster for it: 4096 x 4096, affine 4-bit, one row:
+// split 4 / 16 warps 5.25 us, unsplit / 12 warps 4.63; at eight rows 5.3 and 5.7. But the split orders the partial sums.)
 struct FragPlans {
   FragPlan few, many, one;
 };
@@ -507,8 +508,7 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
       // Estimate in microseconds: the warps' runs of tiles, a tile every 0.075 us of an SM that is
       // full of warps or one per 0.9 us and warp in one that is not; staging; the hand-over in a cluster.
       const double run = (double)((panels * c.umax + w - 1) / w);
-      c.staging = 0.05 * c.umax * groups;
-      c.cost = run * std::max(0.9, 0.075 * w) * (groups == 2 ? 1.3 : 1.0) + c.staging + (s > 1 ? 0.5 + 0.05 * s : 0.0);
+      c.cost = run * std::max(0.9, 0.075 * w) * (groups == 2 ? 1.3 : 1.0) + 0.05 * c.umax * groups + (s > 1 ? 0.5 + 0.05 * s : 0.0);
       c.tiles_bytes = (size_t)c.P * c.units * c.tile_bytes;
       c.ok = true;
       *out = c;
@@ -983,30 +983,28 @@ ishi_status ishi_verify_matmul(ishi_ctx *ctx, const void *x, int rows, const voi
 
 // ---- projection: the PackedLinear counterpart ---------------------------------------------------
 
-// The tile layout does not depend on the launch plan, so the plans of the three launches (two to eight rows, nine to
-// sixteen, one) can be chosen by measurement: the planner's best candidates run a few times on the
-// projection's own tiles (activations of zeros) and the fastest stays.
+// The tile layout does not depend on the launch plan, so the plans of both launches (up to eight rows, and nine to
+// sixteen) can be chosen by measurement: the planner's best candidates run a few times on the
+// projection's own tiles (activations of zeros, eight or sixteen rows) and the fastest stays.
 // What the measurement costs counts, since the first projection of every shape pays for it: one pair of buffers
-// for all launches, one wait per pass, and no more candidates and launches than the choice needs (create
-// for 17408 x 5120, Q4_K 4.3 ms, Q6_K 5.4, 4096 x 4096 affine 4-bit 2.8; ten, eight and eight candidates, four finalists and up to sixteen
-// launches of each 5.7, 7.5 and 3.5). Over sixteen (format, shape) pairs, eight times each, against all 72 plans of one to
-// eight ranges, 12 to 24 warps, rings of two to four, timed on weights from HBM: the choice is the best one or within 3 % of it in
-// 47 of 48, at most 10 % behind (Q4_K 5120 x 17408, one row, two of eight times). One launch per
+// for both launches, one wait per pass, and no more candidates and launches than the choice needs. The first create of a
+// shape, tiling included, in ms: 17408 x 5120 Q4_K 2.9, Q6_K 5.9, IQ2_XS 3.8, 11003 x 3840 IQ3_S 4.7, 1024 x 5120 Q4_K 1.4 (with a third
+// measured launch, of one row, 3.7, 7.1, 4.4, 6.1 and 1.8). Over sixteen (format, shape) pairs, eight times each, against all 72 plans of one to
+// eight ranges, 12 to 24 warps, rings of two to four, timed on weights from HBM: the choice is the best one or within 3 % of it. One launch per
 // candidate in the first pass is up to 30 % behind. Copies of the tiles that exceed L2, so that the weight comes from HBM as in use,
 // chose no better and cost 1 ms.
 static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragPlan> *few, std::vector<FragPlan> *many) {
-  constexpr int kRows[3] = {8, 16, 1};
-  constexpr size_t kTuned[3] = {8, 7, 6}, kFinalists = 3;
-  constexpr int kLaunches = 3, kFinalLaunches[3] = {12, 8, 8};
+  constexpr size_t kTuned[2] = {8, 7}, kFinalists = 3;
+  constexpr int kLaunches = 3, kFinalLaunches[2] = {12, 8};
   constexpr float kBehind = 1.15f;  // a candidate this far behind in the first pass is no finalist
   typedef std::pair<float, const FragPlan *> Timed;
   const size_t x_bytes = (size_t)16 * p->d.k * sizeof(__half), y_bytes = (size_t)16 * p->d.n * sizeof(__half);
   uint8_t *buffer = nullptr;  // x, then y
   cudaEvent_t marks[2 * kTuned[0]] = {nullptr};
-  for (int kind = 0; kind < 3; ++kind) {
-    const int rows = kRows[kind];
-    std::vector<FragPlan> *candidates = rows == 16 ? many : few;
-    FragPlan *plan = rows == 16 ? &p->frag.many : rows == 1 ? &p->frag.one : &p->frag.few;
+  for (int groups = 1; groups <= 2; ++groups) {
+    const int rows = 8 * groups;
+    std::vector<FragPlan> *candidates = groups == 2 ? many : few;
+    FragPlan *plan = groups == 2 ? &p->frag.many : &p->frag.few;
     if (candidates->size() < 2) continue;
     // a shape measured before on this context keeps its plan (all layers of a model then agree)
     const auto key = std::make_tuple((const void *)plan->ops, (long long)p->d.n, (long long)p->d.k, rows);
@@ -1030,7 +1028,7 @@ static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragP
     auto time_plans = [&](std::vector<Timed> *plans, int launches) {
       auto launch = [&](const FragPlan &c) {
         FragPlans both;
-        both.few = both.many = both.one = c;
+        both.few = both.many = c;
         return run_frag(ctx, both, p->ws, p->d, buffer, rows, buffer + x_bytes, p->d.n, 0, false, true, false, 0) == ISHI_OK;
       };
       for (size_t i = 0; ok && i < plans->size(); ++i) {
@@ -1050,13 +1048,13 @@ static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragP
     // a first pass over all candidates, then the best few again with more launches (the first pass
     // alone picks among near-equal plans by noise)
     std::vector<Timed> timed, finals;
-    for (const FragPlan &c : *candidates) timed.push_back({(float)(c.cost - (rows == 1 ? c.staging : 0.0)), &c});
+    for (const FragPlan &c : *candidates) timed.push_back({(float)c.cost, &c});
     std::sort(timed.begin(), timed.end(), [](const Timed &a, const Timed &b) { return a.first < b.first; });
-    if (timed.size() > kTuned[kind]) timed.resize(kTuned[kind]);
+    if (timed.size() > kTuned[groups - 1]) timed.resize(kTuned[groups - 1]);
     if (ok) time_plans(&timed, kLaunches);
     for (const Timed &t : timed)
       if (ok && finals.size() < kFinalists && t.first <= timed[0].first * kBehind) finals.push_back(t);
-    if (ok) time_plans(&finals, kFinalLaunches[kind]);
+    if (ok) time_plans(&finals, kFinalLaunches[groups - 1]);
     if (!ok) {
       cudaGetLastError();  // keep the estimate's choice
       continue;
@@ -1073,7 +1071,7 @@ static void tune_frag_plans(ishi_ctx *ctx, ishi_projection *p, std::vector<FragP
     *plan = *best;
     ctx->tuned[key] = {best->S, best->W, best->ring};
     if (getenv("ISHI_DEBUG_PLAN")) {
-      fprintf(stderr, "ishi plan n=%lld k=%lld rows %d measured: split %d, %d clusters, %d warps, ring %d: %.2f us;", (long long)p->d.n,
+      fprintf(stderr, "ishi plan n=%lld k=%lld rows<=%d measured: split %d, %d clusters, %d warps, ring %d: %.2f us;", (long long)p->d.n,
               (long long)p->d.k, rows, best->S, best->NC, best->W, best->ring, finals[0].first * 1e3f);
       for (const auto &c : timed) fprintf(stderr, " %d/%d/%d:%.1f", c.second->S, c.second->W, c.second->ring, c.first * 1e3f);
       fprintf(stderr, "\n");
@@ -1123,11 +1121,11 @@ static ishi_status create_projection(ishi_ctx *ctx, const ishi_weight_desc *desc
   // again afterwards.
   std::vector<FragPlan> few, many;
   if (make_frag_plan(ctx, p->d, 1, &p->frag.few, &few)) {
-    p->frag.one = p->frag.few;
     make_frag_plan(ctx, p->d, 2, &p->frag.many, &many);
     s = ensure_workspace(ctx, &p->ws, 0, 0, p->frag.few.tiles_bytes, 0);
     if (s == ISHI_OK) s = tile_weight_frag(ctx, p->frag.few, descs, count, n_total, p->ws.tiles, 0, gated);
     if (s == ISHI_OK && !getenv("ISHI_NO_AUTOTUNE") && !getenv("ISHI_FRAG_PLAN")) tune_frag_plans(ctx, p, &few, &many);
+    p->frag.one = p->frag.few;
   } else if (count > 1) {
     delete p;
     return fail(ctx, ISHI_E_UNSUPPORTED, "only the warp-level kernel's formats can be stacked into one projection");
@@ -1221,7 +1219,7 @@ ishi_status ishi_projection_set_plan(ishi_projection *p, const int plan[4]) {
   if (!p->frag.few.ok) return fail(ctx, ISHI_E_UNSUPPORTED, "this projection's kernel has one launch plan only");
   std::lock_guard<std::mutex> g(ctx->lock);
   const int many = (plan[3] >> 8) & 0x1fff;
-  const int one = (int)((unsigned)plan[3] >> 21);  // (0: the launch of two to eight rows' plan)
+  const int one = (int)((unsigned)plan[3] >> 21);  // (0: as two to eight rows)
   FragPlans both;
   bool fine = plan[1] > 0 && plan[2] > 0 && plan[1] <= kFragMaxWarps && plan[2] <= kFragMaxWarps &&
               frag_plan(ctx, p->d, 1, plan[0], plan[1] * plan[2], plan[3] & 255, &both.few);

@@ -341,7 +341,7 @@ class PackedLinear:
     @property
     def plan(self) -> tuple[int, int, int, int]:
         """The launch plan create settled on (K split, two factors of the warps per CTA, ring and the
-        launch of 9...16 rows); zeros for a format outside the warp-level kernel."""
+        launches of 9...16 rows and of one); zeros for a format outside the warp-level kernel."""
         out = (ctypes.c_int * 4)()
         self.ctx.check(self.ctx.lib.ishi_projection_plan(self.handle, out), declined=())
         return tuple(int(v) for v in out)

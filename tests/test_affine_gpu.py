@@ -202,6 +202,22 @@ def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(bits, gs, dtype):
     here.ctx.poll()
 
 
+@pytest.mark.parametrize("bits,gs,dtype,block", [(2, 128, "f16", 0), (2, 128, "bf16", 128), (2, 128, "bf16", 32)])
+@pytest.mark.parametrize("n,k", [(4096, 4096), (1024, 5120), (1000, 1536)])
+def test_a_rows_product_does_not_depend_on_the_rows_beside_it(bits, gs, dtype, block, n, k):
+    """A row has the same product bit for bit alone and in calls of two to eight rows, rotated on the way or not."""
+    rng = np.random.default_rng(bits * 1000 + gs + block)
+    w, s, b, sd, bd, bf16 = make_pack(rng, n, k, bits, gs, dtype)
+    lin = PackedLinear(dev(w), sd, bd, None, block, groupSize=gs, bits=bits)
+    x = dev(synth.activations(rng, 8, k))
+    want = lin(x)
+    for row in range(8):
+        assert torch.equal(lin(x[row:row + 1]), want[row:row + 1]), row
+    for m in range(2, 8):
+        assert torch.equal(lin(x[:m]), want[:m]), m
+    lin.ctx.poll()
+
+
 @pytest.mark.parametrize("bits,gs", [(8, 32), (8, 64), (4, 32), (4, 64), (4, 128), (2, 64), (2, 128)])
 def test_an_infinite_activation_stays_in_its_row(bits, gs):
     """The group sums of x come from MMAs over several rows at once, the bias term from their pieces in tf32: an infinity or

@@ -469,6 +469,22 @@ def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(type_id):
     here.ctx.poll()
 
 
+@pytest.mark.parametrize("type_id", [t for t in TYPES if t not in (GGMLType.q2K, GGMLType.q4K, GGMLType.q6K)])
+@pytest.mark.parametrize("n,k", [(4096, 4096), (1024, 5120), (1000, 1536)])
+def test_a_rows_product_does_not_depend_on_the_rows_beside_it(type_id, n, k):
+    """A row has the same product bit for bit alone and in calls of two to eight rows, under the measured plan:
+    the verify step of a draft and plain decoding agree on every token, near-ties included."""
+    rng = np.random.default_rng(int(type_id) + 910)
+    lin = PackedLinear(ggml=GGUFBlocks(dev(synth.ggml_blocks(rng, int(type_id), n, k)), type_id, (n, k)))
+    x = dev(synth.activations(rng, 8, k))
+    want = lin(x)
+    for row in range(8):
+        assert torch.equal(lin(x[row:row + 1]), want[row:row + 1]), row
+    for m in range(2, 8):
+        assert torch.equal(lin(x[:m]), want[:m]), m
+    lin.ctx.poll()
+
+
 @pytest.mark.parametrize("type_id", TYPES)
 def test_an_infinite_activation_stays_in_its_row(type_id):
     """The sums of x that the decoders need come from MMAs over several rows at once: an infinity or a NaN in one

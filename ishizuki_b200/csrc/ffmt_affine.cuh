@@ -163,6 +163,19 @@ struct FragAffine {
     }
   }
 
+  // The sums of activation row g's groups from those of its inputs 64 t ... + 31 (s0) and + 32 ... + 63 (s1), if the row is `mine`
+  static __device__ __forceinline__ void store_sums(uint32_t base, int lane, float s0, float s1, bool mine) {
+    const int g = lane >> 2, t = lane & 3;
+    if (GS == 128) s0 += s1, s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+    if (!mine) return;
+    if (GS == 32) {
+      store_sum(base, g, 2 * t, s0), store_sum(base, g, 2 * t + 1, s1);
+    } else {
+      if (GS == 64) s0 += s1;
+      if (GS == 64 || !(t & 1)) store_sum(base, g, GS == 64 ? t : t >> 1, s0);
+    }
+  }
+
   // After the copies: a warp task per unit and four rows. The sums by MMAs with a weight of ones, as in ffmt_q4k.cuh: lane (g, t) gets those of
   // inputs 64 t ... + 31 and + 32 ... + 63 of activation row g.
   static __device__ __forceinline__ void row_sums(const FragArgs &a, uint32_t xfrag, int rows, int uc) {
@@ -187,15 +200,7 @@ struct FragAffine {
         mma16816(c, kOnes, kOnes, kOnes, kOnes, v[e].z, v[e].w);
         if (g == r0 + e) s0 = c[0], s1 = c[1];
       }
-      if (GS == 128) s0 += s1, s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-      if ((g & 4) != r0) continue;
-      const uint32_t base = sums_of(a, x, u);
-      if (GS == 32) {
-        store_sum(base, g, 2 * t, s0), store_sum(base, g, 2 * t + 1, s1);
-      } else {
-        if (GS == 64) s0 += s1;
-        if (GS == 64 || !(t & 1)) store_sum(base, g, GS == 64 ? t : t >> 1, s0);
-      }
+      store_sums(sums_of(a, x, u), lane, s0, s1, (g & 4) == r0);
     }
   }
 
@@ -218,6 +223,14 @@ struct FragAffine {
                             a.rot_signs ? a.rot_signs + (long long)(ub0 + u) * 256 + lane * 8 : nullptr, lane);
       sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, kRows && m.staged != 1 ? v : arranged(v, lane));
       if (kRows && m.staged != 1) return;
+      if (kRows) {  // as row_sums() has them: a row's product has the same bits alone and beside others
+        constexpr uint32_t kOnes = 0x3c003c00u;
+        float c[4];
+        mma16816_first(c, kOnes, kOnes, kOnes, kOnes, v.x, v.y);
+        mma16816(c, kOnes, kOnes, kOnes, kOnes, v.z, v.w);
+        store_sums(sums_of(a, xfrag, u), lane, c[0], c[1], (lane >> 2) == r);
+        return;
+      }
       const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
       const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
       const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));

@@ -105,6 +105,15 @@ struct FragQ4K {
 
   static __device__ __forceinline__ uint32_t row_stride(const FragArgs &a) { return (uint32_t)a.umax * 512u + 64u; }
 
+  // The sums of sub-blocks 2t and 2t + 1 of activation row g as fp16 hi + lo: the B fragment of the minimum-term MMA, whose k
+  // index runs over sub-blocks
+  static __device__ __forceinline__ void store_sums(uint32_t base, int lane, float s0, float s1) {
+    const __half h0 = __float2half_rn(s0), h1 = __float2half_rn(s1);
+    const __half l0 = __float2half_rn(s0 - __half2float(h0)), l1 = __float2half_rn(s1 - __half2float(h1));
+    sts64(base + (uint32_t)lane * 8u, (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
+          (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16));
+  }
+
   // Sub-block sums of x for the minimum term, a warp task per unit and four rows. The sixteen bytes of lane l are part of
   // sub-block l / 4: as B registers (column l / 4, any k) two MMAs with a weight of ones give the row's eight
   // sums, the same in every row of C, and lane (g, t) keeps sub-blocks 2t and 2t + 1 of activation row g. (One accumulator per row, not
@@ -128,42 +137,26 @@ struct FragQ4K {
         if (g == r0 + e) s0 = c[0], s1 = c[1];
       }
       if ((g & 4) != r0) continue;
-      // as fp16 hi + lo: the B fragment of the minimum-term MMA, whose k index runs over sub-blocks
-      const __half h0 = __float2half_rn(s0), h1 = __float2half_rn(s1);
-      const __half l0 = __float2half_rn(s0 - __half2float(h0)), l1 = __float2half_rn(s1 - __half2float(h1));
       const uint32_t base = x + 8u * R + (uint32_t)u * kSumBytes;
-      sts64(base + (uint32_t)lane * 8u, (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
-            (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16));
+      store_sums(base, lane, s0, s1);
       if (g == 0)  // fp32 sums of activation row 0 (the single-row kernel's minimum term)
         sts64(base + 256u + (uint32_t)lane * 8u, __float_as_uint(s0), __float_as_uint(s1));
     }
   }
 
-  // The same for a single activation row, stored and added up on its way from x: a warp task is (unit, row).
+  // The same for a single activation row, stored and added up on its way from x: a warp task is (unit, row). The same MMAs: a row has
+  // the same sums, and so the same product bit for bit, alone and beside others.
   template <class Then>
   static __device__ __forceinline__ void stage_x(const FragArgs &a, const FragRows &m, uint32_t xfrag, int ub0, int uc, Then then) {
     const int lane = threadIdx.x & 31;
     const uint32_t R = row_stride(a), sums = xfrag + 8u * R;
-    const int jj = lane >> 3;
+    constexpr uint32_t kOnes = 0x3c003c00u;
     frag_stage_rows(a, m, ub0, uc, then, [&](int u, int r, uint4 v) {
       sts128u(xfrag + (uint32_t)r * R + (uint32_t)u * 512u + (uint32_t)lane * 16u, v);
-      const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-      const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-      const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
-      const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
-      float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      const float o = __shfl_xor_sync(0xffffffffu, s, 4);
-      const uint32_t base = sums + (uint32_t)u * kSumBytes;
-      if ((lane & 7) == 0) {
-        // sub-blocks 2t' and 2t' + 1 (t' = lane / 8) of activation row r, as fp16 hi + lo: the B
-        // fragment of the minimum-term MMA, whose k index runs over sub-blocks
-        const __half h0 = __float2half_rn(s), h1 = __float2half_rn(o);
-        const __half l0 = __float2half_rn(s - __half2float(h0)), l1 = __float2half_rn(o - __half2float(h1));
-        sts64(base + (uint32_t)(r * 4 + jj) * 8u, (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
-              (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16));
-      }
+      float c[4];
+      mma16816_first(c, kOnes, kOnes, kOnes, kOnes, v.x, v.y);
+      mma16816(c, kOnes, kOnes, kOnes, kOnes, v.z, v.w);
+      if ((lane >> 2) == r) store_sums(sums + (uint32_t)u * kSumBytes, lane, c[0], c[1]);
     });
   }
 

@@ -481,25 +481,19 @@ __device__ __forceinline__ void frag_rows_by_16(uint32_t xfrag, uint32_t R, uint
     if ((g & 4) == r0) frag_store_sums16(sums + (uint32_t)u * sum_bytes, lane, s);
   }
 }
-// The same for rows that are stored and added up on their way from x: lane l's values v of the unit whose row begins at `row`.
+// The same for rows that are stored and added up on their way from x: lane l's values v of the unit whose row begins at `row`. By the
+// same MMAs: a row has the same sums, and so the same product bit for bit, in calls of one to sixteen rows.
 template <bool SCALED>
 __device__ __forceinline__ void frag_put_by_16(uint32_t row, uint32_t sums, int r, uint4 v, uint32_t factor) {
   const int lane = threadIdx.x & 31;
   const uint32_t to = row + frag_pair_slot(lane);
   sts64(to, SCALED ? frag_times(v.x, factor) : v.x, SCALED ? frag_times(v.y, factor) : v.y);
   sts64(to + 16u, SCALED ? frag_times(v.z, factor) : v.z, SCALED ? frag_times(v.w, factor) : v.w);
-  const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-  const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-  const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&v.z));
-  const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
-  float s = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-  s += __shfl_xor_sync(0xffffffffu, s, 1);  // the group's sixteen values
-  if ((lane & 1) == 0) {
-    const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-    const uint32_t at = sums + (uint32_t)((r * 4 + (lane >> 3)) * 16 + (lane & 6));
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(hi)) : "memory");
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + 8u), "h"(__half_as_ushort(lo)) : "memory");
-  }
+  const uint32_t first = lane & 2 ? 0u : 0x3c003c00u, second = lane & 2 ? 0x3c003c00u : 0u;
+  float c[4];
+  mma16816_first(c, first, second, first, second, v.x, v.y);
+  mma16816(c, first, second, first, second, v.z, v.w);
+  if ((lane >> 2) == r) frag_store_sums16(sums, lane, {c[0], c[2], c[1], c[3]});
 }
 
 // A decoder's shared-memory tables (kExtraBytes, a multiple of 16), laid out once per device from

@@ -202,7 +202,9 @@ def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(bits, gs, dtype):
     here.ctx.poll()
 
 
-@pytest.mark.parametrize("bits,gs,dtype,block", [(2, 128, "f16", 0), (2, 128, "bf16", 128), (2, 128, "bf16", 32)])
+@pytest.mark.parametrize("bits,gs,dtype,block", [(8, 32, "f16", 0), (8, 64, "bf16", 64), (8, 128, "f16", 0), (4, 32, "bf16", 0), (4, 64, "f16", 0),
+                                                 (4, 64, "f16", 256), (4, 128, "bf16", 0), (2, 64, "f16", 0), (2, 64, "f16", 128), (2, 128, "f16", 0),
+                                                 (2, 128, "bf16", 128), (2, 128, "bf16", 32)])
 @pytest.mark.parametrize("n,k", [(4096, 4096), (1024, 5120), (1000, 1536)])
 def test_a_rows_product_does_not_depend_on_the_rows_beside_it(bits, gs, dtype, block, n, k):
     """A row has the same product bit for bit alone and in calls of two to eight rows, rotated on the way or not."""

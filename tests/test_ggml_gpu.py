@@ -469,7 +469,7 @@ def test_a_rows_product_does_not_depend_on_its_half_of_a_panel(type_id):
     here.ctx.poll()
 
 
-@pytest.mark.parametrize("type_id", [t for t in TYPES if t not in (GGMLType.q2K, GGMLType.q4K, GGMLType.q6K)])
+@pytest.mark.parametrize("type_id", TYPES)
 @pytest.mark.parametrize("n,k", [(4096, 4096), (1024, 5120), (1000, 1536)])
 def test_a_rows_product_does_not_depend_on_the_rows_beside_it(type_id, n, k):
     """A row has the same product bit for bit alone and in calls of two to eight rows, under the measured plan:

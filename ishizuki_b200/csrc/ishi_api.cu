@@ -528,7 +528,8 @@ bool make_frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, FragPl
   const int units = (int)(d.k / 256);
   if (fs > 0 && fper > 0 && fpp > 0) {
     const int lane = ((units + fs - 1) / fs + fper - 1) / fper;
-    if (!frag_plan(ctx, d, groups, fs, lane * fpp, fring, &best)) return false;
+    // (no deeper a ring than ishi_projection_plan can report)
+    if (!frag_plan(ctx, d, groups, fs, lane * fpp, std::min(fring, groups == 2 ? 15 : 255), &best)) return false;
     best.lane_warps = lane;
     *pl = best;
     return true;
@@ -1207,8 +1208,9 @@ ishi_status ishi_projection_plan(const ishi_projection *p, int plan[4]) {
   const FragPlan &f = p->frag.few, &m = p->frag.many, &o = p->frag.one;
   if (f.ok) {
     plan[0] = f.S, plan[1] = f.lane_warps, plan[2] = f.W / f.lane_warps;
-    plan[3] = (int)((unsigned)f.ring | (m.ok ? (unsigned)(m.ring << 8 | m.S << 12 | m.W << 16) : 0u) |
-                    (unsigned)(o.W | (o.S - 1) << 5 | (o.ring - 1) << 8) << 21);
+    // (three bits for the ring of one row: a deeper one can only be the ring of two to eight rows, which is what no part means)
+    const unsigned one = o.ring <= 8 ? (unsigned)(o.W | (o.S - 1) << 5 | (o.ring - 1) << 8) : 0u;
+    plan[3] = (int)((unsigned)f.ring | (m.ok ? (unsigned)(m.ring << 8 | m.S << 12 | m.W << 16) : 0u) | one << 21);
   }
   return ISHI_OK;
 }

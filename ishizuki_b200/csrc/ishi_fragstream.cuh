@@ -65,8 +65,6 @@ constexpr int kFragRows = 16;
 // Q4_K, ternary and the other affine 4-bit 1 to 2 % less, Q6_K 24.2 / 29.6 -> 23.8 / 28.4; Q2_K 21.2 / 24.3
 // -> 21.6 / 26.0, affine 2-bit 19.4 / 21.7 -> 19.5 / 22.4, IQ2_S the same: these stay at 20.
 constexpr int kFragMaxWarps = ISHI_FRAG_MAX_WARPS;
-constexpr int kFragMaxRing = 4;   // most tiles per warp-private ring (FragArgs::ring of them are used:
-                                  // one is decoded while the others are in flight)
 constexpr int kFragMaxSplit = 8;  // portable cluster size
 constexpr int kFragMaxPeers = 8;  // GPUs of one NVSwitch box
 
@@ -78,7 +76,7 @@ struct FragArgs {
   int out_transposed;
   int M, N, K;
   int units, S, P, NC;  // NC clusters of S CTAs
-  int ring;             // tiles per warp-private ring, 2 ... kFragMaxRing
+  int ring;             // tiles per warp-private ring, two or more: one is decoded while the others are in flight
   int ahead;            // of them, tiles asked for before the dependency wait, 1 ... ring - 1
   int led;              // most panels a CTA leads (S > 1)
   // ceil(2^32 / d) for d = S, NC, warps, umax, umax - 1, or 0 for d = 1: see frag_div()

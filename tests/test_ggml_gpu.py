@@ -530,6 +530,35 @@ def test_the_plan_of_a_single_row(type_id):
     lin.ctx.poll()
 
 
+def test_a_reported_plan_is_accepted_whatever_its_ring(monkeypatch):
+    """The ring of one row has three bits in the plan's last word: a deeper one that it shares with up to eight rows comes back with them."""
+    rng = np.random.default_rng(75)
+    n, k = 64, 4096
+    blocks = synth.q4k_blocks(rng, n, k)
+    x = synth.activations(rng, 8, k)
+    want32, _ = oracle.ggml_matmul(int(GGMLType.q4K), blocks, x, n)
+
+    def check(lin, ring):
+        plan = lin.plan
+        assert plan[3] & 255 == ring
+        before = lin(dev(x))
+        lin.set_plan(plan)
+        assert lin.plan == plan
+        assert torch.equal(lin(dev(x)), before)
+        assert rel_err(before.cpu().numpy(), want32) < TOL
+        assert torch.equal(lin(dev(x[:1])), before[:1])
+
+    lin = PackedLinear(ggml=GGUFBlocks(dev(blocks), GGMLType.q4K, (n, k)))
+    for ring in (2, 7, 8, 9, 16, 17):
+        lin.set_plan((1, 1, 2, ring))
+        check(lin, ring)
+    monkeypatch.setenv("ISHI_FRAG_PLAN", "2,8,2,18")  # deeper than the four bits of nine to sixteen rows
+    lin = PackedLinear(ggml=GGUFBlocks(dev(blocks), GGMLType.q4K, (n, k)))
+    check(lin, 18)
+    assert (lin.plan[3] >> 8) & 0x1fff == 15 | 2 << 4 | 2 << 8
+    lin.ctx.poll()
+
+
 @pytest.mark.parametrize("type_id,units", [(GGMLType.q2K, 46), (GGMLType.q6K, 42), (GGMLType.iq4Xs, 42), (GGMLType.iq2Xs, 35)])
 def test_the_widest_inputs_of_the_warp_level_kernel(type_id, units):
     """Eight column ranges of as many units as shared memory has ever taken: the activations leave room for a few warps only."""

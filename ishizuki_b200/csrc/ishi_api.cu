@@ -487,6 +487,7 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
   c.umax = (c.units + s - 1) / s;
   c.xregion = (uint32_t)(c.umax * ops->x_bytes + ops->x_fixed);
   c.NC = std::min(ctx->sm_count / s, c.P);
+  const int stride = frag_ring_stride(c.tile_bytes), least = (groups * 1024 + stride - 1) / stride;  // a drained ring holds a partial tile
   // shared memory depends on the clusters (fewer of them lead more panels each), which depend on it
   for (int tries = 0; tries < 3; ++tries) {
     const int panels = (c.P + c.NC - 1) / c.NC;
@@ -494,8 +495,7 @@ bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int 
     if ((long long)panels * c.umax * std::max(kFragMaxWarps * kFragMaxWarps, c.umax) >= (1ll << 32)) return false;
     c.led = s > 1 ? (panels + s - 1) / s : 0;
     bool fits = false;
-    for (int r = ring ? ring : ring_for(groups, s, w); r >= (ring ? ring : 2) && !fits; --r) {
-      if (r * frag_ring_stride(c.tile_bytes) < groups * 1024) break;  // a drained ring holds a partial tile
+    for (int r = ring ? ring : std::max(ring_for(groups, s, w), least); r >= std::max(ring ? ring : 2, least) && !fits; --r) {
       c.ring = r;
       c.smem = frag_smem_bytes((size_t)groups * c.xregion + ops->x_extra, w, c.led, s, groups, c.tile_bytes, r);
       fits = c.smem <= budget;
@@ -544,7 +544,7 @@ bool make_frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, FragPl
   // inputs so wide that the activations leave no room for four warps
   for (int s = 1; !best.ok && s <= kFragMaxSplit && s <= units; ++s)
     for (int w : {2, 1})
-      if (!best.ok) frag_plan(ctx, d, groups, s, w, 2, &best);
+      if (!best.ok) frag_plan(ctx, d, groups, s, w, 0, &best);
   if (!best.ok) return false;
   *pl = best;
   return true;

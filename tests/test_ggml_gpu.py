@@ -530,6 +530,24 @@ def test_the_plan_of_a_single_row(type_id):
     lin.ctx.poll()
 
 
+@pytest.mark.parametrize("type_id", [GGMLType.iq1S, GGMLType.iq1M])
+@pytest.mark.parametrize("units", [3, 64, 192])
+def test_sixteen_rows_of_small_tiles_are_one_launch(monkeypatch, type_id, units):
+    """Two tiles of these types through the dense decoder are shorter than the partial tile of sixteen rows that a drained ring holds:
+    they have a plan of three. (192 units: the widest that sixteen rows have taken.)"""
+    monkeypatch.setenv("ISHI_DENSE_DECODER", "1")
+    rng = np.random.default_rng(int(type_id) + 76)
+    n, k = 40, units * 256
+    blocks = synth.ggml_blocks(rng, int(type_id), n, k)
+    lin = PackedLinear(ggml=GGUFBlocks(dev(blocks), type_id, (n, k)))
+    assert (lin.plan[3] >> 8) & 15 >= 3
+    for m in (9, 16):
+        x = synth.activations(rng, m, k)
+        want32, _ = oracle.ggml_matmul(int(type_id), blocks, x, n)
+        assert rel_err(lin(dev(x)).cpu().numpy(), want32) < TOL
+    lin.ctx.poll()
+
+
 def test_a_reported_plan_is_accepted_whatever_its_ring(monkeypatch):
     """The ring of one row has three bits in the plan's last word: a deeper one that it shares with up to eight rows comes back with them."""
     rng = np.random.default_rng(75)

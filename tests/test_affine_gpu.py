@@ -247,7 +247,7 @@ def test_an_infinite_activation_stays_in_its_row(bits, gs):
     lin.ctx.poll()
 
 
-@pytest.mark.parametrize("bits,gs,units", [(8, 64, 44), (4, 64, 48), (4, 128, 48), (2, 128, 50)])
+@pytest.mark.parametrize("bits,gs,units", [(8, 32, 42), (8, 64, 44), (8, 128, 44), (4, 32, 46), (4, 64, 48), (4, 128, 48), (2, 64, 50), (2, 128, 50)])
 def test_the_widest_inputs_of_the_warp_level_kernel(bits, gs, units):
     """Eight column ranges of as many units as shared memory has ever taken: the activations leave room for a few warps only."""
     rng = np.random.default_rng(bits * 100 + gs + 1)

@@ -469,7 +469,10 @@ __device__ __forceinline__ void frag_rows_by_16(uint32_t xfrag, uint32_t R, uint
       mma16816(c, first, second, first, second, v[e].z, v[e].w);
       if (g == r0 + e) s[0] = c[0], s[1] = c[2], s[2] = c[1], s[3] = c[3];
     }
-    __syncwarp();  // every lane has its values of the four rows (the MMAs took them all)
+    // every lane has its values of the four rows, which other lanes' stores overwrite
+#pragma unroll
+    for (int e = 0; e < 4; ++e) values_ready(v[e]);
+    __syncwarp();
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const uint32_t to = at + (uint32_t)e * R + frag_pair_slot(lane);

@@ -113,6 +113,7 @@ __device__ __forceinline__ uint32_t stage_acquire(uint32_t addr) {
 __device__ __forceinline__ void values_ready(float &a, float &b, float &c, float &d) {
   asm volatile("" : "+f"(a), "+f"(b), "+f"(c), "+f"(d)::"memory");
 }
+__device__ __forceinline__ void values_ready(uint4 &v) { asm volatile("" : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)::"memory"); }
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;

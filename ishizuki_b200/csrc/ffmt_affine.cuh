@@ -45,7 +45,7 @@
 namespace ishi {
 
 template <int BITS, int GS, bool BF16>
-struct FragAffine {
+struct FragAffine : FragCopying {
   static_assert(BITS == 8 || BITS == 4 || BITS == 2, "8-, 4- and 2-bit codes");
   static_assert(GS == 32 || GS == 64 || GS == 128, "group sizes of the reference");
   static_assert(BITS != 2 || GS >= 64, "a 2-bit k-step spans 64 inputs");
@@ -64,8 +64,7 @@ struct FragAffine {
   // the packs that are rotated on the tensor cores all by loads and stores: both ways in one kernel take registers from the loop
   // (34816 x 5120, ternary, eight rows: 17.5 us against 17.1).
   static constexpr bool kRows = !(BITS == 2 && GS == 128), kRowSums = kRows;
-  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
-  static constexpr bool kSumsLater = true;  // do several rows that are not copied leave the sums to row_sums()?
+  static constexpr bool kSumsLater = true;
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

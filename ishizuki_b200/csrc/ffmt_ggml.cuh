@@ -24,15 +24,13 @@
 namespace ishi {
 
 template <int TYPE>
-struct FragGGML {
+struct FragGGML : FragCopying {
   static constexpr int kBlock = ggml_type_bytes(TYPE);
   static_assert(kBlock > 0, "a GGML type with a decoder");
   static constexpr int kTileBytes = 16 * kBlock;
   static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 16;  // a staged region: per unit eight rows of 512 bytes; the rows' skews
   static constexpr double kUnit = 1.0;  // unit of the tile results
   static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
-  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
-  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;     // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

@@ -38,7 +38,7 @@ namespace ishi {
 
 // TYPE: the GGML type number, 19 IQ1_S, 29 IQ1_M
 template <int TYPE>
-struct FragIQ1 {
+struct FragIQ1 : FragCopying {
   static_assert(TYPE == 19 || TYPE == 29, "IQ1_S or IQ1_M");
   static constexpr int kBlock = TYPE == 19 ? 50 : 56;
   static constexpr int kD = 1024;
@@ -47,8 +47,6 @@ struct FragIQ1 {
   static constexpr int kXBytes = 8 * 512 + 1024, kXFixed = 8 * 16;
   static constexpr double kUnit = 1.0;  // unit of the tile results
   static constexpr bool kRows = false, kRowSums = false;  // staged by loads and stores: the entry sums come from the registers (a pass over copied rows: 0.4 us a launch more)
-  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
-  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = 2048 * 32;  // the grid, four copies interleaved
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

@@ -59,7 +59,7 @@ static __device__ const uint16_t g_iq2xs_frag_codes[512] = {ISHI_IQ2XS_CODES_LIS
 
 // TYPE: the GGML type number, 17 IQ2_XS, 16 IQ2_XXS, 22 IQ2_S
 template <int TYPE>
-struct FragIQ2 {
+struct FragIQ2 : FragCopying {
   static_assert(TYPE == 17 || TYPE == 16 || TYPE == 22, "IQ2_XS, IQ2_XXS or IQ2_S");
   static constexpr bool kWide = TYPE == 22;                  // IQ2_S: ten index bits, eight explicit signs
   static constexpr int kBlock = TYPE == 17 ? 74 : TYPE == 16 ? 66 : 82;
@@ -75,8 +75,6 @@ struct FragIQ2 {
   static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 16;    // a staged region: per unit eight rows of 512 bytes; the rows' skews
   static constexpr double kUnit = 0.125;         // tile results come in units of 1/8
   static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
-  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
-  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = kEntries * kCopies * 16;  // the grid as fp16, its copies interleaved
   static constexpr bool kRowMode = false;        // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

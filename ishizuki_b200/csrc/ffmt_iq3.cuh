@@ -32,7 +32,7 @@ namespace ishi {
 
 // TYPE: the GGML type number, 18 IQ3_XXS, 21 IQ3_S
 template <int TYPE>
-struct FragIQ3 {
+struct FragIQ3 : FragCopying {
   static_assert(TYPE == 18 || TYPE == 21, "IQ3_XXS or IQ3_S");
   static constexpr bool kNine = TYPE == 21;  // nine index bits, explicit signs
   static constexpr int kBlock = kNine ? 110 : 98;
@@ -43,8 +43,6 @@ struct FragIQ3 {
   static constexpr int kXBytes = FragIQ2<17>::kXBytes, kXFixed = FragIQ2<17>::kXFixed;
   static constexpr double kUnit = kNine ? 1.0 : 0.25;  // unit of the tile results
   static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
-  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
-  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = kEntries * 128;  // the grid as fp16, sixteen copies interleaved
   static constexpr bool kRowMode = false;  // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

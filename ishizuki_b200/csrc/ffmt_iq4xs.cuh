@@ -24,13 +24,11 @@
 
 namespace ishi {
 
-struct FragIQ4XS {
+struct FragIQ4XS : FragCopying {
   static constexpr int kTileBytes = 2048 + 128 + 32;
   static constexpr int kXBytes = 8 * 512, kXFixed = 8 * 64;  // a staged region: per unit eight rows of 512 bytes; the rows' skews
   static constexpr double kUnit = 1.0;  // unit of the tile results
   static constexpr bool kRows = true, kRowSums = false;  // the activations as they lie in x
-  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
-  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = 256 * 128;       // the pair table: entry e of lane l's copy at e * 128 + l * 4
   static constexpr bool kRowMode = false;             // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

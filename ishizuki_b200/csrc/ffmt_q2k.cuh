@@ -28,7 +28,7 @@
 
 namespace ishi {
 
-struct FragQ2K {
+struct FragQ2K : FragCopying {
   static constexpr int kTileBytes = 16 * 84;
   static constexpr int kSumBytes = 512;         // per unit: [lane][hi hi | lo lo] sub-block sums
   static constexpr int kXBytes = 8 * 512 + kSumBytes, kXFixed = 8 * 64;  // a staged region: per unit eight rows and the sums; the rows' skews
@@ -36,7 +36,6 @@ struct FragQ2K {
   static constexpr bool kRows = true, kRowSums = true;  // the activations as they lie in x, then put in order and added up
   // five to eight rows by loads and stores, which arrange and add up on the way (4096 x 4096 at eight rows, copied: 5.66 us against 5.45)
   static constexpr int kCopyRows = 4;
-  static constexpr bool kSumsLater = false;
   static constexpr int kExtraBytes = 0;
   static constexpr bool kRowMode = false;       // one activation row runs through the MMA path as well
   static constexpr int kFewWarps = 16;  // most warps of the smaller block size at up to eight rows

@@ -41,12 +41,10 @@
 
 namespace ishi {
 
-struct FragQ4K {
+struct FragQ4K : FragCopying {
   static constexpr int kTileBytes = 2048 + 16 * 16 + 16 * 4;
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr bool kRows = true, kRowSums = true;  // the activations as they lie in x
-  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
-  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = true;  // MODE 1: one activation row on CUDA cores
   static constexpr int kFewWarps = 20;  // most warps of the smaller block size at up to eight rows

@@ -400,6 +400,12 @@ __device__ __forceinline__ void frag_stage_rows(const FragArgs &a, const FragRow
   } while (i0 < tasks);
 }
 
+// How a decoder that copies its activations and adds them up (Fmt::kRows, Fmt::kRowSums) does it, if it says nothing else
+struct FragCopying {
+  static constexpr int kCopyRows = 8;  // most rows that are copied at up to eight
+  static constexpr bool kSumsLater = false;  // do several rows that are not copied leave the sums to row_sums()?
+};
+
 // The activations of a decoder that reads them as they lie in x (Fmt::kRows): a bulk copy per row, asked for by
 // one warp, all counted on `bar`. No thread's load or store is in the way: alone on the GPU 80 KB are there 1500
 // cycles after the request where loads and stores by all warps take 2200 to 2500 (10 KB: 720 against 1150). Launches over weights

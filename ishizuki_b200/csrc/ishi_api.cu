@@ -473,7 +473,7 @@ int ring_for(int groups, int s, int w) { return groups == 2 || w > 16 || (w > 12
 bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int w, int ring, FragPlan *out) {
   const FragOps *ops = frag_ops_for(d);
   if (!ops) return false;
-  const size_t budget = (size_t)std::min(kSmemPerSm, ctx->smem_optin) - 1024 - 256;  // (room beside it for a CTA of the norm)
+  const size_t budget = (size_t)std::min(kSmemPerSm, ctx->smem_optin) - 1024 - 256;  // (1280 bytes beside it for a CTA of the norm or of the host copies)
   if (configure_once(ctx, ops, ops->configure, (int)budget) != ISHI_OK) return false;
   FragPlan c;
   c.ops = ops;

@@ -29,9 +29,10 @@ __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { retu
 // A row is a cluster of CTAs of 128 threads, eight values per thread in 16-byte loads, held in registers between the
 // two passes. Bound by latency alone (a row is 10-20 KB): x and w are hinted into L2 ahead of the wait
 // (hints only: either may be the output of the launch before), the rest is one exchange of the warps' sums through
-// distributed shared memory and one cluster barrier. The CTAs are as small as the product kernel's leave room for (4096
-// registers, 1280 bytes of shared memory of an SM), so they sit beside the products: one CTA of 1024 threads per row kept
-// its SM from the product behind it, whose CTA there started 3 us and was ready 1.2 us after the others.
+// distributed shared memory and one cluster barrier. The CTAs are as small as the product kernel's leave room for: 4096
+// registers (20 warps of 96, 24 of 80, 16 of 120; 16 warps of 128, as Q6_K has at nine to sixteen rows, leave none) and 1280 bytes of
+// shared memory of an SM. So most sit beside the products: one CTA of 1024 threads per row kept its SM from the product
+// behind it, whose CTA there started 3 us and was ready 1.2 us after the others.
 // Two decoder layers of the 27B shape, four norms: Q4_K at eight rows 110.7 -> 109.0 us, at one 103.4 -> 102.2, ternary at four 96.5 -> 95.0.
 // Sums: a warp's 256 squares, then the warps' sums, each by a butterfly, whatever the number of CTAs.
 constexpr int kNormThreads = 128, kNormPer = 8, kNormWarps = 32;  // threads of a CTA, values of one, most warps of a row
@@ -146,7 +147,7 @@ namespace {
 // The inputs of a host batch, a kernel between two products that copies those of the next few. The copy
 // engine takes 4.7 us a copy on top of the bytes and an event between two products, which idles the
 // SMs for 2.5 us; this kernel is a link of the chain of programmatic launches and runs beside the
-// product before it, whose CTAs leave 4096 registers and 1 KB of shared memory of an SM free: a CTA
+// product before it, whose CTAs leave 4096 registers (most of them, see above) and 1280 bytes of shared memory of an SM free: a CTA
 // of this kernel. The copies are one range of 16-byte pieces over all CTAs: one after the other, each
 // would add the bus's 2 us of latency. 32 CTAs keep 128 KB on the way; 16 are slower by 8 % of a
 // whole batch, more gain nothing. (Outputs stay with the copy engine: written to the host by a

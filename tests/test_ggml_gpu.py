@@ -593,8 +593,8 @@ def test_the_widest_inputs_of_the_warp_level_kernel(type_id, units):
 
 
 def test_a_chain_of_early_launches_reads_what_the_one_before_wrote():
-    """gather, norm, projection and gather again without a wait between them, each starting while the one before ends and reading
-    or writing over its arrays: the same bits as with a wait after every call."""
+    """gather, norm and projection without a wait between them, then gather again by ids that the host framework's kernels make
+    of the product: the same bits as with a wait after every call."""
     from ishizuki_b200.interface import rmsNorm
     rng = np.random.default_rng(73)
     n, k, rows = 5000, 2048, 8
@@ -615,6 +615,57 @@ def test_a_chain_of_early_launches_reads_what_the_one_before_wrote():
 
     for a, b in zip(chain(20, False), chain(20, True)):
         assert torch.equal(a, b)
+
+
+def test_early_launches_wait_for_the_arrays_they_share():
+    """Launches of the library directly behind one another, each of which may start while the one before ends: blocks, rows and inputs that
+    the launch before wrote, and outputs over what the launch before still reads. `spread`, `x` and `f` are written over and over; the
+    results have the bits that they have with a wait after every call."""
+    rng = np.random.default_rng(74)
+    n, k, rows, steps = 4096, 2048, 8, 6
+    per_row = k // 256 * 144  # bytes of a row of blocks
+    src = [dev(synth.q4k_blocks(rng, n, k)) for _ in range(3)]
+    lin = PackedLinear(ggml=GGUFBlocks(dev(synth.q4k_blocks(rng, n, k)), GGMLType.q4K, (n, k)))
+    ctx, q4k, blocks, last = lin.ctx, int(GGMLType.q4K), n * k // 256, 40000
+    ids = dev(rng.integers(n * k * 2 // per_row - 500, n * k * 2 // per_row, 2048).astype(np.int32))  # rows that the last blocks wrote
+    others = dev(rng.integers(0, n, 2048).astype(np.int32))
+    w = torch.ones(k, dtype=torch.float16, device="cuda")
+
+    def run(wait):
+        spread = torch.zeros(n * k, dtype=torch.float16, device="cuda")  # one expansion's output, the next one's blocks
+        x = torch.zeros(2048, k, dtype=torch.float16, device="cuda")
+        f = torch.zeros(2048, k, dtype=torch.float32, device="cuda")
+        again = [torch.zeros(last * 256, dtype=torch.float16, device="cuda") for _ in range(steps)]
+        y = [torch.zeros(rows, n, dtype=torch.float16, device="cuda") for _ in range(2 * steps)]
+        normed = [torch.zeros(2048, k, dtype=torch.float16, device="cuda") for _ in range(steps)]
+        offset = (n * k * 2 // 144 - last) * 144
+        torch.cuda.synchronize()
+
+        def call(name, *args):
+            assert getattr(ctx.lib, name)(*args, _stream()) == _lib.OK, ctx.last_error()
+            if wait:
+                torch.cuda.synchronize()
+
+        def at(t, offset=0):
+            return _ptr(t.view(torch.uint8).reshape(-1)[offset:])
+
+        for i in range(steps):
+            call("ishi_ggml_dequantize", ctx.handle, q4k, at(src[i % 3]), blocks, at(spread), _lib.DT_F16)
+            call("ishi_ggml_dequantize", ctx.handle, q4k, at(spread, offset), last, at(again[i]), _lib.DT_F16)  # blocks of the launch before
+            call("ishi_ggml_dequantize", ctx.handle, q4k, at(src[(i + 1) % 3]), blocks, at(spread), _lib.DT_F16)  # over what that one reads
+            call("ishi_ggml_gather", ctx.handle, _ptr(ids), 2048, at(spread), n * k * 2, q4k, n * k * 2 // per_row, k, _ptr(x), _lib.DT_F16)
+            call("ishi_projection_apply", lin.handle, _ptr(x), rows, _ptr(y[2 * i]), n, 0)  # rows of the launch before
+            call("ishi_ggml_gather", ctx.handle, _ptr(others), 2048, at(src[i % 3]), n * per_row, q4k, n, k, _ptr(x), _lib.DT_F16)  # over its input
+            call("ishi_projection_apply", lin.handle, at(x, (2048 - rows) * k * 2), rows, _ptr(y[2 * i + 1]), n, 0)
+            call("ishi_ggml_gather", ctx.handle, _ptr(others), 2048, at(src[i % 3]), n * per_row, q4k, n, k, _ptr(f), _lib.DT_F32)
+            call("ishi_rms_norm", ctx.handle, _ptr(f), _lib.DT_F32, 2048, k, _ptr(w), _lib.DT_F16, 1e-6, _ptr(normed[i]))
+            call("ishi_ggml_dequantize", ctx.handle, q4k, at(src[(i + 2) % 3]), 2048 * k // 256, _ptr(f), _lib.DT_F32)  # over what the norm reads
+        torch.cuda.synchronize()
+        return [t.view(torch.int16) for t in (*again, *y, *normed)]
+
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
+    ctx.poll()
 
 
 @pytest.mark.parametrize("type_id", [GGMLType.q4K, GGMLType.q6K])

@@ -151,7 +151,8 @@ int ishi_projection_crossover_rows(const ishi_projection *p);
  * for the other kernels), and a way to impose one. The order in which partial sums are added follows the
  * plan, so two projections of the same weight agree bit for bit only under the same plan (the tiled
  * copy does not depend on it). create runs one row as it runs two to eight: a row's product has the
- * same bits in all calls of up to eight rows. An imposed plan may give one row a launch of its own
+ * same bits in all calls of up to eight rows on the tensor cores (ISHI_ROUTE_GEMV adds up in
+ * another order). An imposed plan may give one row a launch of its own
  * (without that part it runs as two to eight do), whose products can then differ in the last bit.
  * set_plan accepts what ishi_projection_plan of a projection of the same shape returned. */
 ishi_status ishi_projection_plan(const ishi_projection *p, int plan[4]);

@@ -58,7 +58,7 @@ struct FragAffine : FragCopying {
   static constexpr int kBiases = kHeader + 16 * kRowScales;
   static constexpr int kTileBytes = kBiases + 16 * kRowScales;
   static constexpr int kSkew = BITS == 2 ? 16 : 64;  // of the rows against one another: 32 or 16 bytes of a row per lane and load
-  static constexpr int kSumBytes = GS == 32 ? 640 : GS == 64 ? 320 : 256;  // per unit: the group sums' pieces, see store_sum()
+  static constexpr int kSumBytes = GS == 32 ? 640 : GS == 64 ? 384 : 256;  // per unit: the group sums' pieces, see store_sum()
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   // The activations as they lie in x, then a pass that scales and adds up; a single row and rotated ones by loads and stores. Of
   // the packs that are rotated on the tensor cores all by loads and stores: both ways in one kernel take registers from the loop
@@ -137,7 +137,7 @@ struct FragAffine : FragCopying {
   // (r, t) find them: groups of 64: group t = j, [lane][hi mid] and behind them [lane][lo]; of 32: groups 2t and 2t + 1,
   // [hi hi], [mid mid], [lo lo]; of 128: group t / 2, [hi lo] in the even lane, [mid 0] in the odd one.
   // hi and mid take eleven bits each of the 24, lo has two at most: it is exact in a bf16, as which it is kept for
-  // groups of 64 and 32 (the widest inputs of these packs have no room for more).
+  // groups of 32 (the widest inputs have no room for more).
   struct Pieces {
     uint32_t hi, mid, lo;
   };
@@ -157,7 +157,7 @@ struct FragAffine : FragCopying {
     const Pieces p = pieces_of(sum);
     if (GS == 64) {
       sts64(base + (uint32_t)((r * 4 + j) * 8), p.hi, p.mid);
-      store_lo(base + 256u + (uint32_t)((r * 4 + j) * 2), p.lo);
+      sts32(base + 256u + (uint32_t)((r * 4 + j) * 4), p.lo);
     } else if (GS == 32) {
       const uint32_t at = base + (uint32_t)((r * 4 + (j >> 1)) * 8 + (j & 1) * 4);
       sts32(at, p.hi), sts32(at + 256u, p.mid);
@@ -410,7 +410,7 @@ struct FragAffine : FragCopying {
             }
           } else {
             const uint2 p = lds64(xs);
-            if (GS == 64) mma1684_tf32(acc[nb], b0, b1, lds16(xs + 256u - (uint32_t)lane * 6u) << 16);
+            if (GS == 64) mma1684_tf32(acc[nb], b0, b1, lds32(xs + 256u - (uint32_t)lane * 4u));
             mma1688_tf32(acc[nb], b0, b1, b0, b1, p.x, p.y);
           }
         }
@@ -431,7 +431,7 @@ struct FragAffine : FragCopying {
         } else {
           const float2 p = lds64f(xs);
           float s = p.x + p.y;
-          if (GS == 64) s += __uint_as_float(lds16(xs + 256u - (uint32_t)t * 6u) << 16);
+          if (GS == 64) s += lds32f(xs + 256u - (uint32_t)t * 4u);
           acc[0][0] += b0 * s, acc[0][2] += b1 * s;
         }
       }

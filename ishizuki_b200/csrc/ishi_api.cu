@@ -473,8 +473,10 @@ int ring_for(int groups, int s, int w) { return groups == 2 || w > 16 || (w > 12
 bool frag_plan(ishi_ctx *ctx, const ishi_weight_desc &d, int groups, int s, int w, int ring, FragPlan *out) {
   const FragOps *ops = frag_ops_for(d);
   if (!ops) return false;
-  const size_t budget = (size_t)std::min(kSmemPerSm, ctx->smem_optin) - 1024 - 256;  // (1280 bytes beside it for a CTA of the norm or of the host copies)
-  if (configure_once(ctx, ops, ops->configure, (int)budget) != ISHI_OK) return false;
+  const size_t most_smem = (size_t)std::min(kSmemPerSm, ctx->smem_optin);
+  // 1280 bytes beside it for a CTA of the norm or of the host copies, but where the activations leave room for one or two warps
+  const size_t budget = most_smem - (w > 2 ? 1280 : 0);
+  if (configure_once(ctx, ops, ops->configure, (int)most_smem) != ISHI_OK) return false;
   FragPlan c;
   c.ops = ops;
   c.units = (int)(d.k / 256);

@@ -50,7 +50,7 @@ struct FragQ6K : FragCopying {
   static constexpr int kXBytes = 8 * 512 + kSumBytes, kXFixed = 8 * 64;  // a staged region: per unit eight rows and the sums; the rows' skews
   static constexpr double kUnit = 16777216.0;  // tile results come in units of 2^24: masked codes are q * 2^-24
   static constexpr bool kRows = true, kRowSums = true;  // the activations as they lie in x, then put in order and added up
-  // five to eight rows by loads and stores, which arrange and add up on the way (4096 x 4096 at eight rows, copied: 6.6 us against 6.35)
+  // five to eight rows by loads and stores, which arrange and add up on the way (4096 x 4096 at eight rows, copied: 6.36 us against 6.28)
   static constexpr int kCopyRows = 4;
   static constexpr int kExtraBytes = 0;  // shared memory per CTA beyond the staged regions
   static constexpr bool kRowMode = false;         // one activation row runs through the MMA path as well

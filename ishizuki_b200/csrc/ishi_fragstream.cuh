@@ -489,7 +489,7 @@ __device__ __forceinline__ void frag_rows_by_16(uint32_t xfrag, uint32_t R, uint
   }
 }
 // The same for rows that are stored and added up on their way from x: lane l's values v of the unit whose row begins at `row`. By the
-// same MMAs: a row has the same sums, and so the same product bit for bit, in calls of one to sixteen rows.
+// same MMAs: a row has the same sums, and so under one plan the same product bit for bit, whatever rows are beside it.
 template <bool SCALED>
 __device__ __forceinline__ void frag_put_by_16(uint32_t row, uint32_t sums, int r, uint4 v, uint32_t factor) {
   const int lane = threadIdx.x & 31;
